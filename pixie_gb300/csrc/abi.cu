@@ -112,6 +112,7 @@ __global__ void k_setup(PathJob* jobs, Arena A, int maxBands);
 const void* rows_kernel(int v);
 size_t rows_smem(int v);
 int rows_warps(int v);
+bool rows_fast(int mode, long long W);
 void launch_rows(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
                  const Arena& A, const uint8_t* tbl, long long items, int rpi);
 __global__ void k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl);
@@ -122,8 +123,17 @@ int scene_rec_warps();
 const void* scene_kernel();
 int scene_warps();
 int scene_tile();
+const void* scene_big_kernel(int v);
+size_t scene_big_smem(int v);
+int scene_big_warps(int v);
+void launch_scene_big(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A);
+const void* scene_rest_kernel();
+size_t scene_rest_smem();
+int scene_rest_warps();
 void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
-                      long long items, const Arena& A, unsigned char* wide, long long slots);
+                      long long items, int rpi, const Arena& A);
+void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, unsigned char* wide,
+                       long long slots);
 void launch_scene(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns, long long items,
                   const Arena& A, const uint8_t* tbl, int sliceW);
 size_t scene_wide_bytes();
@@ -131,9 +141,7 @@ size_t setup_smem(int maxBands);
 int draw_masks_tiles();
 void launch_draw_masks(int tile, uint32_t* page, long long W, long long H, const void* items, int n,
                        const uint8_t* masks, int mode, const uint8_t* tbl, cudaStream_t st);
-size_t rows_smem_fast();
 size_t rows_smem_wide();
-int rows_warps_fast();
 struct SmoothArgs {
   float px, py, dxx, dxy, dyx, dyy;
   float seg[4][4];
@@ -258,8 +266,8 @@ struct Ctx {
   long long mdraw_cap = 0;
   int4* prog = nullptr;           // scene row programs
   long long prog_cap = 0;
-  int* rowidx = nullptr;          // scene rows -> program
-  long long rowidx_cap = 0;
+  int4* rowhdr = nullptr;         // scene rows: what each draws
+  long long rowhdr_cap = 0;
   uint8_t* cov8 = nullptr;        // scene coverage bytes (rows that fit; the rest keep spans)
   long long cov8_cap = 0;
   unsigned char* wide = nullptr;  // per-warp wide row scratch of the scene recording kernel
@@ -298,8 +306,8 @@ struct Ctx {
   size_t ringSmemMax = 0;
   float last_ms = 0;
   long long stats[6] = {0, 0, 0, 0, 0, 0};  // last fill launch: paths, prims, segments, entries, blends, wide rows
-  int rows_ctas_per_sm[2] = {1, 1};  // resident CTAs of each row-kernel variant
-  int scene_ctas_per_sm[2] = {1, 1};  // resident CTAs of the scene recording and drawing kernels
+  int rows_ctas_per_sm[4] = {1, 1, 1, 1};  // resident CTAs of each row-kernel variant
+  int scene_ctas_per_sm[5] = {1, 1, 1, 1, 1};  // resident CTAs of the scene recording, drawing, rest and big-row kernels
   int scene_slice = 256;              // pixels of a row one warp of the drawing pass owns (0: chosen per launch)
   bool stroke_gpu = true;             // outline strokes without dashes on the GPU (stroke.cu)
   float2* sk_pts = nullptr;           // outline kernel inputs: polyline points, shapes
@@ -354,7 +362,7 @@ void init_locked(int device) {
   }
   CU(cudaMalloc(&g.tbl, kTblBytes));
   CU(cudaMemcpy(g.tbl, t.data(), kTblBytes, cudaMemcpyHostToDevice));
-  for (int v = 0; v < 2; v++) {
+  for (int v = 0; v < 4; v++) {
     CU(cudaFuncSetAttribute(rows_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(v)));
     int per = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rows_kernel(v), rows_warps(v) * 32, rows_smem(v)));
@@ -367,6 +375,18 @@ void init_locked(int device) {
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_rec_kernel(), scene_rec_warps() * 32,
                                                      scene_rec_smem()));
     g.scene_ctas_per_sm[0] = std::max(1, per);
+    for (int v = 0; v < 2; v++) {
+      CU(cudaFuncSetAttribute(scene_big_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)scene_big_smem(v)));
+      CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_big_kernel(v), scene_big_warps(v) * 32,
+                                                       scene_big_smem(v)));
+      g.scene_ctas_per_sm[3 + v] = std::max(1, per);
+    }
+    CU(cudaFuncSetAttribute(scene_rest_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)scene_rest_smem()));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_rest_kernel(), scene_rest_warps() * 32,
+                                                     scene_rest_smem()));
+    g.scene_ctas_per_sm[2] = std::max(1, per);
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_kernel(), scene_warps() * 32, 0));
     g.scene_ctas_per_sm[1] = std::max(1, per);
   }
@@ -581,7 +601,7 @@ Staged stage(const std::vector<PathJob>& run, const void* extra, size_t extraByt
   A.primcnt_cap = g.primcnt_cap;
   A.prog = g.prog;
   A.prog_cap = g.prog_cap;
-  A.rowidx = g.rowidx;
+  A.rowhdr = g.rowhdr;
   A.cov8 = g.cov8;
   A.cov8_cap = g.cov8_cap;
   A.counters = reinterpret_cast<unsigned long long*>(g.d_up + S.jobsBytes);
@@ -629,8 +649,8 @@ void grow_needs(const unsigned long long* ctr, long long& seg_need, long long& l
 // Row-kernel configuration of a fill launch: scratch variant and rows per
 // work item.
 struct RowsCfg {
-  int variant = 0;
-  int rpi = 1;
+  int variant = 0;  // 0 (masks: 3), 1 (masks only)
+  int rpi = 0;      // 0: chosen per launch
 };
 
 // A captured launch sequence (upload, setup, rows, status read-back), replayed
@@ -660,7 +680,18 @@ struct RunOpts {
 // alone, after the others were drawn.  Returns per-job status.
 void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::vector<int>& status,
               const RunOpts& opts = RunOpts()) {
-  const RowsCfg cfg = opts.cfg;
+  RowsCfg cfg = opts.cfg;
+  if (cfg.variant == 0 && !jobs.empty() && jobs[0].a8) cfg.variant = 3;
+  if (cfg.rpi == 0) {
+    // a row per warp while the launch's rows are few (the chain of a chunk is
+    // as long as its rows); whole band chunks once every resident warp has some
+    long long rows = 0;
+    for (const PathJob& j : jobs) rows += j.H;
+    const long long slots = (long long)g.nsm * g.rows_ctas_per_sm[cfg.variant] * rows_warps(cfg.variant);
+    cfg.rpi = rows >= 4 * slots ? 4 : rows >= 2 * slots ? 2 : 1;
+  }
+  for (const PathJob& j : jobs)
+    if (!rows_fast(j.mode, j.W)) cfg = RowsCfg{2, 1};  // the general row kernel, row by row
   const int nj = (int)jobs.size();
   status.assign((size_t)nj, kOk);
   std::vector<int> todo(nj);
@@ -899,6 +930,15 @@ int scene_slice_for(const std::vector<HostRun>& runs) {
   return (int)w;
 }
 
+// Rows of a recording work item.  Whole band chunks (a band's entries are
+// clipped once for its rows) when every resident warp has hundreds of rows;
+// otherwise single rows, because the launch lasts as long as its last chunk
+// and a row of a wide stroke takes tens of times a simple one's.
+int scene_rec_rows(long long rows) {
+  const long long slots = (long long)g.nsm * g.scene_ctas_per_sm[0] * scene_rec_warps();
+  return rows >= 256 * slots ? 4 : rows >= 128 * slots ? 2 : 1;
+}
+
 // Paints several runs (distinct canvases) in one setup + scene launch pair,
 // repeating for runs whose workspace ran out.  MaskBlend paths must not be
 // inside a run (their clears reach outside the rows the run owns).
@@ -917,6 +957,10 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     std::vector<size_t> which;  // launch run -> runs index
     long long items = 0, recItems = 0, riTotal = 0, maxH = 1;
     const int slice = scene_slice_for(runs);
+    long long pathRows = 0;
+    for (const HostRun& r : runs)
+      if (r.status == kOk && r.j0 < r.j1) pathRows += (long long)(r.j1 - r.j0) * r.canvas->height;
+    const int rpi = scene_rec_rows(pathRows);
     for (size_t ri = 0; ri < runs.size(); ri++) {
       HostRun& r = runs[ri];
       if (r.status != kOk || r.j0 >= r.j1) continue;
@@ -938,8 +982,8 @@ void run_scene_runs(std::vector<HostRun>& runs) {
         pj.img = r.canvas->data;
         pj.W = r.canvas->width;
         pj.H = r.canvas->height;
-        pj.row_off = recItems;  // recording items: one per row of the canvas
-        recItems += pj.H;
+        pj.row_off = recItems;
+        recItems += (pj.H + rpi - 1) / rpi;
         pj.ri_off = s.ri_base + (long long)(j - r.j0);
         pj.ri_stride = nrun;
         pj.status = kOk;
@@ -956,9 +1000,10 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     const int nj = (int)dev.size();
     const int maxBands = setup_max_bands(maxH);
     ensure_arena(seg_need, list_need, (long long)nj * maxBands, pc, 1);
-    if (prog_need == 0) prog_need = std::max<long long>(1 << 20, std::min<long long>(recItems * 3, 1LL << 27));
+    dev_grow(g.ovf, g.ovf_cap, 3 * std::max<long long>(riTotal, 1));
+    if (prog_need == 0) prog_need = std::max<long long>(1 << 20, std::min<long long>(riTotal / 4, 1LL << 27));
     dev_grow(g.prog, g.prog_cap, prog_need);
-    dev_grow(g.rowidx, g.rowidx_cap, std::max<long long>(riTotal, 1));
+    dev_grow(g.rowhdr, g.rowhdr_cap, std::max<long long>(riTotal, 1));
     if (!g.cov8) {  // coverage-byte arena: up to 4 GB, at most an eighth of the free memory
       size_t fr = 0, tot = 0;
       CU(cudaMemGetInfo(&fr, &tot));
@@ -970,7 +1015,10 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     const long long recBlocks = std::max<long long>(
         1, std::min<long long>((recItems + scene_rec_warps() - 1) / scene_rec_warps(),
                                (long long)g.nsm * g.scene_ctas_per_sm[0]));
-    const long long slots = recBlocks * scene_rec_warps();
+    const long long restBlocks =
+        std::max<long long>(1, std::min<long long>((riTotal + scene_rest_warps() - 1) / scene_rest_warps(),
+                                                   (long long)g.nsm * g.scene_ctas_per_sm[2]));
+    const long long slots = restBlocks * scene_rest_warps();
     if (slots > g.wide_slots) {
       if (g.wide) cudaFree(g.wide);
       g.wide = nullptr;
@@ -981,11 +1029,22 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     const long long blocks = std::max<long long>(
         1, std::min<long long>((items + scene_warps() - 1) / scene_warps(), (long long)g.nsm * g.scene_ctas_per_sm[1]));
     Staged S = stage(dev, sr.data(), sizeof(SceneRun) * sr.size(), std::vector<Prim>());
+    S.A.ovf_cap = g.ovf_cap / 3;  // three lists
     k_setup<<<nj, 256, setup_smem(maxBands), g.stream>>>(S.dj, S.A, maxBands); note_launch();
     CU(cudaGetLastError());
-    CU(cudaMemsetAsync(g.rowidx, 0xff, sizeof(int) * (size_t)std::max<long long>(riTotal, 1), g.stream));
+    CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
     launch_scene_rec((unsigned)recBlocks, g.stream, S.dj, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(),
-                     recItems, S.A, g.wide, g.wide_slots);
+                     recItems, rpi, S.A);
+    note_launch();
+    CU(cudaGetLastError());
+    for (int v = 0; v < 2; v++) {
+      const long long bigBlocks = std::min<long long>((riTotal + scene_big_warps(v) - 1) / scene_big_warps(v),
+                                                      (long long)g.nsm * g.scene_ctas_per_sm[3 + v]);
+      launch_scene_big(v, (unsigned)std::max<long long>(1, bigBlocks), g.stream, S.dj, S.A);
+      note_launch();
+      CU(cudaGetLastError());
+    }
+    launch_scene_rest((unsigned)restBlocks, g.stream, S.dj, S.A, g.wide, g.wide_slots);
     note_launch();
     CU(cudaGetLastError());
     launch_scene((unsigned)blocks, g.stream, S.dj, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(), items,
@@ -1358,7 +1417,7 @@ void srv_step(pxg_server* sv) {
 // seen.  Every configuration computes the same bytes; only speed differs.
 // ---------------------------------------------------------------------------
 enum TuneOp { kTuneMaskRows = 0, kTuneMaskDraw = 1 };
-const RowsCfg kMaskRowsCands[] = {{0, 1}, {1, 1}, {1, 2}, {1, 4}};
+const RowsCfg kMaskRowsCands[] = {{0, 4}, {1, 1}, {1, 2}, {1, 4}};
 constexpr int kNumMaskRowsCands = 4;
 
 struct Tuner {

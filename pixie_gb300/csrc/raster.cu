@@ -840,6 +840,7 @@ __device__ __forceinline__ int stable_rank_i(const int* keys, int n, int i) {
 __device__ __forceinline__ int stable_rank_f(const float* keys, int n, int i) {
   float ki = keys[i];
   int r = 0;
+#pragma unroll 2
   for (int j = 0; j < n; j++) {
     float kj = keys[j];
     r += (kj < ki) || (kj == ki && j < i);
@@ -903,6 +904,80 @@ __device__ void clear_span_linear(const PathJob& J, const Arena& A, int job, Row
   }
 }
 
+// The covered area of pixel x in the left sliver of a trapezoid pair: the edge
+// (m, b) crosses the row's top and bottom at t0 and t1; xs is the sliver's
+// first pixel (:1752-1788).
+__device__ __forceinline__ float trap_left_area(float m, float b, float t0, float t1, long long x, long long xs,
+                                                long long y) {
+  const bool inv = t0 < t1;
+  const float sliverStart = nmin(t0, t1), rectStart = nmax(t0, t1);
+  float prevPen = x == xs ? sliverStart : (float)x;
+  float pen = (float)(x + 1);
+  float rightRectArea = 0;
+  if (pen > rectStart) {
+    rightRectArea = pen - rectStart;
+    pen = rectStart;
+  }
+  float prevPenY = x == xs ? (inv ? (float)y : (float)(y + 1)) : m * (float)x + b;
+  float penY = m * pen + b;
+  float run = pen - prevPen;
+  float tri = 0.5f * run * fabsf(penY - prevPenY);
+  float rect = inv ? (prevPenY - (float)y) * run : ((float)(y + 1) - prevPenY) * run;
+  return tri + rect + rightRectArea;
+}
+// ... and in the right sliver (:1790-1828)
+__device__ __forceinline__ float trap_right_area(float m, float b, float t0, float t1, long long x, long long xs,
+                                                 long long y) {
+  const bool inv = t0 > t1;
+  const float rectEnd = nmin(t0, t1), sliverEnd = nmax(t0, t1);
+  float prevPen = x == xs ? rectEnd : (float)x;
+  float pen = (float)(x + 1);
+  float ap = fabsf(prevPen);
+  float leftRectArea = ap - floorf(ap);  // vmath fractional: fractional part of |v|
+  if (pen > sliverEnd) pen = sliverEnd;
+  float prevPenY = x == xs ? (inv ? (float)(y + 1) : (float)y) : m * (float)x + b;
+  float penY = m * pen + b;
+  float run = pen - prevPen;
+  float tri = 0.5f * run * fabsf(penY - prevPenY);
+  float rect = inv ? (penY - (float)y) * run : ((float)(y + 1) - penY) * run;
+  return leftRectArea + tri + rect;
+}
+
+// The pixels [x0, x1) of a row filled (op_fill), 16-byte quads between the
+// ragged ends of an RGBX row.
+template <bool A8>
+__device__ __forceinline__ void fill_span(RowPx<A8> row, int mode, const uint8_t* tbl, uint32_t rgbx, long long x0,
+                                          long long x1, int lane, unsigned* cnt = nullptr) {
+  if (!A8 && x1 - x0 >= 64) {
+    uint32_t* p = reinterpret_cast<uint32_t*>(row.base) + (x0 - row.x0);
+    const long long n = x1 - x0;
+    const int head = (int)((4 - ((reinterpret_cast<uintptr_t>(p) >> 2) & 3)) & 3);
+    const long long nq = (n - head) >> 2;
+    const int tail = (int)(n - head - 4 * nq);
+    if (lane < head) p[lane] = op_fill(mode, tbl, p[lane], rgbx);
+    if (lane < tail) p[n - tail + lane] = op_fill(mode, tbl, p[n - tail + lane], rgbx);
+    uint4* q = reinterpret_cast<uint4*>(p + head);
+    if (mode == kOverwrite || (mode == kNormal && (rgbx >> 24) == 255)) {
+      for (long long i = lane; i < nq; i += 32) q[i] = make_uint4(rgbx, rgbx, rgbx, rgbx);
+    } else {
+      for (long long i = lane; i < nq; i += 32) {
+        uint4 v = q[i];
+        v.x = op_fill(mode, tbl, v.x, rgbx);
+        v.y = op_fill(mode, tbl, v.y, rgbx);
+        v.z = op_fill(mode, tbl, v.z, rgbx);
+        v.w = op_fill(mode, tbl, v.w, rgbx);
+        q[i] = v;
+      }
+    }
+    if (cnt) *cnt += (unsigned)((lane < head) + (lane < tail) + 4 * ((nq - lane + 31) / 32));
+    return;
+  }
+  for (long long x = x0 + lane; x < x1; x += 32) {
+    row[x] = op_fill(mode, tbl, row[x], rgbx);
+    if (cnt) ++*cnt;
+  }
+}
+
 // The trapezoid path's pixels for one pair of entries, left (Lm, Lb) and
 // right (Rm, Rb), crossing the row at tl0/tl1 and tr0/tr1 (:1752-1835), drawn
 // within [xa, xb).
@@ -915,54 +990,22 @@ __device__ __forceinline__ void apply_trap_pair(RowPx<A8> row, int mode, const u
   const long long leftCoverEnd = nim_int(ceilf(leftMaxX));
   const long long rightCoverBegin = nim_int(truncf(rightMinX));
   {  // left sliver (:1752-1788)
-    const bool inv = tl0 < tl1;
-    const float sliverStart = nmin(tl0, tl1), rectStart = leftMaxX;
-    const long long xs = nim_int(sliverStart), xe = nim_int(ceilf(rectStart));
-    for (long long x = max(max(xs, 0LL), xa) + lane; x < min(min(xe, W), xb); x += 32) {
-      float prevPen = x == xs ? sliverStart : (float)x;
-      float pen = (float)(x + 1);
-      float rightRectArea = 0;
-      if (pen > rectStart) {
-        rightRectArea = pen - rectStart;
-        pen = rectStart;
-      }
-      float prevPenY = x == xs ? (inv ? (float)y : (float)(y + 1)) : Lm * (float)x + Lb;
-      float penY = Lm * pen + Lb;
-      float run = pen - prevPen;
-      float tri = 0.5f * run * fabsf(penY - prevPenY);
-      float rect = inv ? (prevPenY - (float)y) * run : ((float)(y + 1) - prevPenY) * run;
-      float area = tri + rect + rightRectArea;
-      row[x] = blend_row(mode, tbl, row[x], mul_f(rgbx, area));
+    const long long xs = nim_int(nmin(tl0, tl1));
+    for (long long x = max(max(xs, 0LL), xa) + lane; x < min(min(leftCoverEnd, W), xb); x += 32) {
+      row[x] = blend_row(mode, tbl, row[x], mul_f(rgbx, trap_left_area(Lm, Lb, tl0, tl1, x, xs, y)));
       if (cnt) ++*cnt;
     }
   }
   {  // right sliver (:1790-1828)
-    const bool inv = tr0 > tr1;
-    const float rectEnd = rightMinX, sliverEnd = nmax(tr0, tr1);
-    const long long xs = nim_int(rectEnd), xe = nim_int(ceilf(sliverEnd));
+    const long long xs = nim_int(rightMinX), xe = nim_int(ceilf(nmax(tr0, tr1)));
     for (long long x = max(max(xs, 0LL), xa) + lane; x < min(min(xe, W), xb); x += 32) {
-      float prevPen = x == xs ? rectEnd : (float)x;
-      float pen = (float)(x + 1);
-      float ap = fabsf(prevPen);
-      float leftRectArea = ap - floorf(ap);  // vmath fractional: fractional part of |v|
-      if (pen > sliverEnd) pen = sliverEnd;
-      float prevPenY = x == xs ? (inv ? (float)(y + 1) : (float)y) : Rm * (float)x + Rb;
-      float penY = Rm * pen + Rb;
-      float run = pen - prevPen;
-      float tri = 0.5f * run * fabsf(penY - prevPenY);
-      float rect = inv ? (penY - (float)y) * run : ((float)(y + 1) - penY) * run;
-      float area = leftRectArea + tri + rect;
-      row[x] = blend_row(mode, tbl, row[x], mul_f(rgbx, area));
+      row[x] = blend_row(mode, tbl, row[x], mul_f(rgbx, trap_right_area(Rm, Rb, tr0, tr1, x, xs, y)));
       if (cnt) ++*cnt;
     }
   }
-  {  // the fully covered middle (:1830-1835)
-    long long fb = max(min(max(leftCoverEnd, 0LL), W), xa), fe = min(min(max(rightCoverBegin, 0LL), W), xb);
-    for (long long x = fb + lane; x < fe; x += 32) {
-      row[x] = op_fill(mode, tbl, row[x], rgbx);
-      if (cnt) ++*cnt;
-    }
-  }
+  // the fully covered middle (:1830-1835)
+  const long long fb = max(min(max(leftCoverEnd, 0LL), W), xa), fe = min(min(max(rightCoverBegin, 0LL), W), xb);
+  if (fe > fb) fill_span<A8>(row, mode, tbl, rgbx, fb, fe, lane, cnt);
 }
 
 // computeCoverage's accumulation of the sample spans (prevAt, at) in 24.8
@@ -1079,27 +1122,33 @@ __device__ void apply_hits(RowPx<A8> row, int mode, const uint8_t* tbl, uint32_t
 
 // Row programs: what a row of a path draws, recorded by the scene's first
 // pass and replayed by its second.  A program is a header unit then data:
-//   kRecFill  [minX, maxX) filled            (the non-AA two-edge case)
 //   kRecCov   n sample spans, coverage step  (computeCoverage + fillCoverage)
 //   kRecHits  n spans                        (fillHits, non-AA)
 //   kRecTrap  n pairs: {Lm, Lb, Rm, Rb}, {tl0, tl1, tr0, tr1} per pair
-//   kRecCov8  the coverage bytes of pixels [lo, hi), at a 64-bit offset in
-//             Arena::cov8 (the accumulation done once, at record time)
-enum RecKind { kRecFill = 1, kRecCov = 2, kRecHits = 3, kRecTrap = 4, kRecCov8 = 5 };
+// Each row of each path has a header {kind, place, lo, hi} in Arena::rowhdr;
+// zero: the row draws nothing.
+//   kRecFill  pixels [lo, hi) filled, nothing else stored
+//   kRecCov8  coverage bytes of pixels [lo, hi) -- lo a multiple of 16 -- from
+//             unit `place` (16 bytes) of Arena::cov8 (the accumulation done
+//             once, at record time); zero: the pixel is left alone
+//   kRecCov8Z a list at unit `place` of Arena::prog: {cov8 unit, n} and n
+//             pixels that are blended with an empty source besides
+//   kRecProg  a program at unit `place` of Arena::prog
+enum RecKind { kRecFill = 1, kRecCov = 2, kRecHits = 3, kRecTrap = 4, kRecCov8 = 5, kRecCov8Z = 6, kRecProg = 7 };
 
 // Allocates `units` 16-byte units for row y of job J's program, stores its
-// index for the row, and returns it (lane-uniform); -1 if the arena is full.
-__device__ __forceinline__ long long rec_alloc(const PathJob& J, const Arena& A, long long y, int units,
-                                               int lane) {
+// place for the row (drawn within [lo, hi)), and returns it (lane-uniform);
+// -1 if the arena is full.
+__device__ __forceinline__ long long rec_alloc(const PathJob& J, const Arena& A, long long y, int kind, int units,
+                                               long long lo, long long hi, int lane) {
   unsigned long long base = 0;
   if (lane == 0) {
     base = atomicAdd(&A.counters[kCtrProg], (unsigned long long)units);
     if ((long long)(base + units) > A.prog_cap || base + units > (unsigned long long)INT_MAX) {
       atomicOr(&A.counters[kCtrProgFull], 1ull);
-      A.rowidx[J.ri_off + y * J.ri_stride] = -1;
       base = ~0ull;
     } else {
-      A.rowidx[J.ri_off + y * J.ri_stride] = (int)base;
+      A.rowhdr[J.ri_off + y * J.ri_stride] = make_int4(kind, (int)base, (int)lo, (int)hi);
     }
   }
   base = __shfl_sync(0xffffffffu, base, 0);
@@ -1164,8 +1213,8 @@ __device__ bool process_row(const PathJob& J, const Arena& A, const uint8_t* tbl
     long long minX = min(max(nim_int(E[0].ax), 0LL), W);
     long long maxX = min(max(nim_int(E[1].ax), 0LL), W);
     if (REC) {
-      const long long at = rec_alloc(J, A, y, 1, lane);
-      if (at >= 0 && lane == 0) A.prog[at] = make_int4(kRecFill, 0, (int)minX, (int)maxX);
+      if (lane == 0 && maxX > minX)
+        A.rowhdr[J.ri_off + y * J.ri_stride] = make_int4(kRecFill, 0, (int)minX, (int)maxX);
       return true;
     }
     for (long long x = xa + lane; x < xb; x += 32) {
@@ -1275,7 +1324,7 @@ __device__ bool process_row(const PathJob& J, const Arena& A, const uint8_t* tbl
     }
     if (simple && REC) {
       const int np = n / 2;
-      const long long at = rec_alloc(J, A, y, 1 + 2 * np, lane);
+      const long long at = rec_alloc(J, A, y, kRecProg, 1 + 2 * np, 0, W, lane);
       if (at >= 0) {
         if (lane == 0) A.prog[at] = make_int4(kRecTrap, np, 0, 0);
         for (int p = lane; p < np; p += 32) {
@@ -1432,12 +1481,10 @@ __device__ bool process_row(const PathJob& J, const Arena& A, const uint8_t* tbl
       }
       lo = max(lo, J.startX);
       hi = min(hi, J.startX + J.pathWidth);
-      if (hi <= lo) {
-        if (lane == 0) A.rowidx[J.ri_off + y * J.ri_stride] = -1;
-        return true;
-      }
+      if (hi <= lo) return true;
       // coverage bytes when the arena has room (else the spans are recorded)
-      const unsigned long long nbytes = (unsigned long long)((hi - lo + 15) & ~15LL);
+      const long long lo16 = lo & ~15LL;
+      const unsigned long long nbytes = (unsigned long long)((hi - lo16 + 15) & ~15LL);
       unsigned long long cb = 0;
       if (lane == 0) {
         cb = atomicAdd(&A.counters[kCtrCov8], nbytes);
@@ -1445,24 +1492,22 @@ __device__ bool process_row(const PathJob& J, const Arena& A, const uint8_t* tbl
       }
       cb = __shfl_sync(0xffffffffu, cb, 0);
       if (cb != ~0ull) {
-        const long long at = rec_alloc(J, A, y, 2, lane);
-        if (at < 0) return true;
-        if (lane == 0) {
-          A.prog[at] = make_int4(kRecCov8, 0, (int)lo, (int)hi);
-          A.prog[at + 1] = make_int4((int)(cb & 0xffffffffu), (int)(cb >> 32), 0, 0);
-        }
+        if (lane == 0)
+          A.rowhdr[J.ri_off + y * J.ri_stride] = make_int4(kRecCov8, (int)(cb >> 4), (int)lo16, (int)hi);
         uint8_t* dst = A.cov8 + cb;
+        for (int i = lane; i < (int)(lo - lo16); i += 32) dst[i] = 0;
+        for (long long i = hi - lo16 + lane; i < (long long)nbytes; i += 32) dst[i] = 0;
         for (long long tx0 = lo; tx0 < hi; tx0 += XT) {
           const long long tx1 = min(tx0 + (long long)XT, hi);
           cov_tile<XT>(S.sp, nsp, sc, tx0, tx1, S.acc, lane);
-          for (int i = lane; i < (int)(tx1 - tx0); i += 32) dst[tx0 - lo + i] = (uint8_t)(S.acc[i] & 255);
+          for (int i = lane; i < (int)(tx1 - tx0); i += 32) dst[tx0 - lo16 + i] = (uint8_t)(S.acc[i] & 255);
           __syncwarp();
         }
         return true;
       }
     }
-    const long long at = nsp > 0 ? rec_alloc(J, A, y, 1 + (nsp + 1) / 2, lane) : -1;
-    if (nsp == 0 && lane == 0) A.rowidx[J.ri_off + y * J.ri_stride] = -1;
+    const long long at =
+        nsp > 0 ? rec_alloc(J, A, y, kRecProg, 1 + (nsp + 1) / 2, aa ? J.startX : 0, aa ? J.startX + J.pathWidth : W, lane) : -1;
     if (at >= 0) {
       if (lane == 0) A.prog[at] = make_int4(aa ? kRecCov : kRecHits, nsp, sc, 0);
       int2* d = reinterpret_cast<int2*>(A.prog + at + 1);
@@ -1496,13 +1541,53 @@ __device__ bool process_row(const PathJob& J, const Arena& A, const uint8_t* tbl
   return true;
 }
 
+}  // namespace pxg
+#include "rowfast.cuh"
+namespace pxg {
+
 constexpr int kFastMaxH = 256, kFastXT = 1024, kFastWarps = 4;
 constexpr int kWideMaxH = 2048, kWideXT = 1024;
 
-// The persistent row kernel: every warp takes work items -- RPI consecutive
-// rows of one job -- from a device queue (one atomic per item) until the
-// queue is empty, so jobs of uneven height share the GPU evenly.  Rows whose
-// crossings exceed MAXH go to the wide kernel.
+// The persistent row kernel: every warp takes work items -- rpi consecutive
+// rows of one job's path -- from a device queue (one atomic per item, issued
+// while the item before is drawn) until the queue is empty, so jobs of uneven
+// height share the GPU evenly.  Rows the engine hands on go to the wide
+// kernel.  NB = 64 with a 256-pixel tile is for small paths such as glyphs:
+// a quarter of the shared memory per warp.
+template <int OUT, int NB, int XT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) k_rows_fast(PathJob* jobs, const long long* offs, int njobs, Arena A,
+                                                          const uint8_t* tbl, long long totalItems, int rpi) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  FastRow<NB, XT>& S = reinterpret_cast<FastRow<NB, XT>*>(rsm)[warp];
+  init_fast_row(S, lane);
+  pdl_trigger();
+  pdl_wait();  // the setup's segments, bands and queue counters
+  unsigned long long q = 0;
+  if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue], 1ull);
+  while (true) {
+    const long long item = (long long)__shfl_sync(0xffffffffu, q, 0);
+    if (item >= totalItems) break;
+    if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue], 1ull);
+    int lo = 0, hi = njobs - 1;  // job with row_off <= item (offs: the jobs' row_off, packed)
+    while (lo < hi) {
+      int mid = (lo + hi + 1) >> 1;
+      if (offs[mid] <= item) lo = mid;
+      else hi = mid - 1;
+    }
+    const PathJob& J = jobs[lo];
+    if (J.status != kOk) continue;
+    const long long yA = J.startY + (item - J.row_off) * rpi, yB = min(yA + rpi, J.pathHeight);
+    if (yA < yB) fast_rows<OUT, NB, XT>(J, A, tbl, lo, (int)yA, (int)yB, S, lane);
+  }
+}
+constexpr int kRowsNB = 256, kRowsXT = 1024, kRowsWarps = 4;
+constexpr int kGlyphNB = 64, kGlyphXT = 256, kGlyphWarps = 8;
+
+// The general row kernel (launches with MaskBlend paths, whose clears reach
+// outside the path, or images too wide for the row engine's sort keys): the same queue,
+// over all rows of the images.  Rows whose crossings exceed MAXH go to the
+// wide kernel.
 template <int MAXH, int XT, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_rows(PathJob* jobs, const long long* offs, int njobs, Arena A,
                                                      const uint8_t* tbl, long long totalItems, int rpi) {
@@ -1546,12 +1631,6 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows(PathJob* jobs, const long l
   }
 }
 
-constexpr int kSmallMaxH = 32, kSmallXT = 256, kSmallWarps = 8;
-template __global__ void k_rows<kFastMaxH, kFastXT, kFastWarps>(PathJob*, const long long*, int, Arena,
-                                                                 const uint8_t*, long long, int);
-template __global__ void k_rows<kSmallMaxH, kSmallXT, kSmallWarps>(PathJob*, const long long*, int, Arena,
-                                                                   const uint8_t*, long long, int);
-
 // Rows whose crossings exceed the fast kernel's capacity: one warp per CTA
 // with room for kWideMaxH crossings.
 __global__ void __launch_bounds__(32) k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl) {
@@ -1593,24 +1672,83 @@ __global__ void k_xclears(PathJob* jobs, Arena A) {
 }
 
 // Dense scenes, in two passes.
-// k_scene_rec: every (path, row) of the launch, independent of the pixels, so
-// all of them run in parallel from a device queue: the row's band entries,
-// crossings, sort and walk, recorded as the row's program (RecKind).  Rows
-// with more crossings than the shared-memory scratch holds take a per-warp
-// global-memory scratch of kWideMaxH.
+// k_scene_rec: every row of every path of the launch, independent of the
+// pixels, in chunks from a device queue (rowfast.cuh): the row's coverage
+// bytes (or, rarely, its program: RecKind).  k_scene_big and
+// k_scene_rest record the rows it hands on.
 // k_scene: a warp owns a slice of one canvas row (sliceW pixels) and replays
 // every path's program for that row in submission order, so each pixel sees
 // the paths in the order the reference's sequence of fillPath/strokePath
 // calls applies them.  A path that failed in setup stops its run there (the
-// reference raises at that call); a path whose bounds miss the slice is
-// skipped (outside its bounds a non-mask fill writes nothing).  If the
-// program arena overflowed, k_scene draws nothing and the host reruns the
-// launch with a larger arena.
-constexpr int kRecXT = 256;  // coverage tile of the recording pass
+// reference raises at that call).  If the program arena overflowed, k_scene
+// draws nothing and the host reruns the launch with a larger arena.
+constexpr int kRecNB = 128, kRecRowXT = 1024, kRecRowWarps = 4;
+__global__ void __launch_bounds__(kRecRowWarps * 32, 7) k_scene_rec(PathJob* jobs, const SceneRun* runs, int nruns,
+                                                                 long long totalItems, int rpi, Arena A) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  FastRow<kRecNB, kRecRowXT>& S = reinterpret_cast<FastRow<kRecNB, kRecRowXT>*>(rsm)[warp];
+  init_fast_row(S, lane);
+  pdl_trigger();
+  pdl_wait();
+  unsigned long long q = 0;
+  if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue], 1ull);
+  while (true) {
+    const long long item = (long long)__shfl_sync(0xffffffffu, q, 0);
+    if (item >= totalItems) break;
+    if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue], 1ull);
+    // items run by run, path by path, chunk of rpi rows by chunk: rec_off + (j - j0) * chunks + c
+    int r0 = 0, r1 = nruns - 1;
+    while (r0 < r1) {
+      int mid = (r0 + r1 + 1) >> 1;
+      if (runs[mid].rec_off <= item) r0 = mid;
+      else r1 = mid - 1;
+    }
+    const long long local = item - runs[r0].rec_off, chunks = (runs[r0].H + rpi - 1) / rpi;
+    const int lo = runs[r0].j0 + (int)(local / chunks);
+    const PathJob& J = jobs[lo];
+    if (J.status != kOk) continue;
+    const long long yA = J.startY + (local % chunks) * rpi, yB = min(yA + rpi, J.pathHeight);
+    if (yA >= yB) continue;
+    if (J.W >= fast_max_w(kRecNB)) {
+      for (long long y = yA; y < yB; y++) push_row(A, lo, (int)y, lane);
+      continue;
+    }
+    fast_rows<kOutRec, kRecNB, kRecRowXT>(J, A, nullptr, lo, (int)yA, (int)yB, S, lane);
+  }
+}
+
+// The rows k_scene_rec handed on (list 0): up to NB crossings -- stroke
+// outlines overlap themselves hundreds of times a row.  The instance for
+// 512 hands the rest on to list 1, the one for 2048 (a warp per CTA, its keys
+// in shared memory) to list 2.
+template <int NB, int XT, int WARPS, int FROM>
+__global__ void __launch_bounds__(WARPS * 32) k_scene_big(PathJob* jobs, Arena A) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  FastRow<NB, XT>& S = reinterpret_cast<FastRow<NB, XT>*>(rsm)[warp];
+  init_fast_row(S, lane);
+  pdl_trigger();
+  pdl_wait();
+  const long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[FROM ? kCtrOvfRows2 : kCtrOvfRows]);
+#pragma unroll 1
+  for (long long i = (long long)blockIdx.x * WARPS + warp; i < n; i += (long long)gridDim.x * WARPS) {
+    const long long v = A.ovf_rows[FROM * A.ovf_cap + i];
+    const int job = (int)(v >> 32), y = (int)(v & 0xffffffffLL);
+    const PathJob& J = jobs[job];
+    if (J.W >= fast_max_w(NB)) push_row(A, job, y, lane, FROM + 1);
+    else fast_rows<kOutRec, NB, XT, FROM + 1>(J, A, nullptr, job, y, y + 1, S, lane);
+  }
+}
+constexpr int kBigNB = 512, kBigXT = 1024, kBigWarps = 4;
+constexpr int kHugeNB = 2048, kHugeXT = 1024, kHugeWarps = 1;
+
+// The rows k_scene_big handed on (list 2), by the general row code; those with
+// more than MAXH crossings take a per-warp global scratch.
+constexpr int kRecXT = 256;  // coverage tile of the general recording code
 template <int MAXH, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) k_scene_rec(PathJob* jobs, const SceneRun* runs, int nruns,
-                                                          long long totalItems, Arena A, unsigned char* wide,
-                                                          long long wideSlots) {
+__global__ void __launch_bounds__(WARPS * 32) k_scene_rest(PathJob* jobs, Arena A, unsigned char* wide,
+                                                           long long wideSlots) {
   extern __shared__ __align__(16) unsigned char rsm[];
   using Scratch = RowScratch<MAXH, kRecXT>;
   using Wide = RowScratch<kWideMaxH, kWideXT>;
@@ -1619,34 +1757,19 @@ __global__ void __launch_bounds__(WARPS * 32) k_scene_rec(PathJob* jobs, const S
   pdl_wait();
   Scratch& S = reinterpret_cast<Scratch*>(rsm)[warp];
   const long long gw = (long long)blockIdx.x * WARPS + warp;
-  while (true) {
-    unsigned long long q = 0;
-    if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue], 1ull);
-    const long long item = (long long)__shfl_sync(0xffffffffu, q, 0);
-    if (item >= totalItems) break;
-    // items run by run, path by path, row by row: rec_off + (j - j0) * H + y
-    int r0 = 0, r1 = nruns - 1;
-    while (r0 < r1) {
-      int mid = (r0 + r1 + 1) >> 1;
-      if (runs[mid].rec_off <= item) r0 = mid;
-      else r1 = mid - 1;
-    }
-    const long long local = item - runs[r0].rec_off, H = runs[r0].H;
-    const int lo = runs[r0].j0 + (int)(local / H);
-    const long long y = local % H;
+  const long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[kCtrOvfRows3]);
+  for (long long i = gw; i < n; i += (long long)gridDim.x * WARPS) {
+    const long long v = A.ovf_rows[2 * A.ovf_cap + i];
+    const int lo = (int)(v >> 32);
+    const long long y = v & 0xffffffffLL;
     const PathJob& J = jobs[lo];
-    if (J.status != kOk || y < J.startY || y >= J.pathHeight) continue;
     bool ok = process_row<MAXH, kRecXT, false, true>(J, A, nullptr, lo, y, S, lane, 0, J.W);
     if (!ok && gw < wideSlots) {
-      if (lane == 0) atomicAdd(&A.counters[kCtrOvfRows], 1ull);  // rows taking the wide scratch
       __syncwarp();
       ok = process_row<kWideMaxH, kWideXT, false, true>(J, A, nullptr, lo, y, reinterpret_cast<Wide*>(wide)[gw],
                                                         lane, 0, J.W);
     }
-    if (!ok && lane == 0) {
-      atomicMin(&A.counters[kCtrRowErr], (unsigned long long)lo);
-      A.rowidx[J.ri_off + y * J.ri_stride] = -1;
-    }
+    if (!ok && lane == 0) atomicMin(&A.counters[kCtrRowErr], (unsigned long long)lo);
     __syncwarp();
   }
 }
@@ -1695,33 +1818,31 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
     for (int c0 = R.j0; c0 < R.j1; c0 += 32) {
       const int j = c0 + lane;
       const bool valid = j < R.j1;
-      int st = kNothing, at = -1, mode = 0;
+      int st = kNothing, mode = 0;
       uint32_t rgbx = 0;
-      long long sx = 0, pw = 0;
+      int4 rh = make_int4(0, 0, 0, 0);
       if (valid) {
         const PathJob& J = jobs[j];
         st = J.status;
-        at = A.rowidx[rb + (j - R.j0)];
-        sx = J.startX;
-        pw = J.pathWidth;
+        rh = A.rowhdr[rb + (j - R.j0)];
         mode = J.mode;
         rgbx = J.rgbx;
       }
       // the first failed path stops the run: it and the paths after it draw nothing
       const unsigned bad = __ballot_sync(0xffffffffu, valid && st != kOk && st != kNothing);
       const int lim = bad ? __ffs(bad) - 1 : 32;
-      const bool draws = valid && lane < lim && st == kOk && at >= 0 && sx < xb && sx + pw > xa;
-      int4 h = make_int4(0, 0, 0, 0);
-      if (draws) h = A.prog[at];
+      const bool draws = valid && lane < lim && st == kOk && rh.x != 0 && rh.z < xb && rh.w > xa;
+      int4 h = rh;
+      if (draws && rh.x == kRecProg) h = A.prog[rh.y];
       unsigned dm = __ballot_sync(0xffffffffu, draws);
       while (dm) {
         const int i = __ffs(dm) - 1;
         dm &= dm - 1;
         const int hx = __shfl_sync(0xffffffffu, h.x, i), hy = __shfl_sync(0xffffffffu, h.y, i);
         const int hz = __shfl_sync(0xffffffffu, h.z, i), hw = __shfl_sync(0xffffffffu, h.w, i);
-        const int ai = __shfl_sync(0xffffffffu, at, i), mi = __shfl_sync(0xffffffffu, mode, i);
+        const int ai = __shfl_sync(0xffffffffu, rh.y, i), mi = __shfl_sync(0xffffffffu, mode, i);
         const uint32_t ci = __shfl_sync(0xffffffffu, rgbx, i);
-        const long long sxi = __shfl_sync(0xffffffffu, sx, i), pwi = __shfl_sync(0xffffffffu, pw, i);
+        const int p0 = __shfl_sync(0xffffffffu, rh.z, i), p1 = __shfl_sync(0xffffffffu, rh.w, i);
         if (hx == kRecFill) {
           for (long long x = max((long long)hz, xa) + lane; x < min((long long)hw, xb); x += 32) {
             row[x] = op_fill(mi, tbl, row[x], ci);
@@ -1729,10 +1850,11 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
           }
         } else if (hx == kRecCov) {
           apply_cov<false, XT>(row, mi, tbl, ci, reinterpret_cast<const int2*>(A.prog + ai + 1), hy, hz,
-                               max(sxi, xa), min(sxi + pwi, xb), acc, lane, &painted);
-        } else if (hx == kRecCov8) {
-          const int4 u = A.prog[ai + 1];
-          const uint8_t* cv8 = A.cov8 + (((long long)(unsigned)u.y << 32) | (unsigned)u.x) - hz;
+                               max((long long)p0, xa), min((long long)p1, xb), acc, lane, &painted);
+        } else if (hx == kRecCov8 || hx == kRecCov8Z) {
+          int4 u = make_int4(ai, 0, 0, 0);
+          if (hx == kRecCov8Z) u = A.prog[ai];
+          const uint8_t* cv8 = A.cov8 + ((long long)(unsigned)u.x << 4) - hz;
           const long long x0 = max((long long)hz, xa), x1 = min((long long)hw, xb);
           uint32_t cvN = 0, bdN = 0;
           if (x0 + lane < x1) {
@@ -1749,6 +1871,13 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
             }
             if (cv) {
               row[x] = op_cov(mi, tbl, bd, ci, cv);
+              ++painted;
+            }
+          }
+          if (lane < u.y) {
+            const int x = reinterpret_cast<const int*>(A.prog + ai + 1)[lane];
+            if (x >= xa && x < xb) {
+              row[x] = blend_any(mi, tbl, row[x], 0u);
               ++painted;
             }
           }
@@ -1778,20 +1907,39 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
   }
 }
 
-// Scene kernels: the recording pass holds 128 crossings per row in shared
-// memory (8 warps per CTA); the drawing pass keeps one 256-pixel coverage
-// tile per warp.
+// Scene kernels: the general recording code holds 128 crossings per row in
+// shared memory (8 warps per CTA); the drawing pass keeps one 256-pixel
+// coverage tile per warp.
 constexpr int kRecMaxH = 128, kRecWarps = 8, kSceneXT = 256, kSceneWarps = 8;
-const void* scene_rec_kernel() { return (const void*)k_scene_rec<kRecMaxH, kRecWarps>; }
-size_t scene_rec_smem() { return sizeof(RowScratch<kRecMaxH, kRecXT>) * kRecWarps; }
-int scene_rec_warps() { return kRecWarps; }
+const void* scene_rec_kernel() { return (const void*)k_scene_rec; }
+size_t scene_rec_smem() { return sizeof(FastRow<kRecNB, kRecRowXT>) * kRecRowWarps; }
+int scene_rec_warps() { return kRecRowWarps; }
+// the two big-row instances (0: 512 crossings, 1: 2048)
+constexpr auto kSceneBig = k_scene_big<kBigNB, kBigXT, kBigWarps, 0>;
+constexpr auto kSceneHuge = k_scene_big<kHugeNB, kHugeXT, kHugeWarps, 1>;
+const void* scene_big_kernel(int v) { return v ? (const void*)kSceneHuge : (const void*)kSceneBig; }
+size_t scene_big_smem(int v) {
+  return v ? sizeof(FastRow<kHugeNB, kHugeXT>) * kHugeWarps : sizeof(FastRow<kBigNB, kBigXT>) * kBigWarps;
+}
+int scene_big_warps(int v) { return v ? kHugeWarps : kBigWarps; }
+void launch_scene_big(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A) {
+  launch_pdl(v ? kSceneHuge : kSceneBig, dim3(blocks), dim3(scene_big_warps(v) * 32), scene_big_smem(v), st, jobs, A);
+}
+const void* scene_rest_kernel() { return (const void*)k_scene_rest<kRecMaxH, kRecWarps>; }
+size_t scene_rest_smem() { return sizeof(RowScratch<kRecMaxH, kRecXT>) * kRecWarps; }
+int scene_rest_warps() { return kRecWarps; }
 const void* scene_kernel() { return (const void*)k_scene<kSceneXT, kSceneWarps>; }
 int scene_warps() { return kSceneWarps; }
 int scene_tile() { return kSceneXT; }
 void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
-                      long long items, const Arena& A, unsigned char* wide, long long slots) {
-  launch_pdl(k_scene_rec<kRecMaxH, kRecWarps>, dim3(blocks), dim3(kRecWarps * 32), scene_rec_smem(), st, jobs, runs,
-             nruns, items, A, wide, slots);
+                      long long items, int rpi, const Arena& A) {
+  launch_pdl(k_scene_rec, dim3(blocks), dim3(kRecRowWarps * 32), scene_rec_smem(), st, jobs, runs, nruns, items, rpi,
+             A);
+}
+void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, unsigned char* wide,
+                       long long slots) {
+  launch_pdl(k_scene_rest<kRecMaxH, kRecWarps>, dim3(blocks), dim3(kRecWarps * 32), scene_rest_smem(), st, jobs, A,
+             wide, slots);
 }
 void launch_scene(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns, long long items,
                   const Arena& A, const uint8_t* tbl, int sliceW) {
@@ -1808,29 +1956,35 @@ size_t setup_smem(int maxBands) {  // counts and flags, then per warp: band coun
 
 size_t scene_wide_bytes() { return sizeof(RowScratch<kWideMaxH, kWideXT>); }
 
-size_t rows_smem_fast() { return sizeof(RowScratch<kFastMaxH, kFastXT>) * kFastWarps; }
 size_t rows_smem_wide() { return sizeof(RowScratch<kWideMaxH, kWideXT>); }
-int rows_warps_fast() { return kFastWarps; }
 
-// Row kernel variants: 0 = 256 crossings / 1024-px coverage tiles / 4 warps
-// per CTA, 1 = 32 crossings / 256-px tiles / 8 warps (small paths such as
-// glyphs: eight times less shared memory per warp, more warps per SM).
+// Row kernel variants: 0 = RGBX images, 1 = masks of small paths such as
+// glyphs (64 crossings and 256-px tiles, a quarter of the shared memory per
+// warp), 2 = the general code, 3 = masks.
+constexpr auto kRowsRgbx = k_rows_fast<kOutRgbx, kRowsNB, kRowsXT, kRowsWarps>;
+constexpr auto kRowsGlyph = k_rows_fast<kOutA8, kGlyphNB, kGlyphXT, kGlyphWarps>;
+constexpr auto kRowsMask = k_rows_fast<kOutA8, kRowsNB, kRowsXT, kRowsWarps>;
+constexpr auto kRowsGeneral = k_rows<kFastMaxH, kFastXT, kFastWarps>;
 const void* rows_kernel(int v) {
-  return v == 1 ? (const void*)k_rows<kSmallMaxH, kSmallXT, kSmallWarps>
-                : (const void*)k_rows<kFastMaxH, kFastXT, kFastWarps>;
+  return v == 0 ? (const void*)kRowsRgbx
+                : v == 1 ? (const void*)kRowsGlyph : v == 2 ? (const void*)kRowsGeneral : (const void*)kRowsMask;
 }
 size_t rows_smem(int v) {
-  return v == 1 ? sizeof(RowScratch<kSmallMaxH, kSmallXT>) * kSmallWarps : rows_smem_fast();
+  return v == 1   ? sizeof(FastRow<kGlyphNB, kGlyphXT>) * kGlyphWarps
+         : v == 2 ? sizeof(RowScratch<kFastMaxH, kFastXT>) * kFastWarps
+                  : sizeof(FastRow<kRowsNB, kRowsXT>) * kRowsWarps;
 }
-int rows_warps(int v) { return v == 1 ? kSmallWarps : kFastWarps; }
+int rows_warps(int v) { return v == 1 ? kGlyphWarps : v == 2 ? kFastWarps : kRowsWarps; }
+// Whether a job's rows can take the row engine (every variant but 2).
+bool rows_fast(int mode, long long W) { return mode != kMask && W < fast_max_w(kRowsNB); }
 void launch_rows(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
                  const Arena& A, const uint8_t* tbl, long long items, int rpi) {
-  if (v == 1)
-    launch_pdl(k_rows<kSmallMaxH, kSmallXT, kSmallWarps>, dim3(blocks), dim3(kSmallWarps * 32), rows_smem(1), st, jobs,
-               offs, njobs, A, tbl, items, rpi);
-  else
-    launch_pdl(k_rows<kFastMaxH, kFastXT, kFastWarps>, dim3(blocks), dim3(kFastWarps * 32), rows_smem(0), st, jobs,
-               offs, njobs, A, tbl, items, rpi);
+  const dim3 b(blocks), t(rows_warps(v) * 32);
+  const size_t sm = rows_smem(v);
+  if (v == 0) launch_pdl(kRowsRgbx, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
+  else if (v == 1) launch_pdl(kRowsGlyph, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
+  else if (v == 2) launch_pdl(kRowsGeneral, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
+  else launch_pdl(kRowsMask, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
 }
 
 }  // namespace pxg

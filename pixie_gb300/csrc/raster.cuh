@@ -60,7 +60,7 @@ struct PathJob {
   uint8_t* img;  // RGBX or A8, row-major, W*H pixels
   long long W, H;
   long long row_off;  // prefix of row-kernel work items over the batch
-  long long ri_off;     // scenes: row y of the job is Arena::rowidx[ri_off + y * ri_stride]
+  long long ri_off;     // scenes: row y of the job is Arena::rowhdr[ri_off + y * ri_stride]
   long long ri_stride;
   int stroke_gpu;       // host: the primitives are a GPU-outlined stroke (scene: in its stroke region)
   int pad_;
@@ -95,8 +95,8 @@ struct SceneRun {
   long long row_off;  // prefix of (row, slice) work items over the launch's runs
   long long W, H;
   uint8_t* img;       // the canvas (RGBX)
-  long long ri_base;  // row y, path j: Arena::rowidx[ri_base + y * (j1 - j0) + j - j0]
-  long long rec_off;  // recording items of the run: rec_off + (j - j0) * H + y
+  long long ri_base;  // row y, path j: Arena::rowhdr[ri_base + y * (j1 - j0) + j - j0]
+  long long rec_off;  // recording items of the run: rec_off + (j - j0) * ceil(H / rpi) + chunk
   int j0, j1;
 };
 
@@ -109,7 +109,7 @@ struct MaskDraw {
 
 enum ArenaCounter {
   kCtrSegs = 0, kCtrBands, kCtrOvfRows, kCtrXClears, kCtrBandSegs, kCtrRowErr, kCtrQueue,
-  kCtrProg, kCtrProgFull, kCtrQueue2, kCtrCov8, kCtrPainted, kNumCounters
+  kCtrProg, kCtrProgFull, kCtrQueue2, kCtrCov8, kCtrPainted, kCtrOvfRows2, kCtrOvfRows3, kNumCounters
 };
 
 struct Arena {
@@ -126,11 +126,11 @@ struct Arena {
   long long primcnt_cap;
   int4* prog;          // scenes: row programs (16-byte units)
   long long prog_cap;
-  int* rowidx;         // scenes: per row and job, the first unit of its program (-1: none)
-  uint8_t* cov8;       // scenes: coverage bytes of rows recorded as kRecCov8
+  int4* rowhdr;        // scenes: per row and job, what it draws (RecKind)
+  uint8_t* cov8;       // scenes: coverage bytes of rows recorded as kRecCov8 (16-byte units)
   long long cov8_cap;
   unsigned long long* counters;
-  long long* ovf_rows;  // packed (job << 32 | y) rows whose crossings exceed the fast kernel
+  long long* ovf_rows;  // packed (job << 32 | y) rows a row kernel hands on (scenes: three lists of ovf_cap)
   long long ovf_cap;
   long long* xclears;   // (job, start, end) linear-pixel clears that reach into earlier rows
   long long xclear_cap;
