@@ -255,74 +255,59 @@ __device__ __forceinline__ float softLight1(float cb, float cs, const float* dsl
   if (cs <= 0.5f) return cb - ((1.0f - 2.0f * cs) * cb) * (1.0f - cb);
   return cb + (2.0f * cs - 1.0f) * (dsl[v] - cb);
 }
-// One float mode, inlined where the mode is a compile-time constant (draw).
-template <int MODE>
-__device__ __forceinline__ uint32_t blendFloatT(const uint8_t* tbl, uint32_t bp, uint32_t sp);
-
-static __device__ __noinline__ uint32_t blendFloat(const uint8_t* tbl, uint32_t bp, uint32_t sp, int mode) {
-  Px b8 = straight8(tbl, bp), s8 = straight8(tbl, sp);
+// One float mode (mode a compile-time constant where a kernel is made for it).
+// Over an opaque backdrop -- a canvas or background filled once stays opaque
+// under every blend mode -- the composite needs no division: with ab = 1 the
+// output alpha as + (1 - as) is exactly 1 for each of the 256 alphas, the
+// mixed source (1 - ab) cs + ab m is m, and the result needs no
+// premultiplication.  The same floats, so the same bytes.  2048 x 2048 draws
+// back to back over opaque images, before -> after: SoftLight 28.6 -> 22.2 us,
+// Hue 40.2 -> 33.6, Saturation 42.5 -> 35.8, Color 31.6 -> 24.7, Luminosity
+// 31.3 -> 24.4; over images of every alpha 29.0 -> 26.6, 38.6 -> 36.1,
+// 41.5 -> 39.1, 29.8 -> 27.2, 32.3 -> 29.6.  (Gathers from the tables under a
+// test for opaque pixels cost more than they save: they no longer overlap.)
+__device__ __forceinline__ uint32_t blend_float(int mode, const uint8_t* tbl, uint32_t bp, uint32_t sp) {
+  const Px b8 = straight8(tbl, bp), s8 = straight8(tbl, sp);
   const float* u = reinterpret_cast<const float*>(tbl + kTblUnitOff);  // u[v] = v / 255.0f
   const float* dsl = reinterpret_cast<const float*>(tbl + kTblSoftOff);
-  F3 cb{u[b8.r], u[b8.g], u[b8.b]};
-  F3 cs{u[s8.r], u[s8.g], u[s8.b]};
-  float ab = u[b8.a], as = u[s8.a];
+  const F3 cb{u[b8.r], u[b8.g], u[b8.b]};
+  const F3 cs{u[s8.r], u[s8.g], u[s8.b]};
+  const float as = u[s8.a];
   F3 m;
-  switch (mode) {
-    case kSoftLight:
-      m = F3{softLight1(cb.r, cs.r, dsl, b8.r), softLight1(cb.g, cs.g, dsl, b8.g),
-             softLight1(cb.b, cs.b, dsl, b8.b)};
-      break;
-    case kHue: m = setLum(setSat(cs, sat3(cb)), lum3(cb)); break;
-    case kSaturation: m = setLum(setSat(cb, sat3(cs)), lum3(cb)); break;
-    case kColor: m = setLum(cs, lum3(cb)); break;
-    default: m = setLum(cb, lum3(cs)); break;
+  if (mode == kSoftLight) {
+    m = F3{softLight1(cb.r, cs.r, dsl, b8.r), softLight1(cb.g, cs.g, dsl, b8.g), softLight1(cb.b, cs.b, dsl, b8.b)};
+  } else {
+    // Hue: setLum(setSat(cs, sat(cb)), lum(cb)); Saturation: setLum(setSat(cb, sat(cs)), lum(cb));
+    // Color: setLum(cs, lum(cb)); Luminosity: setLum(cb, lum(cs))
+    F3 c = mode == kHue || mode == kColor ? cs : cb;
+    if (mode == kHue || mode == kSaturation) c = setSat(c, sat3(mode == kHue ? cb : cs));
+    m = setLum(c, lum3(mode == kLuminosity ? cs : cb));
   }
-  float ao = as + ab * (1.0f - as);
+  if (b8.a == 255) {
+    const float k = 1.0f - as;
+    return pack(unit_to_u8(as * m.r + k * cb.r), unit_to_u8(as * m.g + k * cb.g), unit_to_u8(as * m.b + k * cb.b),
+                255u);
+  }
+  const float ab = u[b8.a];
+  const float ao = as + ab * (1.0f - as);
   if (!(ao > 0.0f)) return 0u;
-  float k = (1.0f - as) * ab;
-  float csr = (1.0f - ab) * cs.r + ab * m.r;
-  float csg = (1.0f - ab) * cs.g + ab * m.g;
-  float csb = (1.0f - ab) * cs.b + ab * m.b;
+  const float k = (1.0f - as) * ab;
+  const float csr = (1.0f - ab) * cs.r + ab * m.r;
+  const float csg = (1.0f - ab) * cs.g + ab * m.g;
+  const float csb = (1.0f - ab) * cs.b + ab * m.b;
   const float yo = __frcp_rn(ao);
-  float orr = div_rcp(as * csr + k * cb.r, ao, yo);
-  float og = div_rcp(as * csg + k * cb.g, ao, yo);
-  float ob = div_rcp(as * csb + k * cb.b, ao, yo);
+  const float orr = div_rcp(as * csr + k * cb.r, ao, yo);
+  const float og = div_rcp(as * csg + k * cb.g, ao, yo);
+  const float ob = div_rcp(as * csb + k * cb.b, ao, yo);
   return premul8(pack(unit_to_u8(orr), unit_to_u8(og), unit_to_u8(ob), unit_to_u8(ao)));
 }
-
 template <int MODE>
 __device__ __forceinline__ uint32_t blendFloatT(const uint8_t* tbl, uint32_t bp, uint32_t sp) {
-  constexpr int mode = MODE;
-  Px b8 = straight8(tbl, bp), s8 = straight8(tbl, sp);
-  const float* u = reinterpret_cast<const float*>(tbl + kTblUnitOff);  // u[v] = v / 255.0f
-  const float* dsl = reinterpret_cast<const float*>(tbl + kTblSoftOff);
-  F3 cb{u[b8.r], u[b8.g], u[b8.b]};
-  F3 cs{u[s8.r], u[s8.g], u[s8.b]};
-  float ab = u[b8.a], as = u[s8.a];
-  F3 m;
-  switch (mode) {
-    case kSoftLight:
-      m = F3{softLight1(cb.r, cs.r, dsl, b8.r), softLight1(cb.g, cs.g, dsl, b8.g),
-             softLight1(cb.b, cs.b, dsl, b8.b)};
-      break;
-    case kHue: m = setLum(setSat(cs, sat3(cb)), lum3(cb)); break;
-    case kSaturation: m = setLum(setSat(cb, sat3(cs)), lum3(cb)); break;
-    case kColor: m = setLum(cs, lum3(cb)); break;
-    default: m = setLum(cb, lum3(cs)); break;
-  }
-  float ao = as + ab * (1.0f - as);
-  if (!(ao > 0.0f)) return 0u;
-  float k = (1.0f - as) * ab;
-  float csr = (1.0f - ab) * cs.r + ab * m.r;
-  float csg = (1.0f - ab) * cs.g + ab * m.g;
-  float csb = (1.0f - ab) * cs.b + ab * m.b;
-  const float yo = __frcp_rn(ao);
-  float orr = div_rcp(as * csr + k * cb.r, ao, yo);
-  float og = div_rcp(as * csg + k * cb.g, ao, yo);
-  float ob = div_rcp(as * csb + k * cb.b, ao, yo);
-  return premul8(pack(unit_to_u8(orr), unit_to_u8(og), unit_to_u8(ob), unit_to_u8(ao)));
+  return blend_float(MODE, tbl, bp, sp);
 }
-
+static __device__ __noinline__ uint32_t blendFloat(const uint8_t* tbl, uint32_t bp, uint32_t sp, int mode) {
+  return blend_float(mode, tbl, bp, sp);
+}
 
 // floor(n / d) for integers held exactly in floats, 0 <= n, n + d < 2^24,
 // 1 <= d, n / d < 2^21.  rd is rcp.approx(d) (relative error below 2^-22), so
@@ -345,26 +330,33 @@ __device__ __forceinline__ uint32_t fdiv_floor(float n, float d, float rd) {
 }
 // ColorBurn / ColorDodge (blends.nim:111-126, :158-173) with the divisions
 // done as above: the same integers as the reference's integer divisions.
-template <bool BURN>
-__device__ __forceinline__ uint32_t blendBurnDodge(const uint8_t* tbl, uint32_t bv, uint32_t sv) {
+// Burn is 255 - dodge of the complements.  Over an opaque backdrop (2048 x 2048
+// ColorBurn draws 28.0 -> 20.3 us) alphaFix's
+// quotient (t1 m + t2 b) / 65025 with t1 = 255 sa, t2 = 255 (255 - sa) is
+// (sa m + (255 - sa) b) / 255, and the result's alpha is 255.
+__device__ __forceinline__ uint32_t blend_burn_dodge(bool burn, const uint8_t* tbl, uint32_t bv, uint32_t sv) {
   const Px bd = straight8(tbl, bv), sr = straight8(tbl, sv);
-  auto mix = [](uint32_t b, uint32_t s) -> uint32_t {
-    if (BURN) {
-      if (b == 255) return 255u;
-      if (s == 0) return 0u;
-      const float sf = small_to_f(s);
-      const uint32_t v = fdiv_floor(small_to_f(255u * (255u - b)), sf, rcp_approx(sf));
-      return 255u - (v < 255u ? v : 255u);
+  const uint32_t flip = burn ? 255u : 0u;
+  auto mix = [&](uint32_t b, uint32_t s) -> uint32_t {
+    b ^= flip;
+    s ^= flip;
+    uint32_t v = 0;
+    if (b != 0) {
+      v = 255;
+      if (s != 255) {
+        const float df = small_to_f(255u - s);
+        v = min(fdiv_floor(small_to_f(255u * b), df, rcp_approx(df)), 255u);
+      }
     }
-    if (b == 0) return 0u;
-    if (s == 255) return 255u;
-    const float df = small_to_f(255u - s);
-    const uint32_t v = fdiv_floor(small_to_f(255u * b), df, rcp_approx(df));
-    return v < 255u ? v : 255u;
+    return v ^ flip;
   };
   const uint32_t mr = mix(bd.r, sr.r), mg = mix(bd.g, sr.g), mb = mix(bd.b, sr.b);
   // alphaFix (blends.nim:18-39): (t0 src + t1 mixed + t2 backdrop) / a / 255 = ... / (255 a)
   const uint32_t sa = sr.a, ba = bd.a;
+  if (ba == 255) {
+    const uint32_t sk = 255 - sa;
+    return pack((sa * mr + sk * bd.r) / 255, (sa * mg + sk * bd.g) / 255, (sa * mb + sk * bd.b) / 255, 255u);
+  }
   const uint32_t a = sa + ba * (255 - sa) / 255;
   if (a == 0) return 0u;
   const float t0 = small_to_f(sa * (255 - ba)), t1 = small_to_f(sa * ba), t2 = small_to_f((255 - sa) * ba);
@@ -373,6 +365,10 @@ __device__ __forceinline__ uint32_t blendBurnDodge(const uint8_t* tbl, uint32_t 
   const float g = fmaf(t0, small_to_f(sr.g), fmaf(t1, small_to_f(mg), t2 * small_to_f(bd.g)));
   const float b = fmaf(t0, small_to_f(sr.b), fmaf(t1, small_to_f(mb), t2 * small_to_f(bd.b)));
   return premul8(pack(fdiv_floor(r, d, rd), fdiv_floor(g, d, rd), fdiv_floor(b, d, rd), a));
+}
+template <bool BURN>
+__device__ __forceinline__ uint32_t blendBurnDodge(const uint8_t* tbl, uint32_t bv, uint32_t sv) {
+  return blend_burn_dodge(BURN, tbl, bv, sv);
 }
 
 // blender(mode)(backdrop, source)  blends.nim:275-299
@@ -385,10 +381,12 @@ __device__ __forceinline__ uint32_t blend_px(int mode, const uint8_t* tbl, uint3
   }
   Px b = unpack(bv), s = unpack(sv);
   switch (mode) {
-    case kDarken: {  // :72-84
-      auto f = [](uint32_t bc, uint32_t ba, uint32_t sc, uint32_t sa) {
+    case kDarken:  // :72-84
+    case kLighten: {  // :128-140
+      const bool dark = mode == kDarken;
+      auto f = [&](uint32_t bc, uint32_t ba, uint32_t sc, uint32_t sa) {
         uint32_t x = bc + ((255 - ba) * sc) / 255, y = sc + ((255 - sa) * bc) / 255;
-        return (x < y ? x : y) & 255u;
+        return (dark ? min(x, y) : max(x, y)) & 255u;
       };
       return pack(f(b.r, b.a, s.r, s.a), f(b.g, b.a, s.g, s.a), f(b.b, b.a, s.b, s.a), blendAlpha(b.a, s.a));
     }
@@ -398,21 +396,14 @@ __device__ __forceinline__ uint32_t blend_px(int mode, const uint8_t* tbl, uint3
       };
       return pack(f(b.r, b.a, s.r, s.a), f(b.g, b.a, s.g, s.a), f(b.b, b.a, s.b, s.a), blendAlpha(b.a, s.a));
     }
-    case kLighten: {  // :128-140
-      auto f = [](uint32_t bc, uint32_t ba, uint32_t sc, uint32_t sa) {
-        uint32_t x = bc + ((255 - ba) * sc) / 255, y = sc + ((255 - sa) * bc) / 255;
-        return (x > y ? x : y) & 255u;
-      };
-      return pack(f(b.r, b.a, s.r, s.a), f(b.g, b.a, s.g, s.a), f(b.b, b.a, s.b, s.a), blendAlpha(b.a, s.a));
-    }
     case kScreen:  // :142-146
       return pack(screen1(b.r, s.r), screen1(b.g, s.g), screen1(b.b, s.b), blendAlpha(b.a, s.a));
-    case kOverlay:  // :175-179
-      return pack(hardLight1(s.r, s.a, b.r, b.a), hardLight1(s.g, s.a, b.g, b.a),
-                  hardLight1(s.b, s.a, b.b, b.a), blendAlpha(b.a, s.a));
-    case kHardLight:  // :184-188
-      return pack(hardLight1(b.r, b.a, s.r, s.a), hardLight1(b.g, b.a, s.g, s.a),
-                  hardLight1(b.b, b.a, s.b, s.a), blendAlpha(b.a, s.a));
+    case kOverlay:     // :175-179: HardLight with the two exchanged
+    case kHardLight: {  // :184-188
+      const Px x = mode == kOverlay ? s : b, y = mode == kOverlay ? b : s;
+      return pack(hardLight1(x.r, x.a, y.r, y.a), hardLight1(x.g, x.a, y.g, y.a), hardLight1(x.b, x.a, y.b, y.a),
+                  blendAlpha(b.a, s.a));
+    }
     case kDifference: {  // :190-204; (bc + sc) wraps as uint8
       auto f = [](uint32_t bc, uint32_t ba, uint32_t sc, uint32_t sa) {
         uint32_t m1 = bc * sa, m2 = sc * ba;
@@ -428,8 +419,8 @@ __device__ __forceinline__ uint32_t blend_px(int mode, const uint8_t* tbl, uint3
       };
       return pack(f(b.r, s.r), f(b.g, s.g), f(b.b, s.b), blendAlpha(b.a, s.a));
     }
-    case kColorBurn: return blendBurnDodge<true>(tbl, bv, sv);
-    case kColorDodge: return blendBurnDodge<false>(tbl, bv, sv);
+    case kColorBurn:
+    case kColorDodge: return blend_burn_dodge(mode == kColorBurn, tbl, bv, sv);
     case kSoftLight:
     case kHue:
     case kSaturation:
