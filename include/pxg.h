@@ -273,7 +273,7 @@ int pxg_scene_record_batch(pxg_scene* scene, int64_t n, const int32_t* kinds, co
 int pxg_image_draw_scene(pxg_image* image, const pxg_scene* scene);
 /* Scene drawing configuration (every choice writes the same bytes):
  * slice_width is the part of a canvas row one warp of the drawing pass owns
- * (>= 32 pixels; default 256), or 0 to choose it per launch from the canvas
+ * (>= 32 pixels), or 0 -- and by default -- chosen per launch from the canvas
  * rows and the GPU's resident warps.  coverage_bytes >= 0 replaces the arena
  * in which the recording pass stores rows' coverage bytes (default: 4 GB or
  * an eighth of free memory); rows that do not fit are recorded as sample

@@ -120,9 +120,8 @@ __global__ void k_xclears(PathJob* jobs, Arena A);
 const void* scene_rec_kernel();
 size_t scene_rec_smem();
 int scene_rec_warps();
-const void* scene_kernel();
+const void* scene_kernel(int ppl);
 int scene_warps();
-int scene_tile();
 const void* scene_big_kernel(int v);
 size_t scene_big_smem(int v);
 int scene_big_warps(int v);
@@ -134,8 +133,8 @@ void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const Sce
                       long long items, int rpi, const Arena& A);
 void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, unsigned char* wide,
                        long long slots);
-void launch_scene(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns, long long items,
-                  const Arena& A, const uint8_t* tbl, int sliceW);
+void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
+                  long long items, const Arena& A, const uint8_t* tbl, int sliceW);
 size_t scene_wide_bytes();
 size_t setup_smem(int maxBands);
 int draw_masks_tiles();
@@ -268,6 +267,8 @@ struct Ctx {
   long long prog_cap = 0;
   int4* rowhdr = nullptr;         // scene rows: what each draws
   long long rowhdr_cap = 0;
+  uint2* pinfo = nullptr;         // scene paths: colour, mode, status
+  long long pinfo_cap = 0;
   uint8_t* cov8 = nullptr;        // scene coverage bytes (rows that fit; the rest keep spans)
   long long cov8_cap = 0;
   unsigned char* wide = nullptr;  // per-warp wide row scratch of the scene recording kernel
@@ -308,7 +309,7 @@ struct Ctx {
   long long stats[6] = {0, 0, 0, 0, 0, 0};  // last fill launch: paths, prims, segments, entries, blends, wide rows
   int rows_ctas_per_sm[4] = {1, 1, 1, 1};  // resident CTAs of each row-kernel variant
   int scene_ctas_per_sm[5] = {1, 1, 1, 1, 1};  // resident CTAs of the scene recording, drawing, rest and big-row kernels
-  int scene_slice = 256;              // pixels of a row one warp of the drawing pass owns (0: chosen per launch)
+  int scene_slice = 0;                // pixels of a row one warp of the drawing pass owns (0: chosen per launch)
   bool stroke_gpu = true;             // outline strokes without dashes on the GPU (stroke.cu)
   float2* sk_pts = nullptr;           // outline kernel inputs: polyline points, shapes
   long long sk_pts_cap = 0;
@@ -387,7 +388,7 @@ void init_locked(int device) {
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_rest_kernel(), scene_rest_warps() * 32,
                                                      scene_rest_smem()));
     g.scene_ctas_per_sm[2] = std::max(1, per);
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_kernel(), scene_warps() * 32, 0));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_kernel(4), scene_warps() * 32, 0));
     g.scene_ctas_per_sm[1] = std::max(1, per);
   }
   g.setupSmemMax = allow_max_smem((const void*)k_setup);
@@ -602,6 +603,7 @@ Staged stage(const std::vector<PathJob>& run, const void* extra, size_t extraByt
   A.prog = g.prog;
   A.prog_cap = g.prog_cap;
   A.rowhdr = g.rowhdr;
+  A.pinfo = nullptr;
   A.cov8 = g.cov8;
   A.cov8_cap = g.cov8_cap;
   A.counters = reinterpret_cast<unsigned long long*>(g.d_up + S.jobsBytes);
@@ -910,24 +912,19 @@ const Prim* scene_device_prims(const pxg_scene* sc) {
   return sc->dprims;
 }
 
-// The row slice of the drawing pass.  Each work item replays every path of
-// its run, so items are long and the kernel lasts as long as its busiest
-// warp: the slice is chosen so that the launch has about three items per
-// resident warp (at most 256 pixels, the shared-memory stage), unless a
-// width was set with pxg_scene_config.
-int scene_slice_for(const std::vector<HostRun>& runs) {
-  if (g.scene_slice > 0) return g.scene_slice;
-  long long rows = 0, wmax = 1;
-  for (const HostRun& r : runs) {
-    if (r.status != kOk || r.j0 >= r.j1) continue;
-    rows += r.canvas->height;
-    wmax = std::max<long long>(wmax, r.canvas->width);
-  }
+// The row slice of the drawing pass (a multiple of 4 pixels) and its pixels
+// per lane.  Each work item replays every path of its run, so the kernel lasts
+// as long as its busiest warp: 128-pixel slices, four pixels a lane, when
+// those give every resident warp one; 32-pixel slices, one pixel a lane,
+// below that.  A width set with pxg_scene_config is kept.
+int scene_slice_for(const std::vector<HostRun>& runs, int& ppl) {
+  long long items = 0;
+  for (const HostRun& r : runs)
+    if (r.status == kOk && r.j0 < r.j1) items += r.canvas->height * ((r.canvas->width + 127) / 128);
   const long long slots = (long long)g.nsm * g.scene_ctas_per_sm[1] * scene_warps();
-  const long long per_row = std::max<long long>(1, (3 * slots + rows - 1) / std::max<long long>(rows, 1));
-  long long w = (wmax + per_row - 1) / per_row;
-  w = std::max<long long>(32, std::min<long long>(w, scene_tile()));
-  return (int)w;
+  ppl = items >= slots ? 4 : 1;
+  if (g.scene_slice > 0) return std::min((g.scene_slice + 3) / 4 * 4, 1 << 20);
+  return 32 * ppl;
 }
 
 // Rows of a recording work item.  Whole band chunks (a band's entries are
@@ -956,7 +953,8 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     std::vector<SceneRun> sr;
     std::vector<size_t> which;  // launch run -> runs index
     long long items = 0, recItems = 0, riTotal = 0, maxH = 1;
-    const int slice = scene_slice_for(runs);
+    int ppl = 4;
+    const int slice = scene_slice_for(runs, ppl);
     long long pathRows = 0;
     for (const HostRun& r : runs)
       if (r.status == kOk && r.j0 < r.j1) pathRows += (long long)(r.j1 - r.j0) * r.canvas->height;
@@ -1030,6 +1028,8 @@ void run_scene_runs(std::vector<HostRun>& runs) {
         1, std::min<long long>((items + scene_warps() - 1) / scene_warps(), (long long)g.nsm * g.scene_ctas_per_sm[1]));
     Staged S = stage(dev, sr.data(), sizeof(SceneRun) * sr.size(), std::vector<Prim>());
     S.A.ovf_cap = g.ovf_cap / 3;  // three lists
+    dev_grow(g.pinfo, g.pinfo_cap, (long long)nj);
+    S.A.pinfo = g.pinfo;
     k_setup<<<nj, 256, setup_smem(maxBands), g.stream>>>(S.dj, S.A, maxBands); note_launch();
     CU(cudaGetLastError());
     CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
@@ -1047,7 +1047,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     launch_scene_rest((unsigned)restBlocks, g.stream, S.dj, S.A, g.wide, g.wide_slots);
     note_launch();
     CU(cudaGetLastError());
-    launch_scene((unsigned)blocks, g.stream, S.dj, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(), items,
+    launch_scene(ppl, (unsigned)blocks, g.stream, S.dj, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(), items,
                  S.A, g.tbl, slice);
     note_launch();
     CU(cudaGetLastError());

@@ -395,6 +395,11 @@ __device__ long long block_excl_scan(long long v, long long* s_warp, long long& 
 // ---------------------------------------------------------------------------
 // k_setup: flatten -> segments -> bounds -> partitions (one CTA per job)
 // ---------------------------------------------------------------------------
+// The job's outcome, and beside its colour and mode for the drawing pass.
+__device__ __forceinline__ void set_status(PathJob& J, const Arena& A, int st) {
+  J.status = st;
+  if (A.pinfo) A.pinfo[blockIdx.x] = make_uint2(J.rgbx, (uint32_t)J.mode | ((uint32_t)st << 8));
+}
 __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBands) {
   pdl_trigger();  // the row kernel may be set up while this runs; it waits for the segments
   pdl_wait();
@@ -460,7 +465,7 @@ __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBa
   }
   __syncthreads();
   if (s_err != LLONG_MAX) {
-    if (tid == 0) J.status = (int)(s_err & 255);
+    if (tid == 0) set_status(J, A, (int)(s_err & 255));
     return;
   }
   // exclusive prefix of the counts, in primitive order
@@ -480,7 +485,7 @@ __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBa
   }
   __syncthreads();
   if (s_status != kOk) {
-    if (tid == 0) J.status = s_status;
+    if (tid == 0) set_status(J, A, s_status);
     return;
   }
 
@@ -583,7 +588,7 @@ __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBa
   }
   __syncthreads();
   if (s_status != kOk) {
-    if (tid == 0) J.status = s_status;
+    if (tid == 0) set_status(J, A, s_status);
     return;
   }
   const long long startY = s_hdr[1], pathHeight = s_hdr[3];
@@ -661,7 +666,7 @@ __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBa
   }
   __syncthreads();
   if (s_status != kOk) {
-    if (tid == 0) J.status = s_status;
+    if (tid == 0) set_status(J, A, s_status);
     return;
   }
   // Phase E: each band's entry list, segment indices ascending -- the order in
@@ -690,7 +695,7 @@ __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBa
   }
   __syncthreads();
   if (s_status != kOk) {
-    if (tid == 0) J.status = s_status;
+    if (tid == 0) set_status(J, A, s_status);
     return;
   }
   int* L = A.bandseg + s_listbase;
@@ -734,7 +739,7 @@ __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBa
     }
     if (tid == 0) {
       J.band_off = s_bandbase;
-      J.status = kOk;
+      set_status(J, A, kOk);
     }
     return;
   }
@@ -780,7 +785,7 @@ __global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBa
   }
   if (tid == 0) {
     J.band_off = s_bandbase;
-    J.status = kOk;
+    set_status(J, A, kOk);
   }
 }
 
@@ -1774,18 +1779,54 @@ __global__ void __launch_bounds__(WARPS * 32) k_scene_rest(PathJob* jobs, Arena 
   }
 }
 
-template <int XT, int WARPS>
+// A recorded program (RecKind) drawn within [xa, xb) of a row by the general
+// code; out of line, for rows are rarely recorded so.  Returns the number of
+// blends.
+template <int XT>
+static __device__ __noinline__ unsigned draw_program(RowPx<false> row, int mode, const uint8_t* tbl, uint32_t rgbx,
+                                                     const int4* prog, int lo, int hi, long long y, int W, int xa,
+                                                     int xb, int* acc, int lane) {
+  unsigned cnt = 0;
+  const int4 g = prog[0];
+  if (g.x == kRecCov) {
+    apply_cov<false, XT>(row, mode, tbl, rgbx, reinterpret_cast<const int2*>(prog + 1), g.y, g.z, max(lo, xa),
+                         min(hi, xb), acc, lane, &cnt);
+  } else if (g.x == kRecHits) {
+    apply_hits<false>(row, mode, tbl, rgbx, reinterpret_cast<const int2*>(prog + 1), g.y, xa, xb, lane, &cnt);
+  } else if (g.x == kRecTrap) {
+#pragma unroll 1
+    for (int t = 0; t < g.y; t++) {
+      const int4 e = prog[1 + 2 * t], u = prog[2 + 2 * t];
+      apply_trap_pair<false>(row, mode, tbl, rgbx, y, W, __int_as_float(e.x), __int_as_float(e.y), __int_as_float(e.z),
+                             __int_as_float(e.w), __int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z),
+                             __int_as_float(u.w), xa, xb, lane, &cnt);
+    }
+  }
+  return __reduce_add_sync(0xffffffffu, cnt);
+}
+
+// The drawing pass.  What bounds it: issue -- a blend is 40 to 250 instructions
+// a pixel and the modes of a scene differ path by path -- and the latency of
+// one warp's path sequence.  A lane keeps PPL pixels of a step (pixels lane,
+// lane + 32, ...) in registers while the launch's paths are applied, so a path
+// costs its coverage bytes (one word per lane, requested a path ahead, dealt
+// out by shuffles) and no pixel traffic; 32-pixel groups a path does not touch
+// are skipped, and each mode's blend exists once (the lane's pixels rotate
+// through it), which keeps the kernel within the instruction cache.  PPL = 4;
+// PPL = 1 for launches with too few rows to fill the GPU, where a path's time
+// on its warp matters and not the instructions per pixel.
+template <int PPL, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const SceneRun* runs, int nruns,
-                                                      long long totalItems, Arena A, const uint8_t* tbl,
-                                                      int sliceW) {
-  __shared__ int accs[WARPS][XT + 1];
-  __shared__ uint32_t pix[WARPS][XT];  // the warp's row slice while its paths are applied
+                                                         long long totalItems, Arena A, const uint8_t* tbl,
+                                                         int sliceW) {
+  constexpr int SW = 32 * PPL;          // pixels of a step
+  __shared__ int accs[WARPS][SW + 1];   // recorded programs: a coverage tile and the step's pixels
+  __shared__ uint32_t pix[WARPS][SW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_trigger();
   pdl_wait();
-  int* acc = accs[warp];
-  const bool staged = sliceW <= XT;
   if (A.counters[kCtrProgFull]) return;  // programs incomplete: the host reruns the launch
+#pragma unroll 1
   while (true) {
     unsigned long long q = 0;
     if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue2], 1ull);
@@ -1797,120 +1838,127 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
       if (runs[mid].row_off <= item) lo = mid;
       else hi = mid - 1;
     }
-    const SceneRun R = runs[lo];
+    const SceneRun& R = runs[lo];
+    const int W = (int)R.W, njobs = R.j1 - R.j0;
     const long long ns = (R.W + sliceW - 1) / sliceW;
     const long long local = item - R.row_off;
-    const long long y = local / ns;
-    const long long xa = (local % ns) * sliceW, xb = min(xa + sliceW, R.W);
-    if (y >= R.H) continue;
-    uint32_t* grow = reinterpret_cast<uint32_t*>(R.img) + y * R.W;
-    if (staged) {
-      for (long long x = xa + lane; x < xb; x += 32) pix[warp][x - xa] = grow[x];
-      __syncwarp();
-    }
-    const RowPx<false> row = staged ? RowPx<false>{reinterpret_cast<unsigned char*>(pix[warp]), xa}
-                                    : RowPx<false>{reinterpret_cast<unsigned char*>(grow), 0};
+    const int y = (int)(local / ns);
+    const int xs = (int)(local % ns) * sliceW, xe = min(xs + sliceW, W);
+    uint32_t* grow = reinterpret_cast<uint32_t*>(R.img) + (long long)y * W;
+    const int4* hdr = A.rowhdr + R.ri_base + (long long)y * njobs;
+    const uint2* info = A.pinfo + R.j0;
     unsigned painted = 0;  // pixel blends of this item (reported as a launch counter)
-    // 32 paths at a time: each lane loads one path's row program index and
-    // header (the row's indices are contiguous), then the warp replays the
-    // programs in path order.
-    const long long rb = R.ri_base + y * (long long)(R.j1 - R.j0);
-    for (int c0 = R.j0; c0 < R.j1; c0 += 32) {
-      const int j = c0 + lane;
-      const bool valid = j < R.j1;
-      int st = kNothing, mode = 0;
-      uint32_t rgbx = 0;
-      int4 rh = make_int4(0, 0, 0, 0);
-      if (valid) {
-        const PathJob& J = jobs[j];
-        st = J.status;
-        rh = A.rowhdr[rb + (j - R.j0)];
-        mode = J.mode;
-        rgbx = J.rgbx;
-      }
-      // the first failed path stops the run: it and the paths after it draw nothing
-      const unsigned bad = __ballot_sync(0xffffffffu, valid && st != kOk && st != kNothing);
-      const int lim = bad ? __ffs(bad) - 1 : 32;
-      const bool draws = valid && lane < lim && st == kOk && rh.x != 0 && rh.z < xb && rh.w > xa;
-      int4 h = rh;
-      if (draws && rh.x == kRecProg) h = A.prog[rh.y];
-      unsigned dm = __ballot_sync(0xffffffffu, draws);
-      while (dm) {
-        const int i = __ffs(dm) - 1;
-        dm &= dm - 1;
-        const int hx = __shfl_sync(0xffffffffu, h.x, i), hy = __shfl_sync(0xffffffffu, h.y, i);
-        const int hz = __shfl_sync(0xffffffffu, h.z, i), hw = __shfl_sync(0xffffffffu, h.w, i);
-        const int ai = __shfl_sync(0xffffffffu, rh.y, i), mi = __shfl_sync(0xffffffffu, mode, i);
-        const uint32_t ci = __shfl_sync(0xffffffffu, rgbx, i);
-        const int p0 = __shfl_sync(0xffffffffu, rh.z, i), p1 = __shfl_sync(0xffffffffu, rh.w, i);
-        if (hx == kRecFill) {
-          for (long long x = max((long long)hz, xa) + lane; x < min((long long)hw, xb); x += 32) {
-            row[x] = op_fill(mi, tbl, row[x], ci);
-            ++painted;
-          }
-        } else if (hx == kRecCov) {
-          apply_cov<false, XT>(row, mi, tbl, ci, reinterpret_cast<const int2*>(A.prog + ai + 1), hy, hz,
-                               max((long long)p0, xa), min((long long)p1, xb), acc, lane, &painted);
-        } else if (hx == kRecCov8 || hx == kRecCov8Z) {
-          int4 u = make_int4(ai, 0, 0, 0);
-          if (hx == kRecCov8Z) u = A.prog[ai];
-          const uint8_t* cv8 = A.cov8 + ((long long)(unsigned)u.x << 4) - hz;
-          const long long x0 = max((long long)hz, xa), x1 = min((long long)hw, xb);
-          uint32_t cvN = 0, bdN = 0;
-          if (x0 + lane < x1) {
-            cvN = cv8[x0 + lane];
-            if (cvN) bdN = row[x0 + lane];
-          }
 #pragma unroll 1
-          for (long long x = x0 + lane; x < x1; x += 32) {
-            const uint32_t cv = cvN, bd = bdN;
-            cvN = 0;
-            if (x + 32 < x1) {
-              cvN = cv8[x + 32];
-              if (cvN) bdN = row[x + 32];
-            }
-            if (cv) {
-              row[x] = op_cov(mi, tbl, bd, ci, cv);
-              ++painted;
-            }
-          }
-          if (lane < u.y) {
-            const int x = reinterpret_cast<const int*>(A.prog + ai + 1)[lane];
-            if (x >= xa && x < xb) {
-              row[x] = blend_any(mi, tbl, row[x], 0u);
-              ++painted;
-            }
-          }
-        } else if (hx == kRecHits) {
-          apply_hits<false>(row, mi, tbl, ci, reinterpret_cast<const int2*>(A.prog + ai + 1), hy, xa, xb, lane,
-                            &painted);
-        } else if (hx == kRecTrap) {
-          for (int p = 0; p < hy; p++) {
-            const int4 e = A.prog[ai + 1 + 2 * p], t = A.prog[ai + 2 + 2 * p];
-            apply_trap_pair<false>(row, mi, tbl, ci, y, R.W, __int_as_float(e.x), __int_as_float(e.y),
-                                   __int_as_float(e.z), __int_as_float(e.w), __int_as_float(t.x),
-                                   __int_as_float(t.y), __int_as_float(t.z), __int_as_float(t.w), xa, xb, lane,
-                                   &painted);
-          }
-        }
-        __syncwarp();
-      }
-      if (bad) break;
-    }
-    if (staged) {
-      for (long long x = xa + lane; x < xb; x += 32) grow[x] = pix[warp][x - xa];
-      __syncwarp();
-    }
+    for (int xa = xs; xa < xe; xa += SW) {
+      const int xb = min(xa + SW, xe);
+      uint32_t p[PPL];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) painted += __shfl_xor_sync(0xffffffffu, painted, o);
+      for (int i = 0; i < PPL; i++) p[i] = xa + i * 32 + lane < xb ? grow[xa + i * 32 + lane] : 0u;
+      // 32 paths at a time: each lane loads one path's row header (contiguous
+      // over the paths) and colour, then the warp applies them in path order
+#pragma unroll 1
+      for (int c0 = 0; c0 < njobs; c0 += 32) {
+        uint2 in = make_uint2(0u, (uint32_t)kNothing << 8);
+        int4 h = make_int4(0, 0, 0, 0);
+        if (c0 + lane < njobs) {
+          in = info[c0 + lane];
+          h = hdr[c0 + lane];
+        }
+        // the first failed path stops the run: it and the paths after it draw nothing
+        const int st = (int)(in.y >> 8);
+        const unsigned bad = __ballot_sync(0xffffffffu, st != kOk && st != kNothing);
+        const int lim = bad ? __ffs(bad) - 1 : 32;
+        unsigned dm = __ballot_sync(0xffffffffu, lane < lim && st == kOk && h.x != 0 && h.z < xb && h.w > xa);
+        int next = -1;      // the path after the current one, and its coverage
+        uint32_t nextCov = 0;
+        bool first = true;
+#pragma unroll 1
+        while (true) {
+          const int cur = next;
+          const uint32_t cov = nextCov;
+          next = -1;
+          if (dm) {
+            next = __ffs(dm) - 1;
+            dm &= dm - 1;
+            const int kind = __shfl_sync(0xffffffffu, h.x, next), hlo = __shfl_sync(0xffffffffu, h.z, next);
+            const int hhi = __shfl_sync(0xffffffffu, h.w, next), x = xa + 4 * lane;
+            unsigned unit = (unsigned)__shfl_sync(0xffffffffu, h.y, next);
+            nextCov = 0;
+            if (kind == kRecFill) {
+              const int b0 = min(max(hlo - x, 0), 4), b1 = min(max(min(hhi, xb) - x, 0), 4);
+              if (b1 > b0) nextCov = (uint32_t)((1ull << (8 * b1)) - (1ull << (8 * b0)));
+            } else if (kind != kRecProg) {
+              if (kind == kRecCov8Z) unit = (unsigned)A.prog[unit].x;
+              // whole words: lo is a multiple of 16, the bytes past hi are zero
+              if (lane < 8 * PPL && x >= hlo && x < hhi && x < xb)
+                nextCov = *reinterpret_cast<const uint32_t*>(A.cov8 + ((long long)unit << 4) + (x - hlo));
+            }
+          }
+          if (cur < 0) {
+            if (!first || next < 0) break;
+            first = false;
+            continue;
+          }
+          first = false;
+          const uint32_t col = __shfl_sync(0xffffffffu, in.x, cur);
+          const int mode = (int)(__shfl_sync(0xffffffffu, in.y, cur) & 255u);
+          if (__any_sync(0xffffffffu, cov != 0)) {
+#pragma unroll 1
+            for (int i = 0; i < PPL; i++) {
+              const uint32_t k = (__shfl_sync(0xffffffffu, cov, i * 8 + (lane >> 2)) >> (8 * (lane & 3))) & 255u;
+              uint32_t v = p[0];
+              const unsigned on = __ballot_sync(0xffffffffu, k != 0);
+              painted += __popc(on);
+              if (k) {
+                const uint32_t s = mul_c(col, k);
+                v = mode == kNormal ? blendNormal(v, s) : blend_px(mode, tbl, v, s);
+              }
+#pragma unroll
+              for (int t = 0; t + 1 < PPL; t++) p[t] = p[t + 1];
+              p[PPL - 1] = v;
+            }
+          }
+          const int ck = __shfl_sync(0xffffffffu, h.x, cur);
+          if (ck != kRecCov8Z && ck != kRecProg) continue;
+          const int cp = __shfl_sync(0xffffffffu, h.y, cur);
+          if (ck == kRecCov8Z) {  // and the listed pixels with an empty source
+            const int nz = A.prog[cp].y;
+#pragma unroll 1
+            for (int z = 0; z < nz; z++) {
+              const int x = reinterpret_cast<const int*>(A.prog + cp + 1)[z];
+              if (x < xa || x >= xb) continue;
+              ++painted;
+#pragma unroll
+              for (int i = 0; i < PPL; i++)
+                if (xa + i * 32 + lane == x) p[i] = blend_any(mode, tbl, p[i], 0u);
+            }
+            continue;
+          }
+          // a program: the general code, on the step's pixels in shared memory
+#pragma unroll
+          for (int i = 0; i < PPL; i++) pix[warp][i * 32 + lane] = p[i];
+          __syncwarp();
+          const RowPx<false> row{reinterpret_cast<unsigned char*>(pix[warp]), xa};
+          const int plo = __shfl_sync(0xffffffffu, h.z, cur), phi = __shfl_sync(0xffffffffu, h.w, cur);
+          painted += draw_program<SW>(row, mode, tbl, col, A.prog + cp, plo, phi, y, W, xa, xb, accs[warp], lane);
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < PPL; i++) p[i] = pix[warp][i * 32 + lane];
+          __syncwarp();
+        }
+        if (bad) break;
+      }
+#pragma unroll
+      for (int i = 0; i < PPL; i++)
+        if (xa + i * 32 + lane < xb) grow[xa + i * 32 + lane] = p[i];
+    }
     if (lane == 0 && painted) atomicAdd(&A.counters[kCtrPainted], (unsigned long long)painted);
   }
 }
 
 // Scene kernels: the general recording code holds 128 crossings per row in
-// shared memory (8 warps per CTA); the drawing pass keeps one 256-pixel
-// coverage tile per warp.
-constexpr int kRecMaxH = 128, kRecWarps = 8, kSceneXT = 256, kSceneWarps = 8;
+// shared memory (8 warps per CTA).
+constexpr int kRecMaxH = 128, kRecWarps = 8, kSceneWarps = 8;
 const void* scene_rec_kernel() { return (const void*)k_scene_rec; }
 size_t scene_rec_smem() { return sizeof(FastRow<kRecNB, kRecRowXT>) * kRecRowWarps; }
 int scene_rec_warps() { return kRecRowWarps; }
@@ -1928,9 +1976,10 @@ void launch_scene_big(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, co
 const void* scene_rest_kernel() { return (const void*)k_scene_rest<kRecMaxH, kRecWarps>; }
 size_t scene_rest_smem() { return sizeof(RowScratch<kRecMaxH, kRecXT>) * kRecWarps; }
 int scene_rest_warps() { return kRecWarps; }
-const void* scene_kernel() { return (const void*)k_scene<kSceneXT, kSceneWarps>; }
+const void* scene_kernel(int ppl) {
+  return ppl == 1 ? (const void*)k_scene<1, kSceneWarps> : (const void*)k_scene<4, kSceneWarps>;
+}
 int scene_warps() { return kSceneWarps; }
-int scene_tile() { return kSceneXT; }
 void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
                       long long items, int rpi, const Arena& A) {
   launch_pdl(k_scene_rec, dim3(blocks), dim3(kRecRowWarps * 32), scene_rec_smem(), st, jobs, runs, nruns, items, rpi,
@@ -1941,10 +1990,10 @@ void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Ar
   launch_pdl(k_scene_rest<kRecMaxH, kRecWarps>, dim3(blocks), dim3(kRecWarps * 32), scene_rest_smem(), st, jobs, A,
              wide, slots);
 }
-void launch_scene(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns, long long items,
-                  const Arena& A, const uint8_t* tbl, int sliceW) {
-  launch_pdl(k_scene<kSceneXT, kSceneWarps>, dim3(blocks), dim3(kSceneWarps * 32), 0, st, jobs, runs, nruns, items,
-             A, tbl, sliceW);
+void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
+                  long long items, const Arena& A, const uint8_t* tbl, int sliceW) {
+  launch_pdl(ppl == 1 ? k_scene<1, kSceneWarps> : k_scene<4, kSceneWarps>, dim3(blocks), dim3(kSceneWarps * 32), 0, st,
+             jobs, runs, nruns, items, A, tbl, sliceW);
 }
 
 // Dynamic shared memory of k_setup for a launch whose images have at most
