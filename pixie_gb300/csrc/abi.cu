@@ -108,7 +108,9 @@ struct pxg_server {
 };
 
 namespace pxg {
-__global__ void k_setup(PathJob* jobs, Arena A, int maxBands);
+__global__ void k_setup(PathJob* jobs, Arena A, int maxBands, int C);
+int setup_cluster(long long njobs, long long maxWork, int maxBands);
+cudaError_t launch_setup(int njobs, int C, int maxBands, cudaStream_t st, PathJob* jobs, const Arena& A);
 const void* rows_kernel(int v);
 size_t rows_smem(int v);
 int rows_warps(int v);
@@ -237,7 +239,7 @@ struct Ctx {
   bool ready = false;
   int dev = 0, nsm = 0;
   size_t smemOptin = 48 * 1024;
-  size_t setupSmemMax = 0, blurSmemMax = 0;
+  size_t blurSmemMax = 0;
   cudaStream_t own = nullptr, stream = nullptr;
   // Non-blocking mode: uploads and downloads run on their own streams.  Each
   // call's compute waits for the copies issued before it (copies_pending); a
@@ -283,8 +285,6 @@ struct Ctx {
   long long pt_stops_cap = 0;
   uint32_t* sm_buf[2] = {nullptr, nullptr};  // minify/magnify pre-pass images (ping-pong)
   long long sm_cap[2] = {0, 0};
-  uint8_t* fsteps = nullptr;  // flattening step records (fill setup)
-  long long fsteps_cap = 0;
   // upload area: jobs | counters | prims (device and pinned mirror)
   unsigned char* d_up = nullptr;
   unsigned char* h_up = nullptr;
@@ -391,7 +391,7 @@ void init_locked(int device) {
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_kernel(4), scene_warps() * 32, 0));
     g.scene_ctas_per_sm[1] = std::max(1, per);
   }
-  g.setupSmemMax = allow_max_smem((const void*)k_setup);
+  allow_max_smem((const void*)k_setup);
   g.blurSmemMax = std::min(allow_max_smem((const void*)k_blur_x), allow_max_smem((const void*)k_blur_y));
   g.blurSmemMax = std::min(g.blurSmemMax, allow_max_smem((const void*)k_blurf_x));
   g.blurSmemMax = std::min(g.blurSmemMax, allow_max_smem((const void*)k_blurf_y));
@@ -521,15 +521,16 @@ int64_t nim_round_int(float v) {
   return (int64_t)r;
 }
 
-// Lanes per curve in the setup kernel's flattening: the 256 threads of a job's
-// CTA shared out over its curves (a power of two, 1..32).
-int curve_group(const std::vector<Prim>& prims, long long off, int n) {
-  long long curves = 0;
+// Quadratics and cubics among a job's primitives (the setup kernel shares its
+// threads out over them).
+int count_curves(const std::vector<Prim>& prims, long long off, int n) {
+  int curves = 0;
   for (int i = 0; i < n; i++) curves += prims[(size_t)(off + i)].kind != kPrimLine;
-  int gsz = 1;
-  while (gsz < 32 && curves * gsz * 2 <= 256) gsz *= 2;
-  return gsz;
+  return curves;
 }
+// What the setup kernel spends on a job, in lines: a curve's search takes some
+// tens of them.
+long long setup_work(const PathJob& j) { return j.nprims + 24LL * j.curves; }
 
 // Workspace of the fill kernels, grown on demand (never shrunk).
 void ensure_arena(long long seg_need, long long list_need, long long nbands, long long nprims, long long rows) {
@@ -611,12 +612,6 @@ Staged stage(const std::vector<PathJob>& run, const void* extra, size_t extraByt
   A.ovf_cap = g.ovf_cap;
   A.xclears = g.xcl;
   A.xclear_cap = g.xcl_cap / 3;
-  if (!g.fsteps) {  // step records of the first 16 setup CTAs of a launch (512 steps x 256 groups each)
-    CU(cudaMalloc(&g.fsteps, (size_t)16 * 256 * 512));
-    g.fsteps_cap = (long long)16 * 256 * 512;
-  }
-  A.fsteps = g.fsteps;
-  A.fsteps_cap = g.fsteps_cap;
   return S;
 }
 
@@ -631,7 +626,8 @@ void note_stats(long long paths, long long prims, const unsigned long long* ctr)
 
 int setup_max_bands(long long maxH) {
   const int maxBands = (int)(std::max<long long>(1, maxH / 4) + 1);
-  if (setup_smem(maxBands) > g.setupSmemMax) throw ApiError{"Image too tall for the fill kernels"};
+  // 8 bytes of shared memory per band beside 9296 fixed ones
+  if (maxBands > 1024 && (size_t)maxBands * 8 + 9296 > g.smemOptin) throw ApiError{"Image too tall for the fill kernels"};
   return maxBands;
 }
 
@@ -703,11 +699,11 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
   long long list_need = seg_need * 4;
   for (int attempt = 0; attempt < 12 && !todo.empty(); attempt++) {
     std::vector<PathJob> run;
-    long long rows = 0, maxH = 1;
+    long long rows = 0, maxH = 1, maxWork = 0;
     long long items = 0;
     for (int i : todo) {
       PathJob j = jobs[i];
-      if (j.group == 0) j.group = curve_group(prims, j.prim_off, j.nprims);
+      if (j.curves < 0) j.curves = count_curves(prims, j.prim_off, j.nprims);
       j.pc_off = j.prim_off;
       if (!opts.dprims) j.prims = nullptr;  // the staged copy
       else j.prims = opts.dprims;
@@ -716,10 +712,12 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
       rows += j.H;
       maxH = std::max<long long>(maxH, j.H);
       j.status = kOk;
+      maxWork = std::max(maxWork, setup_work(j));
       run.push_back(j);
     }
     const int nr = (int)run.size();
     const int maxBands = setup_max_bands(maxH);
+    const int setupC = setup_cluster(nr, maxWork, maxBands);
     ensure_arena(seg_need, list_need, (long long)nr * maxBands, nprims, rows);
     const bool graphed = opts.graph && attempt == 0 && g.stream != nullptr;
     std::vector<long long> offs((size_t)nr);
@@ -736,9 +734,8 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
     auto issue = [&](bool count) {
       if (attempt == 0 && opts.zero) CU(cudaMemsetAsync(opts.zero, 0, (size_t)opts.zero_bytes, g.stream));
       CU(cudaMemcpyAsync(g.d_up, g.h_up, S.upBytes, cudaMemcpyHostToDevice, g.stream));
-      k_setup<<<nr, 256, setup_smem(maxBands), g.stream>>>(dj, A, maxBands);
+      CU(launch_setup(nr, setupC, maxBands, g.stream, dj, A));
       if (count) note_launch();
-      CU(cudaGetLastError());
       if (timeRows) CU(cudaEventRecord(g.evr0, g.stream));
       launch_rows(v, (unsigned)blocks, g.stream, dj, reinterpret_cast<const long long*>(S.extra), nr, A, g.tbl, items,
                   cfg.rpi);
@@ -753,7 +750,7 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
                                     (long long)(uintptr_t)g.bandseg, g.bandseg_cap,
                                     (long long)(uintptr_t)g.bands, g.band_cap, (long long)(uintptr_t)g.primcnt,
                                     g.primcnt_cap, (long long)(uintptr_t)g.ovf, g.ovf_cap,
-                                    (long long)(uintptr_t)g.xcl, g.xcl_cap, v, cfg.rpi, blocks, maxBands,
+                                    (long long)(uintptr_t)g.xcl, g.xcl_cap, v, cfg.rpi, blocks, maxBands, setupC,
                                     (long long)(uintptr_t)opts.zero, opts.zero_bytes,
                                     (long long)(uintptr_t)g.stream, (long long)(uintptr_t)opts.dprims};
       GraphCache& gc = *opts.graph;
@@ -835,13 +832,6 @@ struct HostRun {
   int status;                  // first failure (kOk when every path was painted)
   const Prim* dstroke = nullptr;   // GPU-outlined strokes' primitives (jobs with stroke_gpu)
 };
-
-// Lanes per curve of a path with `curves` curve primitives (curve_group).
-int group_for(long long curves) {
-  int gsz = 1;
-  while (gsz < 32 && curves * gsz * 2 <= 256) gsz *= 2;
-  return gsz;
-}
 
 // Builds the outline primitives of sg into dout (stroke.cu): uploads the
 // polylines, runs the outline kernel, then rebuilds on the host, with the C
@@ -952,7 +942,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     long long pc = 0;
     std::vector<SceneRun> sr;
     std::vector<size_t> which;  // launch run -> runs index
-    long long items = 0, recItems = 0, riTotal = 0, maxH = 1;
+    long long items = 0, recItems = 0, riTotal = 0, maxH = 1, maxWork = 0;
     int ppl = 4;
     const int slice = scene_slice_for(runs, ppl);
     long long pathRows = 0;
@@ -973,7 +963,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
       const long long nrun = (long long)(r.j1 - r.j0);
       for (size_t j = r.j0; j < r.j1; j++) {
         PathJob pj = (*r.jobs)[j];
-        if (pj.group == 0) pj.group = curve_group(*r.prims, pj.prim_off, pj.nprims);
+        if (pj.curves < 0) pj.curves = count_curves(*r.prims, pj.prim_off, pj.nprims);
         pj.prims = pj.stroke_gpu ? r.dstroke : r.dprims;
         pj.pc_off = pc;
         pc += pj.nprims;
@@ -985,6 +975,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
         pj.ri_off = s.ri_base + (long long)(j - r.j0);
         pj.ri_stride = nrun;
         pj.status = kOk;
+        maxWork = std::max(maxWork, setup_work(pj));
         dev.push_back(pj);
       }
       s.j1 = (int)dev.size();
@@ -1030,8 +1021,8 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     S.A.ovf_cap = g.ovf_cap / 3;  // three lists
     dev_grow(g.pinfo, g.pinfo_cap, (long long)nj);
     S.A.pinfo = g.pinfo;
-    k_setup<<<nj, 256, setup_smem(maxBands), g.stream>>>(S.dj, S.A, maxBands); note_launch();
-    CU(cudaGetLastError());
+    CU(launch_setup(nj, setup_cluster(nj, maxWork, maxBands), maxBands, g.stream, S.dj, S.A));
+    note_launch();
     CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
     launch_scene_rec((unsigned)recBlocks, g.stream, S.dj, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(),
                      recItems, rpi, S.A);
@@ -1087,6 +1078,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
 PathJob make_job(pxg_image* img, uint32_t rgbx, int blend, const float* mat, float ps, int winding) {
   PathJob j;
   memset(&j, 0, sizeof j);
+  j.curves = -1;
   j.winding = winding;
   j.ems = error_margin_sq(ps);
   j.identity = is_identity(mat) ? 1 : 0;
@@ -1762,7 +1754,7 @@ int pxg_image_stroke_path(pxg_image* im, const float* cmds, int64_t n, const flo
       std::vector<PathJob> jobs(1, make_job(im, rgbx, blend, mat, ps, 0));
       jobs[0].prim_off = 0;
       jobs[0].nprims = (int)sg.nprims;
-      jobs[0].group = group_for(sg.ncurves);
+      jobs[0].curves = (int)sg.ncurves;
       RunOpts opts;
       opts.dprims = g.sk_prims;
       opts.ndprims = sg.nprims;
@@ -1876,7 +1868,7 @@ int pxg_scene_fill_path(pxg_scene* sc, const float* cmds, int64_t n, const float
     PathJob j = make_job(nullptr, rgbx, blend, mat, ps, winding);
     j.prim_off = (long long)sc->prims.size();
     j.nprims = (int)prims.size();
-    j.group = curve_group(prims, 0, j.nprims);
+    j.curves = count_curves(prims, 0, j.nprims);
     sc->prims.insert(sc->prims.end(), prims.begin(), prims.end());
     sc->jobs.push_back(j);
     sc->dirty = true;
@@ -1903,7 +1895,7 @@ int pxg_scene_stroke_path(pxg_scene* sc, const float* cmds, int64_t n, const flo
       if (sg.nprims > INT32_MAX) throw ApiError{"Path too complex"};
       j.stroke_gpu = 1;
       j.nprims = (int)sg.nprims;
-      j.group = group_for(sg.ncurves);
+      j.curves = (int)sg.ncurves;
       j.prim_off = append_stroke(sc->sk, sg);
       sc->jobs.push_back(j);
       sc->dirty = true;
@@ -1913,7 +1905,7 @@ int pxg_scene_stroke_path(pxg_scene* sc, const float* cmds, int64_t n, const flo
     build_stroke_prims(cmds, n, ps, width, cap, join, miterLimit, dashes, nd, prims);
     j.prim_off = (long long)sc->prims.size();
     j.nprims = (int)prims.size();
-    j.group = curve_group(prims, 0, j.nprims);
+    j.curves = count_curves(prims, 0, j.nprims);
     sc->prims.insert(sc->prims.end(), prims.begin(), prims.end());
     sc->jobs.push_back(j);
     sc->dirty = true;
@@ -2009,12 +2001,12 @@ int pxg_scene_record_batch(pxg_scene* sc, int64_t n, const int32_t* kinds, const
       if (r.state != 1) continue;
       if (r.job.stroke_gpu) {
         r.job.nprims = (int)r.sg.nprims;
-        r.job.group = group_for(r.sg.ncurves);
+        r.job.curves = (int)r.sg.ncurves;
         r.job.prim_off = append_stroke(sc->sk, r.sg);
       } else {
         r.job.prim_off = (long long)sc->prims.size();
         r.job.nprims = (int)r.prims.size();
-        r.job.group = curve_group(r.prims, 0, r.job.nprims);
+        r.job.curves = count_curves(r.prims, 0, r.job.nprims);
         sc->prims.insert(sc->prims.end(), r.prims.begin(), r.prims.end());
       }
       sc->jobs.push_back(r.job);
@@ -2097,7 +2089,7 @@ int pxg_masks_add_path(pxg_masks* m, const float* cmds, int64_t n, int64_t width
     j.H = height;
     j.prim_off = (long long)m->prims.size();
     j.nprims = (int)prims.size();
-    j.group = curve_group(prims, 0, j.nprims);
+    j.curves = count_curves(prims, 0, j.nprims);
     m->prims.insert(m->prims.end(), prims.begin(), prims.end());
     m->jobs.push_back(j);
     m->dirty = true;
@@ -2173,7 +2165,7 @@ int pxg_masks_add_paths(pxg_masks* m, int64_t n, const float* cmds, const int64_
       Rec& r = rec[(size_t)i];
       r.job.prim_off = (long long)m->prims.size();
       r.job.nprims = (int)r.prims.size();
-      r.job.group = curve_group(r.prims, 0, r.job.nprims);
+      r.job.curves = count_curves(r.prims, 0, r.job.nprims);
       m->prims.insert(m->prims.end(), r.prims.begin(), r.prims.end());
       m->jobs.push_back(r.job);
       m->offs.push_back(m->bytes);

@@ -14,6 +14,7 @@
 //           coverage -> paint -> blend write of the row.
 // Float math is compiled with -fmad=false: every expression keeps the
 // reference's float32 operation order.
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 
@@ -24,7 +25,6 @@ namespace pxg {
 
 static __device__ constexpr float kEps = (float)(0.0001 * 3.141592653589793);  // paths.nim:44
 static constexpr long long kIterCap = 1LL << 24;
-static constexpr int kSegTile = 1024;  // segment band ranges staged per pass of the band-list build
 static constexpr int kBallotBands = 1024;  // band count up to which the ballot band-list build runs
 
 struct V2 {
@@ -55,227 +55,8 @@ __device__ __forceinline__ V2 quadAt(V2 a, V2 c, V2 to, float t) {
   return a * ((t2 - 2 * t) + 1) + c * (-2 * t2 + 2 * t) + to * t2;
 }
 
-// The adaptive loops of addCubic/addQuadratic (paths.nim:677-762) with the
-// halvings of one search evaluated side by side.  After a segment is
-// accepted the loop tries steps s0, s0/2, s0/4, ... until one passes the
-// error test (or drops to float32 epsilon, which raises).  Every quantity the
-// test at level k reads -- next = f(t + s0/2^k), halfway = f(t + s0/2^(k+1)),
-// the tangent at t + s0/2^(k+1) -- depends only on (t, s0, prev): halving a
-// normal float is exact, so the sequential loop's recomputed `next = halfway`
-// and `t + step/4` equal these values bit for bit.  A group of G lanes tests
-// levels base..base+G-1 at once; the first level that accepts (or is at or
-// below epsilon) is the one the sequential loop would have stopped at.  With
-// G = 1 this is the reference's loop unchanged.  Calls emit(prev, next) for
-// every segment addSegment keeps (zero-length ones dropped, :669-675);
-// returns a JobStatus.  All G lanes of the group run the loop in lockstep.
 __device__ __forceinline__ float pow2neg(int k) {  // 2^-k for 0 <= k < 126
   return __int_as_float((127 - k) << 23);
-}
-template <class Emit>
-__device__ int flatten_curve_group(const Prim& p, float ems, int G, int gl, int leader,
-                                   unsigned gmask, Emit&& emit) {
-  const bool cubic = p.kind == kPrimCubic;
-  const V2 at{p.x[0], p.y[0]}, c1{p.x[1], p.y[1]};
-  const V2 c2{p.x[2], p.y[2]}, to{cubic ? p.x[3] : p.x[2], cubic ? p.y[3] : p.y[2]};
-  float t = 0, s0 = 1;
-  bool halfStepping = false;
-  V2 prev = at;
-  long long rounds = 0;
-  while (true) {
-    int kdec = 0;
-    V2 nxt{0, 0};
-    for (int base = 0;; base += G) {
-      if (++rounds > kIterCap) return kErrIterLimit;
-      const int k = base + gl;
-      const float sk = k < 100 ? s0 * pow2neg(k) : 0.0f;
-      const bool invalid = sk <= FLT_EPSILON;
-      bool accept = false;
-      V2 nx{0, 0};
-      if (!invalid) {
-        const float sh = sk * 0.5f;
-        if (cubic) {
-          nx = cubicAt(at, c1, c2, to, t + sk);
-          const V2 halfway = cubicAt(at, c1, c2, to, t + sh);
-          const V2 midpoint = (prev + nx) / 2;
-          const V2 lineTangent = midpoint - prev;
-          const V2 curveTangent = cubicDeriv(at, c1, c2, to, t + sh);
-          const V2 scaled = (curveTangent / length(curveTangent)) * length(lineTangent);
-          const float error = lengthSq(midpoint - halfway);
-          const float errorTangent = lengthSq(lineTangent - scaled);
-          accept = !(error + errorTangent > ems);
-        } else {
-          nx = quadAt(at, c1, c2, t + sk);
-          const V2 halfway = quadAt(at, c1, c2, t + sh);
-          const V2 midpoint = (prev + nx) / 2;
-          accept = !(lengthSq(midpoint - halfway) > ems);
-        }
-      }
-      const unsigned dec = (__ballot_sync(gmask, invalid || accept) >> leader) & (G == 32 ? 0xffffffffu : ((1u << G) - 1));
-      if (dec) {
-        const int src = leader + __ffs(dec) - 1;
-        if (__shfl_sync(gmask, (int)invalid, src)) return cubic ? kErrCubic : kErrQuad;
-        nxt.x = __shfl_sync(gmask, nx.x, src);
-        nxt.y = __shfl_sync(gmask, nx.y, src);
-        kdec = base + __ffs(dec) - 1;
-        break;
-      }
-    }
-    const float step = s0 * pow2neg(kdec);
-    if (prev.x - nxt.x != 0.0f || prev.y - nxt.y != 0.0f) emit(prev, nxt);
-    t += step;
-    if (t == 1) break;
-    prev = nxt;
-    if (kdec > 0) halfStepping = true;
-    s0 = (!cubic && halfStepping) ? nmin(step, 1 - t) : nmin(step * 2, 1 - t);
-  }
-  return kOk;
-}
-
-// Every group of a warp flattens its curves (primitives gid, gid + NG, ...,
-// lines skipped) with the search of flatten_curve_group, but the groups step
-// together: one search window per iteration of a warp-wide loop, so the warp
-// never serialises its groups' divergent loops.  A group that finishes a
-// curve starts its next one in the same loop.  emit(p, prev, next) is called
-// by every lane of the group for each segment addSegment keeps.  Returns the
-// lane's group's error status for the first failing curve it met (kOk if
-// none) and that curve's index in errp.
-template <class Emit, class Done>
-__device__ int flatten_curves_converged(const Prim* P, int np, float ems, int G, int gid, int NG, int gl, int leader,
-                                        int& errp, Emit&& emit, Done&& done, uint8_t* rec = nullptr, int cap = 0,
-                                        int* nrec = nullptr) {
-  const unsigned gbits = G == 32 ? 0xffffffffu : ((1u << G) - 1);
-  auto next_curve = [&](int q) {
-    while (q < np && P[q].kind == kPrimLine) q += NG;
-    return q;
-  };
-  int p = next_curve(gid);
-  bool cubic = false;
-  V2 at{0, 0}, c1{0, 0}, c2{0, 0}, to{0, 0}, prev{0, 0};
-  float t = 0, s0 = 1;
-  bool halfStepping = false;
-  int base = 0;
-  long long rounds = 0;
-  auto start = [&]() {
-    if (p >= np) return;
-    const Prim& q = P[p];
-    cubic = q.kind == kPrimCubic;
-    at = V2{q.x[0], q.y[0]};
-    c1 = V2{q.x[1], q.y[1]};
-    c2 = V2{q.x[2], q.y[2]};
-    to = V2{cubic ? q.x[3] : q.x[2], cubic ? q.y[3] : q.y[2]};
-    t = 0;
-    s0 = 1;
-    prev = at;
-    halfStepping = false;
-    base = 0;
-    rounds = 0;
-  };
-  start();
-  int status = kOk;
-  while (true) {
-    const bool active = p < np;
-    if (!__any_sync(0xffffffffu, active)) break;
-    const int k = base + gl;
-    const float sk = k < 100 ? s0 * pow2neg(k) : 0.0f;
-    const bool invalid = sk <= FLT_EPSILON;
-    bool accept = false;
-    V2 nx{0, 0};
-    if (active && !invalid) {
-      const float sh = sk * 0.5f;
-      if (cubic) {
-        nx = cubicAt(at, c1, c2, to, t + sk);
-        const V2 halfway = cubicAt(at, c1, c2, to, t + sh);
-        const V2 midpoint = (prev + nx) / 2;
-        const V2 lineTangent = midpoint - prev;
-        const V2 curveTangent = cubicDeriv(at, c1, c2, to, t + sh);
-        const V2 scaled = (curveTangent / length(curveTangent)) * length(lineTangent);
-        const float error = lengthSq(midpoint - halfway);
-        const float errorTangent = lengthSq(lineTangent - scaled);
-        accept = !(error + errorTangent > ems);
-      } else {
-        nx = quadAt(at, c1, c2, t + sk);
-        const V2 halfway = quadAt(at, c1, c2, t + sh);
-        const V2 midpoint = (prev + nx) / 2;
-        accept = !(lengthSq(midpoint - halfway) > ems);
-      }
-    }
-    const unsigned b = __ballot_sync(0xffffffffu, active && (invalid || accept));
-    const unsigned mine = (b >> leader) & gbits;
-    const int src = leader + (mine ? __ffs(mine) - 1 : 0);
-    const int srcInvalid = __shfl_sync(0xffffffffu, (int)invalid, src);
-    const float nxx = __shfl_sync(0xffffffffu, nx.x, src);
-    const float nxy = __shfl_sync(0xffffffffu, nx.y, src);
-    if (!active) continue;
-    if (++rounds > kIterCap) {
-      status = kErrIterLimit;
-      errp = p;
-      p = np;
-      continue;
-    }
-    if (!mine) {
-      base += G;
-      continue;
-    }
-    if (srcInvalid) {
-      status = cubic ? kErrCubic : kErrQuad;
-      errp = p;
-      p = np;
-      continue;
-    }
-    const int kdec = base + __ffs(mine) - 1;
-    if (rec) {  // record the step's halving level for the replay
-      if (*nrec < cap && gl == 0) rec[*nrec] = (uint8_t)kdec;
-      ++*nrec;
-    }
-    const float step = s0 * pow2neg(kdec);
-    const V2 nxt{nxx, nxy};
-    if (prev.x - nxt.x != 0.0f || prev.y - nxt.y != 0.0f) emit(p, prev, nxt);
-    t += step;
-    if (t == 1) {
-      done(p);
-      p = next_curve(p + NG);
-      start();
-      continue;
-    }
-    prev = nxt;
-    if (kdec > 0) halfStepping = true;
-    s0 = (!cubic && halfStepping) ? nmin(step, 1 - t) : nmin(step * 2, 1 - t);
-    base = 0;
-  }
-  return status;
-}
-
-// The group's curves again from the halving levels the search recorded: the
-// accepted point of a step is cubicAt/quadAt at t + s0 * 2^-level, the same
-// expression the search evaluated, so the same segments come out without
-// the search.  emit and done as for flatten_curves_converged.
-template <class Emit, class Done>
-__device__ void replay_curves(const Prim* P, int np, int gid, int NG, const uint8_t* rec, int nrec, Emit&& emit,
-                              Done&& done) {
-  int n = 0;
-  for (int p = gid; p < np; p += NG) {
-    const Prim& q = P[p];
-    if (q.kind == kPrimLine) continue;
-    const bool cubic = q.kind == kPrimCubic;
-    const V2 at{q.x[0], q.y[0]}, c1{q.x[1], q.y[1]}, c2{q.x[2], q.y[2]};
-    const V2 to{cubic ? q.x[3] : q.x[2], cubic ? q.y[3] : q.y[2]};
-    float t = 0, s0 = 1;
-    bool halfStepping = false;
-    V2 prev = at;
-    while (true) {
-      if (n >= nrec) return;  // a complete record ends with the last curve's t == 1
-      const int kdec = rec[n++];
-      const float step = s0 * pow2neg(kdec);
-      const V2 nxt = cubic ? cubicAt(at, c1, c2, to, t + step) : quadAt(at, c1, c2, t + step);
-      if (prev.x - nxt.x != 0.0f || prev.y - nxt.y != 0.0f) emit(p, prev, nxt);
-      t += step;
-      if (t == 1) break;
-      prev = nxt;
-      if (kdec > 0) halfStepping = true;
-      s0 = (!cubic && halfStepping) ? nmin(step, 1 - t) : nmin(step * 2, 1 - t);
-    }
-    done(p);
-  }
 }
 
 // transform + shapesToSegments for one emitted pair (paths.nim:1059-1096).
@@ -285,11 +66,14 @@ __device__ __forceinline__ float quantize256(float v) {
   float sgn = v >= 0 ? 1.0f : -1.0f;
   return sgn * (floorf(fabsf(v) / n) * n);
 }
-__device__ __forceinline__ bool make_seg(const PathJob& J, V2 a, V2 b, float4& s, int& w) {
-  if (!J.identity) {
-    const float* m = J.mat;
-    a = V2{m[0] * a.x + m[3] * a.y + m[6], m[1] * a.x + m[4] * a.y + m[7]};
-    b = V2{m[0] * b.x + m[3] * b.y + m[6], m[1] * b.x + m[4] * b.y + m[7]};
+struct SegMat {  // the job's transform: (x, y) -> (mx . (x, y, 1), my . (x, y, 1))
+  float mx[3], my[3];
+  int identity;
+};
+__device__ __forceinline__ bool make_seg(const SegMat& M, V2 a, V2 b, float4& s, int& w) {
+  if (!M.identity) {
+    a = V2{M.mx[0] * a.x + M.mx[1] * a.y + M.mx[2], M.my[0] * a.x + M.my[1] * a.y + M.my[2]};
+    b = V2{M.mx[0] * b.x + M.mx[1] * b.y + M.mx[2], M.my[0] * b.x + M.my[1] * b.y + M.my[2]};
   }
   a.y = quantize256(a.y);
   b.y = quantize256(b.y);
@@ -357,436 +141,6 @@ __device__ __forceinline__ Entry make_entry(float4 s, int w, float top, float bo
   e.bx = b.x;
   e.by = b.y;
   return e;
-}
-
-__device__ __forceinline__ long long warp_sum_ll(long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-// Block-wide exclusive scan of one value per thread (blockDim.x <= 1024).
-__device__ long long block_excl_scan(long long v, long long* s_warp, long long& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  long long x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    long long y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  __syncthreads();
-  if (lane == 31) s_warp[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    long long t = lane < nw ? s_warp[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      long long y = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += y;
-    }
-    if (lane < nw) s_warp[lane] = t;
-  }
-  __syncthreads();
-  total = s_warp[nw - 1];
-  long long before = warp > 0 ? s_warp[warp - 1] : 0;
-  __syncthreads();
-  return before + x - v;
-}
-
-// ---------------------------------------------------------------------------
-// k_setup: flatten -> segments -> bounds -> partitions (one CTA per job)
-// ---------------------------------------------------------------------------
-// The job's outcome, and beside its colour and mode for the drawing pass.
-__device__ __forceinline__ void set_status(PathJob& J, const Arena& A, int st) {
-  J.status = st;
-  if (A.pinfo) A.pinfo[blockIdx.x] = make_uint2(J.rgbx, (uint32_t)J.mode | ((uint32_t)st << 8));
-}
-__global__ void __launch_bounds__(256) k_setup(PathJob* jobs, Arena A, int maxBands) {
-  pdl_trigger();  // the row kernel may be set up while this runs; it waits for the segments
-  pdl_wait();
-  extern __shared__ int dsm[];
-  int* bandc = dsm;             // per band: entry count
-  int* bandf = dsm + maxBands;  // per band: flags
-  __shared__ long long s_warp[32];
-  __shared__ long long s_err;
-  __shared__ int s_status;
-  __shared__ long long s_segbase, s_bandbase, s_nseg, s_listbase;
-  __shared__ uint2 s_tile[kSegTile];
-  __shared__ uint32_t s_lohi[66];
-  __shared__ float s_red[4][32];
-  __shared__ long long s_hdr[6];
-
-  PathJob& J = jobs[blockIdx.x];
-  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned lt32 = (1u << lane) - 1;
-  if (tid == 0) {
-    s_err = LLONG_MAX;
-    s_status = kOk;
-  }
-  __syncthreads();
-
-  const Prim* P = J.prims + J.prim_off;
-  const int np = J.nprims;
-  int* PC = A.primcnt + J.pc_off;
-  // curves: groups of G lanes (G divides 32), one curve per group at a time
-  const int G = J.group;
-  const int NG = T / G, gid = tid / G, gl = tid % G, leader = lane - gl;
-  const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1) << leader);
-
-  // Phase A: count the segments each primitive emits
-  for (int p = tid; p < np; p += T) {
-    if (P[p].kind != kPrimLine) continue;
-    float4 s;
-    int w;
-    V2 a{P[p].x[0], P[p].y[0]}, b{P[p].x[1], P[p].y[1]};
-    PC[p] = ((a.x - b.x != 0.0f || a.y - b.y != 0.0f) && make_seg(J, a, b, s, w)) ? 1 : 0;
-  }
-  // each group's record of halving levels, for the emitting pass to replay
-  constexpr int kStepCap = 512;
-  uint8_t* rec = nullptr;
-  if (A.fsteps && ((long long)blockIdx.x + 1) * 256 * kStepCap <= A.fsteps_cap)
-    rec = A.fsteps + ((long long)blockIdx.x * 256 + gid) * kStepCap;
-  int nrec = 0;
-  {
-    int cnt = 0, errp = 0;
-    const int st = flatten_curves_converged(
-        P, np, J.ems, G, gid, NG, gl, leader, errp,
-        [&](int, V2 a, V2 b) {
-          float4 s;
-          int w;
-          if (make_seg(J, a, b, s, w)) cnt++;
-        },
-        [&](int p) {
-          if (gl == 0) PC[p] = cnt;
-          cnt = 0;
-        },
-        rec, kStepCap, &nrec);
-    if (st != kOk && gl == 0)  // the reference raises at the first failing primitive
-      atomicMin(&s_err, ((long long)errp << 8) | st);
-  }
-  __syncthreads();
-  if (s_err != LLONG_MAX) {
-    if (tid == 0) set_status(J, A, (int)(s_err & 255));
-    return;
-  }
-  // exclusive prefix of the counts, in primitive order
-  long long total = 0;
-  for (int c0 = 0; c0 < np; c0 += T) {
-    const int p = c0 + tid;
-    long long v = p < np ? PC[p] : 0, tot;
-    long long ex = block_excl_scan(v, s_warp, tot);
-    if (p < np) PC[p] = (int)(total + ex);
-    total += tot;
-  }
-  if (tid == 0) {
-    unsigned long long base = atomicAdd(&A.counters[kCtrSegs], (unsigned long long)total);
-    s_segbase = (long long)base;
-    s_nseg = total;
-    if ((long long)base + total > A.seg_cap || total > INT_MAX) s_status = kErrArenaFull;
-  }
-  __syncthreads();
-  if (s_status != kOk) {
-    if (tid == 0) set_status(J, A, s_status);
-    return;
-  }
-
-  // Phase B: emit the segments in order and reduce the bounds (:1098-1117)
-  float xmin = INFINITY, xmax = -INFINITY, ymin = INFINITY, ymax = -INFINITY;
-  auto put = [&](long long o, float4 s, int w) {
-    A.segs[o] = s;
-    A.segw[o] = w;
-    xmin = nmin(xmin, nmin(s.x, s.z));
-    xmax = nmax(xmax, nmax(s.x, s.z));
-    ymin = nmin(ymin, s.y);
-    ymax = nmax(ymax, s.w);
-  };
-  for (int p = tid; p < np; p += T) {
-    if (P[p].kind != kPrimLine) continue;
-    float4 s;
-    int w;
-    V2 a{P[p].x[0], P[p].y[0]}, b{P[p].x[1], P[p].y[1]};
-    if ((a.x - b.x != 0.0f || a.y - b.y != 0.0f) && make_seg(J, a, b, s, w)) put(s_segbase + PC[p], s, w);
-  }
-  {
-    int cnt = 0, errp = 0;
-    auto emitB = [&](int p, V2 a, V2 b) {
-      float4 s;
-      int w;
-      if (make_seg(J, a, b, s, w)) {
-        if (gl == 0) put(s_segbase + PC[p] + cnt, s, w);
-        cnt++;
-      }
-    };
-    auto doneB = [&](int) { cnt = 0; };
-    // replay where every group of the warp kept its whole record, else search again
-    if (__all_sync(0xffffffffu, rec != nullptr && nrec <= kStepCap))
-      replay_curves(P, np, gid, NG, rec, nrec, emitB, doneB);
-    else
-      flatten_curves_converged(P, np, J.ems, G, gid, NG, gl, leader, errp, emitB, doneB);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    xmin = nmin(xmin, __shfl_xor_sync(0xffffffffu, xmin, o));
-    xmax = nmax(xmax, __shfl_xor_sync(0xffffffffu, xmax, o));
-    ymin = nmin(ymin, __shfl_xor_sync(0xffffffffu, ymin, o));
-    ymax = nmax(ymax, __shfl_xor_sync(0xffffffffu, ymax, o));
-  }
-  if (lane == 0) {
-    s_red[0][warp] = xmin;
-    s_red[1][warp] = xmax;
-    s_red[2][warp] = ymin;
-    s_red[3][warp] = ymax;
-  }
-  __syncthreads();
-
-  // Phase C: bounds -> pixel window, partition geometry (:1602-1619, :1172-1192)
-  const long long W = J.W, H = J.H;
-  if (tid == 0) {
-    const int nw = (T + 31) >> 5;
-    float x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
-    for (int i = 0; i < nw; i++) {
-      x0 = nmin(x0, s_red[0][i]);
-      x1 = nmax(x1, s_red[1][i]);
-      y0 = nmin(y0, s_red[2][i]);
-      y1 = nmax(y1, s_red[3][i]);
-    }
-    float bx = 0, by = 0, bw = 0, bh = 0;
-    if (!(isnan(x0) || isnan(x1) || isnan(y0) || isnan(y1))) {
-      bx = x0;
-      by = y0;
-      bw = x1 - x0;
-      bh = y1 - y0;
-    }
-    float sx = floorf(bx), sw = ceilf(bx + bw) - sx;  // snapToPixels common.nim:92-101
-    float sy = floorf(by), sh = ceilf(by + bh) - sy;
-    long long startX = max(0LL, nim_int(sx)), startY = max(0LL, nim_int(sy));
-    long long pathWidth = startX < W ? min(nim_int(sw), W - startX) : 0LL;
-    long long pathHeight = min(H, nim_int(sy + sh));
-    int status = kOk;
-    if (pathWidth == 0) status = kNothing;
-    else if (pathWidth < 0) status = kErrIntOverflow;
-    long long height = pathHeight - startY;
-    long long nseg = s_nseg;
-    uint32_t maxP = (uint32_t)max(1LL, height / 4);
-    uint32_t numP = min(maxP, (uint32_t)max(1LL, nseg / 2));
-    uint32_t ph = (uint32_t)height / numP;
-    if (status == kOk && numP > (uint32_t)maxBands) status = kErrArenaFull;
-    s_status = status;
-    s_hdr[0] = startX;
-    s_hdr[1] = startY;
-    s_hdr[2] = pathWidth;
-    s_hdr[3] = pathHeight;
-    s_hdr[4] = numP;
-    s_hdr[5] = ph;
-    J.seg_off = s_segbase;
-    J.nseg = (int)nseg;
-    J.startX = startX;
-    J.startY = startY;
-    J.pathWidth = pathWidth;
-    J.pathHeight = pathHeight;
-    J.nb = (int)numP;
-    J.ph = ph;
-  }
-  __syncthreads();
-  if (s_status != kOk) {
-    if (tid == 0) set_status(J, A, s_status);
-    return;
-  }
-  const long long startY = s_hdr[1], pathHeight = s_hdr[3];
-  const uint32_t numP = (uint32_t)s_hdr[4], ph = (uint32_t)s_hdr[5];
-  const long long height = pathHeight - startY;
-  const long long nseg = s_nseg, segbase = s_segbase;
-  const float fStartY = (float)(uint32_t)startY;
-
-  auto bandRange = [&](float4 s, uint32_t& a, uint32_t& b) {  // partitionRange :1201-1213
-    if (numP == 1) {
-      a = b = 0;
-      return;
-    }
-    a = nim_u32(nmax(0.0f, s.y - fStartY)) / ph;
-    b = nim_u32(nmax(0.0f, s.w - fStartY)) / ph;
-    a = min(a, numP - 1);
-    b = min(b, numP - 1);
-  };
-  (void)height;
-
-  // Phase D: each segment's band range (partitionRange :1201-1213), each
-  // band's entry count and anti-aliasing flag (:1215-1234).  With at most
-  // kBallotBands bands each warp owns a contiguous run of segments and counts
-  // its entries per band (the list build below places them); otherwise
-  // shared-memory atomics per band.
-  const bool ballot = numP <= (uint32_t)kBallotBands && maxBands <= kBallotBands;
-  const int NW = T >> 5;
-  int* wc = dsm + 2 * maxBands;  // [warp][band]: entries, then each warp's start
-  const long long per = ((nseg + NW - 1) / NW + 31) / 32 * 32;
-  const long long ws0 = min(nseg, (long long)warp * per), ws1 = min(nseg, ws0 + per);
-  int* mine = wc + warp * (int)numP;
-  for (uint32_t k = tid; k < numP; k += T) {
-    bandc[k] = 0;
-    bandf[k] = 0;
-  }
-  if (ballot)
-    for (int k = tid; k < 2 * NW * (int)numP; k += T) wc[k] = 0;  // counts and band masks
-  __syncthreads();
-  if (ballot) {
-    for (long long i = ws0 + lane; i < ws1; i += 32) {
-      const float4 sg = A.segs[segbase + i];
-      uint32_t a, b;
-      bandRange(sg, a, b);
-      A.segband[segbase + i] = make_uint2(a, b);
-      const bool aa = segRequiresAA(sg);
-      for (uint32_t k = a; k <= b; k++) {
-        atomicAdd(&mine[k], 1);
-        if (aa) atomicOr(&bandf[k], kBandAA);
-      }
-    }
-    __syncthreads();
-    for (uint32_t k = tid; k < numP; k += T) {
-      int c = 0;
-      for (int w = 0; w < NW; w++) c += wc[w * numP + k];
-      bandc[k] = c;
-    }
-  } else {
-    for (long long i = tid; i < nseg; i += T) {
-      float4 sg = A.segs[segbase + i];
-      uint32_t a, b;
-      bandRange(sg, a, b);
-      A.segband[segbase + i] = make_uint2(a, b);
-      bool aa = segRequiresAA(sg);
-      for (uint32_t k = a; k <= b; k++) {
-        atomicAdd(&bandc[k], 1);
-        if (aa) atomicOr(&bandf[k], kBandAA);
-      }
-    }
-  }
-  __syncthreads();
-  if (tid == 0) {
-    unsigned long long base = atomicAdd(&A.counters[kCtrBands], (unsigned long long)numP);
-    s_bandbase = (long long)base;
-    if ((long long)base + numP > A.band_cap) s_status = kErrArenaFull;
-  }
-  __syncthreads();
-  if (s_status != kOk) {
-    if (tid == 0) set_status(J, A, s_status);
-    return;
-  }
-  // Phase E: each band's entry list, segment indices ascending -- the order in
-  // which partitionSegments appends them (:1215-1234).  Offsets by a scan of
-  // the counts; then either each warp writes its run's entries (ballot build)
-  // or every thread owns bands and walks the segments in order.
-  long long etotal = 0;
-  for (uint32_t c0 = 0; c0 < numP; c0 += T) {
-    const uint32_t k = c0 + tid;
-    long long v = k < numP ? bandc[k] : 0, tot;
-    long long ex = block_excl_scan(v, s_warp, tot);
-    if (k < numP) {
-      Band bd;
-      bd.off = etotal + ex;  // relative until the base is known
-      bd.count = bandc[k];
-      bd.flags = bandf[k];
-      A.bands[s_bandbase + k] = bd;
-      bandc[k] = (int)(etotal + ex);  // cursor
-    }
-    etotal += tot;
-  }
-  if (tid == 0) {
-    unsigned long long base = atomicAdd(&A.counters[kCtrBandSegs], (unsigned long long)etotal);
-    s_listbase = (long long)base;
-    if ((long long)base + etotal > A.bandseg_cap || etotal > INT_MAX) s_status = kErrArenaFull;
-  }
-  __syncthreads();
-  if (s_status != kOk) {
-    if (tid == 0) set_status(J, A, s_status);
-    return;
-  }
-  int* L = A.bandseg + s_listbase;
-  for (uint32_t k = tid; k < numP; k += T) A.bands[s_bandbase + k].off += s_listbase;
-  if (ballot) {
-    // each warp's start in every band: the band's offset plus the earlier
-    // warps' entries; then the warp writes its run's entries: O(entries) work
-    for (uint32_t k = tid; k < numP; k += T) {
-      int run = bandc[k];
-      for (int w = 0; w < NW; w++) {
-        const int t = wc[w * numP + k];
-        wc[w * numP + k] = run;
-        run += t;
-      }
-    }
-    __syncthreads();
-    // per batch of 32 segments: every lane marks the bands its segment
-    // touches in the warp's band masks; a segment's place in band k is the
-    // warp's cursor plus the number of lower lanes in k's mask (the reference's
-    // append order); each band's lowest lane then advances the cursor and
-    // clears the mask
-    uint32_t* bm = reinterpret_cast<uint32_t*>(wc + NW * (int)numP) + warp * (int)numP;
-    for (long long c0 = ws0; c0 < ws1; c0 += 32) {
-      const long long i = c0 + lane;
-      const bool valid = i < ws1;
-      uint2 r = make_uint2(1u, 0u);  // empty range
-      if (valid) r = A.segband[segbase + i];
-      const uint32_t bit = 1u << lane;
-      for (uint32_t k = r.x; k <= r.y; k++) atomicOr(&bm[k], bit);
-      __syncwarp();
-      for (uint32_t k = r.x; k <= r.y; k++) L[mine[k] + __popc(bm[k] & lt32)] = (int)i;
-      __syncwarp();
-      for (uint32_t k = r.x; k <= r.y; k++) {
-        const uint32_t m = bm[k];
-        if (!(m & lt32)) mine[k] += __popc(m);
-      }
-      __syncwarp();
-      for (uint32_t k = r.x; k <= r.y; k++)
-        if (!(bm[k] & lt32)) bm[k] = 0u;
-      __syncwarp();
-    }
-    if (tid == 0) {
-      J.band_off = s_bandbase;
-      set_status(J, A, kOk);
-    }
-    return;
-  }
-  for (long long t0 = 0; t0 < nseg; t0 += kSegTile) {
-    const int tl = (int)min((long long)kSegTile, nseg - t0);
-    uint32_t lo = UINT_MAX, hi = 0;
-    for (int j = tid; j < tl; j += T) {
-      uint2 r = A.segband[segbase + t0 + j];
-      s_tile[j] = r;
-      lo = min(lo, r.x);
-      hi = max(hi, r.y);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if (lane == 0) {
-      s_lohi[warp] = lo;
-      s_lohi[32 + warp] = hi;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      for (int i = 1; i < (T + 31) / 32; i++) {
-        lo = min(lo, s_lohi[i]);
-        hi = max(hi, s_lohi[32 + i]);
-      }
-      s_lohi[64] = lo;
-      s_lohi[65] = hi;
-    }
-    __syncthreads();
-    const uint32_t tlo = s_lohi[64], thi = s_lohi[65];
-    for (uint32_t k = tid; k < numP; k += T) {
-      if (k < tlo || k > thi) continue;
-      int cur = bandc[k];
-      for (int j = 0; j < tl; j++) {
-        const uint2 r = s_tile[j];
-        if (r.x <= k && k <= r.y) L[cur++] = (int)(t0 + j);
-      }
-      bandc[k] = cur;
-    }
-    __syncthreads();
-  }
-  if (tid == 0) {
-    J.band_off = s_bandbase;
-    set_status(J, A, kOk);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1548,6 +902,7 @@ __device__ bool process_row(const PathJob& J, const Arena& A, const uint8_t* tbl
 
 }  // namespace pxg
 #include "rowfast.cuh"
+#include "setup.cuh"
 namespace pxg {
 
 constexpr int kFastMaxH = 256, kFastXT = 1024, kFastWarps = 4;
@@ -1997,10 +1352,45 @@ void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, cons
 }
 
 // Dynamic shared memory of k_setup for a launch whose images have at most
-// maxBands bands: per band a count and flags, plus per warp and band a cursor
-// for the ballot band-list build.
-size_t setup_smem(int maxBands) {  // counts and flags, then per warp: band counts/cursors and band masks
-  return (size_t)maxBands * 8 + (maxBands <= kBallotBands ? (size_t)2 * (256 / 32) * maxBands * 4 : 0);
+// maxBands bands: per band a count and an anti-aliasing flag; with the ballot
+// build also a place, per warp a count and a lane mask, and the step records.
+size_t setup_smem(int maxBands) {
+  if (maxBands > kBallotBands) return (size_t)(2 * maxBands + 2) * 4;
+  return (size_t)(3 * maxBands + 3 + 2 * kSetupWarps * (maxBands + 1)) * 4 + kStepBytes;
+}
+// CTAs per job: the longest job's time shrinks with them, while each CTA of a
+// launch beyond the first four per SM costs a wave's fixed part.  In
+// microseconds, as measured: 0.014 per unit of work, 15 per wave (0.025 per CTA
+// on 152 SMs), 4 for the cluster's barriers.  One heart: 10 us with 1 CTA, 15
+// with 8; 64 cubics: 90 and 38; a 14,540-primitive stroke: 600 and 83; 4096
+// glyphs: 100 with 1, 243 with 2; 240 local paths: 970 and 175; 2000 paths over
+// 1024 x 1024: 6400 and 2250.
+int setup_cluster(long long njobs, long long maxWork, int maxBands) {
+  if (maxBands > kBallotBands) return 1;
+  int best = 1;
+  double cost = 0;
+  for (int c = 1; c <= 8; c *= 2) {
+    const double t = 0.014 * (double)maxWork / c + 0.025 * (double)njobs * c + (c > 1 ? 4.0 : 0.0);
+    if (c == 1 || t < cost) {
+      best = c;
+      cost = t;
+    }
+  }
+  return best;
+}
+cudaError_t launch_setup(int njobs, int C, int maxBands, cudaStream_t st, PathJob* jobs, const Arena& A) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(njobs * C));
+  cfg.blockDim = dim3(kSetupThreads);
+  cfg.dynamicSmemBytes = setup_smem(maxBands);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)C;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k_setup, jobs, A, maxBands, C);
 }
 
 size_t scene_wide_bytes() { return sizeof(RowScratch<kWideMaxH, kWideXT>); }

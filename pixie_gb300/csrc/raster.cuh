@@ -55,7 +55,7 @@ struct PathJob {
   int identity, mode;
   uint32_t rgbx;  // premultiplied paint colour
   float mat[9];
-  int group;     // lanes that flatten one curve together (1, 2, 4, 8, 16 or 32)
+  int curves;    // quadratics and cubics among the primitives (-1: not counted yet)
   int a8;        // img is an 8-bit alpha mask (white NormalBlend fills only), else RGBX
   uint8_t* img;  // RGBX or A8, row-major, W*H pixels
   long long W, H;
@@ -135,8 +135,6 @@ struct Arena {
   long long ovf_cap;
   long long* xclears;   // (job, start, end) linear-pixel clears that reach into earlier rows
   long long xclear_cap;
-  uint8_t* fsteps;      // fill setup: the halving level of every accepted flattening step, per group
-  long long fsteps_cap; // (the second pass replays them); bytes
 };
 
 }  // namespace pxg
