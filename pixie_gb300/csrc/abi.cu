@@ -140,8 +140,10 @@ void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, cons
 size_t scene_wide_bytes();
 size_t setup_smem(int maxBands);
 int draw_masks_tiles();
-void launch_draw_masks(int tile, uint32_t* page, long long W, long long H, const void* items, int n,
-                       const uint8_t* masks, int mode, const uint8_t* tbl, cudaStream_t st);
+void launch_draw_masks(int tile, uint32_t* page, long long W, long long H, const int4* rects, const MaskDraw* items,
+                       int n, int* bins, const uint8_t* masks, int mode, const uint8_t* tbl, cudaStream_t st);
+long long mask_bins_ints(long long H, int n);
+void preload_draw_masks();
 size_t rows_smem_wide();
 struct SmoothArgs {
   float px, py, dxx, dxy, dyx, dyy;
@@ -263,8 +265,10 @@ struct Ctx {
   long long bandseg_cap = 0;
   int* primcnt = nullptr;
   long long primcnt_cap = 0;
-  MaskDraw* mdraw = nullptr;      // mask positions of pxg_image_draw_masks
+  int4* mdraw = nullptr;          // rectangles and items of pxg_image_draw_masks
   long long mdraw_cap = 0;
+  int* mbins = nullptr;           // masks per row of tiles (counts, lists)
+  long long mbins_cap = 0;
   int4* prog = nullptr;           // scene row programs
   long long prog_cap = 0;
   int4* rowhdr = nullptr;         // scene rows: what each draws
@@ -397,6 +401,7 @@ void init_locked(int device) {
   g.blurSmemMax = std::min(g.blurSmemMax, allow_max_smem((const void*)k_blurf_y));
   g.blurSmemMax = std::min(g.blurSmemMax, allow_max_smem(blurb_kernel(true)));
   g.blurSmemMax = std::min(g.blurSmemMax, allow_max_smem(blurb_kernel(false)));
+  preload_draw_masks();
   CU(cudaEventCreate(&g.ev0));
   CU(cudaEventCreate(&g.ev1));
   CU(cudaEventCreate(&g.evr0));
@@ -1516,25 +1521,37 @@ void render_masks(pxg_masks* m) {
 void draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blend) {
   const int n = (int)m->jobs.size();
   if (n == 0) return;
-  std::vector<MaskDraw> items((size_t)n);
+  // one buffer: the rectangles, then the items (16 bytes each)
+  static_assert(sizeof(MaskDraw) == sizeof(int4), "one buffer holds both");
+  std::vector<int4> buf((size_t)n * 2);
+  MaskDraw* items = reinterpret_cast<MaskDraw*>(buf.data() + n);
   for (int i = 0; i < n; i++) {
-    items[(size_t)i].off = m->offs[(size_t)i];
-    items[(size_t)i].x = xy[2 * i];
-    items[(size_t)i].y = xy[2 * i + 1];
-    items[(size_t)i].w = (int)m->jobs[(size_t)i].W;
-    items[(size_t)i].h = (int)m->jobs[(size_t)i].H;
+    const PathJob& j = m->jobs[(size_t)i];
+    const int64_t x = xy[2 * i], y = xy[2 * i + 1];
+    const bool meets = x < page->width && y < page->height && x > -j.W && y > -j.H;
+    buf[(size_t)i] = meets ? make_int4((int)std::max<int64_t>(x, 0), (int)std::max<int64_t>(y, 0),
+                                       (int)std::min<int64_t>(x + j.W, page->width),
+                                       (int)std::min<int64_t>(y + j.H, page->height))
+                           : make_int4(0, 0, 0, 0);
+    items[i] = MaskDraw{meets ? m->offs[(size_t)i] - y * j.W - x : 0, (int)j.W, 0};
   }
   // a pageable copy: the host vector may go away as soon as the call returns
-  dev_grow(g.mdraw, g.mdraw_cap, (long long)n);
-  CU(cudaMemcpyAsync(g.mdraw, items.data(), sizeof(MaskDraw) * (size_t)n, cudaMemcpyHostToDevice, g.stream));
-  struct {
-    const void* extra;
-  } S{g.mdraw};
+  dev_grow(g.mdraw, g.mdraw_cap, (long long)n * 2);
+  CU(cudaMemcpyAsync(g.mdraw, buf.data(), sizeof(int4) * buf.size(), cudaMemcpyHostToDevice, g.stream));
+  const int4* rects = g.mdraw;
+  const MaskDraw* ditems = reinterpret_cast<const MaskDraw*>(g.mdraw + n);
+  // binning pays from some hundreds of masks on (its launch is 3 us, a tile's
+  // test of 256 masks about one), while its lists stay small
+  int* bins = nullptr;
+  if (n > 512 && mask_bins_ints(page->height, n) <= (64LL << 20)) {
+    dev_grow(g.mbins, g.mbins_cap, mask_bins_ints(page->height, n));
+    bins = g.mbins;
+  }
   const long long pxBytes = page->width * page->height * 4;
   const std::pair<int, long long> key{kTuneMaskDraw, size_bucket(std::max(page->width, page->height)) * 32 +
                                                         count_bucket(n)};
   auto it = g_tune.best.find(key);
-  int tile = 2;
+  int tile = 1;  // 64x32: the fastest of most classes
   if (g_tune.on && it == g_tune.best.end()) {
     // time every tile shape on a copy of the page, then draw with the fastest
     unsigned char* tmp = (unsigned char*)scratch(pxBytes);
@@ -1542,19 +1559,19 @@ void draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blen
     for (int c = 0; c < draw_masks_tiles(); c++) {
       CU(cudaMemcpyAsync(tmp, page->data, (size_t)pxBytes, cudaMemcpyDeviceToDevice, g.stream));
       CU(cudaEventRecord(g.evr0, g.stream));
-      launch_draw_masks(c, (uint32_t*)tmp, page->width, page->height, S.extra, n, m->dev, blend, g.tbl, g.stream);
+      launch_draw_masks(c, (uint32_t*)tmp, page->width, page->height, rects, ditems, n, bins, m->dev, blend, g.tbl, g.stream);
       CU(cudaGetLastError());
       CU(cudaEventRecord(g.evr1, g.stream));
       CU(cudaEventSynchronize(g.evr1));
       CU(cudaEventElapsedTime(&t[(size_t)c], g.evr0, g.evr1));
-      if (t[(size_t)c] < t[(size_t)tile]) tile = c;
     }
+    tile = (int)(std::min_element(t.begin(), t.end()) - t.begin());
     g_tune.best[key] = tile;
     g_tune.ms[key] = t;
   } else if (it != g_tune.best.end()) {
     tile = it->second;
   }
-  launch_draw_masks(tile, (uint32_t*)page->data, page->width, page->height, S.extra, n, m->dev, blend, g.tbl,
+  launch_draw_masks(tile, (uint32_t*)page->data, page->width, page->height, rects, ditems, n, bins, m->dev, blend, g.tbl,
                     g.stream);
   CU(cudaGetLastError());
 }

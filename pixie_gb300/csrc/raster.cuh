@@ -100,11 +100,12 @@ struct SceneRun {
   int j0, j1;
 };
 
-// One mask of a batch drawn onto a page at an integer offset.
+// One mask of a batch drawn onto a page at an integer offset: page pixel (X,
+// Y) within its rectangle (clipped to the page; kept apart as int4 {x0, y0, x1,
+// y1}) takes byte base + Y * w + X of the batch's mask buffer.
 struct MaskDraw {
-  long long off;  // byte offset of the mask in the batch's mask buffer
-  long long x, y;
-  int w, h;
+  long long base;
+  int w, pad;
 };
 
 enum ArenaCounter {
