@@ -273,8 +273,6 @@ struct Ctx {
   long long prog_cap = 0;
   int4* rowhdr = nullptr;         // scene rows: what each draws
   long long rowhdr_cap = 0;
-  uint2* pinfo = nullptr;         // scene paths: colour, mode, status
-  long long pinfo_cap = 0;
   uint8_t* cov8 = nullptr;        // scene coverage bytes (rows that fit; the rest keep spans)
   long long cov8_cap = 0;
   unsigned char* wide = nullptr;  // per-warp wide row scratch of the scene recording kernel
@@ -478,20 +476,30 @@ void* scratch(long long bytes) {
   return g.scratch;
 }
 
+// Times a call's GPU work.  A runner that waits for the GPU itself calls mark()
+// before it does, and done() then neither records nor waits again.
 struct Timed {
   bool force;
+  static bool marked;
   explicit Timed(bool f = false) : force(f) {
+    marked = false;
     if (g.blocking || force) cudaEventRecord(g.ev0, g.stream);
+  }
+  static void mark() {
+    cudaEventRecord(g.ev1, g.stream);
+    marked = true;
   }
   void done() {
     if (!(g.blocking || force)) return;
-    cudaEventRecord(g.ev1, g.stream);
+    if (!marked) cudaEventRecord(g.ev1, g.stream);
+    marked = false;
     CU(cudaEventSynchronize(g.ev1));
     float ms = 0;
     cudaEventElapsedTime(&ms, g.ev0, g.ev1);
     g.last_ms = ms;
   }
 };
+bool Timed::marked = false;
 
 // Reads (and clears) the device error flag; throws if a kernel reported a
 // wait that ran out.
@@ -549,23 +557,29 @@ void ensure_arena(long long seg_need, long long list_need, long long nbands, lon
   dev_grow(g.xcl, g.xcl_cap, 3 * (2 * rows + 1024));
 }
 
-// One host->device copy of jobs | counters | extra | prims through the pinned
-// upload area.
+// One host->device copy of jobs | counters | outcomes | extra | prims through
+// the pinned upload area; counters and outcomes (8 bytes a job, written by the
+// setup kernel) come back in one copy.  fill(jobs) writes the nr jobs in place.
 struct Staged {
   PathJob* dj;
   unsigned char* extra;
-  size_t jobsBytes, ctrBytes, extraBytes, upBytes;
+  size_t jobsBytes, ctrBytes, infoBytes, extraBytes, upBytes;
   Arena A;
+  void read_back() const {
+    CU(cudaMemcpyAsync(g.h_up + jobsBytes, g.d_up + jobsBytes, ctrBytes + infoBytes, cudaMemcpyDeviceToHost, g.stream));
+  }
+  const uint2* outcomes() const { return reinterpret_cast<const uint2*>(g.h_up + jobsBytes + ctrBytes); }
 };
-Staged stage(const std::vector<PathJob>& run, const void* extra, size_t extraBytes,
-             const std::vector<Prim>& prims, bool copy = true) {
+int outcome_status(uint2 o) { return (int)(o.y >> 8); }
+template <class Fill>
+Staged stage(size_t nr, const void* extra, size_t extraBytes, const std::vector<Prim>* prims, bool copy, Fill&& fill) {
   Staged S;
-  const size_t nr = run.size();
   S.jobsBytes = align_up(sizeof(PathJob) * std::max<size_t>(nr, 1), 256);
   S.ctrBytes = 256;
+  S.infoBytes = align_up(sizeof(uint2) * std::max<size_t>(nr, 1), 256);
   S.extraBytes = align_up(extraBytes, 256);
-  const size_t primBytes = sizeof(Prim) * std::max<size_t>(prims.size(), 1);
-  const size_t need = S.jobsBytes + S.ctrBytes + S.extraBytes + primBytes;
+  const size_t primAt = S.jobsBytes + S.ctrBytes + S.infoBytes + S.extraBytes;
+  const size_t need = primAt + sizeof(Prim) * std::max<size_t>(prims ? prims->size() : 0, 1);
   if (need > g.up_cap) {
     CU(cudaStreamSynchronize(g.stream));  // the old area may still be in flight
     if (g.d_up) cudaFree(g.d_up);
@@ -577,23 +591,19 @@ Staged stage(const std::vector<PathJob>& run, const void* extra, size_t extraByt
     CU(cudaMallocHost(&g.h_up, cap));
     g.up_cap = cap;
   }
-  if (nr) memcpy(g.h_up, run.data(), sizeof(PathJob) * nr);
-  {  // jobs without resident primitives read the staged ones
-    const size_t primAt0 = S.jobsBytes + S.ctrBytes + S.extraBytes;
-    PathJob* hj = reinterpret_cast<PathJob*>(g.h_up);
-    for (size_t i = 0; i < nr; i++)
-      if (!hj[i].prims) hj[i].prims = reinterpret_cast<const Prim*>(g.d_up + primAt0);
-  }
+  PathJob* hj = reinterpret_cast<PathJob*>(g.h_up);
+  fill(hj);
+  for (size_t i = 0; i < nr; i++)  // jobs without resident primitives read the staged ones
+    if (!hj[i].prims) hj[i].prims = reinterpret_cast<const Prim*>(g.d_up + primAt);
   unsigned long long* hc = reinterpret_cast<unsigned long long*>(g.h_up + S.jobsBytes);
   memset(hc, 0, S.ctrBytes);
   hc[kCtrRowErr] = ~0ull;
-  if (extraBytes) memcpy(g.h_up + S.jobsBytes + S.ctrBytes, extra, extraBytes);
-  const size_t primAt = S.jobsBytes + S.ctrBytes + S.extraBytes;
-  if (!prims.empty()) memcpy(g.h_up + primAt, prims.data(), sizeof(Prim) * prims.size());
+  if (extraBytes) memcpy(g.h_up + S.jobsBytes + S.ctrBytes + S.infoBytes, extra, extraBytes);
+  if (prims && !prims->empty()) memcpy(g.h_up + primAt, prims->data(), sizeof(Prim) * prims->size());
   S.upBytes = need;
   if (copy) CU(cudaMemcpyAsync(g.d_up, g.h_up, need, cudaMemcpyHostToDevice, g.stream));
   S.dj = reinterpret_cast<PathJob*>(g.d_up);
-  S.extra = g.d_up + S.jobsBytes + S.ctrBytes;
+  S.extra = g.d_up + S.jobsBytes + S.ctrBytes + S.infoBytes;
   Arena& A = S.A;
   A.prims = reinterpret_cast<const Prim*>(g.d_up + primAt);
   A.segs = g.segs;
@@ -609,7 +619,7 @@ Staged stage(const std::vector<PathJob>& run, const void* extra, size_t extraByt
   A.prog = g.prog;
   A.prog_cap = g.prog_cap;
   A.rowhdr = g.rowhdr;
-  A.pinfo = nullptr;
+  A.pinfo = reinterpret_cast<uint2*>(g.d_up + S.jobsBytes + S.ctrBytes);
   A.cov8 = g.cov8;
   A.cov8_cap = g.cov8_cap;
   A.counters = reinterpret_cast<unsigned long long*>(g.d_up + S.jobsBytes);
@@ -676,12 +686,14 @@ struct RunOpts {
   float* rows_ms = nullptr;       // row-kernel time of the first launch (autotuning)
   const Prim* dprims = nullptr;   // primitives already on the device (else staged)
   long long ndprims = -1;         // how many, when `prims` does not hold them (a GPU outline)
+  unsigned char* imgs = nullptr;  // the jobs' images: imgs + (*img_offs)[job] (mask batches), else job.img
+  const std::vector<long long>* img_offs = nullptr;
 };
 
 // Runs fill jobs whose primitives are already in `prims` (job.prim_off set).
 // Jobs must target distinct images: a job whose workspace ran out is rerun
 // alone, after the others were drawn.  Returns per-job status.
-void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::vector<int>& status,
+void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::vector<int>& status,
               const RunOpts& opts = RunOpts()) {
   RowsCfg cfg = opts.cfg;
   if (cfg.variant == 0 && !jobs.empty() && jobs[0].a8) cfg.variant = 3;
@@ -703,32 +715,35 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
   long long seg_need = std::max<long long>(1 << 16, nprims * 8);
   long long list_need = seg_need * 4;
   for (int attempt = 0; attempt < 12 && !todo.empty(); attempt++) {
-    std::vector<PathJob> run;
-    long long rows = 0, maxH = 1, maxWork = 0;
-    long long items = 0;
-    for (int i : todo) {
-      PathJob j = jobs[i];
-      if (j.curves < 0) j.curves = count_curves(prims, j.prim_off, j.nprims);
-      j.pc_off = j.prim_off;
-      if (!opts.dprims) j.prims = nullptr;  // the staged copy
-      else j.prims = opts.dprims;
-      j.row_off = items;
+    const int nr = (int)todo.size();
+    long long rows = 0, maxH = 1, maxWork = 0, items = 0;
+    std::vector<long long> offs((size_t)nr);  // the jobs' first work items
+    for (int r = 0; r < nr; r++) {
+      const PathJob& j = jobs[(size_t)todo[(size_t)r]];
+      offs[(size_t)r] = items;
       items += (j.H + cfg.rpi - 1) / cfg.rpi;
       rows += j.H;
       maxH = std::max<long long>(maxH, j.H);
-      j.status = kOk;
-      maxWork = std::max(maxWork, setup_work(j));
-      run.push_back(j);
     }
-    const int nr = (int)run.size();
     const int maxBands = setup_max_bands(maxH);
-    const int setupC = setup_cluster(nr, maxWork, maxBands);
     ensure_arena(seg_need, list_need, (long long)nr * maxBands, nprims, rows);
     const bool graphed = opts.graph && attempt == 0 && g.stream != nullptr;
-    std::vector<long long> offs((size_t)nr);
-    for (int r = 0; r < nr; r++) offs[(size_t)r] = run[(size_t)r].row_off;
-    Staged S = stage(run, offs.data(), sizeof(long long) * offs.size(), opts.dprims ? std::vector<Prim>() : prims,
-                     false);
+    Staged S = stage((size_t)nr, offs.data(), sizeof(long long) * offs.size(), opts.dprims ? nullptr : &prims, false,
+                     [&](PathJob* dst) {
+                       for (int r = 0; r < nr; r++) {
+                         const size_t i = (size_t)todo[(size_t)r];
+                         PathJob& j = dst[r];
+                         j = jobs[i];
+                         if (opts.imgs) j.img = opts.imgs + (*opts.img_offs)[i];
+                         if (j.curves < 0) j.curves = count_curves(prims, j.prim_off, j.nprims);
+                         j.pc_off = j.prim_off;
+                         j.prims = opts.dprims;  // null: the staged copy
+                         j.row_off = offs[(size_t)r];
+                         j.status = kOk;
+                         maxWork = std::max(maxWork, setup_work(j));
+                       }
+                     });
+    const int setupC = setup_cluster(nr, maxWork, maxBands);
     Arena& A = S.A;
     PathJob* dj = S.dj;
     const int v = cfg.variant;
@@ -747,7 +762,7 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
       if (count) note_launch();
       CU(cudaGetLastError());
       if (timeRows) CU(cudaEventRecord(g.evr1, g.stream));
-      CU(cudaMemcpyAsync(g.h_up, g.d_up, S.jobsBytes + S.ctrBytes, cudaMemcpyDeviceToHost, g.stream));
+      S.read_back();
     };
     if (graphed) {
       std::vector<long long> key = {nr, items, (long long)S.upBytes, (long long)(uintptr_t)g.d_up,
@@ -786,11 +801,13 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
     } else {
       issue(true);
     }
+    Timed::mark();
     CU(cudaStreamSynchronize(g.stream));
     if (timeRows) CU(cudaEventElapsedTime(opts.rows_ms, g.evr0, g.evr1));
     unsigned long long ctr[kNumCounters];
     memcpy(ctr, g.h_up + S.jobsBytes, sizeof ctr);
     note_stats(nr, nprims, ctr);
+    const PathJob* wide = nullptr;
     if (ctr[kCtrOvfRows] > 0 || ctr[kCtrXClears] > 0) {
       if ((long long)ctr[kCtrXClears] > A.xclear_cap) throw ApiError{"Out of workspace memory (cross-row clears)"};
       if (ctr[kCtrOvfRows] > 0) {
@@ -803,16 +820,18 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
         k_xclears<<<(unsigned)b, 256, 0, g.stream>>>(dj, A); note_launch();
         CU(cudaGetLastError());
       }
+      // (the wide kernel's failures are in the jobs alone)
       CU(cudaMemcpyAsync(g.h_up, g.d_up, S.jobsBytes, cudaMemcpyDeviceToHost, g.stream));
+      Timed::mark();
       CU(cudaStreamSynchronize(g.stream));
+      wide = reinterpret_cast<const PathJob*>(g.h_up);
     }
-    const PathJob* out = reinterpret_cast<const PathJob*>(g.h_up);
     std::vector<int> again;
     bool grow = false;
     for (int r = 0; r < nr; r++) {
-      int st = out[r].status;
+      int st = outcome_status(S.outcomes()[r]);
+      if (wide && st == kOk) st = wide[r].status;
       int i = todo[(size_t)r];
-      jobs[(size_t)i] = out[r];
       if (st == kErrArenaFull) {
         again.push_back(i);
         grow = true;
@@ -830,7 +849,7 @@ void run_jobs(std::vector<PathJob>& jobs, const std::vector<Prim>& prims, std::v
 // job's chunk of paths).
 struct HostRun {
   pxg_image* canvas;
-  std::vector<PathJob>* jobs;  // the run's paths, in order; img/W/H are set here
+  const std::vector<PathJob>* jobs;  // the run's paths, in order
   const std::vector<Prim>* prims;  // host primitives (jobs' prim_off index them)
   const Prim* dprims;              // the same primitives on the device
   size_t j0, j1;               // paths still to paint
@@ -943,8 +962,8 @@ void run_scene_runs(std::vector<HostRun>& runs) {
   long long prog_need = 0;
   for (auto& r : runs) r.status = kOk;
   for (int attempt = 0; attempt < 16; attempt++) {
-    std::vector<PathJob> dev;
     long long pc = 0;
+    int nj = 0;
     std::vector<SceneRun> sr;
     std::vector<size_t> which;  // launch run -> runs index
     long long items = 0, recItems = 0, riTotal = 0, maxH = 1, maxWork = 0;
@@ -962,28 +981,14 @@ void run_scene_runs(std::vector<HostRun>& runs) {
       s.W = r.canvas->width;
       s.H = r.canvas->height;
       s.img = r.canvas->data;
-      s.j0 = (int)dev.size();
+      s.j0 = nj;
       s.ri_base = riTotal;
       s.rec_off = recItems;
       const long long nrun = (long long)(r.j1 - r.j0);
-      for (size_t j = r.j0; j < r.j1; j++) {
-        PathJob pj = (*r.jobs)[j];
-        if (pj.curves < 0) pj.curves = count_curves(*r.prims, pj.prim_off, pj.nprims);
-        pj.prims = pj.stroke_gpu ? r.dstroke : r.dprims;
-        pj.pc_off = pc;
-        pc += pj.nprims;
-        pj.img = r.canvas->data;
-        pj.W = r.canvas->width;
-        pj.H = r.canvas->height;
-        pj.row_off = recItems;
-        recItems += (pj.H + rpi - 1) / rpi;
-        pj.ri_off = s.ri_base + (long long)(j - r.j0);
-        pj.ri_stride = nrun;
-        pj.status = kOk;
-        maxWork = std::max(maxWork, setup_work(pj));
-        dev.push_back(pj);
-      }
-      s.j1 = (int)dev.size();
+      for (size_t j = r.j0; j < r.j1; j++) pc += (*r.jobs)[j].nprims;
+      nj += (int)nrun;
+      s.j1 = nj;
+      recItems += nrun * ((s.H + rpi - 1) / rpi);
       riTotal += s.H * nrun;
       items += s.H * ((s.W + slice - 1) / slice);
       maxH = std::max<long long>(maxH, s.H);
@@ -991,7 +996,6 @@ void run_scene_runs(std::vector<HostRun>& runs) {
       which.push_back(ri);
     }
     if (sr.empty()) return;
-    const int nj = (int)dev.size();
     const int maxBands = setup_max_bands(maxH);
     ensure_arena(seg_need, list_need, (long long)nj * maxBands, pc, 1);
     dev_grow(g.ovf, g.ovf_cap, 3 * std::max<long long>(riTotal, 1));
@@ -1022,10 +1026,31 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     }
     const long long blocks = std::max<long long>(
         1, std::min<long long>((items + scene_warps() - 1) / scene_warps(), (long long)g.nsm * g.scene_ctas_per_sm[1]));
-    Staged S = stage(dev, sr.data(), sizeof(SceneRun) * sr.size(), std::vector<Prim>());
+    Staged S = stage((size_t)nj, sr.data(), sizeof(SceneRun) * sr.size(), nullptr, true, [&](PathJob* dst) {
+      long long at = 0, item = 0;
+      for (size_t k = 0; k < sr.size(); k++) {
+        const HostRun& r = runs[which[k]];
+        const SceneRun& s = sr[k];
+        for (size_t j = r.j0; j < r.j1; j++) {
+          PathJob& pj = *dst++;
+          pj = (*r.jobs)[j];
+          if (pj.curves < 0) pj.curves = count_curves(*r.prims, pj.prim_off, pj.nprims);
+          pj.prims = pj.stroke_gpu ? r.dstroke : r.dprims;
+          pj.pc_off = at;
+          at += pj.nprims;
+          pj.img = s.img;
+          pj.W = s.W;
+          pj.H = s.H;
+          pj.row_off = item;
+          item += (s.H + rpi - 1) / rpi;
+          pj.ri_off = s.ri_base + (long long)(j - r.j0);
+          pj.ri_stride = s.j1 - s.j0;
+          pj.status = kOk;
+          maxWork = std::max(maxWork, setup_work(pj));
+        }
+      }
+    });
     S.A.ovf_cap = g.ovf_cap / 3;  // three lists
-    dev_grow(g.pinfo, g.pinfo_cap, (long long)nj);
-    S.A.pinfo = g.pinfo;
     CU(launch_setup(nj, setup_cluster(nj, maxWork, maxBands), maxBands, g.stream, S.dj, S.A));
     note_launch();
     CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
@@ -1047,7 +1072,8 @@ void run_scene_runs(std::vector<HostRun>& runs) {
                  S.A, g.tbl, slice);
     note_launch();
     CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(g.h_up, g.d_up, S.jobsBytes + S.ctrBytes, cudaMemcpyDeviceToHost, g.stream));
+    S.read_back();
+    Timed::mark();
     CU(cudaStreamSynchronize(g.stream));
     unsigned long long ctr[kNumCounters];
     memcpy(ctr, g.h_up + S.jobsBytes, sizeof ctr);
@@ -1056,13 +1082,12 @@ void run_scene_runs(std::vector<HostRun>& runs) {
       prog_need = std::max<long long>(prog_need * 2, (long long)(ctr[kCtrProg] + ctr[kCtrProg] / 4));
       continue;
     }
-    const PathJob* out = reinterpret_cast<const PathJob*>(g.h_up);
     bool grow = false;
     for (size_t k = 0; k < sr.size(); k++) {
       HostRun& r = runs[which[k]];
       size_t done = r.j1;
       for (int j = sr[k].j0; j < sr[k].j1; j++) {
-        const int st = out[j].status;
+        const int st = outcome_status(S.outcomes()[j]);
         if (st == kOk || st == kNothing) continue;
         done = r.j0 + (size_t)(j - sr[k].j0);
         if (st == kErrArenaFull) grow = true;
@@ -1357,7 +1382,7 @@ void srv_step(pxg_server* sv) {
     while (e < pj.size() && e - j->next < lim && pj[e].mode != kMask) e++;
     if (e == j->next) continue;
     rowBudget -= (long long)(e - j->next) * j->H;
-    runs.push_back(HostRun{&j->canvas, const_cast<std::vector<PathJob>*>(&pj), &j->scene->prims,
+    runs.push_back(HostRun{&j->canvas, &pj, &j->scene->prims,
                            scene_device_prims(j->scene), j->next, e, kOk, j->scene->dstroke});
     owners.push_back(j);
     budget -= (long long)(e - j->next);
@@ -1482,8 +1507,6 @@ const Prim* masks_device_prims(pxg_masks* m) {
 void render_masks(pxg_masks* m) {
   if (m->jobs.empty()) return;
   dev_grow(m->dev, m->dev_cap, std::max<long long>(m->bytes, 16));
-  std::vector<PathJob> jobs = m->jobs;
-  for (size_t i = 0; i < jobs.size(); i++) jobs[i].img = m->dev + m->offs[i];
   if (!m->graph) m->graph = new GraphCacheHolder();
   const std::pair<int, long long> key{kTuneMaskRows, mask_class(m)};
   auto it = g_tune.best.find(key);
@@ -1492,26 +1515,29 @@ void render_masks(pxg_masks* m) {
     std::vector<float> t(kNumMaskRowsCands, 0.0f);
     int best = 0;
     for (int c = 0; c < kNumMaskRowsCands; c++) {
-      std::vector<PathJob> jc = jobs;
       RunOpts o;
+      o.imgs = m->dev;
+      o.img_offs = &m->offs;
       o.cfg = kMaskRowsCands[c];
       o.zero = m->dev;
       o.zero_bytes = m->bytes;
       o.rows_ms = &t[(size_t)c];
       o.dprims = masks_device_prims(m);
-      run_jobs(jc, m->prims, st, o);
+      run_jobs(m->jobs, m->prims, st, o);
       if (t[(size_t)c] < t[(size_t)best]) best = c;
     }
     g_tune.best[key] = best;
     g_tune.ms[key] = t;
   } else {
     RunOpts o;
+    o.imgs = m->dev;
+    o.img_offs = &m->offs;
     o.cfg = kMaskRowsCands[it == g_tune.best.end() ? 1 : it->second];
     o.zero = m->dev;
     o.zero_bytes = m->bytes;
     o.graph = &m->graph->gc;
     o.dprims = masks_device_prims(m);
-    run_jobs(jobs, m->prims, st, o);
+    run_jobs(m->jobs, m->prims, st, o);
   }
   for (size_t i = 0; i < st.size(); i++)
     if (st[i] != kOk) throw ApiError{status_message(st[i])};
@@ -2037,7 +2063,7 @@ int pxg_image_draw_scene(pxg_image* im, const pxg_scene* sc) {
   return guarded([&] {
     check_image(im);
     if (!sc) throw ApiError{"Invalid scene handle"};
-    std::vector<PathJob> jobs = sc->jobs;
+    const std::vector<PathJob>& jobs = sc->jobs;
     Timed t(true);
     const Prim* dp = scene_device_prims(sc);
     size_t i = 0;
@@ -2210,9 +2236,9 @@ int pxg_masks_render_config(pxg_masks* m, int variant, int rows_per_item) {
     if (variant < 0 || variant > 1 || rows_per_item < 1 || rows_per_item > 64) throw ApiError{"Invalid configuration"};
     if (m->jobs.empty()) return;
     dev_grow(m->dev, m->dev_cap, std::max<long long>(m->bytes, 16));
-    std::vector<PathJob> jobs = m->jobs;
-    for (size_t i = 0; i < jobs.size(); i++) jobs[i].img = m->dev + m->offs[i];
     RunOpts o;
+    o.imgs = m->dev;
+    o.img_offs = &m->offs;
     o.cfg.variant = variant;
     o.cfg.rpi = rows_per_item;
     o.zero = m->dev;
@@ -2220,7 +2246,7 @@ int pxg_masks_render_config(pxg_masks* m, int variant, int rows_per_item) {
     o.dprims = masks_device_prims(m);
     std::vector<int> st;
     Timed t(true);
-    run_jobs(jobs, m->prims, st, o);
+    run_jobs(m->jobs, m->prims, st, o);
     t.done();
     for (size_t i = 0; i < st.size(); i++)
       if (st[i] != kOk) throw ApiError{status_message(st[i])};

@@ -128,7 +128,7 @@ struct Arena {
   int4* prog;          // scenes: row programs (16-byte units)
   long long prog_cap;
   int4* rowhdr;        // scenes: per row and job, what it draws (RecKind)
-  uint2* pinfo;        // scenes: per job {colour, mode | status << 8}
+  uint2* pinfo;        // per job {colour, mode | status << 8}, written by the setup kernel
   uint8_t* cov8;       // scenes: coverage bytes of rows recorded as kRecCov8 (16-byte units)
   long long cov8_cap;
   unsigned long long* counters;

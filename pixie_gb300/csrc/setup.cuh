@@ -309,10 +309,11 @@ __device__ __forceinline__ int block_scan_excl(int v, int* s_warp, int& total) {
   return before + x - v;
 }
 
-// The job's outcome, and beside its colour and mode for the drawing pass.
+// The job's outcome: for the host, and with its colour and mode for the
+// drawing pass.
 __device__ __forceinline__ void set_status(PathJob& J, const Arena& A, int job, int st) {
   J.status = st;
-  if (A.pinfo) A.pinfo[job] = make_uint2(J.rgbx, (uint32_t)J.mode | ((uint32_t)st << 8));
+  A.pinfo[job] = make_uint2(J.rgbx, (uint32_t)J.mode | ((uint32_t)st << 8));
 }
 
 // C: CTAs per job (the cluster size; 1: a plain launch).
