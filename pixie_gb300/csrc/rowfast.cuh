@@ -16,9 +16,11 @@
 // is 4-7 rows high for all but the tallest shapes).
 //
 // Measured against process_row (GB300, kernel times): recording 2000 paths on
-// 1024 x 1024 (2 M rows) 21.3 -> 7.2 ms, with 1.0 ms for the rows of more than
-// 128 crossings; the rows of 4096 glyphs 1.23 -> 0.57 ms; of one 512 x 512
-// path of 64 cubics 46 -> 30 us.
+// 1024 x 1024 (2 M rows) 21.3 -> 6.6 ms, with 1.0 ms for the rows of more than
+// 128 crossings; the rows of 4096 glyphs 1.23 -> 0.38 ms; of one 512 x 512
+// path of 64 cubics 46 -> 30 us.  The recording kernel's hot code is at the
+// instruction cache's edge: 49 KB of it run at 6.6 ms, 54 KB (with the groups
+// of cov_samples) at 8.6 ms, a miss rate of 8 against 18 per cent.
 //
 // Included by raster.cu after the shared row helpers (make_entry, blends, the
 // trapezoid areas).
@@ -37,15 +39,22 @@ enum RowOut { kOutRgbx = 0, kOutA8 = 1, kOutRec = 2 };
 
 template <int NB, int XT>
 struct __align__(16) FastRow {
-  float ay[NB], by[NB], m[NB], b[NB];  // the chunk's entries, in segment order
-  float key[NB];                       // a sample line's sort keys; midpoints of a trapezoid row
-  float t0[NB], t1[NB];                // a trapezoid row's crossings with its top and bottom; else sample spans
-  uint32_t diff[(XT + 272) / 2];       // coverage differences, two 16-bit pixels per word; zero between rows
-  uint16_t idx[NB], perm[NB];          // the row's entries; their order by midpoint
-  uint8_t wp[NB];                      // winding +1
-  float ends[2][2];                    // clipped x of a two-entry band's entries (top, bottom)
+  float ent[4][NB];               // the chunk's entries, in segment order: ay, by, m, b
+  float key[NB];                  // a sample line's sort keys; midpoints of a trapezoid row
+  float t0[NB], t1[NB];           // a trapezoid row's crossings with its top and bottom; else sample spans
+  uint32_t diff[(XT + 272) / 2];  // coverage differences, two pixels per word; kDiffZero between rows
+  uint16_t idx[NB], perm[NB];     // the row's entries; their order by midpoint
+  uint8_t wp[NB];                 // winding +1
+  float ends[2][2];               // clipped x of a two-entry band's entries (top, bottom)
   int nzero, zero[kZeroCap];
+  __device__ __forceinline__ float& ay(int j) { return ent[0][j]; }
+  __device__ __forceinline__ float& by(int j) { return ent[1][j]; }
+  __device__ __forceinline__ float& m(int j) { return ent[2][j]; }
+  __device__ __forceinline__ float& b(int j) { return ent[3][j]; }
 };
+// Two signed 16-bit sums per word: the lower one is kept above zero, so adding
+// a negative difference to it never borrows from the upper one.
+constexpr uint32_t kDiffZero = 0x4000u;
 
 // A loop-invariant value the compiler is not to specialise loops for: a copy
 // of a loop per value of a flag doubles the code.
@@ -224,11 +233,9 @@ struct CovTile {
 };
 
 // diff[x] += v: contributions left of the tile carry into its first pixel,
-// those right of it are dropped.  Both halves of a word take signed 16-bit
-// sums; a lower half's borrow is undone where the word is read.
+// those right of it end at its last.
 __device__ __forceinline__ void cov_add(uint32_t* diff, const CovTile& T, int x, int v) {
-  if (x >= T.t1) return;
-  const int i = max(x, T.t0) - T.x0;
+  const int i = min(max(x, T.t0), T.t1) - T.x0;
   atomicAdd(&diff[i >> 1], (uint32_t)v << ((i & 1) << 4));
 }
 // pixels [a, b) += v
@@ -274,117 +281,159 @@ __device__ __forceinline__ void cov_span(uint32_t* diff, CovTile& T, int prevAt,
   }
 }
 
-// The walk of computeCoverage over one sample line's nh sorted crossings
-// (paths.nim:1298-1334); the spans it draws are appended to sp.  A crossing's
+// 32 crossings of computeCoverage's walk over a sample line's nh sorted ones
+// (paths.nim:1298-1334), for one line or for several with a group of lanes
+// each; the spans it draws are appended to sp.  A crossing's
 // winding count is the number of +1 minus -1 crossings before it.  What the
 // walk does at one position -- draws a span up to it, only moves prevAt
 // there, or neither -- is decided by the first of its crossings that does
 // either (a second span there would be empty), which the lane of the
 // position's first crossing finds: crossings that cancel their successor are
 // skipped with it, and a nonzero count that stays nonzero does nothing.
+// i: the lane's crossing (keys[i]; none at or past nh); group: the lanes of the
+// same line; count and prevAt: the walk's before them, moved past them unless
+// the line ends with them.
 template <int TAG>
-__device__ __forceinline__ void walk_keys(const uint32_t* keys, int nh, int winding, int2* sp, int& ns, int lane) {
-  const unsigned lt = (1u << lane) - 1;
-  int carry = 0, prevCarry = 0;
+__device__ __forceinline__ void walk_step(const uint32_t* keys, int i, int nh, unsigned group, bool last, int& count,
+                                          int& prevAt, int winding, int2* sp, int& ns, int lane) {
+  const unsigned lt = (1u << lane) - 1, before = lt & group;
+  const bool valid = i < nh;
+  uint32_t key = valid ? keys[i] : kNoKey;
+  const uint32_t prev = valid && i > 0 ? keys[i - 1] : kNoKey;
+  const int at = (int)(key >> TAG);
+  const unsigned V = __ballot_sync(0xffffffffu, valid), P = __ballot_sync(0xffffffffu, valid && (key & 1));
+  int c = count + 2 * __popc(P & before) - __popc(V & before);
+  bool span = false, upd = false;
+  const bool nonzero = opaque(winding) == 0;
+  if (valid && at > 0 && ((key ^ prev) >> TAG) != 0) {
 #pragma unroll 1
-  for (int c0 = 0; c0 < nh; c0 += 32) {
-    int i = c0 + lane;
-    const bool valid = i < nh;
-    uint32_t key = valid ? keys[i] : kNoKey;
-    const uint32_t before = valid && i > 0 ? keys[i - 1] : kNoKey;
-    const int at = (int)(key >> TAG);
-    const unsigned P = __ballot_sync(0xffffffffu, valid && (key & 1)), N = __ballot_sync(0xffffffffu, valid && !(key & 1));
-    int count = carry + __popc(P & lt) - __popc(N & lt);
-    carry += __popc(P) - __popc(N);
-    bool span = false, upd = false;
-    const bool nonzero = opaque(winding) == 0;
-    if (valid && at > 0 && ((key ^ before) >> TAG) != 0) {
-      while (true) {
-        if ((nonzero ? count : count & 1) == 0) {
-          upd = true;
-          break;
-        }
-        const uint32_t nx = i + 1 < nh ? keys[i + 1] : kNoKey;
-        const bool same = ((key ^ nx) >> TAG) == 0;
-        const int w = (key & 1) ? 1 : -1;
-        if (same && ((key ^ nx) & 1)) {
-          i += 2;
-          key = i < nh ? keys[i] : kNoKey;
-        } else if (nonzero && i < nh - 1 && count + w != 0) {
-          count += w;
-          i++;
-          key = nx;
-        } else {
-          span = upd = true;
-          break;
-        }
-        if ((int)(key >> TAG) != at) break;
+    while (true) {
+      if ((nonzero ? c : c & 1) == 0) {
+        upd = true;
+        break;
       }
+      const uint32_t nx = i + 1 < nh ? keys[i + 1] : kNoKey;
+      const int w = (key & 1) ? 1 : -1;
+      if (((key ^ nx) >> TAG) == 0 && ((key ^ nx) & 1)) {
+        i += 2;
+        key = i < nh ? keys[i] : kNoKey;
+      } else if (nonzero && i < nh - 1 && c + w != 0) {
+        c += w;
+        i++;
+        key = nx;
+      } else {
+        span = upd = true;
+        break;
+      }
+      if ((int)(key >> TAG) != at) break;
     }
-    const unsigned um = __ballot_sync(0xffffffffu, upd), below = um & lt;
-    const unsigned em = __ballot_sync(0xffffffffu, span);
-    const int pa = __shfl_sync(0xffffffffu, at, below ? 31 - __clz(below) : lane);
-    if (span) sp[ns + __popc(em & lt)] = make_int2(below ? pa : prevCarry, at);
-    const int last = __shfl_sync(0xffffffffu, at, um ? 31 - __clz(um) : 0);
-    if (um) prevCarry = last;
-    ns += __popc(em);
+  }
+  const unsigned um = __ballot_sync(0xffffffffu, upd), below = um & before;
+  const unsigned em = __ballot_sync(0xffffffffu, span);
+  const int pa = __shfl_sync(0xffffffffu, at, below ? 31 - __clz(below) : lane);
+  if (span) sp[ns + __popc(em & lt)] = make_int2(below ? pa : prevAt, at);
+  ns += __popc(em);
+  if (!last) {
+    count += 2 * __popc(P) - __popc(V);
+    const int moved = __shfl_sync(0xffffffffu, at, um ? 31 - __clz(um) : 0);
+    if (um) prevAt = moved;
   }
 }
 
+// A line's key for the row's entry e (the chunk's j): where it crosses yLine,
+// over its place among equals and its winding.
+template <int TAG, int NB, int XT>
+__device__ __forceinline__ uint32_t crossing_key(FastRow<NB, XT>& S, int j, int e, float yLine, float Wf) {
+  const float m = S.m(j), b = S.b(j);
+  const float x = m == 0 ? b : (yLine - b) / m;
+  const int fx = nim_i32(nmin(x, Wf) * 256.0f);
+  // crossings at or left of 0 only add to the winding count, in any order
+  return ((uint32_t)max(fx, 0) << TAG) | ((uint32_t)e << 1) | S.wp[j];
+}
 // The sample lines of row y (:1350-1397): the row's n entries (S.idx) against
-// each line, sorted, walked, accumulated into S.diff over the tile T.  The
-// entries are ordered once by where they cross the middle of the row (or end
-// nearest to it); a line's crossings, gathered in that order, are then nearly
-// sorted.  Only the exact sort of a line's own keys decides.
-template <int NB, int XT>
+// each line, sorted, walked, accumulated into S.diff over the tile T.
+// Up to kGroupN entries -- most rows of drawn shapes have 2 to 8 -- the lanes
+// take as many lines at once as fit, a group of n lanes each, and a crossing's
+// rank is counted (GROUPED; the recording kernel is faster without the code).
+// With more, the entries are ordered once by where they cross the middle of the
+// row (or end nearest to it); a line's crossings, gathered in that order, are
+// then nearly sorted.  Only the exact sort of a line's own keys decides.
+constexpr int kGroupN = 16;
+template <bool GROUPED, int NB, int XT>
 __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, float Wf, int winding, bool aa,
                                             CovTile& T, int lane) {
+  constexpr int TAG = tag_bits(NB);
   const unsigned lt = (1u << lane) - 1;
   uint32_t* keys = reinterpret_cast<uint32_t*>(S.key);
   int2* sp = reinterpret_cast<int2*>(S.t0);
-  constexpr int TAG = tag_bits(NB);
-  const int cap = NB <= 64 || n <= 64 ? 64 : NB <= 512 ? NB : 0;
+  const int lines = aa ? 5 : 1;
   const float offset = aa ? 1.0f / 5.0f : 1.0f;
   const float initialOffset = offset / 2 + kEps;
   float yLine = (float)y + initialOffset - offset;
-  int ns = 0;
+  const bool grouped = GROUPED && n <= kGroupN;
+  const int sets = grouped ? 32 / n : 1;
+  // the lane's place: line s of a step, entry i of its group, keys from kb on
+  const int s = grouped ? lane / n : 0, kb = s * n, i = lane - kb;
+  const unsigned group = grouped ? ((1u << n) - 1) << kb : 0xffffffffu;
+  const int cap = NB <= 64 || n <= 64 ? 64 : NB <= 512 ? NB : 0;
+  int ns = 0, done = grouped ? 0 : -1;  // lines done (-1: the ordering is to come)
+  if (grouped) {                        // the first step's lines are s ahead
 #pragma unroll 1
-  for (int q = aa ? 6 : 2; q > 0; q--) {  // the ordering, then the sample lines
-    const bool ordering = opaque(q) == (aa ? 6 : 2);
+    for (int k = 0; k < min(s, lines); k++) yLine += offset;
+  }
+#pragma unroll 1
+  while (done < lines) {
+    const bool ordering = !grouped && opaque(done) < 0;
+    int nh = 0;  // the crossings of the lane's line
     if (!ordering) yLine += offset;
-    int nh = 0;
+    if (grouped) {
+      const int j = S.idx[i];
+      const bool hit = s < sets && done + s < lines && S.ay(j) <= yLine && S.by(j) >= yLine;
+      const uint32_t key = hit ? crossing_key<TAG>(S, j, i, yLine, Wf) : kNoKey;
+      int rank = 0;
 #pragma unroll 1
-    for (int e0 = 0; e0 < n; e0 += 32) {
-      const int i = min(e0 + lane, n - 1), e = ordering ? i : S.perm[i], j = S.idx[e];
-      const float ay = S.ay[j], by = S.by[j];
-      const float yl = ordering ? fminf(fmaxf((float)y + 0.5f, ay), by) : yLine;
-      const bool hit = e0 + lane < n && (ordering || (ay <= yl && by >= yl));
-      const unsigned msk = __ballot_sync(0xffffffffu, hit);
-      if (hit) {
-        const float m = S.m[j], b = S.b[j];
-        const float x = m == 0 ? b : (yl - b) / m;
-        const int fx = nim_i32(nmin(x, Wf) * 256.0f);
-        // crossings at or left of 0 only add to the winding count, in any order
-        keys[nh + __popc(msk & lt)] = ((uint32_t)max(fx, 0) << TAG) | ((uint32_t)e << 1) | S.wp[j];
+      for (int d = 1, o = i + 1; d < n; d++, o++) {
+        if (o == n) o = 0;
+        rank += __shfl_sync(0xffffffffu, key, kb + o) < key;
       }
-      nh += __popc(msk);
-    }
+      nh = __popc(__ballot_sync(0xffffffffu, hit) & group);
+      if (hit) keys[kb + rank] = key;
+      // the lane's next line is `sets` further on: sets - 1 of them here
 #pragma unroll 1
-    for (int i = nh + lane; i < cap; i += 32) keys[i] = kNoKey;
-    __syncwarp();
-    if (cap == 64) sort_keys<2>(keys, nh, ordering, lane);
-    else if (NB <= 512) sort_keys<NB <= 512 ? NB / 32 : 2>(keys, nh, ordering, lane);
-    else sort_keys_shared(keys, nh, ordering, lane);
+      for (int k = 1; k < sets && done + sets < lines; k++) yLine += offset;
+    } else {
+#pragma unroll 1
+      for (int e0 = 0; e0 < n; e0 += 32) {
+        const int at = min(e0 + lane, n - 1), e = ordering ? at : S.perm[at], j = S.idx[e];
+        const float ay = S.ay(j), by = S.by(j);
+        const float yl = ordering ? fminf(fmaxf((float)y + 0.5f, ay), by) : yLine;
+        const bool hit = e0 + lane < n && (ordering || (ay <= yl && by >= yl));
+        const unsigned msk = __ballot_sync(0xffffffffu, hit);
+        if (hit) keys[nh + __popc(msk & lt)] = crossing_key<TAG>(S, j, e, yl, Wf);
+        nh += __popc(msk);
+      }
+#pragma unroll 1
+      for (int k = nh + lane; k < cap; k += 32) keys[k] = kNoKey;
+      __syncwarp();
+      if (cap == 64) sort_keys<2>(keys, nh, ordering, lane);
+      else if (NB <= 512) sort_keys<NB <= 512 ? NB / 32 : 2>(keys, nh, ordering, lane);
+      else sort_keys_shared(keys, nh, ordering, lane);
+    }
     __syncwarp();
     if (ordering) {
 #pragma unroll 1
-      for (int i = lane; i < nh; i += 32) S.perm[i] = (uint16_t)((keys[i] >> 1) & ((1u << (TAG - 1)) - 1));
-    }
-    if (!ordering) walk_keys<TAG>(keys, nh, winding, sp, ns, lane);
-    __syncwarp();
-    if (ns > NB / 2 || q == 1) {  // a line has at most NB / 2 spans, and there is room for NB
+      for (int k = lane; k < nh; k += 32) S.perm[k] = (uint16_t)((keys[k] >> 1) & ((1u << (TAG - 1)) - 1));
+    } else {
+      int count = 0, prevAt = 0;  // after the 32 crossings before
 #pragma unroll 1
-      for (int i = lane; i < ns; i += 32) cov_span(S.diff, T, sp[i].x, sp[i].y, opaque(aa) != 0);
+      for (int c0 = 0; c0 < (grouped ? 1 : nh); c0 += 32)
+        walk_step<TAG>(keys + kb, c0 + i, nh, group, grouped, count, prevAt, winding, sp, ns, lane);
+    }
+    __syncwarp();
+    done += sets;
+    if (ns > NB / 2 || done >= lines) {  // a line has at most NB / 2 spans, and there is room for NB
+#pragma unroll 1
+      for (int k = lane; k < ns; k += 32) cov_span(S.diff, T, sp[k].x, sp[k].y, opaque(aa) != 0);
       ns = 0;
       __syncwarp();
     }
@@ -399,55 +448,56 @@ __device__ __forceinline__ int warp_scan_incl(int v, int lane) {
   }
   return v;
 }
-__device__ __forceinline__ void unpack_diff(uint32_t w, int& a, int& b) {
-  a = (int)(short)(w & 0xffffu);
-  b = (int)(w - (uint32_t)a) >> 16;
-}
-
 // Takes the difference array from index i0 (a multiple of 8) through iEnd,
-// leaving it zero, N (4 or 8) pixels per lane: out(i, c) gets the prefix sums
-// of indices i .. i + N - 1, 0 at or past iLim.
+// leaving it at zero, 2 N pixels (N = 2 or 4 words) per lane: out(i, f) gets the
+// prefix sums of indices i .. i + 2 N - 1, two per word.  A word's two prefix
+// sums are w + (w << 16), the sum before it is added to both halves at once;
+// the sums themselves are not negative, so the halves come out exact.
 template <int N, class Out>
-__device__ __forceinline__ void flush_diff(uint32_t* diff, int i0, int iEnd, int iLim, int lane, Out&& out) {
+__device__ __forceinline__ void flush_diff(uint32_t* diff, int i0, int iEnd, int lane, Out&& out) {
   int carry = 0;
 #pragma unroll 1
-  for (int i = i0; i <= iEnd; i += 32 * N) {
-    const int ii = i + lane * N;
-    int c[N];
-    if (N == 8) {
+  for (int i = i0; i <= iEnd; i += 64 * N) {
+    const int ii = i + lane * 2 * N;
+    uint32_t w[N];
+    if (N == 4) {
       uint4* p = reinterpret_cast<uint4*>(diff + (ii >> 1));
       const uint4 q = *p;
-      *p = make_uint4(0u, 0u, 0u, 0u);
-      unpack_diff(q.x, c[0], c[1]);
-      unpack_diff(q.y, c[2], c[3]);
-      unpack_diff(q.z, c[N - 4], c[N - 3]);
-      unpack_diff(q.w, c[N - 2], c[N - 1]);
+      *p = make_uint4(kDiffZero, kDiffZero, kDiffZero, kDiffZero);
+      w[0] = q.x;
+      w[1] = q.y;
+      w[N - 2] = q.z;
+      w[N - 1] = q.w;
     } else {
       uint2* p = reinterpret_cast<uint2*>(diff + (ii >> 1));
       const uint2 q = *p;
-      *p = make_uint2(0u, 0u);
-      unpack_diff(q.x, c[0], c[1]);
-      unpack_diff(q.y, c[2], c[3]);
+      *p = make_uint2(kDiffZero, kDiffZero);
+      w[0] = q.x;
+      w[1] = q.y;
     }
+    int sum[N];  // through word k
 #pragma unroll
-    for (int k = 1; k < N; k++) c[k] += c[k - 1];
-    const int incl = warp_scan_incl(c[N - 1], lane);
-    const int base = carry + incl - c[N - 1];
+    for (int k = 0; k < N; k++) {
+      sum[k] = ((int)w[k] >> 16) + (int)(w[k] & 0xffffu) - (int)kDiffZero + (k ? sum[k - 1] : 0);
+      w[k] -= kDiffZero;
+      w[k] += w[k] << 16;
+    }
+    const int incl = warp_scan_incl(sum[N - 1], lane);
+    const int base = carry + incl - sum[N - 1];
     carry += __shfl_sync(0xffffffffu, incl, 31);
 #pragma unroll
-    for (int k = 0; k < N; k++) c[k] = ii + k < iLim ? base + c[k] : 0;
-    out(ii, c);
+    for (int k = 0; k < N; k++) w[k] += (uint32_t)(base + (k ? sum[k - 1] : 0)) * 0x00010001u;
+    out(ii, w);
   }
   __syncwarp();
 }
-__device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
-  return (a & 255) | ((b & 255) << 8) | ((c & 255) << 16) | ((uint32_t)d << 24);
-}
+// the low bytes of four prefix sums
+__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x6420); }
 
-// Loads the entries of a band that overlap the rows [c0, c1) into S, in
-// segment order; returns their number, or -1 when they exceed NB.  A band of
-// exactly two entries that are two non-intersecting spanning edges
-// (:1250-1262) sets two and orders them left to right.
+// Loads the entries of a band that overlap the rows [c0, c1) into S, in segment
+// order; returns their number, or -1 when they exceed NB.  A band of exactly two entries that
+// are two non-intersecting spanning edges (:1250-1262) sets two and orders them
+// left to right.
 template <int NB, int XT>
 __device__ __forceinline__ int load_chunk(const PathJob& J, const Arena& A, const Band& bd, float top, float bottom,
                                           float c0, float c1, FastRow<NB, XT>& S, int lane, bool& two) {
@@ -470,10 +520,10 @@ __device__ __forceinline__ int load_chunk(const PathJob& J, const Arena& A, cons
     const unsigned msk = __ballot_sync(0xffffffffu, pred);
     const int p = n + __popc(msk & lt);
     if (pred && p < NB) {
-      S.ay[p] = e.ay;
-      S.by[p] = e.by;
-      S.m[p] = e.m;
-      S.b[p] = e.b;
+      S.ay(p) = e.ay;
+      S.by(p) = e.by;
+      S.m(p) = e.m;
+      S.b(p) = e.b;
       S.wp[p] = e.w > 0;
       if (p < 2) {
         S.ends[p][0] = e.ax;
@@ -484,25 +534,28 @@ __device__ __forceinline__ int load_chunk(const PathJob& J, const Arena& A, cons
   }
   __syncwarp();
   two = false;
+  if (n > NB) return -1;
   if (nb == 2) {
-    const V2 a0{S.ends[0][0], S.ay[0]}, b0{S.ends[0][1], S.by[0]}, a1{S.ends[1][0], S.ay[1]}, b1{S.ends[1][1], S.by[1]};
+    const V2 a0{S.ends[0][0], S.ay(0)}, b0{S.ends[0][1], S.by(0)}, a1{S.ends[1][0], S.ay(1)}, b1{S.ends[1][1], S.by(1)};
     two = !intersectsInside(a0, b0, a1, b1) && a0.y <= top && b0.y >= bottom && a1.y <= top && b1.y >= bottom;
     if (two && (a0.x + b0.x) * 0.5f > (a1.x + b1.x) * 0.5f) {
-      const float m = S.m[lane & 1], b = S.b[lane & 1];
-      const uint8_t w = S.wp[lane & 1];
+      const int p = lane & 1;
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) v[k] = S.ent[k][p];
+      const uint8_t t = S.wp[p];
+      const float x = S.ends[p][0];
       __syncwarp();
       if (lane < 2) {
-        S.ay[1 - lane] = lane ? a1.y : a0.y;
-        S.by[1 - lane] = lane ? b1.y : b0.y;
-        S.m[1 - lane] = m;
-        S.b[1 - lane] = b;
-        S.wp[1 - lane] = w;
-        S.ends[1 - lane][0] = lane ? a1.x : a0.x;
+#pragma unroll
+        for (int k = 0; k < 4; k++) S.ent[k][1 - p] = v[k];
+        S.wp[1 - p] = t;
+        S.ends[1 - p][0] = x;
       }
       __syncwarp();
     }
   }
-  return n <= NB ? n : -1;
+  return n;
 }
 
 // Hands row y of the job on, to list 0, 1 or 2 (which a later kernel takes): more
@@ -528,7 +581,7 @@ __device__ __forceinline__ bool trap_row(FastRow<NB, XT>& S, int n, float yTop, 
 #pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     const int j = S.idx[i];
-    const float m = S.m[j], b = S.b[j];
+    const float m = S.m(j), b = S.b(j);
     const float t0 = entry_x(m, b, yTop), t1 = entry_x(m, b, yBottom), key = (t0 + t1) * 0.5f;
     S.t0[i] = t0;
     S.t1[i] = t1;
@@ -565,8 +618,9 @@ __device__ __forceinline__ bool trap_row(FastRow<NB, XT>& S, int n, float yTop, 
     // partial coverage of neighbours must not overlap (:1721-1731)
     if (i + 1 < n) bad |= nim_trunc(ceilf(nmax(S.t0[j], S.t1[j]))) > nim_trunc(nmin(S.t0[q], S.t1[q]));
     // and pairs must be simple fills (:1733-1750)
-    const unsigned P = __ballot_sync(0xffffffffu, valid && S.wp[S.idx[j]]);
-    const unsigned N = __ballot_sync(0xffffffffu, valid && !S.wp[S.idx[j]]);
+    const bool up = S.wp[S.idx[j]] != 0;
+    const unsigned P = __ballot_sync(0xffffffffu, valid && up);
+    const unsigned N = __ballot_sync(0xffffffffu, valid && !up);
     const int count = carry + __popc(P & le) - __popc(N & le);  // after this entry
     if (valid) bad |= ((opaque(winding) == 0 ? count : count & 1) != 0) != ((i & 1) == 0);
     carry += __popc(P) - __popc(N);
@@ -586,7 +640,7 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
 #pragma unroll 1
   for (int s = 0; s < n; s++) {
     const int i = S.perm[s], j = S.idx[i];
-    const float m = S.m[j], b = S.b[j], t0 = S.t0[i], t1 = S.t1[i];
+    const float m = S.m(j), b = S.b(j), t0 = S.t0[i], t1 = S.t1[i];
     const float lo = nmin(t0, t1), end = ceilf(nmax(t0, t1));
     const long long xs = nim_int(lo);
     const int x1 = nim_clamp(end, T.t0, T.t1);
@@ -621,13 +675,12 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
   const unsigned lt = (1u << lane) - 1;
   const int W = (int)J.W, startY = (int)J.startY, pathHeight = (int)J.pathHeight, ph = (int)J.ph;
   const int winding = J.winding, nb = J.nb;
-  int curK = -1, cnt = 0, validTo = yA;  // validTo: the rows the loaded entries serve
+  int cnt = 0, validTo = yA;  // validTo: the rows the loaded entries serve
   bool aa = false, two = false;
 #pragma unroll 1
   for (int y = yA; y < yB; y++) {
-    const int k = min((y - startY) / ph, nb - 1);
-    if (k != curK || y >= validTo) {
-      curK = k;
+    if (y >= validTo) {
+      const int k = min((y - startY) / ph, nb - 1);
       const Band bd = A.bands[J.band_off + k];
       const int bt = startY + k * ph;  // the band's top and bottom (:1178-1190)
       const int bb = k == nb - 1 ? pathHeight : bt + ph;
@@ -665,7 +718,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
 #pragma unroll 1
         for (int j0 = 0; j0 < cnt; j0 += 32) {
           const int j = j0 + lane;
-          const float ay = j < cnt ? S.ay[j] : yBottom, by = j < cnt ? S.by[j] : yTop;
+          const float ay = j < cnt ? S.ay(j) : yBottom, by = j < cnt ? S.by(j) : yTop;
           const bool pred = !(by <= yTop || ay >= yBottom);
           const unsigned msk = __ballot_sync(0xffffffffu, pred);
           if (pred) S.idx[n + __popc(msk & lt)] = (uint16_t)j;
@@ -735,7 +788,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       }
       CovTile T{xt, max(dl, xt), min(dh, xt + XT), INT_MAX, INT_MIN};
       if (kind == 0) {
-        cov_samples<NB, XT>(S, n, y, (float)W, winding, aa, T, lane);
+        cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane);
       } else {
         if (kind == 1) failed = trap_cov<REC>(S, n, y, T, lane);
         else if (lane == 0) cov_range(S.diff, T, dl, dh, 255);
@@ -745,8 +798,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       __syncwarp();
       const int lo = max(__reduce_min_sync(0xffffffffu, T.lo), T.t0);
       const int hi = min(__reduce_max_sync(0xffffffffu, T.hi), T.t1);
-      const int iLim = T.t1 - xt;
-      int i0 = 0, iEnd = iLim;
+      int i0 = 0, iEnd = T.t1 - xt;
       if (!tiled) {
         if (hi <= lo) break;  // every difference cancelled or was dropped
         i0 = (lo - xt) & ~15;
@@ -763,15 +815,15 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
         failed = (long long)(cb + covBytes) > A.cov8_cap;
       }
       uint8_t* dst = REC ? A.cov8 + cov : base;
-      flush_diff<OUT == kOutRgbx ? 4 : 8>(S.diff, i0, iEnd, iLim, lane, [&](int i, const int* c) {
+      flush_diff<OUT == kOutRgbx ? 2 : 4>(S.diff, i0, iEnd, lane, [&](int i, const uint32_t* f) {
         if (REC) {
           const int o = xt + i - covX;
           if (i < XT && o < (int)covBytes && !failed)
-            *reinterpret_cast<uint2*>(dst + o) = make_uint2(pack4(c[0], c[1], c[2], c[3]), pack4(c[4], c[5], c[6], c[7]));
+            *reinterpret_cast<uint2*>(dst + o) = make_uint2(pack4(f[0], f[1]), pack4(f[2], f[3]));
         } else if (OUT == kOutA8) {
           // a mask job paints white, opaque, Normal onto a cleared mask, each
           // pixel once: the blended alpha is the multiplier
-          const uint32_t a = pack4(c[0], c[1], c[2], c[3]), b = pack4(c[4], c[5], c[6], c[7]);
+          const uint32_t a = pack4(f[0], f[1]), b = pack4(f[2], f[3]);
           const int x = xt + i;
           if (failed || dry || (a | b) == 0) return;
           if (x >= 0 && x + 8 <= W) {
@@ -784,7 +836,8 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
             }
           }
         } else {
-          if (failed || dry || (c[0] | c[1] | c[2] | c[3]) == 0) return;
+          const uint32_t c[4] = {f[0] & 0xffffu, f[0] >> 16, f[1] & 0xffffu, f[1] >> 16};
+          if (failed || dry || (f[0] | f[1]) == 0) return;
           const int x = xt + i;
           uint32_t* p = reinterpret_cast<uint32_t*>(base) + x;
           const bool vec = x >= 0 && x + 4 <= W;
@@ -797,13 +850,13 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
             if (c[2] && x >= -2 && x + 2 < W) v.z = p[2];
             if (c[3] && x >= -3 && x + 3 < W) v.w = p[3];
           }
-          int c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+          uint32_t c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
 #pragma unroll 1
           for (int q = 0; q < 4; q++) {  // one copy of the blend: the pixels rotate through it
             uint32_t r = v.x;
-            if (c0) r = blend_row(J.mode, tbl, r, mul_c(J.rgbx, (uint32_t)c0 & 255u));
+            if (c0) r = blend_row(J.mode, tbl, r, mul_c(J.rgbx, c0 & 255u));
             v = make_uint4(v.y, v.z, v.w, r);
-            const int t = c0;
+            const uint32_t t = c0;
             c0 = c1;
             c1 = c2;
             c2 = c3;
@@ -840,7 +893,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
 template <int NB, int XT>
 __device__ __forceinline__ void init_fast_row(FastRow<NB, XT>& S, int lane) {
 #pragma unroll 1
-  for (int i = lane; i < (XT + 272) / 2; i += 32) S.diff[i] = 0u;
+  for (int i = lane; i < (XT + 272) / 2; i += 32) S.diff[i] = kDiffZero;
   __syncwarp();
 }
 

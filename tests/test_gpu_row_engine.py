@@ -76,7 +76,7 @@ def check(paths, w, h, seed, blends=(0,), windings=(0, 1), color=(0.8, 0.3, 0.1,
                 assert np.array_equal(img.to_numpy(), ref), f"scene {w}x{h} blend {blend} winding {winding}"
 
 
-@pytest.mark.parametrize("n", [2, 3, 31, 32, 33, 63, 64, 65, 66, 127, 128, 129, 130, 255, 256, 257, 258, 511, 512,
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 15, 16, 17, 18, 31, 32, 33, 63, 64, 65, 66, 127, 128, 129, 130, 255, 256, 257, 258, 511, 512,
                                513, 514, 1100, 2047, 2048])
 def test_crossings_per_row(n):
     check([zigzag(n, 700, 9, 2 * n), zigzag(n, 700, 9, 2 * n + 1)], 700, 9, n)
