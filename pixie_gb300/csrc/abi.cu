@@ -126,7 +126,8 @@ const void* scene_kernel(int ppl);
 int scene_warps();
 const void* scene_big_kernel(int v);
 size_t scene_big_smem(int v);
-int scene_big_warps(int v);
+int scene_big_threads(int v);
+int scene_big_rows(int v);
 void launch_scene_big(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A);
 const void* scene_rest_kernel();
 size_t scene_rest_smem();
@@ -381,7 +382,7 @@ void init_locked(int device) {
     for (int v = 0; v < 2; v++) {
       CU(cudaFuncSetAttribute(scene_big_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)scene_big_smem(v)));
-      CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_big_kernel(v), scene_big_warps(v) * 32,
+      CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scene_big_kernel(v), scene_big_threads(v),
                                                        scene_big_smem(v)));
       g.scene_ctas_per_sm[3 + v] = std::max(1, per);
     }
@@ -1059,7 +1060,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     note_launch();
     CU(cudaGetLastError());
     for (int v = 0; v < 2; v++) {
-      const long long bigBlocks = std::min<long long>((riTotal + scene_big_warps(v) - 1) / scene_big_warps(v),
+      const long long bigBlocks = std::min<long long>((riTotal + scene_big_rows(v) - 1) / scene_big_rows(v),
                                                       (long long)g.nsm * g.scene_ctas_per_sm[3 + v]);
       launch_scene_big(v, (unsigned)std::max<long long>(1, bigBlocks), g.stream, S.dj, S.A);
       note_launch();

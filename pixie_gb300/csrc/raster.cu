@@ -1034,8 +1034,8 @@ __global__ void k_xclears(PathJob* jobs, Arena A) {
 // Dense scenes, in two passes.
 // k_scene_rec: every row of every path of the launch, independent of the
 // pixels, in chunks from a device queue (rowfast.cuh): the row's coverage
-// bytes (or, rarely, its program: RecKind).  k_scene_big and
-// k_scene_rest record the rows it hands on.
+// bytes (or, rarely, its program: RecKind).  k_scene_big,
+// k_scene_huge and k_scene_rest record the rows it hands on.
 // k_scene: a warp owns a slice of one canvas row (sliceW pixels) and replays
 // every path's program for that row in submission order, so each pixel sees
 // the paths in the order the reference's sequence of fillPath/strokePath
@@ -1078,32 +1078,68 @@ __global__ void __launch_bounds__(kRecRowWarps * 32, 7) k_scene_rec(PathJob* job
   }
 }
 
-// The rows k_scene_rec handed on (list 0): up to NB crossings -- stroke
-// outlines overlap themselves hundreds of times a row.  The instance for
-// 512 hands the rest on to list 1, the one for 2048 (a warp per CTA, its keys
-// in shared memory) to list 2.
-template <int NB, int XT, int WARPS, int FROM>
-__global__ void __launch_bounds__(WARPS * 32) k_scene_big(PathJob* jobs, Arena A) {
+// The rows k_scene_rec handed on (list 0): up to 512 crossings -- stroke
+// outlines overlap themselves hundreds of times a row -- with fewer warps; the
+// rest to list 1.
+constexpr int kBigNB = 512, kBigXT = 1024, kBigWarps = 4;
+__global__ void __launch_bounds__(kBigWarps * 32) k_scene_big(PathJob* jobs, Arena A) {
   extern __shared__ __align__(16) unsigned char rsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  FastRow<NB, XT>& S = reinterpret_cast<FastRow<NB, XT>*>(rsm)[warp];
+  FastRow<kBigNB, kBigXT>& S = reinterpret_cast<FastRow<kBigNB, kBigXT>*>(rsm)[warp];
   init_fast_row(S, lane);
   pdl_trigger();
   pdl_wait();
-  const long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[FROM ? kCtrOvfRows2 : kCtrOvfRows]);
+  const long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[kCtrOvfRows]);
 #pragma unroll 1
-  for (long long i = (long long)blockIdx.x * WARPS + warp; i < n; i += (long long)gridDim.x * WARPS) {
-    const long long v = A.ovf_rows[FROM * A.ovf_cap + i];
+  for (long long i = (long long)blockIdx.x * kBigWarps + warp; i < n; i += (long long)gridDim.x * kBigWarps) {
+    const long long v = A.ovf_rows[i];
     const int job = (int)(v >> 32), y = (int)(v & 0xffffffffLL);
     const PathJob& J = jobs[job];
-    if (J.W >= fast_max_w(NB)) push_row(A, job, y, lane, FROM + 1);
-    else fast_rows<kOutRec, NB, XT, FROM + 1>(J, A, nullptr, job, y, y + 1, S, lane);
+    if (J.W >= fast_max_w(kBigNB)) push_row(A, job, y, lane, 1);
+    else fast_rows<kOutRec, kBigNB, kBigXT, 1>(J, A, nullptr, job, y, y + 1, S, lane);
   }
 }
-constexpr int kBigNB = 512, kBigXT = 1024, kBigWarps = 4;
-constexpr int kHugeNB = 2048, kHugeXT = 1024, kHugeWarps = 1;
 
-// The rows k_scene_big handed on (list 2), by the general row code; those with
+// List 1: up to 2048 crossings, a CTA per row and a warp per sample line, for
+// these rows are few and each takes long (a warp each, the widest rows of a
+// 240-path scene took 347 us, this way 74); the rest to list 2.
+constexpr int kHugeNB = 2048, kHugeXT = 1024;
+struct HugeRow {
+  FastRow<kHugeNB, kHugeXT> row;
+  LineScratch<kHugeNB> line[kLineWarps];
+  LineWork work;
+};
+__global__ void __launch_bounds__(kLineWarps * 32) k_scene_huge(PathJob* jobs, Arena A) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  HugeRow& S = *reinterpret_cast<HugeRow*>(rsm);
+  pdl_trigger();
+  pdl_wait();
+  if (warp > 0) {  // the other lines of the rows warp 0 publishes
+#pragma unroll 1
+    while (true) {
+      line_barrier();
+      if (S.work.n < 0) break;
+      one_line(S.row, S.work, S.line[warp], warp, lane);
+      line_barrier();
+    }
+    return;
+  }
+  init_fast_row(S.row, lane);
+  const long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[kCtrOvfRows2]);
+#pragma unroll 1
+  for (long long i = blockIdx.x; i < n; i += gridDim.x) {
+    const long long v = A.ovf_rows[A.ovf_cap + i];
+    const int job = (int)(v >> 32), y = (int)(v & 0xffffffffLL);
+    const PathJob& J = jobs[job];
+    if (J.W >= fast_max_w(kHugeNB)) push_row(A, job, y, lane, 2);
+    else fast_rows<kOutRec, kHugeNB, kHugeXT, 2, true>(J, A, nullptr, job, y, y + 1, S.row, lane, &S.work, S.line);
+  }
+  if (lane == 0) S.work.n = -1;
+  line_barrier();
+}
+
+// The rows k_scene_huge handed on (list 2), by the general row code; those with
 // more than MAXH crossings take a per-warp global scratch.
 constexpr int kRecXT = 256;  // coverage tile of the general recording code
 template <int MAXH, int WARPS>
@@ -1317,16 +1353,13 @@ constexpr int kRecMaxH = 128, kRecWarps = 8, kSceneWarps = 8;
 const void* scene_rec_kernel() { return (const void*)k_scene_rec; }
 size_t scene_rec_smem() { return sizeof(FastRow<kRecNB, kRecRowXT>) * kRecRowWarps; }
 int scene_rec_warps() { return kRecRowWarps; }
-// the two big-row instances (0: 512 crossings, 1: 2048)
-constexpr auto kSceneBig = k_scene_big<kBigNB, kBigXT, kBigWarps, 0>;
-constexpr auto kSceneHuge = k_scene_big<kHugeNB, kHugeXT, kHugeWarps, 1>;
-const void* scene_big_kernel(int v) { return v ? (const void*)kSceneHuge : (const void*)kSceneBig; }
-size_t scene_big_smem(int v) {
-  return v ? sizeof(FastRow<kHugeNB, kHugeXT>) * kHugeWarps : sizeof(FastRow<kBigNB, kBigXT>) * kBigWarps;
-}
-int scene_big_warps(int v) { return v ? kHugeWarps : kBigWarps; }
+// the kernels of wide rows: 0 k_scene_big, 1 k_scene_huge
+const void* scene_big_kernel(int v) { return v ? (const void*)k_scene_huge : (const void*)k_scene_big; }
+size_t scene_big_smem(int v) { return v ? sizeof(HugeRow) : sizeof(FastRow<kBigNB, kBigXT>) * kBigWarps; }
+int scene_big_threads(int v) { return (v ? kLineWarps : kBigWarps) * 32; }
+int scene_big_rows(int v) { return v ? 1 : kBigWarps; }  // per CTA
 void launch_scene_big(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A) {
-  launch_pdl(v ? kSceneHuge : kSceneBig, dim3(blocks), dim3(scene_big_warps(v) * 32), scene_big_smem(v), st, jobs, A);
+  launch_pdl(v ? k_scene_huge : k_scene_big, dim3(blocks), dim3(scene_big_threads(v)), scene_big_smem(v), st, jobs, A);
 }
 const void* scene_rest_kernel() { return (const void*)k_scene_rest<kRecMaxH, kRecWarps>; }
 size_t scene_rest_smem() { return sizeof(RowScratch<kRecMaxH, kRecXT>) * kRecWarps; }

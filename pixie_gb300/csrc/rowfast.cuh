@@ -440,6 +440,108 @@ __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, fl
   }
 }
 
+// Rows of hundreds of crossings: a warp per sample line.  The row's warp (0)
+// orders the entries and publishes the row; warps 1 .. 4 take the other lines
+// with keys and spans of their own, all into the row's difference array.
+constexpr int kLineWarps = 5;
+template <int NB>
+struct __align__(16) LineScratch {
+  static_assert(NB >= 1024, "sort_many pads to 1024 keys");
+  uint32_t keys[NB];
+  int2 spans[NB / 2 + 32];
+};
+struct LineWork {  // what warp 0 publishes (n < 0: no more rows), and the warps' touched pixels
+  int n, y, winding, lines, x0, t0, t1;
+  float Wf;
+  int lo[kLineWarps], hi[kLineWarps];
+};
+__device__ __forceinline__ void line_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kLineWarps * 32) : "memory"); }
+
+// n keys of up to 2048: 1024 fit a warp's registers.
+static __device__ __noinline__ void sort_many(uint32_t* keys, int n, bool fresh, int lane) {
+  if (n > 1024) {
+    sort_keys_shared(keys, n, fresh, lane);
+  } else {
+#pragma unroll 1
+    for (int k = n + lane; k < 1024; k += 32) keys[k] = kNoKey;
+    __syncwarp();
+    sort_keys<32>(keys, n, fresh, lane);
+  }
+  __syncwarp();
+}
+
+template <int NB, int XT>
+__device__ __forceinline__ void one_line(FastRow<NB, XT>& S, LineWork& L, LineScratch<NB>& K, int q, int lane) {
+  constexpr int TAG = tag_bits(NB);
+  const unsigned lt = (1u << lane) - 1;
+  CovTile T{L.x0, L.t0, L.t1, INT_MAX, INT_MIN};
+  const int n = L.n;
+  const bool aa = L.lines == 5;
+  if (q < L.lines) {
+    const float offset = aa ? 1.0f / 5.0f : 1.0f;
+    const float initialOffset = offset / 2 + kEps;
+    float yLine = (float)L.y + initialOffset - offset;
+#pragma unroll 1
+    for (int k = 0; k <= q; k++) yLine += offset;
+    int nh = 0;
+#pragma unroll 1
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      const int e = S.perm[min(e0 + lane, n - 1)], j = S.idx[e];
+      const bool hit = e0 + lane < n && S.ay(j) <= yLine && S.by(j) >= yLine;
+      const unsigned msk = __ballot_sync(0xffffffffu, hit);
+      if (hit) K.keys[nh + __popc(msk & lt)] = crossing_key<TAG>(S, j, e, yLine, L.Wf);
+      nh += __popc(msk);
+    }
+    __syncwarp();
+    sort_many(K.keys, nh, false, lane);
+    int count = 0, prevAt = 0, ns = 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < nh; c0 += 32)
+      walk_step<TAG>(K.keys, c0 + lane, nh, 0xffffffffu, false, count, prevAt, L.winding, K.spans, ns, lane);
+    __syncwarp();
+#pragma unroll 1
+    for (int k = lane; k < ns; k += 32) cov_span(S.diff, T, K.spans[k].x, K.spans[k].y, opaque(aa) != 0);
+  }
+  const int lo = __reduce_min_sync(0xffffffffu, T.lo), hi = __reduce_max_sync(0xffffffffu, T.hi);
+  if (lane == 0) {
+    L.lo[q] = lo;
+    L.hi[q] = hi;
+  }
+}
+// cov_samples by kLineWarps warps (called by warp 0).
+template <int NB, int XT>
+__device__ __forceinline__ void cov_lines(FastRow<NB, XT>& S, LineWork& L, LineScratch<NB>& K, int n, int y, float Wf,
+                                          int winding, bool aa, CovTile& T, int lane) {
+  constexpr int TAG = tag_bits(NB);
+#pragma unroll 1
+  for (int i = lane; i < n; i += 32) {
+    const int j = S.idx[i];
+    K.keys[i] = crossing_key<TAG>(S, j, i, fminf(fmaxf((float)y + 0.5f, S.ay(j)), S.by(j)), Wf);
+  }
+  __syncwarp();
+  sort_many(K.keys, n, true, lane);
+#pragma unroll 1
+  for (int i = lane; i < n; i += 32) S.perm[i] = (uint16_t)((K.keys[i] >> 1) & ((1u << (TAG - 1)) - 1));
+  if (lane == 0) {
+    L.n = n;
+    L.y = y;
+    L.winding = winding;
+    L.lines = aa ? 5 : 1;
+    L.x0 = T.x0;
+    L.t0 = T.t0;
+    L.t1 = T.t1;
+    L.Wf = Wf;
+  }
+  line_barrier();
+  one_line(S, L, K, 0, lane);
+  line_barrier();
+#pragma unroll 1
+  for (int q = 0; q < kLineWarps; q++) {
+    T.lo = min(T.lo, L.lo[q]);
+    T.hi = max(T.hi, L.hi[q]);
+  }
+}
+
 __device__ __forceinline__ int warp_scan_incl(int v, int lane) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -668,9 +770,10 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
 // Rows [yA, yB) of job J (non-MaskBlend, narrower than fast_max_w(NB), within the
 // path's rows), drawn into an RGBX image or an 8-bit mask, or recorded; rows it
 // does not take are handed on to list LIST.
-template <int OUT, int NB, int XT, int LIST = 0>
+template <int OUT, int NB, int XT, int LIST = 0, bool LINES = false>
 __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, const uint8_t* tbl, int job, int yA,
-                                          int yB, FastRow<NB, XT>& S, int lane) {
+                                          int yB, FastRow<NB, XT>& S, int lane, LineWork* L = nullptr,
+                                          LineScratch<2048>* K = nullptr) {
   constexpr bool REC = OUT == kOutRec;
   const unsigned lt = (1u << lane) - 1;
   const int W = (int)J.W, startY = (int)J.startY, pathHeight = (int)J.pathHeight, ph = (int)J.ph;
@@ -788,7 +891,8 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       }
       CovTile T{xt, max(dl, xt), min(dh, xt + XT), INT_MAX, INT_MIN};
       if (kind == 0) {
-        cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane);
+        if constexpr (LINES) cov_lines(S, *L, *K, n, y, (float)W, winding, aa, T, lane);
+        else cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane);
       } else {
         if (kind == 1) failed = trap_cov<REC>(S, n, y, T, lane);
         else if (lane == 0) cov_range(S.diff, T, dl, dh, 255);
