@@ -132,7 +132,7 @@ void launch_scene_big(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, co
 const void* scene_rest_kernel();
 size_t scene_rest_smem();
 int scene_rest_warps();
-void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
+void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const RecOrder* order, int njobs,
                       long long items, int rpi, const Arena& A);
 void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, unsigned char* wide,
                        long long slots);
@@ -967,7 +967,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     int nj = 0;
     std::vector<SceneRun> sr;
     std::vector<size_t> which;  // launch run -> runs index
-    long long items = 0, recItems = 0, riTotal = 0, maxH = 1, maxWork = 0;
+    long long items = 0, riTotal = 0, maxH = 1, maxWork = 0;
     int ppl = 4;
     const int slice = scene_slice_for(runs, ppl);
     long long pathRows = 0;
@@ -984,12 +984,10 @@ void run_scene_runs(std::vector<HostRun>& runs) {
       s.img = r.canvas->data;
       s.j0 = nj;
       s.ri_base = riTotal;
-      s.rec_off = recItems;
       const long long nrun = (long long)(r.j1 - r.j0);
       for (size_t j = r.j0; j < r.j1; j++) pc += (*r.jobs)[j].nprims;
       nj += (int)nrun;
       s.j1 = nj;
-      recItems += nrun * ((s.H + rpi - 1) / rpi);
       riTotal += s.H * nrun;
       items += s.H * ((s.W + slice - 1) / slice);
       maxH = std::max<long long>(maxH, s.H);
@@ -997,6 +995,31 @@ void run_scene_runs(std::vector<HostRun>& runs) {
       which.push_back(ri);
     }
     if (sr.empty()) return;
+    // the recording order: by the log2 of a path's primitives, heaviest first (a counting sort)
+    std::vector<unsigned char> extra(align_up(sizeof(SceneRun) * sr.size(), 16) + sizeof(RecOrder) * (size_t)nj);
+    const size_t orderAt = align_up(sizeof(SceneRun) * sr.size(), 16);
+    memcpy(extra.data(), sr.data(), sizeof(SceneRun) * sr.size());
+    RecOrder* order = reinterpret_cast<RecOrder*>(extra.data() + orderAt);
+    long long recItems = 0;
+    {
+      int at[33] = {0};
+      auto bucket = [](const PathJob& j) { return j.nprims > 0 ? __builtin_clz((unsigned)j.nprims) : 32; };
+      auto each = [&](auto&& f) {
+        int job = 0;
+        for (size_t k = 0; k < sr.size(); k++)
+          for (size_t j = runs[which[k]].j0; j < runs[which[k]].j1; j++) f((*runs[which[k]].jobs)[j], sr[k], job++);
+      };
+      each([&](const PathJob& j, const SceneRun&, int) {
+        if (bucket(j) < 32) at[bucket(j) + 1]++;
+      });
+      for (int b = 1; b < 33; b++) at[b] += at[b - 1];
+      each([&](const PathJob& j, const SceneRun& s, int job) { order[at[bucket(j)]++] = RecOrder{(s.H + rpi - 1) / rpi, job, 0}; });
+      for (int k = 0; k < nj; k++) {  // chunk counts -> first items
+        const long long n = order[k].first;
+        order[k].first = recItems;
+        recItems += n;
+      }
+    }
     const int maxBands = setup_max_bands(maxH);
     ensure_arena(seg_need, list_need, (long long)nj * maxBands, pc, 1);
     dev_grow(g.ovf, g.ovf_cap, 3 * std::max<long long>(riTotal, 1));
@@ -1027,8 +1050,8 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     }
     const long long blocks = std::max<long long>(
         1, std::min<long long>((items + scene_warps() - 1) / scene_warps(), (long long)g.nsm * g.scene_ctas_per_sm[1]));
-    Staged S = stage((size_t)nj, sr.data(), sizeof(SceneRun) * sr.size(), nullptr, true, [&](PathJob* dst) {
-      long long at = 0, item = 0;
+    Staged S = stage((size_t)nj, extra.data(), extra.size(), nullptr, true, [&](PathJob* dst) {
+      long long at = 0;
       for (size_t k = 0; k < sr.size(); k++) {
         const HostRun& r = runs[which[k]];
         const SceneRun& s = sr[k];
@@ -1042,8 +1065,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
           pj.img = s.img;
           pj.W = s.W;
           pj.H = s.H;
-          pj.row_off = item;
-          item += (s.H + rpi - 1) / rpi;
+          pj.row_off = 0;
           pj.ri_off = s.ri_base + (long long)(j - r.j0);
           pj.ri_stride = s.j1 - s.j0;
           pj.status = kOk;
@@ -1055,7 +1077,7 @@ void run_scene_runs(std::vector<HostRun>& runs) {
     CU(launch_setup(nj, setup_cluster(nj, maxWork, maxBands), maxBands, g.stream, S.dj, S.A));
     note_launch();
     CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
-    launch_scene_rec((unsigned)recBlocks, g.stream, S.dj, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(),
+    launch_scene_rec((unsigned)recBlocks, g.stream, S.dj, reinterpret_cast<const RecOrder*>(S.extra + orderAt), nj,
                      recItems, rpi, S.A);
     note_launch();
     CU(cudaGetLastError());

@@ -1043,7 +1043,7 @@ __global__ void k_xclears(PathJob* jobs, Arena A) {
 // reference raises at that call).  If the program arena overflowed, k_scene
 // draws nothing and the host reruns the launch with a larger arena.
 constexpr int kRecNB = 128, kRecRowXT = 1024, kRecRowWarps = 4;
-__global__ void __launch_bounds__(kRecRowWarps * 32, 7) k_scene_rec(PathJob* jobs, const SceneRun* runs, int nruns,
+__global__ void __launch_bounds__(kRecRowWarps * 32, 7) k_scene_rec(PathJob* jobs, const RecOrder* order, int njobs,
                                                                  long long totalItems, int rpi, Arena A) {
   extern __shared__ __align__(16) unsigned char rsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1053,28 +1053,30 @@ __global__ void __launch_bounds__(kRecRowWarps * 32, 7) k_scene_rec(PathJob* job
   pdl_wait();
   unsigned long long q = 0;
   if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue], 1ull);
+#pragma unroll 1
   while (true) {
     const long long item = (long long)__shfl_sync(0xffffffffu, q, 0);
     if (item >= totalItems) break;
     if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue], 1ull);
-    // items run by run, path by path, chunk of rpi rows by chunk: rec_off + (j - j0) * chunks + c
-    int r0 = 0, r1 = nruns - 1;
-    while (r0 < r1) {
-      int mid = (r0 + r1 + 1) >> 1;
-      if (runs[mid].rec_off <= item) r0 = mid;
-      else r1 = mid - 1;
+    // chunks of rpi rows, path by path in the launch's recording order
+    int lo = 0, hi = njobs - 1;
+#pragma unroll 1
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (order[mid].first <= item) lo = mid;
+      else hi = mid - 1;
     }
-    const long long local = item - runs[r0].rec_off, chunks = (runs[r0].H + rpi - 1) / rpi;
-    const int lo = runs[r0].j0 + (int)(local / chunks);
-    const PathJob& J = jobs[lo];
+    const int job = order[lo].job;
+    const PathJob& J = jobs[job];
     if (J.status != kOk) continue;
-    const long long yA = J.startY + (local % chunks) * rpi, yB = min(yA + rpi, J.pathHeight);
+    const int yA = (int)J.startY + (int)(item - order[lo].first) * rpi, yB = min(yA + rpi, (int)J.pathHeight);
     if (yA >= yB) continue;
     if (J.W >= fast_max_w(kRecNB)) {
-      for (long long y = yA; y < yB; y++) push_row(A, lo, (int)y, lane);
+#pragma unroll 1
+      for (int y = yA; y < yB; y++) push_row(A, job, y, lane);
       continue;
     }
-    fast_rows<kOutRec, kRecNB, kRecRowXT>(J, A, nullptr, lo, (int)yA, (int)yB, S, lane);
+    fast_rows<kOutRec, kRecNB, kRecRowXT>(J, A, nullptr, job, yA, yB, S, lane);
   }
 }
 
@@ -1368,9 +1370,9 @@ const void* scene_kernel(int ppl) {
   return ppl == 1 ? (const void*)k_scene<1, kSceneWarps> : (const void*)k_scene<4, kSceneWarps>;
 }
 int scene_warps() { return kSceneWarps; }
-void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
+void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const RecOrder* order, int njobs,
                       long long items, int rpi, const Arena& A) {
-  launch_pdl(k_scene_rec, dim3(blocks), dim3(kRecRowWarps * 32), scene_rec_smem(), st, jobs, runs, nruns, items, rpi,
+  launch_pdl(k_scene_rec, dim3(blocks), dim3(kRecRowWarps * 32), scene_rec_smem(), st, jobs, order, njobs, items, rpi,
              A);
 }
 void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, unsigned char* wide,

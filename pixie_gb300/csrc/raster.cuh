@@ -96,8 +96,15 @@ struct SceneRun {
   long long W, H;
   uint8_t* img;       // the canvas (RGBX)
   long long ri_base;  // row y, path j: Arena::rowhdr[ri_base + y * (j1 - j0) + j - j0]
-  long long rec_off;  // recording items of the run: rec_off + (j - j0) * ceil(H / rpi) + chunk
   int j0, j1;
+};
+
+// The recording pass takes a launch's paths from the heaviest to the lightest
+// (the pass lasts as long as its last rows): the k-th path's job and first work
+// item, a chunk of rows each.
+struct RecOrder {
+  long long first;
+  int job, pad;
 };
 
 // One mask of a batch drawn onto a page at an integer offset: page pixel (X,
