@@ -171,9 +171,9 @@ int pxg_stroke_config(int gpu_outline);
 int64_t pxg_stroke_fixups(void);
 
 /* Blur kernels: 3 (default) runs radii 1..8 on register-blocked CUDA-core
- * passes and radii 9..128 on the tensor cores with TMA-fed input rings in
- * tensor memory (images whose sides are multiples of 4; others take mode 1's
- * kernels); 1 runs radii 8..128 on the tensor cores with the warp-specialised
+ * passes and radii 9..128 on the tensor cores with input rings in tensor
+ * memory, as it does radii 6..8 of images large enough to be faster there
+ * (images with a side below 4 take mode 1's kernels); 1 runs radii 8..128 on the tensor cores with the warp-specialised
  * kernel that loads through registers; 2 uses the single-stage tensor-core
  * kernel (radii 8..128); 0 the tiled CUDA-core kernels (which every mode uses
  * for the radii it does not take).  All write the same bytes.  No
@@ -184,8 +184,9 @@ int pxg_blur_config(int use_tensor_cores);
  * mode 3 for radii 1..8, on images the library allocated whose device
  * address was never handed out: the result lands in the library's scratch
  * buffer and the two buffers change owners), 4 (the two small-radius passes
- * of mode 3, in place), 3 (the ring passes), 2, 1 or 0 as above (-1 before
- * any blur).  No counterpart in the reference. */
+ * of mode 3, in place), 3 (the ring passes, sides multiples of 4), 1 (the ring
+ * passes on other sizes, and mode 1's kernel), 2 or 0 as above (-1 before any
+ * blur).  No counterpart in the reference. */
 int pxg_last_blur_kernel(void);
 
 /* Converter trace of the ring blur passes, a profiling aid: enable != 0

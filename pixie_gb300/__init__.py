@@ -611,8 +611,8 @@ def stroke_fixups() -> int:
 
 
 def blur_config(mode):
-    """3 (default): tensor-core blur with TMA-fed input rings (radii 1..128,
-    rows a multiple of 16 bytes); 1: the pipelined tensor-core kernel that
+    """3 (default): tensor-core blur with input rings (radii 9..128, and 6..8
+    of large images; small radii on CUDA cores); 1: the pipelined tensor-core kernel that
     loads through registers (radii 8..128); 2: the single-stage tensor-core
     kernel (radii 8..128); 0: CUDA cores.  Radii or images a mode does not
     take run on the next family (3 -> 1 -> 0)."""

@@ -437,6 +437,21 @@ const uint16_t* weights_for(int64_t r) {
   return d;
 }
 
+// Whether a radius of 1..8 is worth the tensor-core passes.  The CUDA-core
+// kernel's time is its taps' (per pixel and radius), the tensor-core passes'
+// two trips over memory whatever the radius, plus 10 us before the pipeline
+// runs full.  Calls with the CUDA-core kernel / with the ring passes, 30 us of
+// each the call itself: 4096 x 4096 at radius 5 99.7 / 98.2 us, 6 112 / 98,
+// 8 141 / 98; 3000 x 3000 at 5 69.2 / 70.2, 6 75.4 / 68.9; 2048 x 2048 at 6
+// 51.5 / 53.5, 7 56.2 / 54.9; 1600 x 1200 at 8 44.0 / 44.8.  Without tensor
+// maps (rows not whole 16-byte units) the ring pays later: 4095 x 4095 at 6
+// 118 / 121, 7 137 / 121; 2401 x 2001 at 7 59.6 / 62.2, 8 65.1 / 62.4.
+bool ring_takes_small(const uint32_t* img, long long W, long long H, int64_t r) {
+  if (r > 8) return false;
+  const bool mapped = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
+  return mapped ? r >= 6 && r * W * H >= 29000000 : r >= 7 && r * W * H >= 38000000;
+}
+
 // Both blur passes of an RGBX image (img -> tmp -> img) with the configured
 // kernels; a kernel family that does not take this image or radius hands it
 // to the next one.  With swap_ok the caller owns both buffers and lets the
@@ -445,19 +460,28 @@ const uint16_t* weights_for(int64_t r) {
 // buffers.
 // tmp holds tmp_bytes: W * H * 4 at least; the tensor-core passes need
 // blur_scratch_bytes(W, H) (a padded intermediate) and are skipped below that.
+// g.last_blur tells the ring passes' images by their sides: 3 if both are
+// multiples of 4, else 1.
 bool blur_dispatch(uint32_t* img, uint32_t* tmp, long long tmp_bytes, long long W, long long H, int64_t r,
                    uint32_t oob, bool swap_ok = false) {
   const uint16_t* kern = weights_for(r);
+  const bool ring = g.blur_tensor == 3 && g.ring_ok && tmp_bytes >= blur_scratch_bytes(W, H);
+  if (ring && ring_takes_small(img, W, H, r) &&
+      launch_blur_ring(img, tmp, W, H, (int)r, kern, g.weights_f16[r], oob, g.nsm, g.ringSmemMax, g.dev_err,
+                       g.stream)) {
+    g.last_blur = ((W | H) & 3) == 0 ? 3 : 1;
+    return false;
+  }
   if (swap_ok && g.blur_tensor == 3 && launch_blur_small_fused(img, tmp, W, H, (int)r, kern, oob, g.stream)) {
     g.last_blur = 5;
     return true;
   }
   int used = -1;
   if (g.blur_tensor == 3 && launch_blur_small(img, tmp, W, H, (int)r, kern, oob, g.nsm, g.stream)) used = 4;
-  if (used < 0 && g.blur_tensor == 3 && g.ring_ok && tmp_bytes >= blur_scratch_bytes(W, H) &&
+  if (used < 0 && ring &&
       launch_blur_ring(img, tmp, W, H, (int)r, kern, g.weights_f16[r], oob, g.nsm, g.ringSmemMax, g.dev_err,
                        g.stream))
-    used = 3;
+    used = ((W | H) & 3) == 0 ? 3 : 1;
   if (used < 0 && g.blur_tensor == 2 &&
       launch_blur_tc(img, tmp, W, H, (int)r, kern, oob, g.nsm, g.tcSmemMax, g.dev_err, g.stream))
     used = 2;

@@ -1,5 +1,6 @@
-// Gaussian blur passes on the tensor cores: TMA-fed rows, the f16 input ring
-// in tensor memory, transposed outputs.
+// Gaussian blur passes on the tensor cores: rows fed by TMA (or, where the
+// image's rows are not whole 16-byte units, by 4-byte asynchronous copies),
+// the f16 input ring in tensor memory, transposed outputs.
 //
 // One pass of pixie's blur (images.nim:304-365) is, per channel,
 //   out[x] = (sum_t w[t] * p[x - r + t]) div 256 div 255,   t = 0 .. 2r,
@@ -169,13 +170,31 @@ __device__ __forceinline__ void mma_ts_elect(uint32_t tmem_d, uint32_t tmem_a, u
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// 4 bytes from global to shared memory, zeros where !live (nothing is read).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const uint32_t* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(live ? 4u : 0u) : "memory");
+}
+
+// How a pass reads and writes.  A tensor map wants rows of whole 16-byte
+// units.  The intermediate's rows always are (ring_tmp_pitch); the image's
+// are when its width is a multiple of 4.
+constexpr int kIoTma = 0;     // tensor-map loads and stores
+constexpr int kIoLoad4 = 1;   // pass 1 over an image with other rows: 4-byte cp.async, 64 a lane and chunk
+constexpr int kIoStore4 = 2;  // pass 2 back into one: the staged tile goes out with 128-byte warp stores
+// The copies cost issue slots that TMA does not, in warps that wait anyway.
+// Calls (30 us of each the call itself) on the kernel that loads through
+// registers / here: 1237 x 1001 at radius 12 60.2 / 45.2 us, at 100
+// 103 / 51.5; 4095 x 4095 at 12 230 / 120, at 100 762 / 142 (4096 x 4096 by
+// TMA: 98.6 and 125).
+
 // DELTA = (first input position of a chunk) mod 4 = (-r) mod 4, the pixel
 // offset of the chunk inside its 16-byte aligned box, fixed per radius: as a
-// template parameter the converters' word selection is straight-line code.
-template <bool SPLIT, int DELTA>
+// template parameter the converters' word selection is straight-line code
+// (kIoLoad4 stages a chunk from its first position: DELTA 0).
+template <bool SPLIT, int DELTA, int IO>
 __global__ void __launch_bounds__(kRingThreads, 1)
     k_blur_ring(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout, const RingArgs a,
-                const uint16_t* __restrict__ kern, int* err, int late) {
+                const uint16_t* __restrict__ kern, const uint32_t* img_in, uint32_t* img_out, int* err, int late) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~(uintptr_t)1023);
   constexpr int kAcc = SPLIT ? 2 : 4;
@@ -211,7 +230,7 @@ __global__ void __launch_bounds__(kRingThreads, 1)
   }
   if (tid == 0) {
     for (int b = 0; b < kMaxRaw; b++) {
-      mbar_init(rawFull + 8 * b, 1);
+      mbar_init(rawFull + 8 * b, IO == kIoLoad4 ? 32 : 1);
       mbar_init(rawEmpty + 8 * b, kConvWarps / 2);  // one lane of each converter warp of a group
     }
     for (int b = 0; b < kMaxRing; b++) {
@@ -224,8 +243,8 @@ __global__ void __launch_bounds__(kRingThreads, 1)
     }
     mbar_init(doneBar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    tmap_prefetch(&tin);
-    tmap_prefetch(&tout);
+    if (IO != kIoLoad4) tmap_prefetch(&tin);
+    if (IO != kIoStore4) tmap_prefetch(&tout);
   }
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(taddr_s)),
@@ -258,8 +277,26 @@ __global__ void __launch_bounds__(kRingThreads, 1)
           break;
         }
         const int p = s0 - r + kPos * c;  // first input position of the chunk
-        tma_load_2d_elect(base + L.raw + (uint32_t)(slot * a.rawStride), &tin, p - a.delta, kLines * band,
-                          rawFull + 8 * slot, (uint32_t)kRawBytes);
+        const uint32_t dst = base + L.raw + (uint32_t)(slot * a.rawStride);
+        if (IO == kIoLoad4) {
+          const int x = p + lane;
+          const bool in0 = x >= 0 && x < a.alen, in1 = x + 32 >= 0 && x + 32 < a.alen;
+          const uint32_t* src = img_in + (long long)(kLines * band) * a.alen + x;
+          const int lines = min(kLines, a.clen - kLines * band);
+#pragma unroll 8
+          for (int j = 0; j < kLines; j++) {
+            // what is not read names the image's first pixel
+            const bool l0 = in0 && j < lines, l1 = in1 && j < lines;
+            const uint32_t d = dst + (uint32_t)(j * (kRawW * 4) + 4 * lane);
+            cp_async4(d, l0 ? src : img_in, l0);
+            cp_async4(d + 128, l1 ? src + 32 : img_in, l1);
+            src += a.alen;
+          }
+          // this lane's arrival, once its copies have landed
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(rawFull + 8 * slot) : "memory");
+        } else {
+          tma_load_2d_elect(dst, &tin, p - a.delta, kLines * band, rawFull + 8 * slot, (uint32_t)kRawBytes);
+        }
         issued++;
         if (++slot == a.nraw) {
           slot = 0;
@@ -454,7 +491,7 @@ __global__ void __launch_bounds__(kRingThreads, 1)
         if (!ready && lane == 0) atomicExch(err, 1);
         // the staging buffer of this tile was last read by the store two of
         // the group's tiles back
-        if (issuer) bulk_wait_read<1>();
+        if (IO != kIoStore4 && issuer) bulk_wait_read<1>();
         if (epi_bar_or(e, !ready)) {
           ok = false;
           break;
@@ -493,15 +530,32 @@ __global__ void __launch_bounds__(kRingThreads, 1)
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(tEmpty + 8 * cacc);
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        if (IO != kIoStore4) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         epi_bar(e);
-        if (issuer) {
+        if (IO == kIoStore4) {
+          // 32 lines of a position are 128 contiguous bytes; a warp takes every
+          // fourth position (the buffer's next writer comes two barriers later)
+          const int n = min(kPos, a.alen - o0), line = kLines * band + lane;
+          const uint32_t src = stage + ((uint32_t)(lane & 3) << 2);
+          uint32_t* dst = img_out + (long long)(o0 + q) * a.opitch + line;
+          if (line < a.clen) {
+#pragma unroll 4
+            for (int row = q; row < n; row += 4) {
+              uint32_t v;
+              asm volatile("ld.shared.u32 %0, [%1];\n"
+                           : "=r"(v)
+                           : "r"(src + (uint32_t)row * 128u + (((uint32_t)(lane >> 2) ^ ((uint32_t)row & 7u)) << 4)));
+              *dst = v;
+              dst += 4ll * a.opitch;
+            }
+          }
+        } else if (issuer) {
           tma_store_2d(&tout, kLines * band, o0, stage);
           bulk_commit();
         }
       }
     }
-    if (issuer) bulk_wait_all();  // the stores have read shared memory and reached global memory
+    if (IO != kIoStore4 && issuer) bulk_wait_all();  // the stores have read shared memory and reached global memory
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
@@ -573,17 +627,30 @@ bool plan_pass(RingArgs& a, int alen, int clen, int r, int nsm, size_t maxSmem, 
   return true;
 }
 
-template <bool SPLIT>
-void launch_ring_pass(const RingArgs& a, int grid, const CUtensorMap& tin, const CUtensorMap& tout,
-                      const uint16_t* kern, int* err, int late, cudaStream_t st) {
-  // at least 120 KB, so that no second CTA (and tensor-memory allocation) shares an SM
-  const size_t smem = std::max<size_t>(ring_smem(a, SPLIT).total + 1024, 120 * 1024);
-  switch (a.delta) {
-    case 0: launch_pdl(k_blur_ring<SPLIT, 0>, dim3(grid), dim3(kRingThreads), smem, st, tin, tout, a, kern, err, late); break;
-    case 1: launch_pdl(k_blur_ring<SPLIT, 1>, dim3(grid), dim3(kRingThreads), smem, st, tin, tout, a, kern, err, late); break;
-    case 2: launch_pdl(k_blur_ring<SPLIT, 2>, dim3(grid), dim3(kRingThreads), smem, st, tin, tout, a, kern, err, late); break;
-    default: launch_pdl(k_blur_ring<SPLIT, 3>, dim3(grid), dim3(kRingThreads), smem, st, tin, tout, a, kern, err, late); break;
+typedef void (*RingKernel)(CUtensorMap, CUtensorMap, RingArgs, const uint16_t*, const uint32_t*, uint32_t*, int*, int);
+template <bool SPLIT, int IO>
+RingKernel ring_kernel_io(int delta) {
+  if (IO == kIoLoad4) return k_blur_ring<SPLIT, 0, kIoLoad4>;
+  constexpr int io = IO == kIoLoad4 ? kIoTma : IO;
+  switch (delta) {
+    case 0: return k_blur_ring<SPLIT, 0, io>;
+    case 1: return k_blur_ring<SPLIT, 1, io>;
+    case 2: return k_blur_ring<SPLIT, 2, io>;
+    default: return k_blur_ring<SPLIT, 3, io>;
   }
+}
+template <bool SPLIT>
+RingKernel ring_kernel(int io, int delta) {
+  return io == kIoTma ? ring_kernel_io<SPLIT, kIoTma>(delta)
+                      : io == kIoLoad4 ? ring_kernel_io<SPLIT, kIoLoad4>(delta) : ring_kernel_io<SPLIT, kIoStore4>(delta);
+}
+
+void launch_ring_pass(const RingArgs& a, bool split, int io, int grid, const CUtensorMap& tin, const CUtensorMap& tout,
+                      const uint16_t* kern, const uint32_t* in, uint32_t* out, int* err, int late, cudaStream_t st) {
+  // at least 120 KB, so that no second CTA (and tensor-memory allocation) shares an SM
+  const size_t smem = std::max<size_t>(ring_smem(a, split).total + 1024, 120 * 1024);
+  launch_pdl(split ? ring_kernel<true>(io, a.delta) : ring_kernel<false>(io, a.delta), dim3(grid), dim3(kRingThreads),
+             smem, st, tin, tout, a, kern, in, out, err, late);
   note_launch();
 }
 
@@ -617,41 +684,48 @@ bool ring_blur_init(size_t* maxSmem) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const void* ks[8] = {(const void*)k_blur_ring<true, 0>,  (const void*)k_blur_ring<true, 1>,
-                       (const void*)k_blur_ring<true, 2>,  (const void*)k_blur_ring<true, 3>,
-                       (const void*)k_blur_ring<false, 0>, (const void*)k_blur_ring<false, 1>,
-                       (const void*)k_blur_ring<false, 2>, (const void*)k_blur_ring<false, 3>};
-  for (const void* k : ks)
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
+  for (int io = 0; io < 3; io++)
+    for (int d = 0; d < 4; d++)
+      for (int split = 0; split < 2; split++) {
+        const RingKernel k = split ? ring_kernel<true>(io, d) : ring_kernel<false>(io, d);
+        if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) {
+          cudaGetLastError();
+          return false;
+        }
+      }
   *maxSmem = (size_t)optin;
   return true;
 }
 
 // Row pitch (pixels) of the transposed intermediate of a blur of an image H
-// pixels high: H, or H + 4 when H * 4 bytes is a multiple of 1 KB.  Pass 1
-// writes four intermediate rows per warp store and its loads and pass 2's
-// read 32 rows per box; at a pitch of a multiple of 1 KB (4096-pixel rows:
-// 16 KB) those rows fall on the same memory channels and a 4096 x 4096 blur
-// ran 25 % slower than a 4096 x 4100 one.  16 more bytes per row spread them.
-long long ring_tmp_pitch(long long H) { return (H * 4) % 1024 == 0 ? H + 4 : H; }
+// pixels high: H rounded up to whole 16-byte units, and 4 more when that is a
+// multiple of 1 KB.  Pass 1 writes four intermediate rows per warp store and
+// its loads and pass 2's read 32 rows per box; at a pitch of a multiple of
+// 1 KB (4096-pixel rows: 16 KB) those rows fall on the same memory channels
+// and a 4096 x 4096 blur ran 25 % slower than a 4096 x 4100 one.  16 more
+// bytes per row spread them.
+long long ring_tmp_pitch(long long H) {
+  const long long p = (H + 3) / 4 * 4;
+  return (p * 4) % 1024 == 0 ? p + 4 : p;
+}
 
 // Bytes of the intermediate buffer a blur of W x H pixels needs.
 long long blur_scratch_bytes(long long W, long long H) { return W * ring_tmp_pitch(H) * 4; }
 
 // Both passes (img -> tmp transposed -> img) on the ring kernels.  Returns
 // false (and launches nothing) when the image or radius is not for this path:
-// width and height must be multiples of 4 (TMA rows of whole 16-byte units
-// in both orientations) and both buffers 16-byte aligned, r in 1..128.  tmp
-// holds blur_scratch_bytes(W, H) bytes (W rows of ring_tmp_pitch(H) pixels).
+// r in 1..128, sides of 4 to 2^24, tmp 16-byte aligned.  An image whose rows
+// are not whole 16-byte units, or whose base is not at one, is read and
+// written by plain copies (kIoLoad4, kIoStore4); the intermediate always goes
+// by tensor maps, whose width takes the rows' padding in: pixels there hold
+// what pass 1 made of lines past the image, and pass 2 replaces them with the
+// outOfBounds colour as it does every position past the row.  tmp holds
+// blur_scratch_bytes(W, H) bytes (W rows of ring_tmp_pitch(H) pixels).
 bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, int r, const uint16_t* kern,
                       bool exactF16, uint32_t oob, int nsm, size_t maxSmem, int* err, cudaStream_t st) {
-  if (!g_encode || r < 1 || r > 128 || W < 4 || H < 4 || (W & 3) != 0 || (H & 3) != 0 || W > (1 << 24) ||
-      H > (1 << 24))
-    return false;
-  if ((reinterpret_cast<uintptr_t>(img) & 15) || (reinterpret_cast<uintptr_t>(tmp) & 15)) return false;
+  if (!g_encode || r < 1 || r > 128 || W < 4 || H < 4 || W > (1 << 24) || H > (1 << 24)) return false;
+  if (reinterpret_cast<uintptr_t>(tmp) & 15) return false;
+  const bool mapped = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
   // plans and tensor maps of the last few (buffers, size, radius, colour)
   // keys, so a repeated blur costs its two launches on the host (callers
   // hold the library lock)
@@ -663,8 +737,8 @@ bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, in
     bool split;
     RingArgs a1, a2;
     int g1, g2;
-    CUtensorMap m1, m2;    // pass inputs: image rows, intermediate rows
-    CUtensorMap o1, o2;    // pass outputs: intermediate, image (boxes of 32 lines x 64 positions)
+    CUtensorMap m1, m2;    // pass inputs: image rows (if mapped), intermediate rows
+    CUtensorMap o1, o2;    // pass outputs: intermediate, image (if mapped; boxes of 32 lines x 64 positions)
   };
   static Plan cache[8];
   static int ncache = 0, next = 0;
@@ -693,10 +767,13 @@ bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, in
       return false;
     n.a1.oob = n.a2.oob = oob;
     n.a1.opitch = (int)ring_tmp_pitch(H);  // pass 1 writes the intermediate
-    if (!encode_map(&n.m1, img, (int)W, (int)H, W, kRawW, kLines) ||
-        !encode_map(&n.m2, tmp, (int)H, (int)W, ring_tmp_pitch(H), kRawW, kLines) ||
-        !encode_map(&n.o1, tmp, (int)H, (int)W, ring_tmp_pitch(H), kLines, kPos, true) ||
-        !encode_map(&n.o2, img, (int)W, (int)H, W, kLines, kPos, true))
+    if (!mapped) n.a1.delta = 0;
+    const int Hp = (int)((H + 3) / 4 * 4);
+    if (!encode_map(&n.m2, tmp, Hp, (int)W, ring_tmp_pitch(H), kRawW, kLines) ||
+        !encode_map(&n.o1, tmp, Hp, (int)W, ring_tmp_pitch(H), kLines, kPos, true))
+      return false;
+    if (mapped && (!encode_map(&n.m1, img, (int)W, (int)H, W, kRawW, kLines) ||
+                   !encode_map(&n.o2, img, (int)W, (int)H, W, kLines, kPos, true)))
       return false;
     cache[next] = n;
     pl = &cache[next];
@@ -705,15 +782,11 @@ bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, in
   }
   const Span im{img, (size_t)(W * H * 4)}, tm{tmp, (size_t)blur_scratch_bytes(W, H)};
   const int late1 = dep_late(st, {tm}, {im});  // pass 1: image rows -> intermediate
-  if (split)
-    launch_ring_pass<true>(pl->a1, pl->g1, pl->m1, pl->o1, kern, err, late1, st);
-  else
-    launch_ring_pass<false>(pl->a1, pl->g1, pl->m1, pl->o1, kern, err, late1, st);
+  launch_ring_pass(pl->a1, split, mapped ? kIoTma : kIoLoad4, pl->g1, pl->m1, pl->o1, kern, img, nullptr, err, late1,
+                   st);
   const int late2 = dep_late(st, {im}, {tm});  // pass 2 (always waits: it reads pass 1's output)
-  if (split)
-    launch_ring_pass<true>(pl->a2, pl->g2, pl->m2, pl->o2, kern, err, late2, st);
-  else
-    launch_ring_pass<false>(pl->a2, pl->g2, pl->m2, pl->o2, kern, err, late2, st);
+  launch_ring_pass(pl->a2, split, mapped ? kIoTma : kIoStore4, pl->g2, pl->m2, pl->o2, kern, nullptr, img, err, late2,
+                   st);
   return true;
 }
 
