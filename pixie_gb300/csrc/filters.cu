@@ -8,6 +8,8 @@
 // shared memory and run one output pixel per thread.
 // shadow: MaskBlend reads only the mask's alpha and spread writes
 // rgbx(0,0,0,v), so the whole shadow runs on one uint8 alpha plane.
+#include <algorithm>
+
 #include "pxg_device.cuh"
 
 namespace pxg {
@@ -462,7 +464,7 @@ void launch_spread(uint32_t* img, uint8_t* a0, uint8_t* a1, long long W, long lo
   k_alpha_to_rgbx<<<grid_for(n, nsm), 256, 0, st>>>(a0, img, n); note_launch();
 }
 
-// shadow in one pass over 64 x 64 output tiles: the tile and a halo of
+// Shadow in one pass over tiles of 64 columns and th rows: the tile and a halo of
 // |spread| + radius (at most kShadowHalo) of the offset alpha plane are staged
 // in shared memory and the reference's stages run there in order -- spread
 // along x then y (a running max or min over the window clipped to the image:
@@ -470,140 +472,238 @@ void launch_spread(uint32_t* img, uint8_t* a0, uint8_t* a1, long long W, long lo
 // (taps outside the image read 0; integer sums and v div 256 div 255 as the
 // blur passes), then colour * alpha / 255 (the MaskBlend draw of the filled
 // result) written once.
-// The blur radius R is a template parameter (0..kShadowHalo): the taps unroll
-// and each thread forms four neighbouring outputs from one window of inputs.
-constexpr int kShadowTile = 64, kShadowHalo = 32;
-template <int R>
-__global__ void __launch_bounds__(1024) k_shadow_tile(const uint32_t* __restrict__ src, uint32_t* __restrict__ out,
-                                                     int W, int H, int ox, int oy, int m, int grow,
-                                                     const uint16_t* __restrict__ kern, uint32_t color, int late) {
-  constexpr int r = R;
+//
+// What bounds it is instructions: at 1237 x 1001, spread 4 and radius 12 a
+// byte at a time took 31 us of which the image's bytes are 1.5.  So four
+// neighbours are handled at once.  A shrink is a grow of the complement.  A
+// window's four results share its middle.  A blur's are dot products of 16-bit
+// weight pairs with byte pairs of the staged words (dp2a: two taps an
+// instruction, exact), the weights of the four shifts read from one table of
+// pairs (w[d], w[d + 1]); along y the same code runs on a transposed copy.
+// Rows and columns of words have odd pitches, so lanes down a column fall on
+// different banks.  At 1237 x 1001 (spread, radius): (4, 12) 29.7 -> 14.5 us,
+// (0, 12) 18.3 -> 11.1, (4, 0) 15.6 -> 9.4, (0, 4) 13.3 -> 9.0, (0, 32) 37 ->
+// 20.7, (16, 16) 59 -> 24.6.  Three CTAs an SM: at the 56 registers the
+// compiler would take only two fit, and one tile in twenty runs a second wave.
+//
+// 4 Q is the radius rounded up to whole words: what a window's words reach
+// beyond it meets zero weights.
+constexpr int kShadowTile = 64, kShadowHalo = 32, kShadowThreads = 512, kShadowMaxRows = 96;
+struct ShadowDims {  // in shared memory: two byte planes, the weight pairs, the colours by alpha
+  int rows, hx, pitch;  // staged rows, columns left of the tile, words from row to row
+};
+__host__ __device__ inline ShadowDims shadow_dims(int th, int m, int r) {
+  ShadowDims d;
+  d.rows = th + 2 * (m + r);
+  d.hx = (m + 3) / 4 * 4 + (r + 3) / 4 * 4;
+  d.pitch = ((kShadowTile + 2 * d.hx) / 4) | 1;
+  return d;
+}
+// The second plane also takes the transposed columns (64 of th + 8 ceil(r / 4)
+// bytes and a word).
+__host__ __device__ inline int shadow_col_words(int th, int r) { return (th / 4 + 2 * ((r + 3) / 4)) | 1; }
+size_t shadow_tile_smem(int th, int m, int r) {
+  const ShadowDims d = shadow_dims(th, m, r);
+  return (size_t)(2 * ((r + 3) / 4) + 1) * 16 + 256 * 4 + (size_t)d.rows * d.pitch * 4 +
+         std::max((size_t)d.rows * d.pitch, (size_t)kShadowTile * shadow_col_words(th, r)) * 4;
+}
+// Rows of a tile, a multiple of 4: what the busiest SM does (its tiles, their
+// rows and halo, 24 rows' worth before the first) is least.  With 64 rows
+// always, 1237 x 1001 at (4, 12) is three tiles on the busiest of 152 SMs and
+// 17.9 us, at 68 two and 14.5; (0, 32) 24.1 and 20.7.
+int shadow_tile_rows(long long W, long long H, int m, int r, int nsm) {
+  const long long cols = (W + kShadowTile - 1) / kShadowTile;
+  long long best = 0;
+  int th = 64;
+  for (int t = kShadowMaxRows; t >= 16; t -= 4) {
+    const long long tiles = cols * ((H + t - 1) / t), cost = (tiles + nsm - 1) / nsm * (t + 2 * (m + r) + 24);
+    if (best == 0 || cost < best) {
+      best = cost;
+      th = t;
+    }
+  }
+  return th;
+}
+
+// Four outputs' weighted sums over the words p[0 .. 2 Q]: output o takes the
+// bytes from 4 Q - r + o on.  wq[k] holds the weight pairs at d - 1 .. d + 2
+// with d = 4 k - (4 Q - r); those at d - 3 and d - 2 are the word before's.
+template <int Q>
+__device__ __forceinline__ void dot_words(const uint32_t* p, const uint4* wq, uint32_t (&a)[4]) {
+  uint32_t p1 = 0, p2 = 0;
+  a[0] = a[1] = a[2] = a[3] = 0;
+#pragma unroll(Q <= 2 ? 2 * Q + 1 : 3)
+  for (int k = 0; k <= 2 * Q; k++) {
+    const uint32_t v = p[k];
+    const uint4 t = wq[k];
+    a[0] = __dp2a_hi(t.w, v, __dp2a_lo(t.y, v, a[0]));
+    a[1] = __dp2a_hi(t.z, v, __dp2a_lo(t.x, v, a[1]));
+    a[2] = __dp2a_hi(t.y, v, __dp2a_lo(p2, v, a[2]));
+    a[3] = __dp2a_hi(t.x, v, __dp2a_lo(p1, v, a[3]));
+    p1 = t.z;
+    p2 = t.w;
+  }
+}
+// floor(floor(a / 256) / 255) for a < 2^24
+__device__ __forceinline__ uint32_t quot_65280(uint32_t a) { return ((a >> 8) * 0x8081u) >> 23; }
+
+template <int Q>
+__global__ void __launch_bounds__(kShadowThreads, 3) k_shadow_tile(const uint32_t* __restrict__ src,
+                                                                uint32_t* __restrict__ out, int W, int H, int ox,
+                                                                int oy, int th, int m, int r, int grow,
+                                                                const uint16_t* __restrict__ kern, uint32_t color,
+                                                                int late) {
   extern __shared__ __align__(16) unsigned char sh[];
-  const int h = m + r, S = kShadowTile + 2 * h;  // staged side
-  unsigned char* b0 = sh;
-  unsigned char* b1 = sh + S * S;
-  uint32_t* wk = reinterpret_cast<uint32_t*>(sh + ((2 * S * S + 15) & ~15));
-  const int gx0 = blockIdx.x * kShadowTile - h, gy0 = blockIdx.y * kShadowTile - h;  // staged [0][0]
-  const int tid = threadIdx.x, T = blockDim.x;
+  constexpr int kWarps = kShadowThreads / 32, kCols = kShadowTile / 4 + 2 * Q;  // word columns the blur reads
+  const ShadowDims D = shadow_dims(th, m, r);
+  const int S = D.rows, P = 4 * D.pitch, h = m + r;
+  uint4* wq = reinterpret_cast<uint4*>(sh);
+  uint32_t* lut = reinterpret_cast<uint32_t*>(wq + 2 * Q + 1);
+  unsigned char* b0 = reinterpret_cast<unsigned char*>(lut + 256);
+  unsigned char* b1 = b0 + S * P;
+  const int gx0 = blockIdx.x * kShadowTile - D.hx, gy0 = blockIdx.y * th - h;  // staged [0][0]
+  const int tid = threadIdx.x, wi = tid >> 5, ln = tid & 31;
   pdl_late_entry(late);
-  if (r > 0)  // without a blur there is no weight table
-    for (int k = tid; k <= 2 * r; k += T) wk[k] = kern[k];
-  const unsigned char neutral = (m > 0 && !grow) ? 255 : 0;
-  auto inside = [&](int i, int j) {
-    const int gx = gx0 + j, gy = gy0 + i;
-    return gx >= 0 && gx < W && gy >= 0 && gy < H;
-  };
-  // each warp takes rows, its lanes consecutive columns (no divisions by S)
-  const int nw = T >> 5, wi = tid >> 5, ln = tid & 31;
-  // the offset alpha plane (k_alpha_offset), neutral outside the image
-  for (int i = wi; i < S; i += nw)
-    for (int j = ln; j < S; j += 32) {
-      const int gx = gx0 + j, gy = gy0 + i;
-      unsigned char v = neutral;
-      if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-        const int sx = gx - ox, sy = gy - oy;
-        v = (sx >= 0 && sx < W && sy >= 0 && sy < H) ? (unsigned char)(src[(long long)sy * W + sx] >> 24) : 0;
+  if (Q > 0 && tid < 4 * (2 * Q + 1)) {
+    const int d = 4 * (tid >> 2) - (4 * Q - r) - 1 + (tid & 3);
+    const uint32_t w0 = d >= 0 && d <= 2 * r ? kern[d] : 0u, w1 = d + 1 >= 0 && d + 1 <= 2 * r ? kern[d + 1] : 0u;
+    reinterpret_cast<uint32_t*>(wq)[tid] = w0 | (w1 << 16);
+  }
+  if (tid < 256) lut[tid] = mul_div255_px(color, (uint32_t)tid);
+  const uint32_t flip = (m > 0 && !grow) ? 255u : 0u;
+  // the offset alpha plane (k_alpha_offset), complemented for a shrink; 0
+  // (neutral) outside the image.  A warp's rows are loaded eight at a time.
+  const int in0 = max(0, -gy0), inN = max(0, min(S, H - gy0) - in0);  // staged rows in the image
+  const int so0 = max(in0, oy - gy0), soN = max(0, min(in0 + inN, H + oy - gy0) - so0);  // those with a source row
+  const bool whole = gx0 >= max(0, ox) && gx0 + kShadowTile + 2 * D.hx <= min(W, W + ox) && soN == S;
+  for (int j = ln; j < kShadowTile + 2 * D.hx; j += 32) {
+    const int gx = gx0 + j, sx = gx - ox;
+    const bool inx = gx >= 0 && gx < W;
+    const unsigned n = inx ? (unsigned)inN : 0u, nsrc = inx && sx >= 0 && sx < W ? (unsigned)soN : 0u;
+    for (int i0 = wi; i0 < S; i0 += 8 * kWarps) {
+      // the alpha bytes (only read where they lie in the image)
+      const unsigned char* p = reinterpret_cast<const unsigned char*>(src + (long long)(gy0 + i0 - oy) * W + sx) + 3;
+      const long long step = (long long)kWarps * W * 4;
+      uint32_t v[8];
+      if (whole) {
+#pragma unroll
+        for (int k = 0; k < 8; k++, p += step)
+          if (i0 + k * kWarps < S) v[k] = *p;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (i0 + k * kWarps < S) b0[(i0 + k * kWarps) * P + j] = (unsigned char)(v[k] ^ flip);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++, p += step) v[k] = (unsigned)(i0 + k * kWarps - so0) < nsrc ? *p : 0u;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int i = i0 + k * kWarps;
+          if (i < S) b0[i * P + j] = (unsigned)(i - in0) < n ? (unsigned char)(v[k] ^ flip) : 0;
+        }
       }
-      b0[i * S + j] = v;
     }
+  }
   __syncthreads();
-  if (m > 0) {  // spread along x into b1, then along y back into b0 (rows and columns [m, S - m))
-    for (int i = wi; i < S; i += nw)
-      for (int j = m + ln; j < S - m; j += 32) {
-        const unsigned char* p = b0 + i * S + j - m;
-        uint32_t v = neutral;
-        if (grow)
-          for (int t = 0; t <= 2 * m; t++) v = max(v, (uint32_t)p[t]);
-        else
-          for (int t = 0; t <= 2 * m; t++) v = min(v, (uint32_t)p[t]);
-        b1[i * S + j] = (unsigned char)v;
-      }
-    __syncthreads();
-    for (int i = m + wi; i < S - m; i += nw)
-      for (int j = m + ln; j < S - m; j += 32) {
-        const unsigned char* p = b1 + (i - m) * S + j;
-        uint32_t v = neutral;
-        if (grow)
-          for (int t = 0; t <= 2 * m; t++) v = max(v, (uint32_t)p[t * S]);
-        else
-          for (int t = 0; t <= 2 * m; t++) v = min(v, (uint32_t)p[t * S]);
-        b0[i * S + j] = inside(i, j) ? (unsigned char)v : 0;  // blur taps outside the image read 0
-      }
-    __syncthreads();
-  } else if (neutral != 0) {
-    for (int i = wi; i < S; i += nw)
-      for (int j = ln; j < S; j += 32)
-        if (!inside(i, j)) b0[i * S + j] = 0;
-    __syncthreads();
-  }
-  const unsigned char* fin = b0;  // final alpha at [h + y][h + x]
-  if (r > 0) {
-    // blur along x: rows [m, S - m), the tile's columns, into b1 (0 outside the
-    // image); a task is four neighbouring outputs of a row
-    constexpr int NT = 2 * R + 4;
-    for (int task = tid; task < (S - 2 * m) * (kShadowTile / 4); task += T) {
-      const int i = m + task / (kShadowTile / 4), j = h + 4 * (task % (kShadowTile / 4));
-      const unsigned char* p = b0 + i * S + j - r;
-      uint32_t a[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int t = 0; t < NT; t++) {
-        const uint32_t v = p[t];
-#pragma unroll
-        for (int o = 0; o < 4; o++)
-          if (t - o >= 0 && t - o <= 2 * R) a[o] += v * wk[t - o];
-      }
-#pragma unroll
-      for (int o = 0; o < 4; o++) b1[i * S + j + o] = inside(i, j + o) ? (unsigned char)(a[o] / 256 / 255) : 0;
+  if (m > 0) {
+    // spread along x into b1 and along y back into b0 (rows [m, S - m)), the
+    // word columns that the blur reads; of a window's 2 m + 4 inputs for four
+    // outputs the middle ones are in all
+    const int wc0 = (m + 3) / 4;
+    for (int task = tid; task < S * kCols; task += kShadowThreads) {
+      const int i = task / kCols, wc = wc0 + task - i * kCols;
+      const unsigned char* p = b0 + i * P + 4 * wc - m;
+      uint32_t c = 0;
+      for (int t = 3; t <= 2 * m; t++) c = max(c, (uint32_t)p[t]);
+      const uint32_t l0 = p[0], l1 = p[1], l2 = p[2], e1 = p[2 * m + 1], e2 = p[2 * m + 2], e3 = p[2 * m + 3];
+      const uint32_t l12 = max(l1, l2), e12 = max(e1, e2);
+      const uint32_t o0 = max(max(l0, l12), c), o1 = max(max(l12, c), e1), o2 = max(max(l2, c), e12),
+                     o3 = max(max(c, e12), e3);
+      reinterpret_cast<uint32_t*>(b1 + i * P)[wc] = o0 | (o1 << 8) | (o2 << 16) | (o3 << 24);
     }
     __syncthreads();
-    // blur along y: the tile, into b0; a task is four neighbouring outputs of a column
-    for (int task = tid; task < kShadowTile * (kShadowTile / 4); task += T) {
-      const int j = h + task % kShadowTile, i = h + 4 * (task / kShadowTile);
-      const unsigned char* p = b1 + (i - r) * S + j;
-      uint32_t a[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int t = 0; t < NT; t++) {
-        const uint32_t v = p[t * S];
-#pragma unroll
-        for (int o = 0; o < 4; o++)
-          if (t - o >= 0 && t - o <= 2 * R) a[o] += v * wk[t - o];
+    const int rows = S - 2 * m;
+    for (int task = tid; task < (rows + 3) / 4 * kCols; task += kShadowThreads) {
+      const int rg = task / kCols, wc = wc0 + task - rg * kCols;
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(b1) + wc;
+      const auto even = [&](int i) { return p[min(i, S - 1) * D.pitch] & 0x00FF00FFu; };
+      const auto odd = [&](int i) { return (p[min(i, S - 1) * D.pitch] >> 8) & 0x00FF00FFu; };
+      uint32_t ce = 0, co = 0;
+      for (int t = 4 * rg + 3; t <= 4 * rg + 2 * m; t++) {
+        const uint32_t v = p[t * D.pitch];
+        ce = __vmaxu2(ce, v & 0x00FF00FFu);
+        co = __vmaxu2(co, (v >> 8) & 0x00FF00FFu);
       }
+      uint32_t res[4];
+      const auto four = [&](auto get, uint32_t c, int s) {
+        const int i = 4 * rg, e = i + 2 * m;
+        const uint32_t l0 = get(i), l1 = get(i + 1), l2 = get(i + 2), e1 = get(e + 1), e2 = get(e + 2), e3 = get(e + 3);
+        const uint32_t l12 = __vmaxu2(l1, l2), e12 = __vmaxu2(e1, e2);
+        const uint32_t o[4] = {__vmaxu2(__vmaxu2(l0, l12), c), __vmaxu2(__vmaxu2(l12, c), e1),
+                               __vmaxu2(__vmaxu2(l2, c), e12), __vmaxu2(__vmaxu2(c, e12), e3)};
 #pragma unroll
-      for (int o = 0; o < 4; o++) b0[(i + o) * S + j] = (unsigned char)(a[o] / 256 / 255);
+        for (int k = 0; k < 4; k++) res[k] = s ? res[k] | (o[k] << 8) : o[k];
+      };
+      four(even, ce, 0);
+      four(odd, co, 1);
+      uint32_t in = 0;  // blur taps outside the image read 0
+#pragma unroll
+      for (int k = 0; k < 4; k++) in |= gx0 + 4 * wc + k >= 0 && gx0 + 4 * wc + k < W ? 255u << (8 * k) : 0u;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int i = m + 4 * rg + k, gy = gy0 + i;
+        if (i < S - m)
+          reinterpret_cast<uint32_t*>(b0)[i * D.pitch + wc] =
+              gy >= 0 && gy < H ? (res[k] ^ (flip * 0x01010101u)) & in : 0u;
+      }
     }
     __syncthreads();
   }
-  const Px c = unpack(color);
-  for (int idx = tid; idx < kShadowTile * kShadowTile; idx += T) {
-    const int y = idx / kShadowTile, x = idx % kShadowTile;
-    const int gx = gx0 + h + x, gy = gy0 + h + y;
-    if (gx >= W || gy >= H) continue;
-    const uint32_t k = fin[(h + y) * S + h + x];
-    out[(long long)gy * W + gx] = pack((c.r * k) / 255, (c.g * k) / 255, (c.b * k) / 255, (c.a * k) / 255);
+  const int bx = blockIdx.x * kShadowTile, by = blockIdx.y * th;
+  if (Q > 0) {
+    // blur along x: rows [m, S - m), the tile's columns, transposed into b1
+    // (column c's bytes from 4 Q - r on; 0 outside the image).  A warp takes a
+    // word column, its lanes the rows.
+    const int tp = shadow_col_words(th, r);  // words from column to column (odd)
+    static_assert(kWarps == kShadowTile / 4, "one warp for each word column");
+    for (int t = ln; t < S - 2 * m; t += 32) {
+      uint32_t a[4];
+      dot_words<Q>(reinterpret_cast<const uint32_t*>(b0) + (m + t) * D.pitch + D.hx / 4 - Q + wi, wq, a);
+      const int gy = gy0 + m + t;
+      const bool in = gy >= 0 && gy < H;
+#pragma unroll
+      for (int o = 0; o < 4; o++)
+        b1[(4 * wi + o) * 4 * tp + t + 4 * Q - r] = in ? (unsigned char)quot_65280(a[o]) : 0;
+    }
+    __syncthreads();
+    // blur along y: lanes take columns, four rows each
+    const int c = ln + 32 * (wi & 1);
+    if (bx + c < W) {
+#pragma unroll 1
+      for (int yg = wi >> 1; yg < th / 4; yg += kWarps / 2) {
+        uint32_t a[4];
+        dot_words<Q>(reinterpret_cast<const uint32_t*>(b1) + c * tp + yg, wq, a);
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          const int gy = by + 4 * yg + o;
+          if (gy < H) out[(long long)gy * W + bx + c] = lut[quot_65280(a[o]) & 255u];
+        }
+      }
+    }
+  } else {
+    for (int idx = tid; idx < th * kShadowTile; idx += kShadowThreads) {
+      const int y = idx / kShadowTile, x = idx % kShadowTile;
+      if (bx + x < W && by + y < H) out[(long long)(by + y) * W + bx + x] = lut[b0[(h + y) * P + D.hx + x]];
+    }
   }
   pdl_late_exit(late);
 }
-typedef void (*ShadowTileKernel)(const uint32_t*, uint32_t*, int, int, int, int, int, int, const uint16_t*, uint32_t,
-                                 int);
-template <int R>
-struct ShadowTable {
-  static void fill(ShadowTileKernel* t) {
-    t[R] = k_shadow_tile<R>;
-    ShadowTable<R + 1>::fill(t);
-  }
-};
-template <>
-struct ShadowTable<kShadowHalo + 1> {
-  static void fill(ShadowTileKernel*) {}
-};
+typedef void (*ShadowTileKernel)(const uint32_t*, uint32_t*, int, int, int, int, int, int, int, int, const uint16_t*,
+                                 uint32_t, int);
+template <int Q>
 ShadowTileKernel shadow_tile_kernel(int r) {
-  static ShadowTileKernel table[kShadowHalo + 1] = {nullptr};
-  if (!table[0]) ShadowTable<0>::fill(table);
-  return table[r];
-}
-size_t shadow_tile_smem(int h) {
-  const int S = kShadowTile + 2 * h;
-  return (size_t)((2 * S * S + 15) & ~15) + (size_t)(2 * kShadowHalo + 1) * 4;
+  if constexpr (Q < kShadowHalo / 4)
+    if (r > 4 * Q) return shadow_tile_kernel<Q + 1>(r);
+  return k_shadow_tile<Q>;
 }
 
 void launch_shadow(const uint32_t* src, uint32_t* out, uint8_t* a0, uint8_t* a1, long long W,
@@ -613,10 +713,11 @@ void launch_shadow(const uint32_t* src, uint32_t* out, uint8_t* a0, uint8_t* a1,
   const int m = s > 0 ? s : -s;
   if (m + r <= kShadowHalo && W <= (1 << 24) && H <= (1 << 24) && ox > -(1 << 24) && ox < (1 << 24) &&
       oy > -(1 << 24) && oy < (1 << 24)) {
-    const dim3 g((unsigned)((W + kShadowTile - 1) / kShadowTile), (unsigned)((H + kShadowTile - 1) / kShadowTile));
+    const int th = shadow_tile_rows(W, H, m, r, nsm);
+    const dim3 g((unsigned)((W + kShadowTile - 1) / kShadowTile), (unsigned)((H + th - 1) / th));
     const int late = dep_late(st, {Span{out, (size_t)(n * 4)}}, {Span{src, (size_t)(n * 4)}});
-    launch_pdl(shadow_tile_kernel(r), g, dim3(1024), shadow_tile_smem(m + r), st, src, out, (int)W, (int)H, (int)ox,
-               (int)oy, m, (int)(s > 0), kern, color, late);
+    launch_pdl(shadow_tile_kernel<0>(r), g, dim3(kShadowThreads), shadow_tile_smem(th, m, r), st, src, out, (int)W,
+               (int)H, (int)ox, (int)oy, th, m, r, (int)(s > 0), kern, color, late);
     note_launch();
     return;
   }
