@@ -190,7 +190,7 @@ bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, in
 void launch_stroke_outline(const float2* pts, const StrokeShape* shapes, int nshapes, long long nthreads, Prim* out,
                            int2* amb, long long amb_cap, unsigned long long* amb_count, int nsm, cudaStream_t st);
 bool launch_blur_small_fused(const uint32_t* in, uint32_t* out, long long W, long long H, int r,
-                             const uint16_t* kern, uint32_t oob, cudaStream_t st);
+                             const uint16_t* kern, uint32_t oob, int nsm, cudaStream_t st);
 bool launch_blur_small(uint32_t* img, uint32_t* tmp, long long W, long long H, int r, const uint16_t* kern,
                        uint32_t oob, int nsm, cudaStream_t st);
 constexpr int kSmallBlurMaxR = 8;  // the largest radius launch_blur_small(_fused) takes
@@ -472,7 +472,7 @@ bool blur_dispatch(uint32_t* img, uint32_t* tmp, long long tmp_bytes, long long 
     g.last_blur = ((W | H) & 3) == 0 ? 3 : 1;
     return false;
   }
-  if (swap_ok && g.blur_tensor == 3 && launch_blur_small_fused(img, tmp, W, H, (int)r, kern, oob, g.stream)) {
+  if (swap_ok && g.blur_tensor == 3 && launch_blur_small_fused(img, tmp, W, H, (int)r, kern, oob, g.nsm, g.stream)) {
     g.last_blur = 5;
     return true;
   }

@@ -199,16 +199,16 @@ __global__ void __launch_bounds__(256) k_blur_sy(const uint32_t* __restrict__ in
 // DRAM traffic is one read and one write of the image (the halo rows shared
 // by vertical neighbours come from L2).  The arithmetic per output is the
 // two-pass kernels': the same sums, the same floor(S / 65280) between passes.
-constexpr int kFTW = 128, kFTH = 64;  // tile: 128 columns x 64 rows
+constexpr int kFTW = 128;  // columns of a tile
 template <int R>
 __global__ void __launch_bounds__(256) k_blur_fused(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                     int W, int H, const uint16_t* __restrict__ kern, uint32_t oob,
-                                                    int vec, int late) {
+                                                    int th, int vec, int late) {
   constexpr int NI = kOut + 2 * R;
   constexpr int D = (4 - (R & 3)) & 3;
   constexpr int NC = (D + NI + 3) / 4;
-  constexpr int ROWS = kFTH + 2 * R;  // X-pass rows staged
-  __shared__ __align__(16) uint32_t xs[ROWS][kFTW];
+  const int rows = th + 2 * R;  // X-pass rows staged
+  extern __shared__ __align__(16) uint32_t xs[];  // rows of kFTW pixels
   if (late) pdl_trigger();  // else after the start-wait (pdl_late_entry)
   uint64_t w2[2 * R + 1];
 #pragma unroll
@@ -217,11 +217,11 @@ __global__ void __launch_bounds__(256) k_blur_fused(const uint32_t* __restrict__
     w2[t] = f2_pack(w, w);
   }
   const uint64_t nb = f2_pack(-kBias, -kBias), kq = f2_pack(kQuotC, kQuotC), km = f2_pack(kMagic, kMagic);
-  const int tx0 = blockIdx.x * kFTW, ty0 = blockIdx.y * kFTH;
+  const int tx0 = blockIdx.x * kFTW, ty0 = blockIdx.y * th;
   if (!late) pdl_late_entry(0);
   // X pass: (row, 8-pixel group) tasks over the staged rows
   constexpr int GPR = kFTW / kOut;  // groups per staged row
-  for (int task = threadIdx.x; task < ROWS * GPR; task += blockDim.x) {
+  for (int task = threadIdx.x; task < rows * GPR; task += blockDim.x) {
     const int lr = task / GPR, g = task - lr * GPR;
     const int y = ty0 - R + lr;
     const int x0 = tx0 + g * kOut;
@@ -267,14 +267,13 @@ __global__ void __launch_bounds__(256) k_blur_fused(const uint32_t* __restrict__
 #pragma unroll
       for (int o = 0; o < kOut; o++) res[o] = quot_px(arg[o], aba[o], kq, km);
     }
-    uint4* dst = reinterpret_cast<uint4*>(&xs[lr][g * kOut]);
+    uint4* dst = reinterpret_cast<uint4*>(xs + lr * kFTW + g * kOut);
     dst[0] = make_uint4(res[0], res[1], res[2], res[3]);
     dst[1] = make_uint4(res[4], res[5], res[6], res[7]);
   }
   __syncthreads();
   // Y pass: (column, 8-row strip) tasks, consecutive threads on consecutive columns
-  constexpr int STRIPS = kFTH / kOut;
-  for (int task = threadIdx.x; task < STRIPS * kFTW; task += blockDim.x) {
+  for (int task = threadIdx.x; task < th / kOut * kFTW; task += blockDim.x) {
     const int sidx = task / kFTW, c = task - sidx * kFTW;
     const int x = tx0 + c, y0 = ty0 + sidx * kOut;
     if (x >= W || y0 >= H) continue;
@@ -284,7 +283,7 @@ __global__ void __launch_bounds__(256) k_blur_fused(const uint32_t* __restrict__
 #pragma unroll
     for (int t = 0; t < NI; t++) {
       uint64_t rg, ba;
-      px_f2(xs[sidx * kOut + t][c], nb, rg, ba);
+      px_f2(xs[(sidx * kOut + t) * kFTW + c], nb, rg, ba);
 #pragma unroll
       for (int o = 0; o < kOut; o++) {
         if (t - o >= 0 && t - o <= 2 * R) {
@@ -301,14 +300,36 @@ __global__ void __launch_bounds__(256) k_blur_fused(const uint32_t* __restrict__
   pdl_late_exit(late);
 }
 
+// Rows of a tile, a multiple of 8.  A tile's time is its rows' and halo's
+// (0.08 us each at radius 5); the SM with most tiles does them one after the
+// other but for what overlaps, half of one.  Few rows so spread a small image
+// over the chip and many spare a large one the halo.  With 64 rows always /
+// so: 97 x 97 at radius 8 12.0 / 5.3 us, 641 x 641 14.4 / 9.3, 1237 x 1001 at
+// radius 3 10.6 / 8.6 (24 rows) and at 8 19.3 / 16.4 (72), 4096 x 4096 at 5
+// 75.6 / 72.7 (72).
+int fused_rows(long long W, long long H, int r, int nsm) {
+  const long long cols = (W + kFTW - 1) / kFTW;
+  long long best = 0;
+  int th = 64;
+  for (int t = 80; t >= 8; t -= 8) {
+    const long long down = (H + t - 1) / t, rounds = (cols * down + nsm - 1) / nsm, cost = (2 * rounds + 1) * (t + 2 * r);
+    if (down <= 65535 && (best == 0 || cost < best)) {
+      best = cost;
+      th = t;
+    }
+  }
+  return th;
+}
 template <int R>
 void launch_fused(const uint32_t* in, uint32_t* out, int W, int H, const uint16_t* kern, uint32_t oob,
-                  cudaStream_t st) {
+                  int nsm, cudaStream_t st) {
   const int vec = (W % 4 == 0) && ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
-  const dim3 grid((unsigned)((W + kFTW - 1) / kFTW), (unsigned)((H + kFTH - 1) / kFTH));
+  const int th = fused_rows(W, H, R, nsm);
+  const dim3 grid((unsigned)((W + kFTW - 1) / kFTW), (unsigned)((H + th - 1) / th));
   const size_t bytes = (size_t)W * (size_t)H * 4;
   const int late = dep_late(st, {Span{out, bytes}}, {Span{in, bytes}});
-  launch_pdl(k_blur_fused<R>, grid, dim3(256), 0, st, in, out, W, H, kern, oob, vec, late);
+  launch_pdl(k_blur_fused<R>, grid, dim3(256), (size_t)(th + 2 * R) * kFTW * 4, st, in, out, W, H, kern, oob, th, vec,
+             late);
   note_launch();
 }
 
@@ -331,18 +352,18 @@ void launch_small(uint32_t* img, uint32_t* tmp, int W, int H, const uint16_t* ke
 // Both passes in one launch, in -> out (out must not overlap in), for radii
 // 1..8; false if r is not for this kernel.
 bool launch_blur_small_fused(const uint32_t* in, uint32_t* out, long long W, long long H, int r,
-                             const uint16_t* kern, uint32_t oob, cudaStream_t st) {
+                             const uint16_t* kern, uint32_t oob, int nsm, cudaStream_t st) {
   if (r < 1 || r > 8 || W < 1 || H < 1 || W > (1 << 26) || H > (1 << 26)) return false;
-  if ((H + kFTH - 1) / kFTH > 65535) return false;
+  if ((H + 63) / 64 > 65535) return false;
   switch (r) {
-    case 1: launch_fused<1>(in, out, (int)W, (int)H, kern, oob, st); break;
-    case 2: launch_fused<2>(in, out, (int)W, (int)H, kern, oob, st); break;
-    case 3: launch_fused<3>(in, out, (int)W, (int)H, kern, oob, st); break;
-    case 4: launch_fused<4>(in, out, (int)W, (int)H, kern, oob, st); break;
-    case 5: launch_fused<5>(in, out, (int)W, (int)H, kern, oob, st); break;
-    case 6: launch_fused<6>(in, out, (int)W, (int)H, kern, oob, st); break;
-    case 7: launch_fused<7>(in, out, (int)W, (int)H, kern, oob, st); break;
-    default: launch_fused<8>(in, out, (int)W, (int)H, kern, oob, st); break;
+    case 1: launch_fused<1>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
+    case 2: launch_fused<2>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
+    case 3: launch_fused<3>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
+    case 4: launch_fused<4>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
+    case 5: launch_fused<5>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
+    case 6: launch_fused<6>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
+    case 7: launch_fused<7>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
+    default: launch_fused<8>(in, out, (int)W, (int)H, kern, oob, nsm, st); break;
   }
   return true;
 }
