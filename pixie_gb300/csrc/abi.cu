@@ -2775,7 +2775,8 @@ pxg_image temp_image(int i, int64_t w, int64_t h) {  // a zeroed non-owning scra
   return pxg_image{(uint8_t*)g.pt_buf[i], w, h, 0};
 }
 
-void fill_gradient(pxg_image* im, const pxg_paint& p, float opacity) {
+void fill_gradient(pxg_image* im, const pxg_paint& p, float opacity, int out = kOutFill,
+                   const pxg_image* mask = nullptr, uint32_t maskO = 255) {
   const int nh = p.n_handles, ns = p.n_stops;
   if (nh < 0 || ns < 0 || (nh > 0 && !p.handles) || (ns > 0 && !p.stops)) throw ApiError{"Invalid gradient"};
   if (p.kind == 3 && nh != 2) throw ApiError{"Linear gradient requires 2 handles"};
@@ -2812,9 +2813,14 @@ void fill_gradient(pxg_image* im, const pxg_paint& p, float opacity) {
     G.cy = h0.y;
     G.gradientAngle = fix_angle_h(atan2f(n.y, n.x));
   }
-  dev_grow(g.pt_stops, g.pt_stops_cap, 5 * (long long)ns);
-  CU(cudaMemcpyAsync(g.pt_stops, p.stops, sizeof(float) * 5 * (size_t)ns, cudaMemcpyHostToDevice, g.stream));
-  launch_gradient((uint32_t*)im->data, im->width, im->height, G, g.pt_stops, g.nsm, g.stream);
+  if (ns <= kInlineStops) {
+    memcpy(G.inl, p.stops, sizeof(float) * 5 * (size_t)ns);
+  } else {
+    dev_grow(g.pt_stops, g.pt_stops_cap, 5 * (long long)ns);
+    CU(cudaMemcpyAsync(g.pt_stops, p.stops, sizeof(float) * 5 * (size_t)ns, cudaMemcpyHostToDevice, g.stream));
+  }
+  launch_gradient((uint32_t*)im->data, im->width, im->height, G, g.pt_stops, out,
+                  mask ? (const uint32_t*)mask->data : nullptr, maskO, g.nsm, g.stream);
 }
 
 void check_paint(const pxg_paint* p) {
@@ -2827,21 +2833,20 @@ void check_paint(const pxg_paint* p) {
   }
 }
 
-// the paint's own image at opacity 1  paths.nim:2121-2134
+// an image paint's own image at opacity 1  paths.nim:2121-2134
 void paint_fill_image(pxg_image* fill, const pxg_paint& p) {
   M3 m;
   memcpy(m.m, p.image_mat, sizeof m.m);
   if (p.kind == 1)
     draw_transform(fill, p.image, m, 0);
-  else if (p.kind == 2)
-    draw_correct(fill, p.image, m, 0, true);
   else
-    fill_gradient(fill, p, 1.0f);
+    draw_correct(fill, p.image, m, 0, true);
 }
 
 // images.nim:261-277
+uint32_t opacity_u16(float opacity) { return (uint16_t)h_nim_i32(roundf(255 * opacity)); }
 void apply_opacity(pxg_image* im, float opacity) {
-  const uint32_t o = (uint16_t)h_nim_i32(roundf(255 * opacity));
+  const uint32_t o = opacity_u16(opacity);
   if (o == 255) return;
   if (o == 0) {
     CU(cudaMemsetAsync(im->data, 0, (size_t)(im->width * im->height * 4), g.stream));
@@ -2852,11 +2857,23 @@ void apply_opacity(pxg_image* im, float opacity) {
 
 // fill.draw(mask, MaskBlend); image.draw(fill, blendMode)  paths.nim:2136-2142
 void composite_paint(pxg_image* im, pxg_image* mask, const pxg_paint& p) {
+  const float op = p.opacity < 0 ? 0 : (p.opacity > 1 ? 1 : p.opacity);
+  const int64_t W = im->width, H = im->height;
+  if (p.kind >= 3) {  // a gradient's colours go through the mask as they are formed
+    if (p.blend_mode == kNormal) {
+      fill_gradient(im, p, 1.0f, kOutComposite, mask, opacity_u16(op));
+      return;
+    }
+    dev_grow(g.pt_buf[1], g.pt_cap[1], W * H);
+    pxg_image fill{(uint8_t*)g.pt_buf[1], W, H, 0};
+    fill_gradient(&fill, p, 1.0f, kOutMasked, mask, opacity_u16(op));
+    launch_draw((uint32_t*)im->data, (const uint32_t*)fill.data, W, H, W, H, 0, 0, p.blend_mode, g.tbl, g.nsm,
+                g.stream);
+    return;
+  }
   pxg_image fill = temp_image(1, im->width, im->height);
   paint_fill_image(&fill, p);
-  const float op = p.opacity < 0 ? 0 : (p.opacity > 1 ? 1 : p.opacity);
   if (op != 1) apply_opacity(mask, op);
-  const int64_t W = im->width, H = im->height;
   launch_draw((uint32_t*)fill.data, (const uint32_t*)mask->data, W, H, W, H, 0, 0, kMask, g.tbl, g.nsm, g.stream);
   launch_draw((uint32_t*)im->data, (const uint32_t*)fill.data, W, H, W, H, 0, 0, p.blend_mode, g.tbl, g.nsm,
               g.stream);

@@ -155,38 +155,121 @@ __device__ uint32_t gradient_color(const float* __restrict__ st, int n, float op
   return color_rgbx(c[0], c[1], c[2], c[3]);
 }
 
+// The gradient's parameter at a pixel
+template <int KIND>
+__device__ __forceinline__ float gradient_t(const GradientArgs& g, float fx, float fy) {
+  if (KIND == 3) {  // toLineSpace  paints.nim:111-116
+    return (g.dy * (fy - g.aty) + g.dx * (fx - g.atx)) / g.det;
+  } else if (KIND == 4) {  // (mat * xy).length()  :201-203
+    const float vx = g.m[0] * fx + g.m[3] * fy + g.m[6], vy = g.m[1] * fx + g.m[4] * fy + g.m[7];
+    return sqrtf(vx * vx + vy * vy);
+  } else {  // :222-227
+    const float vx = fx - g.cx, vy = fy - g.cy;
+    const float len = sqrtf(vx * vx + vy * vy);
+    const float angle = atan2_cr(vy / len, vx / len);
+    const float f32PI = (float)kPI64;
+    return fix_angle(angle + g.gradientAngle + f32PI / 2) / 2 / f32PI + 0.5f;
+  }
+}
+
+// OUT: what becomes of a pixel's colour c.
+//   kOutFill       img = c
+//   kOutMasked     img = c * (mask's alpha * o div 255) div 255: the paint drawn under MaskBlend
+//   kOutComposite  that, drawn onto img under NormalBlend
+// so a path filled with a gradient takes the mask once and the image once,
+// and no paint image between them.  Bound by instructions (the divisions and
+// roundings of a colour), so pixels the mask leaves out have none formed, a
+// thread takes four neighbours with one division for its row (one for the
+// angular kind, whose arctangent is most of its code), and the stops come as
+// kernel arguments while they fit.  A heart filled with a radial gradient at 1601 x 1203:
+// 42 us in four kernels over whole images (colours 13.5, the mask's opacity 7,
+// the mask 11, the image 10.5) -> 12 in this one; the colours alone 13.5 -> 12.
 // STAGED: the stops are copied into shared memory once per CTA; otherwise
 // (more stops than 48 KB of shared memory holds) they are read from global
 // memory, through the read-only cache.
-template <int KIND, bool STAGED>
-__global__ void __launch_bounds__(256) k_gradient(uint32_t* __restrict__ img, long long W, long long H, GradientArgs g,
-                                                  const float* __restrict__ gstops) {
+template <int KIND, bool STAGED, int OUT>
+__global__ void __launch_bounds__(256) k_gradient(uint32_t* __restrict__ img, long long W, long long n,
+                                                  const __grid_constant__ GradientArgs g,
+                                                  const float* __restrict__ gstops, const uint32_t* __restrict__ mask,
+                                                  uint32_t o, int vec) {
   extern __shared__ float staged[];
   const float* stops = gstops;
   if (STAGED) {
-    for (int i = threadIdx.x; i < 5 * g.nstops; i += blockDim.x) staged[i] = gstops[i];
+    for (int i = threadIdx.x; i < 5 * g.nstops; i += blockDim.x)
+      staged[i] = g.nstops <= kInlineStops ? g.inl[i] : gstops[i];
     __syncthreads();
     stops = staged;
   }
-  const long long n = W * H;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long y = i / W, x = i - y * W;
-    const float fx = (float)x, fy = (float)y;
-    float t;
-    if (KIND == 3) {  // toLineSpace  paints.nim:111-116
-      t = (g.dy * (fy - g.aty) + g.dx * (fx - g.atx)) / g.det;
-    } else if (KIND == 4) {  // (mat * xy).length()  :201-203
-      const float vx = g.m[0] * fx + g.m[3] * fy + g.m[6], vy = g.m[1] * fx + g.m[4] * fy + g.m[7];
-      t = sqrtf(vx * vx + vy * vy);
-    } else {  // :222-227
-      const float vx = fx - g.cx, vy = fy - g.cy;
-      const float len = sqrtf(vx * vx + vy * vy);
-      const float angle = atan2_cr(vy / len, vx / len);
-      const float f32PI = (float)kPI64;
-      t = fix_angle(angle + g.gradientAngle + f32PI / 2) / 2 / f32PI + 0.5f;
+  constexpr int PX = KIND == 5 ? 1 : 4;
+  const bool small = n < (1ll << 31);
+  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * PX; i < n;
+       i += (long long)gridDim.x * blockDim.x * PX) {
+    const bool whole = PX == 4 && vec && i + 4 <= n;
+    uint32_t k[PX], d[PX];
+    if (OUT != kOutFill) {
+      if (whole) {
+        const uint4 v = *reinterpret_cast<const uint4*>(mask + i);
+        k[0] = v.x;
+        k[PX > 1 ? 1 : 0] = PX > 1 ? v.y : v.x;
+        k[PX > 1 ? 2 : 0] = PX > 1 ? v.z : v.x;
+        k[PX > 1 ? 3 : 0] = PX > 1 ? v.w : v.x;
+      } else {
+#pragma unroll
+        for (int q = 0; q < PX; q++) k[q] = i + q < n ? mask[i + q] : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < PX; q++) k[q] = ((k[q] >> 24) * o) / 255;
     }
-    img[i] = gradient_color(stops, g.nstops, g.opacity, t);
+    if (OUT == kOutComposite) {
+      if (whole) {
+        const uint4 v = *reinterpret_cast<const uint4*>(img + i);
+        d[0] = v.x;
+        d[PX > 1 ? 1 : 0] = PX > 1 ? v.y : v.x;
+        d[PX > 1 ? 2 : 0] = PX > 1 ? v.z : v.x;
+        d[PX > 1 ? 3 : 0] = PX > 1 ? v.w : v.x;
+      } else {
+#pragma unroll
+        for (int q = 0; q < PX; q++) d[q] = i + q < n ? img[i + q] : 0u;
+      }
+    }
+    long long y, x;
+    if (small) {
+      y = (unsigned)i / (unsigned)W;
+      x = (unsigned)i - (unsigned)y * (unsigned)W;
+    } else {
+      y = i / W;
+      x = i - y * W;
+    }
+    // (64-bit conversions run at a quarter of the 32-bit rate)
+    const auto to_f = [&](long long v) { return small ? (float)(int)v : (float)v; };
+    float fy = to_f(y);
+    uint32_t c[PX];
+    bool change = false;
+#pragma unroll
+    for (int q = 0; q < PX; q++) {
+      uint32_t v = 0;
+      if (OUT == kOutFill || k[q] != 0) {
+        v = gradient_color(stops, g.nstops, g.opacity, gradient_t<KIND>(g, to_f(x), fy));
+        if (OUT != kOutFill) v = mul_div255_px(v, k[q]);
+      }
+      if (OUT == kOutComposite) {
+        v = blendNormal(d[q], v);
+        change |= v != d[q];
+      }
+      c[q] = v;
+      if (PX > 1 && ++x == W) {
+        x = 0;
+        fy = to_f(++y);
+      }
+    }
+    if (OUT == kOutComposite && !change) continue;
+    if (whole) {
+      *reinterpret_cast<uint4*>(img + i) = make_uint4(c[0], c[PX > 1 ? 1 : 0], c[PX > 1 ? 2 : 0], c[PX > 1 ? 3 : 0]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < PX; q++)
+        if (i + q < n) img[i + q] = c[q];
+    }
   }
 }
 
@@ -283,21 +366,33 @@ struct CorrectTable<kNumBlends> {
 
 }  // namespace
 
-void launch_gradient(uint32_t* img, long long W, long long H, const GradientArgs& g, const float* stops, int nsm,
-                     cudaStream_t st) {
+namespace {
+typedef void (*GradientKernel)(uint32_t*, long long, long long, GradientArgs, const float*, const uint32_t*, uint32_t,
+                               int);
+template <int OUT>
+GradientKernel gradient_kernel(int kind, bool staged) {
+  if (kind == 3) return staged ? k_gradient<3, true, OUT> : k_gradient<3, false, OUT>;
+  if (kind == 4) return staged ? k_gradient<4, true, OUT> : k_gradient<4, false, OUT>;
+  return staged ? k_gradient<5, true, OUT> : k_gradient<5, false, OUT>;
+}
+}  // namespace
+
+// o: the mask's opacity, round(255 * opacity); mask and o are not read for kOutFill
+void launch_gradient(uint32_t* img, long long W, long long H, const GradientArgs& g, const float* stops, int out,
+                     const uint32_t* mask, uint32_t o, int nsm, cudaStream_t st) {
   const long long n = W * H;
   const size_t need = sizeof(float) * 5 * (size_t)g.nstops;
   const bool staged = need <= 48 * 1024;
   const size_t smem = staged ? need : 0;
-  long long blocks = (n + 255) / 256;  // four waves of eight CTAs per SM at most
+  const long long per = g.kind == 5 ? 256 : 1024;
+  long long blocks = (n + per - 1) / per;  // four waves of eight CTAs per SM at most
   if (blocks > (long long)nsm * 32) blocks = (long long)nsm * 32;
   const unsigned gb = (unsigned)(blocks < 1 ? 1 : blocks);
-  if (g.kind == 3)
-    (staged ? k_gradient<3, true> : k_gradient<3, false>)<<<gb, 256, smem, st>>>(img, W, H, g, stops);
-  else if (g.kind == 4)
-    (staged ? k_gradient<4, true> : k_gradient<4, false>)<<<gb, 256, smem, st>>>(img, W, H, g, stops);
-  else
-    (staged ? k_gradient<5, true> : k_gradient<5, false>)<<<gb, 256, smem, st>>>(img, W, H, g, stops);
+  const int vec = ((reinterpret_cast<uintptr_t>(img) | reinterpret_cast<uintptr_t>(mask)) & 15) == 0;
+  const GradientKernel k = out == kOutFill     ? gradient_kernel<kOutFill>(g.kind, staged)
+                           : out == kOutMasked ? gradient_kernel<kOutMasked>(g.kind, staged)
+                                               : gradient_kernel<kOutComposite>(g.kind, staged);
+  k<<<gb, 256, smem, st>>>(img, W, n, g, stops, mask, o, vec);
   note_launch();
 }
 
