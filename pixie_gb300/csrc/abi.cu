@@ -117,7 +117,15 @@ int rows_warps(int v);
 bool rows_fast(int mode, long long W);
 void launch_rows(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
                  const Arena& A, const uint8_t* tbl, long long items, int rpi);
-__global__ void k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl);
+const void* rows_lines_kernel();
+size_t rows_lines_smem();
+int rows_lines_threads();
+void launch_rows_lines(unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
+                       const Arena& A, const uint8_t* tbl, long long items);
+const void* rows_huge_kernel();
+size_t rows_huge_smem();
+void launch_rows_huge(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, const uint8_t* tbl);
+__global__ void k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl, int list);
 __global__ void k_xclears(PathJob* jobs, Arena A);
 const void* scene_rec_kernel();
 size_t scene_rec_smem();
@@ -311,6 +319,7 @@ struct Ctx {
   float last_ms = 0;
   long long stats[6] = {0, 0, 0, 0, 0, 0};  // last fill launch: paths, prims, segments, entries, blends, wide rows
   int rows_ctas_per_sm[4] = {1, 1, 1, 1};  // resident CTAs of each row-kernel variant
+  int lines_ctas_per_sm = 1;               // and of the row kernel with a CTA per row
   int scene_ctas_per_sm[5] = {1, 1, 1, 1, 1};  // resident CTAs of the scene recording, drawing, rest and big-row kernels
   int scene_slice = 0;                // pixels of a row one warp of the drawing pass owns (0: chosen per launch)
   bool stroke_gpu = true;             // outline strokes without dashes on the GPU (stroke.cu)
@@ -372,6 +381,14 @@ void init_locked(int device) {
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rows_kernel(v), rows_warps(v) * 32, rows_smem(v)));
     g.rows_ctas_per_sm[v] = std::max(1, per);
   }
+  {
+    int per = 0;
+    CU(cudaFuncSetAttribute(rows_lines_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_lines_smem()));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rows_lines_kernel(), rows_lines_threads(),
+                                                     rows_lines_smem()));
+    g.lines_ctas_per_sm = std::max(1, per);
+  }
+  CU(cudaFuncSetAttribute(rows_huge_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_huge_smem()));
   CU(cudaFuncSetAttribute(k_rows_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem_wide()));
   {
     CU(cudaFuncSetAttribute(scene_rec_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scene_rec_smem()));
@@ -578,7 +595,7 @@ void ensure_arena(long long seg_need, long long list_need, long long nbands, lon
   dev_grow(g.bands, g.band_cap, nbands);
   dev_grow(g.bandseg, g.bandseg_cap, list_need);
   dev_grow(g.primcnt, g.primcnt_cap, nprims + 1);
-  dev_grow(g.ovf, g.ovf_cap, rows);
+  dev_grow(g.ovf, g.ovf_cap, 2 * rows);  // two lists
   dev_grow(g.xcl, g.xcl_cap, 3 * (2 * rows + 1024));
 }
 
@@ -770,8 +787,20 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
                      });
     const int setupC = setup_cluster(nr, maxWork, maxBands);
     Arena& A = S.A;
+    A.ovf_cap = g.ovf_cap / 2;
     PathJob* dj = S.dj;
     const int v = cfg.variant;
+    // A launch of few rows lasts as long as its busiest one, and a warp per
+    // sample line shortens rows of more than 16 crossings, as paths of some
+    // hundred lines (a curve counts 24) have them: one path of 64 cubics on 512 x
+    // 512 29 us by a warp per row, 21 by a CTA; a stroke's 767 rows of up to 256
+    // crossings 65 and 54.  Beyond two rows per resident CTA the warps' number
+    // counts.  Rows of more than 256 crossings need some thousand lines in the
+    // path: their kernel is launched along then (3 us for nothing), else only
+    // when the call has come back with such rows.
+    const bool byLines = v == 0 && cfg.rpi == 1 && opts.cfg.rpi == 0 && maxWork >= 512 &&
+                         items <= 2LL * g.nsm * g.lines_ctas_per_sm;
+    const bool hugeAlong = v == 0 && maxWork >= 2048;
     long long blocks = (items + rows_warps(v) - 1) / rows_warps(v);
     blocks = std::min<long long>(blocks, (long long)g.nsm * g.rows_ctas_per_sm[v]);
     blocks = std::max<long long>(blocks, 1);
@@ -782,9 +811,14 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
       CU(launch_setup(nr, setupC, maxBands, g.stream, dj, A));
       if (count) note_launch();
       if (timeRows) CU(cudaEventRecord(g.evr0, g.stream));
-      launch_rows(v, (unsigned)blocks, g.stream, dj, reinterpret_cast<const long long*>(S.extra), nr, A, g.tbl, items,
-                  cfg.rpi);
+      const long long* doffs = reinterpret_cast<const long long*>(S.extra);
+      if (byLines) launch_rows_lines((unsigned)items, g.stream, dj, doffs, nr, A, g.tbl, items);
+      else launch_rows(v, (unsigned)blocks, g.stream, dj, doffs, nr, A, g.tbl, items, cfg.rpi);
       if (count) note_launch();
+      if (hugeAlong) {
+        launch_rows_huge((unsigned)g.nsm, g.stream, dj, A, g.tbl);
+        if (count) note_launch();
+      }
       CU(cudaGetLastError());
       if (timeRows) CU(cudaEventRecord(g.evr1, g.stream));
       S.read_back();
@@ -833,11 +867,16 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
     memcpy(ctr, g.h_up + S.jobsBytes, sizeof ctr);
     note_stats(nr, nprims, ctr);
     const PathJob* wide = nullptr;
-    if (ctr[kCtrOvfRows] > 0 || ctr[kCtrXClears] > 0) {
+    // rows handed on and not drawn yet: of list 0, or 1 behind k_rows_huge
+    const unsigned long long more = ctr[hugeAlong ? kCtrOvfRows2 : kCtrOvfRows];
+    if (more > 0 || ctr[kCtrXClears] > 0) {
       if ((long long)ctr[kCtrXClears] > A.xclear_cap) throw ApiError{"Out of workspace memory (cross-row clears)"};
-      if (ctr[kCtrOvfRows] > 0) {
-        long long b = std::min<long long>((long long)ctr[kCtrOvfRows], (long long)g.nsm * 4);
-        k_rows_wide<<<(unsigned)b, 32, rows_smem_wide(), g.stream>>>(dj, A, g.tbl); note_launch();
+      if (more > 0) {
+        long long b = std::min<long long>((long long)more, (long long)g.nsm * 4);
+        if (v == 0 && !hugeAlong) {
+          launch_rows_huge((unsigned)std::min<long long>(b, g.nsm), g.stream, dj, A, g.tbl); note_launch();
+        }
+        k_rows_wide<<<(unsigned)b, 32, rows_smem_wide(), g.stream>>>(dj, A, g.tbl, v == 0); note_launch();
         CU(cudaGetLastError());
       }
       if (ctr[kCtrXClears] > 0) {

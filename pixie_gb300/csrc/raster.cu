@@ -942,6 +942,68 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows_fast(PathJob* jobs, const l
   }
 }
 constexpr int kRowsNB = 256, kRowsXT = 1024, kRowsWarps = 4;
+
+// The same for launches whose rows all fit the GPU at once, a CTA each: the
+// launch lasts as long as the busiest row, and a warp per sample line shortens
+// it (64 cubics on 512 x 512: 29 -> 21 us).
+constexpr int kRowsLineThreads = kLineWarps * 32;
+__global__ void __launch_bounds__(kRowsLineThreads) k_rows_lines(PathJob* jobs, const long long* offs, int njobs,
+                                                                 Arena A, const uint8_t* tbl, long long totalItems) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  LineRow<kRowsNB, kRowsXT>& S = *reinterpret_cast<LineRow<kRowsNB, kRowsXT>*>(rsm);
+  pdl_trigger();
+  pdl_wait();
+  if (warp > 0) {
+    line_warps(S, warp, lane);
+    return;
+  }
+  init_fast_row(S.row, lane);
+#pragma unroll 1
+  for (long long item = blockIdx.x; item < totalItems; item += gridDim.x) {
+    int lo = 0, hi = njobs - 1;
+#pragma unroll 1
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (offs[mid] <= item) lo = mid;
+      else hi = mid - 1;
+    }
+    const PathJob& J = jobs[lo];
+    const int y = (int)(J.startY + (item - J.row_off));
+    if (J.status != kOk || y >= (int)J.pathHeight) continue;
+    fast_rows<kOutRgbx, kRowsNB, kRowsXT, 0, true>(J, A, tbl, lo, y, y + 1, S.row, lane, &S.work, S.line);
+  }
+  line_warps_end(S.work, lane);
+}
+
+// Rows of RGBX launches with more than kRowsNB crossings (list 0), up to
+// kWideMaxH of them; the rest to list 1.  They are few and each takes long: a
+// stroke of 300 points with round joins has five, 160 us by the general code
+// on a warp each after a wait for the host, 56 so.
+__global__ void __launch_bounds__(kRowsLineThreads) k_rows_huge(PathJob* jobs, Arena A, const uint8_t* tbl) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  LineRow<kWideMaxH, kWideXT>& S = *reinterpret_cast<LineRow<kWideMaxH, kWideXT>*>(rsm);
+  pdl_trigger();
+  pdl_wait();
+  if (warp > 0) {
+    line_warps(S, warp, lane);
+    return;
+  }
+  init_fast_row(S.row, lane);
+  const long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[kCtrOvfRows]);
+#pragma unroll 1
+  for (long long i = blockIdx.x; i < n; i += gridDim.x) {
+    const long long v = A.ovf_rows[i];
+    const int job = (int)(v >> 32), y = (int)(v & 0xffffffffLL);
+    const PathJob& J = jobs[job];
+    const int k = min((y - (int)J.startY) / (int)J.ph, J.nb - 1);
+    // a band of more than kWideMaxH entries is an error, which the general kernel reports
+    if (J.W >= fast_max_w(kWideMaxH) || A.bands[J.band_off + k].count > kWideMaxH) push_row(A, job, y, lane, 1);
+    else fast_rows<kOutRgbx, kWideMaxH, kWideXT, 1, true>(J, A, tbl, job, y, y + 1, S.row, lane, &S.work, S.line);
+  }
+  line_warps_end(S.work, lane);
+}
 constexpr int kGlyphNB = 64, kGlyphXT = 256, kGlyphWarps = 8;
 
 // The general row kernel (launches with MaskBlend paths, whose clears reach
@@ -991,16 +1053,16 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows(PathJob* jobs, const long l
   }
 }
 
-// Rows whose crossings exceed the fast kernel's capacity: one warp per CTA
-// with room for kWideMaxH crossings.
-__global__ void __launch_bounds__(32) k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl) {
+// Rows the kernels before handed on (list 0 or 1), by the general row code: one
+// warp per CTA with room for kWideMaxH crossings.
+__global__ void __launch_bounds__(32) k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl, int list) {
   extern __shared__ __align__(16) unsigned char rsm[];
   using Scratch = RowScratch<kWideMaxH, kWideXT>;
   Scratch& S = *reinterpret_cast<Scratch*>(rsm);
   const int lane = threadIdx.x & 31;
-  long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[kCtrOvfRows]);
+  long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[list ? kCtrOvfRows2 : kCtrOvfRows]);
   for (long long i = blockIdx.x; i < n; i += gridDim.x) {
-    long long v = A.ovf_rows[i];
+    long long v = A.ovf_rows[list * A.ovf_cap + i];
     int job = (int)(v >> 32);
     long long y = v & 0xffffffffLL;
     PathJob& J = jobs[job];
@@ -1105,26 +1167,18 @@ __global__ void __launch_bounds__(kBigWarps * 32) k_scene_big(PathJob* jobs, Are
 // List 1: up to 2048 crossings, a CTA per row and a warp per sample line, for
 // these rows are few and each takes long (a warp each, the widest rows of a
 // 240-path scene took 347 us, this way 74); the rest to list 2.
+// (By a CTA per row the rows of up to 512 crossings of 240 local paths take 135
+// us instead of 157, but those of 2000 paths over 1024 x 1024 1156 instead of
+// 944: warp 0's share of a row leaves the other warps idle.)
 constexpr int kHugeNB = 2048, kHugeXT = 1024;
-struct HugeRow {
-  FastRow<kHugeNB, kHugeXT> row;
-  LineScratch<kHugeNB> line[kLineWarps];
-  LineWork work;
-};
 __global__ void __launch_bounds__(kLineWarps * 32) k_scene_huge(PathJob* jobs, Arena A) {
   extern __shared__ __align__(16) unsigned char rsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  HugeRow& S = *reinterpret_cast<HugeRow*>(rsm);
+  LineRow<kHugeNB, kHugeXT>& S = *reinterpret_cast<LineRow<kHugeNB, kHugeXT>*>(rsm);
   pdl_trigger();
   pdl_wait();
-  if (warp > 0) {  // the other lines of the rows warp 0 publishes
-#pragma unroll 1
-    while (true) {
-      line_barrier();
-      if (S.work.n < 0) break;
-      one_line(S.row, S.work, S.line[warp], warp, lane);
-      line_barrier();
-    }
+  if (warp > 0) {
+    line_warps(S, warp, lane);
     return;
   }
   init_fast_row(S.row, lane);
@@ -1137,8 +1191,7 @@ __global__ void __launch_bounds__(kLineWarps * 32) k_scene_huge(PathJob* jobs, A
     if (J.W >= fast_max_w(kHugeNB)) push_row(A, job, y, lane, 2);
     else fast_rows<kOutRec, kHugeNB, kHugeXT, 2, true>(J, A, nullptr, job, y, y + 1, S.row, lane, &S.work, S.line);
   }
-  if (lane == 0) S.work.n = -1;
-  line_barrier();
+  line_warps_end(S.work, lane);
 }
 
 // The rows k_scene_huge handed on (list 2), by the general row code; those with
@@ -1357,7 +1410,7 @@ size_t scene_rec_smem() { return sizeof(FastRow<kRecNB, kRecRowXT>) * kRecRowWar
 int scene_rec_warps() { return kRecRowWarps; }
 // the kernels of wide rows: 0 k_scene_big, 1 k_scene_huge
 const void* scene_big_kernel(int v) { return v ? (const void*)k_scene_huge : (const void*)k_scene_big; }
-size_t scene_big_smem(int v) { return v ? sizeof(HugeRow) : sizeof(FastRow<kBigNB, kBigXT>) * kBigWarps; }
+size_t scene_big_smem(int v) { return v ? sizeof(LineRow<kHugeNB, kHugeXT>) : sizeof(FastRow<kBigNB, kBigXT>) * kBigWarps; }
 int scene_big_threads(int v) { return (v ? kLineWarps : kBigWarps) * 32; }
 int scene_big_rows(int v) { return v ? 1 : kBigWarps; }  // per CTA
 void launch_scene_big(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A) {
@@ -1431,6 +1484,20 @@ cudaError_t launch_setup(int njobs, int C, int maxBands, cudaStream_t st, PathJo
 size_t scene_wide_bytes() { return sizeof(RowScratch<kWideMaxH, kWideXT>); }
 
 size_t rows_smem_wide() { return sizeof(RowScratch<kWideMaxH, kWideXT>); }
+
+const void* rows_lines_kernel() { return (const void*)k_rows_lines; }
+size_t rows_lines_smem() { return sizeof(LineRow<kRowsNB, kRowsXT>); }
+int rows_lines_threads() { return kRowsLineThreads; }
+void launch_rows_lines(unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
+                       const Arena& A, const uint8_t* tbl, long long items) {
+  launch_pdl(k_rows_lines, dim3(blocks), dim3(kRowsLineThreads), rows_lines_smem(), st, jobs, offs, njobs, A, tbl,
+             items);
+}
+const void* rows_huge_kernel() { return (const void*)k_rows_huge; }
+size_t rows_huge_smem() { return sizeof(LineRow<kWideMaxH, kWideXT>); }
+void launch_rows_huge(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, const uint8_t* tbl) {
+  launch_pdl(k_rows_huge, dim3(blocks), dim3(kRowsLineThreads), rows_huge_smem(), st, jobs, A, tbl);
+}
 
 // Row kernel variants: 0 = RGBX images, 1 = masks of small paths such as
 // glyphs (64 crossings and 256-px tiles, a quarter of the shared memory per

@@ -440,13 +440,13 @@ __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, fl
   }
 }
 
-// Rows of hundreds of crossings: a warp per sample line.  The row's warp (0)
-// orders the entries and publishes the row; warps 1 .. 4 take the other lines
-// with keys and spans of their own, all into the row's difference array.
+// Rows whose time on one warp is what a launch waits for: a warp per sample
+// line.  The row's warp (0) orders the entries and publishes the row; warps
+// 1 .. 4 take the other lines with keys and spans of their own, all into the
+// row's difference array.
 constexpr int kLineWarps = 5;
 template <int NB>
 struct __align__(16) LineScratch {
-  static_assert(NB >= 1024, "sort_many pads to 1024 keys");
   uint32_t keys[NB];
   int2 spans[NB / 2 + 32];
 };
@@ -455,18 +455,27 @@ struct LineWork {  // what warp 0 publishes (n < 0: no more rows), and the warps
   float Wf;
   int lo[kLineWarps], hi[kLineWarps];
 };
+template <int NB, int XT>
+struct LineRow {  // a CTA's row
+  FastRow<NB, XT> row;
+  LineScratch<NB> line[kLineWarps];
+  LineWork work;
+};
 __device__ __forceinline__ void line_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kLineWarps * 32) : "memory"); }
 
-// n keys of up to 2048: 1024 fit a warp's registers.
-static __device__ __noinline__ void sort_many(uint32_t* keys, int n, bool fresh, int lane) {
-  if (n > 1024) {
-    sort_keys_shared(keys, n, fresh, lane);
-  } else {
+template <int K>
+__device__ __forceinline__ void sort_padded(uint32_t* keys, int n, bool fresh, int lane) {
 #pragma unroll 1
-    for (int k = n + lane; k < 1024; k += 32) keys[k] = kNoKey;
-    __syncwarp();
-    sort_keys<32>(keys, n, fresh, lane);
-  }
+  for (int k = n + lane; k < 32 * K; k += 32) keys[k] = kNoKey;
+  __syncwarp();
+  sort_keys<K>(keys, n, fresh, lane);
+}
+// n keys of up to NB, in the registers of the warp where they fit.
+template <int NB>
+static __device__ __noinline__ void sort_line(uint32_t* keys, int n, bool fresh, int lane) {
+  if (NB <= 256 && n <= 64) sort_padded<2>(keys, n, fresh, lane);
+  else if (n <= (NB < 1024 ? NB : 1024)) sort_padded<(NB < 1024 ? NB : 1024) / 32>(keys, n, fresh, lane);
+  else sort_keys_shared(keys, n, fresh, lane);
   __syncwarp();
 }
 
@@ -493,7 +502,7 @@ __device__ __forceinline__ void one_line(FastRow<NB, XT>& S, LineWork& L, LineSc
       nh += __popc(msk);
     }
     __syncwarp();
-    sort_many(K.keys, nh, false, lane);
+    sort_line<NB>(K.keys, nh, false, lane);
     int count = 0, prevAt = 0, ns = 0;
 #pragma unroll 1
     for (int c0 = 0; c0 < nh; c0 += 32)
@@ -519,7 +528,7 @@ __device__ __forceinline__ void cov_lines(FastRow<NB, XT>& S, LineWork& L, LineS
     K.keys[i] = crossing_key<TAG>(S, j, i, fminf(fmaxf((float)y + 0.5f, S.ay(j)), S.by(j)), Wf);
   }
   __syncwarp();
-  sort_many(K.keys, n, true, lane);
+  sort_line<NB>(K.keys, n, true, lane);
 #pragma unroll 1
   for (int i = lane; i < n; i += 32) S.perm[i] = (uint16_t)((K.keys[i] >> 1) & ((1u << (TAG - 1)) - 1));
   if (lane == 0) {
@@ -773,7 +782,7 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
 template <int OUT, int NB, int XT, int LIST = 0, bool LINES = false>
 __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, const uint8_t* tbl, int job, int yA,
                                           int yB, FastRow<NB, XT>& S, int lane, LineWork* L = nullptr,
-                                          LineScratch<2048>* K = nullptr) {
+                                          LineScratch<NB>* K = nullptr) {
   constexpr bool REC = OUT == kOutRec;
   const unsigned lt = (1u << lane) - 1;
   const int W = (int)J.W, startY = (int)J.startY, pathHeight = (int)J.pathHeight, ph = (int)J.ph;
@@ -891,8 +900,11 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       }
       CovTile T{xt, max(dl, xt), min(dh, xt + XT), INT_MAX, INT_MIN};
       if (kind == 0) {
-        if constexpr (LINES) cov_lines(S, *L, *K, n, y, (float)W, winding, aa, T, lane);
-        else cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane);
+        if (LINES && (REC || NB > 512 || n > kGroupN)) {
+          if constexpr (LINES) cov_lines(S, *L, *K, n, y, (float)W, winding, aa, T, lane);
+        } else {
+          cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane);
+        }
       } else {
         if (kind == 1) failed = trap_cov<REC>(S, n, y, T, lane);
         else if (lane == 0) cov_range(S.diff, T, dl, dh, 255);
@@ -992,6 +1004,23 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       }
     }
   }
+}
+
+// The warps of a CTA that take a row's other sample lines, until warp 0 has no
+// more rows; what warp 0 calls then.
+template <int NB, int XT>
+__device__ __forceinline__ void line_warps(LineRow<NB, XT>& S, int warp, int lane) {
+#pragma unroll 1
+  while (true) {
+    line_barrier();
+    if (S.work.n < 0) break;
+    one_line(S.row, S.work, S.line[warp], warp, lane);
+    line_barrier();
+  }
+}
+__device__ __forceinline__ void line_warps_end(LineWork& W, int lane) {
+  if (lane == 0) W.n = -1;
+  line_barrier();
 }
 
 template <int NB, int XT>

@@ -129,3 +129,13 @@ def test_masks(variant):
         ref = pxo.new_image(w, h)
         pxo.fill_path(ref, cmds, [1, 1, 1, 1], 1.0, 0, None, wind)
         assert np.array_equal(m.mask(i), ref[..., 3]), f"mask {i}"
+
+
+@pytest.mark.parametrize("lines", [600, 2200])
+@pytest.mark.parametrize("n,w", [(2, 60), (16, 700), (17, 700), (18, 700), (40, 1100), (64, 700), (65, 700), (66, 700),
+                                 (128, 300), (255, 700), (256, 1100), (257, 700), (600, 1100)])
+def test_paths_of_many_lines(n, w, lines):
+    """A path of so many lines that each row takes a CTA (the lines are
+    horizontal, so the crossings are the zigzag's)."""
+    flat = poly([(10 + k % 7, 3.0) for k in range(lines)])
+    check([joined([zigzag(n, w, 9, 2 * n + 1), flat]), joined([flat, rects(n // 2 + 1, w, 9, 1.0, n)])], w, 9, n)
