@@ -255,6 +255,17 @@ __device__ __forceinline__ float softLight1(float cb, float cs, const float* dsl
   if (cs <= 0.5f) return cb - ((1.0f - 2.0f * cs) * cb) * (1.0f - cb);
   return cb + (2.0f * cs - 1.0f) * (dsl[v] - cb);
 }
+// The mixed colour of a float mode.  Hue: setLum(setSat(cs, sat(cb)), lum(cb));
+// Saturation: setLum(setSat(cb, sat(cs)), lum(cb)); Color: setLum(cs, lum(cb));
+// Luminosity: setLum(cb, lum(cs)).  br, bg, bb: the backdrop's straight bytes.
+__device__ __forceinline__ F3 mix_float(int mode, const float* dsl, F3 cb, F3 cs, uint32_t br, uint32_t bg,
+                                        uint32_t bb) {
+  if (mode == kSoftLight)
+    return F3{softLight1(cb.r, cs.r, dsl, br), softLight1(cb.g, cs.g, dsl, bg), softLight1(cb.b, cs.b, dsl, bb)};
+  F3 c = mode == kHue || mode == kColor ? cs : cb;
+  if (mode == kHue || mode == kSaturation) c = setSat(c, sat3(mode == kHue ? cb : cs));
+  return setLum(c, lum3(mode == kLuminosity ? cs : cb));
+}
 // One float mode (mode a compile-time constant where a kernel is made for it).
 // Over an opaque backdrop -- a canvas or background filled once stays opaque
 // under every blend mode -- the composite needs no division: with ab = 1 the
@@ -273,16 +284,7 @@ __device__ __forceinline__ uint32_t blend_float(int mode, const uint8_t* tbl, ui
   const F3 cb{u[b8.r], u[b8.g], u[b8.b]};
   const F3 cs{u[s8.r], u[s8.g], u[s8.b]};
   const float as = u[s8.a];
-  F3 m;
-  if (mode == kSoftLight) {
-    m = F3{softLight1(cb.r, cs.r, dsl, b8.r), softLight1(cb.g, cs.g, dsl, b8.g), softLight1(cb.b, cs.b, dsl, b8.b)};
-  } else {
-    // Hue: setLum(setSat(cs, sat(cb)), lum(cb)); Saturation: setLum(setSat(cb, sat(cs)), lum(cb));
-    // Color: setLum(cs, lum(cb)); Luminosity: setLum(cb, lum(cs))
-    F3 c = mode == kHue || mode == kColor ? cs : cb;
-    if (mode == kHue || mode == kSaturation) c = setSat(c, sat3(mode == kHue ? cb : cs));
-    m = setLum(c, lum3(mode == kLuminosity ? cs : cb));
-  }
+  const F3 m = mix_float(mode, dsl, cb, cs, b8.r, b8.g, b8.b);
   if (b8.a == 255) {
     const float k = 1.0f - as;
     return pack(unit_to_u8(as * m.r + k * cb.r), unit_to_u8(as * m.g + k * cb.g), unit_to_u8(as * m.b + k * cb.b),
@@ -328,6 +330,22 @@ __device__ __forceinline__ uint32_t fdiv_floor(float n, float d, float rd) {
   qi += rem >= d ? 1u : 0u;
   return qi;
 }
+// A channel of ColorBurn / ColorDodge (blends.nim:111-126, :158-173), straight
+// values; burn is 255 - dodge of the complements.
+__device__ __forceinline__ uint32_t mix_burn_dodge(bool burn, uint32_t b, uint32_t s) {
+  const uint32_t flip = burn ? 255u : 0u;
+  b ^= flip;
+  s ^= flip;
+  uint32_t v = 0;
+  if (b != 0) {
+    v = 255;
+    if (s != 255) {
+      const float df = small_to_f(255u - s);
+      v = min(fdiv_floor(small_to_f(255u * b), df, rcp_approx(df)), 255u);
+    }
+  }
+  return v ^ flip;
+}
 // ColorBurn / ColorDodge (blends.nim:111-126, :158-173) with the divisions
 // done as above: the same integers as the reference's integer divisions.
 // Burn is 255 - dodge of the complements.  Over an opaque backdrop (2048 x 2048
@@ -336,20 +354,7 @@ __device__ __forceinline__ uint32_t fdiv_floor(float n, float d, float rd) {
 // (sa m + (255 - sa) b) / 255, and the result's alpha is 255.
 __device__ __forceinline__ uint32_t blend_burn_dodge(bool burn, const uint8_t* tbl, uint32_t bv, uint32_t sv) {
   const Px bd = straight8(tbl, bv), sr = straight8(tbl, sv);
-  const uint32_t flip = burn ? 255u : 0u;
-  auto mix = [&](uint32_t b, uint32_t s) -> uint32_t {
-    b ^= flip;
-    s ^= flip;
-    uint32_t v = 0;
-    if (b != 0) {
-      v = 255;
-      if (s != 255) {
-        const float df = small_to_f(255u - s);
-        v = min(fdiv_floor(small_to_f(255u * b), df, rcp_approx(df)), 255u);
-      }
-    }
-    return v ^ flip;
-  };
+  auto mix = [&](uint32_t b, uint32_t s) { return mix_burn_dodge(burn, b, s); };
   const uint32_t mr = mix(bd.r, sr.r), mg = mix(bd.g, sr.g), mb = mix(bd.b, sr.b);
   // alphaFix (blends.nim:18-39): (t0 src + t1 mixed + t2 backdrop) / a / 255 = ... / (255 a)
   const uint32_t sa = sr.a, ba = bd.a;
@@ -369,6 +374,110 @@ __device__ __forceinline__ uint32_t blend_burn_dodge(bool burn, const uint8_t* t
 template <bool BURN>
 __device__ __forceinline__ uint32_t blendBurnDodge(const uint8_t* tbl, uint32_t bv, uint32_t sv) {
   return blend_burn_dodge(BURN, tbl, bv, sv);
+}
+
+// v / 255.0f correctly rounded (every byte checked against the exact quotient):
+// 1 / 255 as the sum of two floats, one product rounded by the FMA.
+__device__ __forceinline__ float unit_f(uint32_t v) {
+  const float f = small_to_f(v);
+  return fmaf(f, 0x1.010102p-8f, f * -0x1.fdfdfep-33f);
+}
+// Whether a source's channels are no larger than its alpha.
+__device__ __forceinline__ bool premultiplied(uint32_t s) {
+  const uint32_t a = s >> 24;
+  return (s & 255u) <= a && ((s >> 8) & 255u) <= a && ((s >> 16) & 255u) <= a;
+}
+// mul_c without its shortcuts: the same bytes for every k
+__device__ __forceinline__ uint32_t mul_c_flat(uint32_t c, uint32_t k) {
+  return div255_lanes((c & 0x00FF00FFu) * k + 0x007F007Fu) |
+         (div255_lanes(((c >> 8) & 0x00FF00FFu) * k + 0x007F007Fu) << 8);
+}
+// blendNormal without its shortcuts but the one over a backdrop of alpha 0
+// (whose colour need not be 0), for premultiplied sources; where the pixel is
+// not drawn (on = false) the source is 0 and the backdrop stays.
+__device__ __forceinline__ uint32_t blend_normal_flat(uint32_t bv, uint32_t sv, bool on) {
+  const uint32_t k = 255 - (sv >> 24);
+  const uint32_t rb = div255_lanes((bv & 0x00FF00FFu) * k) + (sv & 0x00FF00FFu);
+  const uint32_t ga = div255_lanes(((bv >> 8) & 0x00FF00FFu) * k) + ((sv >> 8) & 0x00FF00FFu);
+  const uint32_t v = rb | (ga << 8);
+  return on && bv < 0x01000000u ? sv : v;
+}
+// The 16 colour modes (mode < kMask) over an opaque backdrop with a
+// premultiplied source.  The backdrop's straight colour is itself, the result
+// is opaque, and the terms of the general formulas (blends.nim:72-213) with a
+// factor 255 - 255 vanish; what is left of the integer modes but Exclusion is
+// one quotient floor(backdrop * M / 255) a channel, with M <= 255 (<= 510
+// where the backdrop is <= 127), so the products fit 16-bit lanes.
+__device__ __forceinline__ uint32_t blend_opaque(int mode, const uint8_t* tbl, uint32_t bv, uint32_t sv) {
+  const uint32_t sa = sv >> 24, sk = 255 - sa;
+  const uint32_t br = bv & 255u, bg = (bv >> 8) & 255u, bb = (bv >> 16) & 255u;
+  const uint32_t sr = sv & 255u, sg = (sv >> 8) & 255u, sb = (sv >> 16) & 255u;
+  const uint32_t Brb = bv & 0x00FF00FFu, Srb = sv & 0x00FF00FFu;
+  uint32_t rb, gg;
+  switch (mode) {
+    case kNormal:
+    case kDarken:  // min, max of the backdrop and s + floor(b (255 - sa) / 255)
+    case kLighten: {
+      rb = div255_lanes(Brb * sk) + Srb;
+      gg = div255_lanes(bg * sk) + sg;
+      if (mode == kDarken) {
+        rb = __vminu2(rb, Brb);
+        gg = min(gg, bg);
+      } else if (mode == kLighten) {
+        rb = __vmaxu2(rb, Brb);
+        gg = max(gg, bg);
+      }
+      break;
+    }
+    case kMultiply:
+      rb = div255_lanes(br * (sk + sr) + ((bb * (sk + sb)) << 16));
+      gg = div255_lanes(bg * (sk + sg));
+      break;
+    case kScreen:
+      rb = Brb + Srb - div255_lanes(br * sr + ((bb * sb) << 16));
+      gg = bg + sg - div255_lanes(bg * sg);
+      break;
+    case kOverlay:
+    case kHardLight: {  // multiply with 2 s + 255 - sa, or screen
+      const bool over = mode == kOverlay;
+      const bool r = over ? br < 128 : 2 * sr <= sa, g = over ? bg < 128 : 2 * sg <= sa;
+      const bool b = over ? bb < 128 : 2 * sb <= sa;
+      const uint32_t qrb = div255_lanes(br * (r ? 2 * sr + sk : sr) + ((bb * (b ? 2 * sb + sk : sb)) << 16));
+      const uint32_t qg = div255_lanes(bg * (g ? 2 * sg + sk : sg));
+      const uint32_t m = (r ? 0xFFFFu : 0u) | (b ? 0xFFFF0000u : 0u);
+      rb = (qrb & m) | ((Brb + Srb - qrb) & ~m);
+      gg = g ? qg : bg + sg - qg;
+      break;
+    }
+    case kDifference:  // b + s - 2 min(floor(b sa / 255), s), as uint8
+      rb = (Brb + Srb - 2 * __vminu2(div255_lanes(Brb * sa), Srb)) & 0x00FF00FFu;
+      gg = (bg + sg - 2 * min(div255_lanes(bg * sa), sg)) & 255u;
+      break;
+    case kExclusion:  // b + s - floor(2 b s / 255) >= 0
+      rb = (br + sr - (2 * br * sr) / 255) | ((bb + sb - (2 * bb * sb) / 255) << 16);
+      gg = bg + sg - (2 * bg * sg) / 255;
+      break;
+    case kColorBurn:
+    case kColorDodge: {  // alphaFix: floor((sa mixed + (255 - sa) backdrop) / 255)
+      const uint8_t* row = tbl + sa * 256;
+      const bool burn = mode == kColorBurn;
+      const uint32_t mr = mix_burn_dodge(burn, br, row[sr]), mg = mix_burn_dodge(burn, bg, row[sg]);
+      const uint32_t mb = mix_burn_dodge(burn, bb, row[sb]);
+      rb = div255_lanes((mr | (mb << 16)) * sa + Brb * sk);
+      gg = div255_lanes(mg * sa + bg * sk);
+      break;
+    }
+    default: {  // blend_float's opaque case
+      const uint8_t* row = tbl + sa * 256;
+      const F3 cb{unit_f(br), unit_f(bg), unit_f(bb)}, cs{unit_f(row[sr]), unit_f(row[sg]), unit_f(row[sb])};
+      const F3 m = mix_float(mode, reinterpret_cast<const float*>(tbl + kTblSoftOff), cb, cs, br, bg, bb);
+      const float as = unit_f(sa), k = 1.0f - as;
+      rb = unit_to_u8(as * m.r + k * cb.r) | (unit_to_u8(as * m.b + k * cb.b) << 16);
+      gg = unit_to_u8(as * m.g + k * cb.g);
+      break;
+    }
+  }
+  return rb | (gg << 8) | 0xFF000000u;
 }
 
 // blender(mode)(backdrop, source)  blends.nim:275-299

@@ -1258,7 +1258,13 @@ static __device__ __noinline__ unsigned draw_program(RowPx<false> row, int mode,
 // costs its coverage bytes (one word per lane, requested a path ahead, dealt
 // out by shuffles) and no pixel traffic; 32-pixel groups a path does not touch
 // are skipped, and each mode's blend exists once (the lane's pixels rotate
-// through it), which keeps the kernel within the instruction cache.  PPL = 4;
+// through it), which keeps the kernel within the instruction cache.  What a
+// path costs besides its blends -- 250 of 290 us for 100 paths of one mode over
+// 1024 x 1024 before, 200 of 240 now -- is kept in two words worked out for 32
+// paths at once, groups of full coverage take the colour as it is, Normal runs
+// through its groups without a branch on the pixels, and steps that were opaque
+// take blend_opaque: 2000 paths 9.65 -> 8.45 ms, 240 local ones 0.16 -> 0.138,
+// Color of 100 paths 0.66 -> 0.54, Screen 0.34 -> 0.31.  PPL = 4;
 // PPL = 1 for launches with too few rows to fill the GPU, where a path's time
 // on its warp matters and not the instructions per pixel.
 template <int PPL, int WARPS>
@@ -1299,7 +1305,13 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
       const int xb = min(xa + SW, xe);
       uint32_t p[PPL];
 #pragma unroll
-      for (int i = 0; i < PPL; i++) p[i] = xa + i * 32 + lane < xb ? grow[xa + i * 32 + lane] : 0u;
+      for (int i = 0; i < PPL; i++) p[i] = xa + i * 32 + lane < xb ? grow[xa + i * 32 + lane] : 0xFF000000u;
+      // whether every pixel of the step is opaque: the colour modes leave it so,
+      // a mask mode ends it
+      bool solid = true;
+#pragma unroll
+      for (int i = 0; i < PPL; i++) solid &= p[i] >= 0xFF000000u;
+      solid = __all_sync(0xffffffffu, solid);
       // 32 paths at a time: each lane loads one path's row header (contiguous
       // over the paths) and colour, then the warp applies them in path order
 #pragma unroll 1
@@ -1314,57 +1326,85 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
         const int st = (int)(in.y >> 8);
         const unsigned bad = __ballot_sync(0xffffffffu, st != kOk && st != kNothing);
         const int lim = bad ? __ffs(bad) - 1 : 32;
-        unsigned dm = __ballot_sync(0xffffffffu, lane < lim && st == kOk && h.x != 0 && h.z < xb && h.w > xa);
+        const bool draws = lane < lim && st == kOk && h.x != 0 && h.z < xb && h.w > xa;
+        unsigned dm = __ballot_sync(0xffffffffu, draws);
+        // what the warp needs of a path, in two words: the step's pixels it may
+        // touch, kind, mode, whether its colour is premultiplied and whether it
+        // meets opaque pixels besides (decided for the step and not for each 32
+        // pixels, for warps that go through both forms of the blends wait for
+        // instructions); and where its coverage would begin at the multiple of 16
+        // pixels up to the step's first (16-byte units: rows of coverage begin at
+        // such multiples and hold whole units, the bytes past the last pixel 0)
+        const int mode0 = (int)(in.y & 255u);
+        const bool plain0 = mode0 < kMask && premultiplied(in.x);
+        const unsigned masks = __ballot_sync(0xffffffffu, draws && mode0 >= kMask);
+        const uint32_t pack0 = (uint32_t)max(h.z - xa, 0) | ((uint32_t)min(h.w - xa, xb - xa) << 8) |
+                               ((uint32_t)h.x << 16) | ((uint32_t)mode0 << 20) | (plain0 ? 1u << 30 : 0u) |
+                               (plain0 && solid && (masks & ((1u << lane) - 1)) == 0 ? 1u << 31 : 0u);
+        solid &= masks == 0;
+        int unit0 = h.y;
+        if (draws && h.x == kRecCov8Z) unit0 = A.prog[(unsigned)h.y].x;
+        unit0 += ((xa & ~15) - h.z) >> 4;
         int next = -1;      // the path after the current one, and its coverage
-        uint32_t nextCov = 0;
-        bool first = true;
+        uint32_t nextCov = 0, nextPack = 0;
 #pragma unroll 1
-        while (true) {
+        while (dm || next >= 0) {
           const int cur = next;
-          const uint32_t cov = nextCov;
+          const uint32_t cov = nextCov, pk = nextPack;
           next = -1;
           if (dm) {
             next = __ffs(dm) - 1;
             dm &= dm - 1;
-            const int kind = __shfl_sync(0xffffffffu, h.x, next), hlo = __shfl_sync(0xffffffffu, h.z, next);
-            const int hhi = __shfl_sync(0xffffffffu, h.w, next), x = xa + 4 * lane;
-            unsigned unit = (unsigned)__shfl_sync(0xffffffffu, h.y, next);
+            nextPack = __shfl_sync(0xffffffffu, pack0, next);
+            const unsigned unit = (unsigned)__shfl_sync(0xffffffffu, unit0, next);
+            const int kind = (int)(nextPack >> 16) & 15, lo = (int)(nextPack & 255u), hi = (int)(nextPack >> 8) & 255;
+            const int x = 4 * lane;
             nextCov = 0;
             if (kind == kRecFill) {
-              const int b0 = min(max(hlo - x, 0), 4), b1 = min(max(min(hhi, xb) - x, 0), 4);
+              const int b0 = min(max(lo - x, 0), 4), b1 = min(max(hi - x, 0), 4);
               if (b1 > b0) nextCov = (uint32_t)((1ull << (8 * b1)) - (1ull << (8 * b0)));
-            } else if (kind != kRecProg) {
-              if (kind == kRecCov8Z) unit = (unsigned)A.prog[unit].x;
-              // whole words: lo is a multiple of 16, the bytes past hi are zero
-              if (lane < 8 * PPL && x >= hlo && x < hhi && x < xb)
-                nextCov = *reinterpret_cast<const uint32_t*>(A.cov8 + ((long long)unit << 4) + (x - hlo));
+            } else if (kind != kRecProg && x >= lo && x < hi) {
+              const int xu = x + (xa & 15);
+              nextCov = *reinterpret_cast<const uint32_t*>(A.cov8 + ((long long)(unit + (xu >> 4)) << 4) + (xu & 15));
             }
           }
-          if (cur < 0) {
-            if (!first || next < 0) break;
-            first = false;
-            continue;
-          }
-          first = false;
+          if (cur < 0) continue;
           const uint32_t col = __shfl_sync(0xffffffffu, in.x, cur);
-          const int mode = (int)(__shfl_sync(0xffffffffu, in.y, cur) & 255u);
-          if (__any_sync(0xffffffffu, cov != 0)) {
+          const int mode = (int)(pk >> 20) & 255;
+          // the lanes with coverage, and with nothing but 255: eight lanes' words
+          // cover a group of 32 pixels
+          unsigned some = __ballot_sync(0xffffffffu, cov != 0), full = __ballot_sync(0xffffffffu, cov == 0xffffffffu);
+          painted += __popc((((cov & 0x7f7f7f7fu) + 0x7f7f7f7fu) | cov) & 0x80808080u);  // its bytes above 0
+          if (((pk >> 20) & 0x4ffu) == 0x400u) {  // Normal, premultiplied
+            if (some) {
+#pragma unroll
+              for (int i = 0; i < PPL; i++) {
+                if (((some >> (8 * i)) & 255u) == 0) continue;
+                uint32_t k = 255, s = col;
+                if (((full >> (8 * i)) & 255u) != 255u) {
+                  k = (__shfl_sync(0xffffffffu, cov, i * 8 + (lane >> 2)) >> (8 * (lane & 3))) & 255u;
+                  s = mul_c_flat(col, k);
+                }
+                p[i] = blend_normal_flat(p[i], s, k != 0);
+              }
+            }
+          } else if (some) {
 #pragma unroll 1
             for (int i = 0; i < PPL; i++) {
-              const uint32_t k = (__shfl_sync(0xffffffffu, cov, i * 8 + (lane >> 2)) >> (8 * (lane & 3))) & 255u;
               uint32_t v = p[0];
-              const unsigned on = __ballot_sync(0xffffffffu, k != 0);
-              painted += __popc(on);
-              if (k) {
-                const uint32_t s = mul_c(col, k);
-                v = mode == kNormal ? blendNormal(v, s) : blend_px(mode, tbl, v, s);
+              if (some & 255u) {
+                const uint32_t k = (__shfl_sync(0xffffffffu, cov, i * 8 + (lane >> 2)) >> (8 * (lane & 3))) & 255u;
+                const uint32_t s = (full & 255u) == 255u ? col : mul_c_flat(col, k);
+                if (k) v = (int)pk < 0 ? blend_opaque(mode, tbl, v, s) : blend_px(mode, tbl, v, s);
               }
+              some >>= 8;
+              full >>= 8;
 #pragma unroll
               for (int t = 0; t + 1 < PPL; t++) p[t] = p[t + 1];
               p[PPL - 1] = v;
             }
           }
-          const int ck = __shfl_sync(0xffffffffu, h.x, cur);
+          const int ck = (int)(pk >> 16) & 15;
           if (ck != kRecCov8Z && ck != kRecProg) continue;
           const int cp = __shfl_sync(0xffffffffu, h.y, cur);
           if (ck == kRecCov8Z) {  // and the listed pixels with an empty source
@@ -1373,7 +1413,7 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
             for (int z = 0; z < nz; z++) {
               const int x = reinterpret_cast<const int*>(A.prog + cp + 1)[z];
               if (x < xa || x >= xb) continue;
-              ++painted;
+              if (lane == 0) ++painted;
 #pragma unroll
               for (int i = 0; i < PPL; i++)
                 if (xa + i * 32 + lane == x) p[i] = blend_any(mode, tbl, p[i], 0u);
@@ -1386,7 +1426,8 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
           __syncwarp();
           const RowPx<false> row{reinterpret_cast<unsigned char*>(pix[warp]), xa};
           const int plo = __shfl_sync(0xffffffffu, h.z, cur), phi = __shfl_sync(0xffffffffu, h.w, cur);
-          painted += draw_program<SW>(row, mode, tbl, col, A.prog + cp, plo, phi, y, W, xa, xb, accs[warp], lane);
+          const unsigned drawn = draw_program<SW>(row, mode, tbl, col, A.prog + cp, plo, phi, y, W, xa, xb, accs[warp], lane);
+          if (lane == 0) painted += drawn;
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < PPL; i++) p[i] = pix[warp][i * 32 + lane];
@@ -1398,6 +1439,7 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
       for (int i = 0; i < PPL; i++)
         if (xa + i * 32 + lane < xb) grow[xa + i * 32 + lane] = p[i];
     }
+    painted = __reduce_add_sync(0xffffffffu, painted);
     if (lane == 0 && painted) atomicAdd(&A.counters[kCtrPainted], (unsigned long long)painted);
   }
 }
