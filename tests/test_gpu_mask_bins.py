@@ -38,3 +38,20 @@ def test_ordered_composite(n, w, h, mode):
     for (x, y), s in zip(at[1:], pick[1:]):
         pxo.draw(ref, s[4], int(x), int(y), mode)
     assert np.array_equal(img.to_numpy(), ref)
+
+
+def test_batches_rendered_again():
+    """The first rendering is issued as launches, later ones replay a graph."""
+    m = px.Masks()
+    paths = []
+    for step in range(3):
+        w, h = 20 + 13 * step, 31 - 5 * step
+        cmds = np.asarray([1, 1.3, 2, 2, w - 2.6, 3.1, 2, w * 0.5, h - 1.4, 0], np.float32)
+        paths.append((cmds, w, h))
+        m.add_path(cmds, w, h)
+        for _ in range(3):
+            m.render()
+            for i, (c, cw, ch) in enumerate(paths):
+                ref = pxo.new_image(cw, ch)
+                pxo.fill_path(ref, c, [1, 1, 1, 1], 1.0, 0, None, 0)
+                assert np.array_equal(m.mask(i), ref[..., 3])
