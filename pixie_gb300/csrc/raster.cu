@@ -1313,9 +1313,14 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
       for (int i = 0; i < PPL; i++) solid &= p[i] >= 0xFF000000u;
       solid = __all_sync(0xffffffffu, solid);
       // 32 paths at a time: each lane loads one path's row header (contiguous
-      // over the paths) and colour, then the warp applies them in path order
+      // over the paths) and colour, then the warp applies them in path order.
+      // Rows with more to them than coverage leave the loop, and it is entered
+      // again behind them (path `from` of the 32): with their calls inside it,
+      // its state went through local memory.
+      int c0 = 0, from = 0;
 #pragma unroll 1
-      for (int c0 = 0; c0 < njobs; c0 += 32) {
+      while (c0 < njobs) {
+        int stop = -1;
         uint2 in = make_uint2(0u, (uint32_t)kNothing << 8);
         int4 h = make_int4(0, 0, 0, 0);
         if (c0 + lane < njobs) {
@@ -1326,7 +1331,7 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
         const int st = (int)(in.y >> 8);
         const unsigned bad = __ballot_sync(0xffffffffu, st != kOk && st != kNothing);
         const int lim = bad ? __ffs(bad) - 1 : 32;
-        const bool draws = lane < lim && st == kOk && h.x != 0 && h.z < xb && h.w > xa;
+        const bool draws = lane >= from && lane < lim && st == kOk && h.x != 0 && h.z < xb && h.w > xa;
         unsigned dm = __ballot_sync(0xffffffffu, draws);
         // what the warp needs of a path, in two words: the step's pixels it may
         // touch, kind, mode, whether its colour is premultiplied and whether it
@@ -1405,35 +1410,45 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const Sc
             }
           }
           const int ck = (int)(pk >> 16) & 15;
-          if (ck != kRecCov8Z && ck != kRecProg) continue;
-          const int cp = __shfl_sync(0xffffffffu, h.y, cur);
-          if (ck == kRecCov8Z) {  // and the listed pixels with an empty source
-            const int nz = A.prog[cp].y;
-#pragma unroll 1
-            for (int z = 0; z < nz; z++) {
-              const int x = reinterpret_cast<const int*>(A.prog + cp + 1)[z];
-              if (x < xa || x >= xb) continue;
-              if (lane == 0) ++painted;
-#pragma unroll
-              for (int i = 0; i < PPL; i++)
-                if (xa + i * 32 + lane == x) p[i] = blend_any(mode, tbl, p[i], 0u);
-            }
-            continue;
+          if (ck == kRecCov8Z || ck == kRecProg) {
+            stop = cur;
+            break;
           }
-          // a program: the general code, on the step's pixels in shared memory
-#pragma unroll
-          for (int i = 0; i < PPL; i++) pix[warp][i * 32 + lane] = p[i];
-          __syncwarp();
-          const RowPx<false> row{reinterpret_cast<unsigned char*>(pix[warp]), xa};
-          const int plo = __shfl_sync(0xffffffffu, h.z, cur), phi = __shfl_sync(0xffffffffu, h.w, cur);
-          const unsigned drawn = draw_program<SW>(row, mode, tbl, col, A.prog + cp, plo, phi, y, W, xa, xb, accs[warp], lane);
-          if (lane == 0) painted += drawn;
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < PPL; i++) p[i] = pix[warp][i * 32 + lane];
-          __syncwarp();
         }
-        if (bad) break;
+        if (stop < 0) {
+          if (bad) break;
+          c0 += 32;
+          from = 0;
+          continue;
+        }
+        // the general code, on the step's pixels in shared memory
+        const int path = c0 + stop;
+        from = stop + 1;  // 32: nothing of these paths is left
+#pragma unroll
+        for (int i = 0; i < PPL; i++) pix[warp][i * 32 + lane] = p[i];
+        __syncwarp();
+        const int4 ph = hdr[path];
+        const uint2 pi = info[path];
+        const int pmode = (int)(pi.y & 255u);
+        if (ph.x == kRecCov8Z) {  // the listed pixels with an empty source
+          const int nz = A.prog[ph.y].y;
+#pragma unroll 1
+          for (int z = 0; z < nz && lane == 0; z++) {
+            const int x = reinterpret_cast<const int*>(A.prog + ph.y + 1)[z];
+            if (x < xa || x >= xb) continue;
+            ++painted;
+            pix[warp][x - xa] = blend_any(pmode, tbl, pix[warp][x - xa], 0u);
+          }
+        } else {
+          const RowPx<false> row{reinterpret_cast<unsigned char*>(pix[warp]), xa};
+          const unsigned drawn = draw_program<SW>(row, pmode, tbl, pi.x, A.prog + ph.y, ph.z, ph.w, y, W, xa, xb,
+                                                  accs[warp], lane);
+          if (lane == 0) painted += drawn;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < PPL; i++) p[i] = pix[warp][i * 32 + lane];
+        __syncwarp();
       }
 #pragma unroll
       for (int i = 0; i < PPL; i++)
