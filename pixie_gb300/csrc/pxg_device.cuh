@@ -8,6 +8,7 @@
 #include <initializer_list>
 #include <utility>
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 namespace pxg {
@@ -255,6 +256,11 @@ __device__ __forceinline__ float softLight1(float cb, float cs, const float* dsl
   if (cs <= 0.5f) return cb - ((1.0f - 2.0f * cs) * cb) * (1.0f - cb);
   return cb + (2.0f * cs - 1.0f) * (dsl[v] - cb);
 }
+// Whether the condition holds for every thread of the warp that is here with
+// this one: the special cases below are worth a branch only when no lane
+// needs the general form besides (both give the same bytes).
+__device__ __forceinline__ bool all_together(bool c) { return cooperative_groups::coalesced_threads().all(c); }
+
 // The mixed colour of a float mode.  Hue: setLum(setSat(cs, sat(cb)), lum(cb));
 // Saturation: setLum(setSat(cb, sat(cs)), lum(cb)); Color: setLum(cs, lum(cb));
 // Luminosity: setLum(cb, lum(cs)).  br, bg, bb: the backdrop's straight bytes.
@@ -277,6 +283,10 @@ __device__ __forceinline__ F3 mix_float(int mode, const float* dsl, F3 cb, F3 cs
 // 31.3 -> 24.4; over images of every alpha 29.0 -> 26.6, 38.6 -> 36.1,
 // 41.5 -> 39.1, 29.8 -> 27.2, 32.3 -> 29.6.  (Gathers from the tables under a
 // test for opaque pixels cost more than they save: they no longer overlap.)
+// A warp with both kinds of pixels takes the general form for all: with a form
+// for each, images that twenty modes in turn have left opaque in part took 45 us
+// of SoftLight at 2048 x 2048 instead of 41, 60 of Saturation instead of 56 (one
+// launch at a time).
 __device__ __forceinline__ uint32_t blend_float(int mode, const uint8_t* tbl, uint32_t bp, uint32_t sp) {
   const Px b8 = straight8(tbl, bp), s8 = straight8(tbl, sp);
   const float* u = reinterpret_cast<const float*>(tbl + kTblUnitOff);  // u[v] = v / 255.0f
@@ -285,7 +295,7 @@ __device__ __forceinline__ uint32_t blend_float(int mode, const uint8_t* tbl, ui
   const F3 cs{u[s8.r], u[s8.g], u[s8.b]};
   const float as = u[s8.a];
   const F3 m = mix_float(mode, dsl, cb, cs, b8.r, b8.g, b8.b);
-  if (b8.a == 255) {
+  if (all_together(b8.a == 255)) {
     const float k = 1.0f - as;
     return pack(unit_to_u8(as * m.r + k * cb.r), unit_to_u8(as * m.g + k * cb.g), unit_to_u8(as * m.b + k * cb.b),
                 255u);
@@ -358,7 +368,7 @@ __device__ __forceinline__ uint32_t blend_burn_dodge(bool burn, const uint8_t* t
   const uint32_t mr = mix(bd.r, sr.r), mg = mix(bd.g, sr.g), mb = mix(bd.b, sr.b);
   // alphaFix (blends.nim:18-39): (t0 src + t1 mixed + t2 backdrop) / a / 255 = ... / (255 a)
   const uint32_t sa = sr.a, ba = bd.a;
-  if (ba == 255) {
+  if (all_together(ba == 255)) {
     const uint32_t sk = 255 - sa;
     return pack((sa * mr + sk * bd.r) / 255, (sa * mg + sk * bd.g) / 255, (sa * mb + sk * bd.b) / 255, 255u);
   }
