@@ -475,7 +475,7 @@ class Scene:
 class Masks:
     """A batch of 8-bit masks: add_path(path, width, height) fills the path
     with color(1, 1, 1, 1) on a transparent width x height image and keeps its
-    alpha; render() renders the whole batch on the GPU (one graph launch);
+    alpha; render() renders the whole batch on the GPU (rendered again: one graph launch);
     Image.draw_masks composites them in order."""
 
     def __init__(self):

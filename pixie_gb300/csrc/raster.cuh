@@ -3,10 +3,10 @@
 //
 // One fill job = one call of fillShapes on one RGBX image.  The host turns the
 // path commands into primitives (lines, quadratics, cubics; arcs and stroke
-// outlines arrive as lines), the setup kernel (one CTA per job) flattens them
+// outlines arrive as lines), the setup kernel (a cluster of CTAs per job) flattens them
 // into pixie's segments, reduces the bounds and derives the row-band
 // partitions (each band's entry list in segment order, its count and
-// anti-aliasing flag); the row kernel (one warp per image row) reads its
+// anti-aliasing flag); the row kernels (a warp per chunk of rows, or a CTA per row) read their
 // band's entries, runs the reference's per-row decision and writes the
 // pixels.
 #pragma once
