@@ -531,10 +531,14 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
     int status = kOk;
     if (pathWidth == 0) status = kNothing;
     else if (pathWidth < 0) status = kErrIntOverflow;
-    long long height = pathHeight - startY;
+    // A path wholly above or below the image, or one whose end is past 2^63 (the
+    // conversion's minimum then), draws no row and needs no partition.  The row
+    // kernels hold rows in 32 bits: theirs are within the image from here on.
+    if (pathHeight <= startY) startY = pathHeight = 0;
+    const long long height = pathHeight - startY;
     uint32_t maxP = (uint32_t)max(1LL, height / 4);
     uint32_t numP = min(maxP, (uint32_t)max(1, nseg / 2));
-    uint32_t ph = (uint32_t)height / numP;
+    uint32_t ph = max(1u, (uint32_t)height / numP);
     if (status == kOk && numP > (uint32_t)maxBands) status = kErrArenaFull;
     s_hdr[0] = status;
     s_hdr[1] = (int)numP;

@@ -1,0 +1,51 @@
+"""The setup kernel at the limits of its arithmetic: paths whose rows lie outside
+what the image, 32 bits or 64 bits hold, byte for byte against the oracle."""
+import numpy as np
+import pytest
+
+import pixie_gb300 as px
+from oracle import pxo
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _init():
+    px.lib().pxg_init(0)
+    pxo.set_golden_mode(False)
+
+
+def zigzag(n, w, y0, y1):
+    """n lines between the heights y0 and y1, closed."""
+    x = np.linspace(0.3, w - 0.4, n + 1)
+    cmds = [1.0, x[0], y0]
+    for k in range(1, n + 1):
+        cmds += [2.0, x[k], y1 if k & 1 else y0]
+    return np.asarray(cmds + [0.0], np.float32)
+
+
+def check(cmds, w, h, modes=(0,)):
+    """A fill, with the modes of a fill path and of a clearing mask, and a scene."""
+    for mode in modes:
+        back = np.random.RandomState(7).randint(0, 256, (h, w, 4)).astype(np.uint8)
+        back[..., :3] = np.minimum(back[..., :3], back[..., 3:])
+        ref = back.copy()
+        pxo.fill_path(ref, cmds, [0.1, 0.7, 0.4, 0.8], 1.0, mode, None, 0)
+        paint = px.Paint(color=(0.1, 0.7, 0.4, 0.8), blend_mode=px.BlendMode(mode))
+        img = px.Image.from_numpy(back)
+        img.fill_path(cmds, paint)
+        assert np.array_equal(img.to_numpy(), ref)
+        sc = px.Scene()
+        sc.fill_path(cmds, paint)
+        img = px.Image.from_numpy(back)
+        img.draw_scene(sc)
+        assert np.array_equal(img.to_numpy(), ref)
+
+
+# the path's last row is past 2^63, its first one in the image; or all rows are far below or above it
+@pytest.mark.parametrize("y0,y1", [(240.0, 1.0e19), (0.0, 3.0e38), (394.75, 3.0e38), (4294967296.0, 4294970000.0),
+                                   (4294967396.0, 9.0e9), (-4294967296.0, -4294967000.0), (-9.0e9, -4294967000.0),
+                                   (-3.0e38, -1.0e19), (400.0, 500.0), (-9.0, 0.0), (1.0e19, 1.0e20)])
+@pytest.mark.parametrize("n", [2, 40, 301, 3000])
+def test_rows_out_of_range(n, y0, y1):
+    check(zigzag(n, 37, y0, y1), 37, 400, (0, 16))
