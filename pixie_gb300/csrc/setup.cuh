@@ -574,7 +574,9 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
 
   // each band's entry count and anti-aliasing flag (:1215-1234): every warp
   // owns a contiguous run of the CTA's segments and counts them as differences
-  // over the bands, so a segment costs two additions however tall it is
+  // over the bands, so a segment costs two additions however tall it is.  A
+  // range may be empty (its first band above its last): a y of 2^32 or more
+  // wraps in partitionRange's conversion, and the segment is in no band.
   const int stride = (int)numP + 1;
   int* mine = wc + warp * stride;
   uint32_t* mask = wm + warp * stride;
@@ -600,6 +602,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
     const float4 sg = A.segs[seg0 + i];
     const uint2 r = bandRange(sg);
     A.segband[seg0 + i] = r;
+    if (r.x > r.y) continue;
     atomicAdd(&counts[r.x], 1);
     atomicAdd(&counts[r.y + 1], -1);
     if (segRequiresAA(sg)) {

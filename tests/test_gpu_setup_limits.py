@@ -1,5 +1,7 @@
 """The setup kernel at the limits of its arithmetic: paths whose rows lie outside
-what the image, 32 bits or 64 bits hold, byte for byte against the oracle."""
+what the image, 32 bits or 64 bits hold, and segments whose band range is empty
+because a coordinate wraps in the reference's 32-bit conversion, byte for byte
+against the oracle."""
 import numpy as np
 import pytest
 
@@ -49,3 +51,20 @@ def check(cmds, w, h, modes=(0,)):
 @pytest.mark.parametrize("n", [2, 40, 301, 3000])
 def test_rows_out_of_range(n, y0, y1):
     check(zigzag(n, 37, y0, y1), 37, 400, (0, 16))
+
+
+# 2^32 and above wrap to small bands; from 2^63 on the conversion yields its minimum
+@pytest.mark.parametrize("far", [4294967296.0, 4294967296.0 + 1024, 3.0e10, 9.0e18, 1.0e19, 3.0e38])
+@pytest.mark.parametrize("n,h", [(2, 400), (40, 400), (301, 400), (3000, 333), (300, 5000)])
+def test_segments_in_no_band(n, h, far):
+    w = 37
+    rs = np.random.RandomState(n + h)
+    for near in (h * 0.6, h - 5.25):
+        cmds = zigzag(n, w, near, far)[:-1]
+        # and a shape of ordinary segments besides
+        pts = rs.rand(6, 2) * (w, h)
+        cmds = np.concatenate([cmds, [0.0, 1.0, *pts[0]], *[[2.0, *p] for p in pts[1:]], [0.0]]).astype(np.float32)
+        try:
+            check(cmds, w, h)
+        except px.PixieError as e:  # the library's limit of 2048 crossings a row
+            assert n > 2048 and "Path too complex" in str(e)
