@@ -564,7 +564,8 @@ const char* status_message(int st) {
     case kErrIntOverflow: return "Path int overflow detected";
     case kErrIterLimit: return "Unable to discretize: flattening did not converge";
     case kErrRowTooComplex: return "Path too complex: a scanline crosses more than 4096 edges";
-    case kErrArenaFull: return "Out of workspace memory";
+    case kErrArenaFull:
+    case kErrTooManyEntries: return "Out of workspace memory";
   }
   return "Unknown error";
 }

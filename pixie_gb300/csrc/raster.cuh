@@ -42,7 +42,8 @@ enum JobStatus {
   kErrIntOverflow = 4,     // "Path int overflow detected"
   kErrArenaFull = 5,       // workspace too small: grow and rerun
   kErrIterLimit = 6,       // flattening did not converge within the iteration cap
-  kErrRowTooComplex = 7    // a row crosses more edges than the largest row kernel holds
+  kErrRowTooComplex = 7,   // a row crosses more edges than the largest row kernel holds
+  kErrTooManyEntries = 8   // more segments, or band entries, than 32-bit places count: no workspace is enough
 };
 
 struct PathJob {

@@ -288,18 +288,18 @@ __device__ __forceinline__ int flatten_chain(const Prim* P, int p0, int p1, floa
 }
 
 // Sum of the values before this thread's, and the block's total.
-__device__ __forceinline__ int block_scan_excl(int v, int* s_warp, int& total) {
+__device__ __forceinline__ long long block_scan_excl(long long v, long long* s_warp, long long& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int x = v;
+  long long x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    const long long y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
   __syncthreads();
   if (lane == 31) s_warp[warp] = x;
   __syncthreads();
-  int before = 0;
+  long long before = 0;
   total = 0;
 #pragma unroll
   for (int w = 0; w < kSetupWarps; w++) {
@@ -332,8 +332,8 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
   int* wc = dsm + 3 * maxBands + 3;                      // [warp][band]: entries, then each warp's next place
   uint32_t* wm = reinterpret_cast<uint32_t*>(wc + kSetupWarps * (maxBands + 1));  // [warp][band]: lanes of a batch
   uint8_t* recs = reinterpret_cast<uint8_t*>(wm + kSetupWarps * (maxBands + 1));
-  __shared__ long long s_err, s_base, s_bandbase, s_listbase;
-  __shared__ int s_warp[kSetupWarps], s_tot, s_status;
+  __shared__ long long s_err, s_base, s_bandbase, s_listbase, s_tot, s_warp[kSetupWarps];
+  __shared__ int s_status;
   __shared__ float s_red[4][kSetupWarps], s_bounds[4];
   __shared__ int s_hdr[6];
   auto cluster = cg::this_cluster();
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
   // Two passes: count the segments each primitive emits, then -- their places
   // known -- emit them in order and reduce the bounds (:1098-1117).
   long long segbase = 0;
-  int off = 0, nseg = 0, mysegs = 0, nrec = 0, kept = -1;
+  int off = 0, nseg = 0, mysegs = 0, nrec = 0, kept = -1;  // (places and counts fit once the total does)
   float xmin = INFINITY, xmax = -INFINITY, ymin = INFINITY, ymax = -INFINITY;
 #pragma unroll 1
   for (int pass = 0; pass < 2; pass++) {
@@ -438,28 +438,29 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
     __syncthreads();
     // exclusive prefix of the counts, in primitive order
     const int m = (p1 - p0 + T - 1) / T, q0 = min(p1, p0 + tid * m), q1 = min(p1, q0 + m);
-    int sum = 0;
+    long long sum = 0, mine = 0, ahead = 0;
     if (s_err == LLONG_MAX) {
 #pragma unroll 1
       for (int p = q0; p < q1; p++) sum += PC[p];
     }
-    int run = block_scan_excl(sum, s_warp, mysegs);
-    if (tid == 0) s_tot = mysegs;
+    const long long first = block_scan_excl(sum, s_warp, mine);
+    if (tid == 0) s_tot = mine;
     sync();
     long long err = LLONG_MAX, total = 0;
 #pragma unroll 1
     for (int q = 0; q < C; q++) {
       err = min(err, *at(&s_err, q));
-      const int v = *at(&s_tot, q);
-      if (q < rank) off += v;
+      const long long v = *at(&s_tot, q);
+      if (q < rank) ahead += v;
       total += v;
     }
     if (rank == 0 && tid == 0) {
       s_base = 0;
       if (err != LLONG_MAX) s_status = (int)(err & 255);
+      else if (total > INT_MAX) s_status = kErrTooManyEntries;
       else {
         s_base = (long long)atomicAdd(&A.counters[kCtrSegs], (unsigned long long)total);
-        if (s_base + total > A.seg_cap || total > INT_MAX) s_status = kErrArenaFull;
+        if (s_base + total > A.seg_cap) s_status = kErrArenaFull;
       }
     }
     sync();
@@ -471,7 +472,9 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
       sync();  // no CTA leaves while another may read its shared memory
       return;
     }
-    run += off;
+    off = (int)ahead;
+    mysegs = (int)mine;
+    int run = (int)(ahead + first);
 #pragma unroll 1
     for (int p = q0; p < q1; p++) {
       const int v = PC[p];
@@ -640,7 +643,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
   // the bands' places in the list, in band order; within a band the CTAs in
   // rank order, so the list holds a band's segments ascending -- the order in
   // which partitionSegments appends them (:1215-1234)
-  int etotal = 0;
+  long long etotal = 0;  // a list of more than INT_MAX entries is an error: its places are 32 bits
 #pragma unroll 1
   for (int k0 = 0; k0 < (int)numP; k0 += T) {
     const int k = k0 + tid;
@@ -654,9 +657,9 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
         aa |= at(bandf, q)[k];
       }
     }
-    int tot;
-    const int ex = etotal + block_scan_excl(v, s_warp, tot);
-    if (k < (int)numP) bandx[k] = ex + before;
+    long long tot;
+    const long long ex = etotal + block_scan_excl(v, s_warp, tot);
+    if (k < (int)numP) bandx[k] = (int)(ex + before);
     if (rank == 0) {
       if (k0 == 0) {  // the bands' records
         if (tid == 0) {
@@ -676,8 +679,12 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
     etotal += tot;
   }
   if (rank == 0 && tid == 0) {
-    s_listbase = (long long)atomicAdd(&A.counters[kCtrBandSegs], (unsigned long long)etotal);
-    if (s_listbase + etotal > A.bandseg_cap) s_status = kErrArenaFull;
+    if (etotal > INT_MAX) {
+      s_status = kErrTooManyEntries;
+    } else {
+      s_listbase = (long long)atomicAdd(&A.counters[kCtrBandSegs], (unsigned long long)etotal);
+      if (s_listbase + etotal > A.bandseg_cap) s_status = kErrArenaFull;
+    }
   }
   sync();
   const int status = *at(&s_status, 0);

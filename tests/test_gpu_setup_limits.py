@@ -68,3 +68,33 @@ def test_segments_in_no_band(n, h, far):
             check(cmds, w, h)
         except px.PixieError as e:  # the library's limit of 2048 crossings a row
             assert n > 2048 and "Path too complex" in str(e)
+
+
+def test_more_band_entries_than_32_bits():
+    """262,200 edges through all 8191 bands of a 32,767-row image are 2^31 + 196,552
+    entries: the call fails, leaves the image alone, and the next calls are whole."""
+    w, h, n = 9, 32767, 262200
+    cmds = np.empty((n, 3), np.float32)
+    cmds[:, 0] = 2.0
+    cmds[0, 0] = 1.0
+    cmds[:, 1] = np.linspace(0.5, w - 0.5, n)
+    cmds[:, 2] = np.where(np.arange(n) & 1, h, 0.0)
+    cmds = np.concatenate([cmds.ravel(), [0.0]]).astype(np.float32)
+    paint = px.Paint(color=(0.1, 0.7, 0.4, 0.8))
+    small = np.asarray([1, 1.3, 2, 2, 7.6, 9.1, 2, 4.5, 90.25, 0], np.float32)
+    ref = pxo.new_image(w, h)
+    pxo.fill_path(ref, small, [0.1, 0.7, 0.4, 0.8], 1.0, 0, None, 0)
+    img = px.Image(w, h)
+    with pytest.raises(px.PixieError, match="Out of workspace memory"):
+        img.fill_path(cmds, paint)
+    assert not img.to_numpy().any()
+    img.fill_path(small, paint)
+    assert np.array_equal(img.to_numpy(), ref)
+    sc = px.Scene()
+    sc.fill_path(small, paint)
+    sc.fill_path(cmds, paint)
+    sc.fill_path(small, paint)
+    img = px.Image(w, h)
+    with pytest.raises(px.PixieError, match="Out of workspace memory"):
+        img.draw_scene(sc)
+    assert np.array_equal(img.to_numpy(), ref)  # the path before it is drawn, as by calls one by one
