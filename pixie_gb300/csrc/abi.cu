@@ -110,7 +110,7 @@ struct pxg_server {
 
 namespace pxg {
 __global__ void k_setup(PathJob* jobs, Arena A, int maxBands, int C);
-int setup_cluster(long long njobs, long long maxWork, int maxBands);
+int setup_cluster(long long njobs, long long maxWork);
 cudaError_t launch_setup(int njobs, int C, int maxBands, cudaStream_t st, PathJob* jobs, const Arena& A);
 const void* rows_kernel(int v);
 size_t rows_smem(int v);
@@ -148,7 +148,6 @@ void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Ar
 void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
                   long long items, const Arena& A, const uint8_t* tbl, int sliceW);
 size_t scene_wide_bytes();
-size_t setup_smem(int maxBands);
 int draw_masks_tiles();
 void launch_draw_masks(int tile, uint32_t* page, long long W, long long H, const int4* rects, const MaskDraw* items,
                        int n, int* bins, const uint8_t* masks, int mode, const uint8_t* tbl, cudaStream_t st);
@@ -685,10 +684,10 @@ void note_stats(long long paths, long long prims, const unsigned long long* ctr)
 }
 
 int setup_max_bands(long long maxH) {
-  const int maxBands = (int)(std::max<long long>(1, maxH / 4) + 1);
-  // 8 bytes of shared memory per band beside 9296 fixed ones
-  if (maxBands > 1024 && (size_t)maxBands * 8 + 9296 > g.smemOptin) throw ApiError{"Image too tall for the fill kernels"};
-  return maxBands;
+  // 111,575 rows are what the fill calls take (a limit of the interface: the
+  // setup kernel itself goes through a tall image's bands in windows)
+  if (maxH > 111575) throw ApiError{"Image too tall for the fill kernels"};
+  return (int)(std::max<long long>(1, maxH / 4) + 1);
 }
 
 // Grows the workspace after a launch in which some job ran out of it.
@@ -788,7 +787,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
                          maxWork = std::max(maxWork, setup_work(j));
                        }
                      });
-    const int setupC = setup_cluster(nr, maxWork, maxBands);
+    const int setupC = setup_cluster(nr, maxWork);
     Arena& A = S.A;
     A.ovf_cap = g.ovf_cap / 2;
     PathJob* dj = S.dj;
@@ -1132,7 +1131,7 @@ void run_scene_chunk(std::vector<HostRun>& runs) {
       }
     });
     S.A.ovf_cap = g.ovf_cap / 3;  // three lists
-    CU(launch_setup(nj, setup_cluster(nj, maxWork, maxBands), maxBands, g.stream, S.dj, S.A));
+    CU(launch_setup(nj, setup_cluster(nj, maxWork), maxBands, g.stream, S.dj, S.A));
     note_launch();
     CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
     launch_scene_rec((unsigned)recBlocks, g.stream, S.dj, reinterpret_cast<const RecOrder*>(S.extra + orderAt), nj,

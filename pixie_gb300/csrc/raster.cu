@@ -25,7 +25,7 @@ namespace pxg {
 
 static __device__ constexpr float kEps = (float)(0.0001 * 3.141592653589793);  // paths.nim:44
 static constexpr long long kIterCap = 1LL << 24;
-static constexpr int kBallotBands = 1024;  // band count up to which the ballot band-list build runs
+static constexpr int kBandWindow = 1024;  // bands the setup kernel counts and lists at a time
 
 struct V2 {
   float x, y;
@@ -1497,11 +1497,11 @@ void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, cons
 }
 
 // Dynamic shared memory of k_setup for a launch whose images have at most
-// maxBands bands: per band a count and an anti-aliasing flag; with the ballot
-// build also a place, per warp a count and a lane mask, and the step records.
+// maxBands bands: per band of a window a count, an anti-aliasing flag and a
+// place, per warp a count and a lane mask, and the step records.
 size_t setup_smem(int maxBands) {
-  if (maxBands > kBallotBands) return (size_t)(2 * maxBands + 2) * 4;
-  return (size_t)(3 * maxBands + 3 + 2 * kSetupWarps * (maxBands + 1)) * 4 + kStepBytes;
+  const int stride = std::min(maxBands, kBandWindow) + 1;
+  return (size_t)((3 + 2 * kSetupWarps) * stride) * 4 + kStepBytes;
 }
 // CTAs per job: the longest job's time shrinks with them, while each CTA of a
 // launch beyond the first four per SM costs a wave's fixed part.  In
@@ -1510,8 +1510,7 @@ size_t setup_smem(int maxBands) {
 // with 8; 64 cubics: 90 and 38; a 14,540-primitive stroke: 600 and 83; 4096
 // glyphs: 100 with 1, 243 with 2; 240 local paths: 970 and 175; 2000 paths over
 // 1024 x 1024: 6400 and 2250.
-int setup_cluster(long long njobs, long long maxWork, int maxBands) {
-  if (maxBands > kBallotBands) return 1;
+int setup_cluster(long long njobs, long long maxWork) {
   int best = 1;
   double cost = 0;
   for (int c = 1; c <= 8; c *= 2) {

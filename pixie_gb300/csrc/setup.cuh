@@ -322,16 +322,15 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
   pdl_trigger();  // the row kernel may be set up while this runs; it waits for the segments
   pdl_wait();
   extern __shared__ int dsm[];
-  // up to kBallotBands bands each warp counts and places its own entries; more
-  // (images over 4096 rows, one CTA per job) are counted together, the list
-  // place of a band takes the count's, and there is no room for step records
-  const bool ballot = maxBands <= kBallotBands;
-  int* bandc = dsm;                 // per band: this CTA's entries
-  int* bandf = dsm + maxBands + 1;  // per band: entries that need anti-aliasing (differences, then sums)
-  int* bandx = ballot ? dsm + 2 * maxBands + 2 : bandc;  // per band: place of this CTA's first entry in the list
-  int* wc = dsm + 3 * maxBands + 3;                      // [warp][band]: entries, then each warp's next place
-  uint32_t* wm = reinterpret_cast<uint32_t*>(wc + kSetupWarps * (maxBands + 1));  // [warp][band]: lanes of a batch
-  uint8_t* recs = reinterpret_cast<uint8_t*>(wm + kSetupWarps * (maxBands + 1));
+  // per band of a window of at most kBandWindow: the CTA's counts and places, and
+  // each warp's own
+  const int wb = min(maxBands, kBandWindow), stride = wb + 1;
+  int* bandc = dsm;              // this CTA's entries
+  int* bandf = dsm + stride;     // entries that need anti-aliasing (differences, then sums)
+  int* bandx = bandf + stride;   // place of this CTA's first entry in the window's list
+  int* wc = bandx + stride;      // [warp][band]: entries, then each warp's next place
+  uint32_t* wm = reinterpret_cast<uint32_t*>(wc + kSetupWarps * stride);  // [warp][band]: lanes of a batch
+  uint8_t* recs = reinterpret_cast<uint8_t*>(wm + kSetupWarps * stride);
   __shared__ long long s_err, s_base, s_bandbase, s_listbase, s_tot, s_warp[kSetupWarps];
   __shared__ int s_status;
   __shared__ float s_red[4][kSetupWarps], s_bounds[4];
@@ -367,9 +366,9 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
   // (chains need room for their points)
   const int most = min(per, (J.curves + C - 1) / C + 1);
   int G = 1;
-  while (G < (ballot ? 32 : 4) && most * G * 2 <= T) G *= 2;
+  while (G < 32 && most * G * 2 <= T) G *= 2;
   const int NG = T / G, gid = tid / G, gl = tid % G, leader = lane - gl;
-  const int cap = ballot ? kStepBytes / NG : 0;
+  const int cap = kStepBytes / NG;
   uint8_t* rec = recs + gid * cap;
 
   // Two passes: count the segments each primitive emits, then -- their places
@@ -556,6 +555,11 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
       J.pathHeight = pathHeight;
       J.nb = (int)numP;
       J.ph = ph;
+      if (status == kOk) {  // the bands' records
+        s_bandbase = (long long)atomicAdd(&A.counters[kCtrBands], (unsigned long long)numP);
+        if (s_bandbase + numP > A.band_cap) s_status = kErrArenaFull;
+        J.band_off = s_bandbase;
+      }
     }
   }
   __syncthreads();
@@ -575,134 +579,123 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
     return r;
   };
 
-  // each band's entry count and anti-aliasing flag (:1215-1234): every warp
+  // Windows of bands, one for images of up to 4096 rows: what the per-warp arrays
+  // hold.  Each has a list of its own, so a tall image costs a pass over the
+  // segments' ranges per window and nothing else.
+  //
+  // A window's entry counts and anti-aliasing flags (:1215-1234): every warp
   // owns a contiguous run of the CTA's segments and counts them as differences
   // over the bands, so a segment costs two additions however tall it is.  A
   // range may be empty (its first band above its last): a y of 2^32 or more
   // wraps in partitionRange's conversion, and the segment is in no band.
-  const int stride = (int)numP + 1;
   int* mine = wc + warp * stride;
   uint32_t* mask = wm + warp * stride;
   const int perw = ((mysegs + kSetupWarps - 1) / kSetupWarps + 31) / 32 * 32;
   const int ws0 = min(mysegs, warp * perw), ws1 = min(mysegs, ws0 + perw);
   const long long seg0 = segbase + off;  // the CTA's first segment
+  long long etotal = 0;  // a job of more than INT_MAX entries is an error: their places are 32 bits
+  int status = kOk;
 #pragma unroll 1
-  for (int k = tid; k < stride; k += T) bandf[k] = 0;
-  if (ballot) {
+  for (int b0 = 0; b0 < (int)numP; b0 += wb) {
+    const int nw = min(wb, (int)numP - b0);  // bands b0 .. b0 + nw - 1
 #pragma unroll 1
-    for (int k = lane; k < stride; k += 32) {
+    for (int k = tid; k <= nw; k += T) bandf[k] = 0;
+#pragma unroll 1
+    for (int k = lane; k <= nw; k += 32) {
       mine[k] = 0;
       mask[k] = 0u;
     }
-  } else {
+    __syncthreads();
 #pragma unroll 1
-    for (int k = tid; k < stride; k += T) bandx[k] = 0;
-  }
-  __syncthreads();
-  int* counts = ballot ? mine : bandx;
-#pragma unroll 1
-  for (int i = ws0 + lane; i < ws1; i += 32) {
-    const float4 sg = A.segs[seg0 + i];
-    const uint2 r = bandRange(sg);
-    A.segband[seg0 + i] = r;
-    if (r.x > r.y) continue;
-    atomicAdd(&counts[r.x], 1);
-    atomicAdd(&counts[r.y + 1], -1);
-    if (segRequiresAA(sg)) {
-      atomicAdd(&bandf[r.x], 1);
-      atomicAdd(&bandf[r.y + 1], -1);
-    }
-  }
-  __syncthreads();
-  // differences -> counts: each warp its own, warp 0 the flags (and, without
-  // per-warp counts, warp 1 the CTA's)
-#pragma unroll 1
-  for (int w = 0; w < 2; w++) {
-    int* d = w == 0 ? (ballot ? mine : warp == 1 ? bandx : nullptr) : warp == 0 ? bandf : nullptr;
-    if (!d) continue;
-    int carry = 0;
-#pragma unroll 1
-    for (int k0 = 0; k0 < (int)numP; k0 += 32) {
-      const int k = k0 + lane;
-      int v = k < (int)numP ? d[k] : 0;
-      v = carry + warp_scan_incl(v, lane);
-      if (k < (int)numP) d[k] = v;
-      carry = __shfl_sync(0xffffffffu, v, 31);
-    }
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int k = tid; k < (int)numP; k += T) {
-    if (!ballot) break;  // bandx is bandc
-    int c = 0;
-#pragma unroll 1
-    for (int w = 0; w < kSetupWarps; w++) c += wc[w * stride + k];
-    bandc[k] = c;
-  }
-  sync();
-  // the bands' places in the list, in band order; within a band the CTAs in
-  // rank order, so the list holds a band's segments ascending -- the order in
-  // which partitionSegments appends them (:1215-1234)
-  long long etotal = 0;  // a list of more than INT_MAX entries is an error: its places are 32 bits
-#pragma unroll 1
-  for (int k0 = 0; k0 < (int)numP; k0 += T) {
-    const int k = k0 + tid;
-    int v = 0, before = 0, aa = 0;
-    if (k < (int)numP) {
-#pragma unroll 1
-      for (int q = 0; q < C; q++) {
-        const int c = at(bandc, q)[k];
-        if (q < rank) before += c;
-        v += c;
-        aa |= at(bandf, q)[k];
+    for (int i = ws0 + lane; i < ws1; i += 32) {
+      const float4 sg = A.segs[seg0 + i];
+      const uint2 r = bandRange(sg);
+      if (b0 == 0) A.segband[seg0 + i] = r;
+      const int x = max((int)r.x - b0, 0), y = min((int)r.y - b0, nw - 1);
+      if (x > y || r.x > r.y) continue;
+      atomicAdd(&mine[x], 1);
+      atomicAdd(&mine[y + 1], -1);
+      if (segRequiresAA(sg)) {
+        atomicAdd(&bandf[x], 1);
+        atomicAdd(&bandf[y + 1], -1);
       }
     }
-    long long tot;
-    const long long ex = etotal + block_scan_excl(v, s_warp, tot);
-    if (k < (int)numP) bandx[k] = (int)(ex + before);
-    if (rank == 0) {
-      if (k0 == 0) {  // the bands' records
-        if (tid == 0) {
-          s_bandbase = (long long)atomicAdd(&A.counters[kCtrBands], (unsigned long long)numP);
-          if (s_bandbase + numP > A.band_cap) s_status = kErrArenaFull;
+    __syncthreads();
+    // differences -> counts: each warp its own, warp 0 the flags
+#pragma unroll 1
+    for (int w = 0; w < 2; w++) {
+      int* d = w == 0 ? mine : warp == 0 ? bandf : nullptr;
+      if (!d) continue;
+      int carry = 0;
+#pragma unroll 1
+      for (int k0 = 0; k0 < nw; k0 += 32) {
+        const int k = k0 + lane;
+        int v = k < nw ? d[k] : 0;
+        v = carry + warp_scan_incl(v, lane);
+        if (k < nw) d[k] = v;
+        carry = __shfl_sync(0xffffffffu, v, 31);
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = tid; k < nw; k += T) {
+      int c = 0;
+#pragma unroll 1
+      for (int w = 0; w < kSetupWarps; w++) c += wc[w * stride + k];
+      bandc[k] = c;
+    }
+    sync();
+    // the bands' places in the list, in band order; within a band the CTAs in
+    // rank order, so the list holds a band's segments ascending -- the order in
+    // which partitionSegments appends them (:1215-1234)
+    long long wtotal = 0;
+#pragma unroll 1
+    for (int k0 = 0; k0 < nw; k0 += T) {
+      const int k = k0 + tid;
+      int v = 0, before = 0, aa = 0;
+      if (k < nw) {
+#pragma unroll 1
+        for (int q = 0; q < C; q++) {
+          const int c = at(bandc, q)[k];
+          if (q < rank) before += c;
+          v += c;
+          aa |= at(bandf, q)[k];
         }
-        __syncthreads();
       }
-      if (k < (int)numP && s_status == kOk) {
+      long long tot;
+      const long long ex = wtotal + block_scan_excl(v, s_warp, tot);
+      if (k < nw) bandx[k] = (int)(ex + before);
+      if (rank == 0 && k < nw && s_status == kOk) {
         Band bd;
         bd.off = ex;  // relative until the base is known
         bd.count = v;
         bd.flags = aa ? kBandAA : 0;
-        A.bands[s_bandbase + k] = bd;
+        A.bands[s_bandbase + b0 + k] = bd;
       }
+      wtotal += tot;
     }
-    etotal += tot;
-  }
-  if (rank == 0 && tid == 0) {
+    etotal += wtotal;
     if (etotal > INT_MAX) {
-      s_status = kErrTooManyEntries;
-    } else {
-      s_listbase = (long long)atomicAdd(&A.counters[kCtrBandSegs], (unsigned long long)etotal);
-      if (s_listbase + etotal > A.bandseg_cap) s_status = kErrArenaFull;
+      status = kErrTooManyEntries;
+      break;
     }
-  }
-  sync();
-  const int status = *at(&s_status, 0);
-  const long long listbase = *at(&s_listbase, 0);
-  if (status != kOk) {
-    if (rank == 0 && tid == 0) set_status(J, A, job, status);
+    if (rank == 0 && tid == 0) {
+      s_listbase = (long long)atomicAdd(&A.counters[kCtrBandSegs], (unsigned long long)wtotal);
+      if (s_listbase + wtotal > A.bandseg_cap) s_status = kErrArenaFull;
+    }
     sync();
-    return;
-  }
-  int* L = A.bandseg + listbase;
-  if (rank == 0) {
+    // (a workspace that is too small is told how much the other windows take)
+    status = *at(&s_status, 0);
+    if (status != kOk) continue;
+    const long long listbase = *at(&s_listbase, 0);
+    int* L = A.bandseg + listbase;
+    if (rank == 0) {
 #pragma unroll 1
-    for (int k = tid; k < (int)numP; k += T) A.bands[s_bandbase + k].off += listbase;
-  }
-  if (ballot) {
+      for (int k = tid; k < nw; k += T) A.bands[s_bandbase + b0 + k].off += listbase;
+    }
     // each warp's start in every band: the CTA's plus the earlier warps' entries
 #pragma unroll 1
-    for (int k = tid; k < (int)numP; k += T) {
+    for (int k = tid; k < nw; k += T) {
       int run = bandx[k];
 #pragma unroll 1
       for (int w = 0; w < kSetupWarps; w++) {
@@ -723,8 +716,13 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
     for (int c0 = ws0; c0 < ws1; c0 += 32) {
       const int i = c0 + lane;
       uint2 r = make_uint2(0xffffffffu, 0u);  // empty range
-      if (i < ws1) r = A.segband[seg0 + i];
+      if (i < ws1) {
+        const uint2 g = A.segband[seg0 + i];
+        const int x = max((int)g.x - b0, 0), y = min((int)g.y - b0, nw - 1);
+        if (x <= y && g.x <= g.y) r = make_uint2((uint32_t)x, (uint32_t)y);
+      }
       const uint32_t kmin = __reduce_min_sync(0xffffffffu, r.x), kmax = __reduce_max_sync(0xffffffffu, r.y);
+      if (kmin > kmax) continue;
       const uint32_t tallest = __reduce_max_sync(0xffffffffu, r.x <= r.y ? r.y - r.x : 0u);
       if ((kmax - kmin) / 32 <= 1 + tallest / 2) {
 #pragma unroll 1
@@ -759,23 +757,9 @@ __global__ void __launch_bounds__(kSetupThreads, 4) k_setup(PathJob* jobs, Arena
       }
       __syncwarp();
     }
-  } else {
-    // more bands than the per-warp arrays hold (images over 4096 rows): every
-    // thread owns bands and walks the CTA's segments in order
-#pragma unroll 1
-    for (int k = tid; k < (int)numP; k += T) {
-      int cur = bandx[k];
-#pragma unroll 1
-      for (int j = 0; j < mysegs; j++) {
-        const uint2 r = A.segband[seg0 + j];
-        if (r.x <= (uint32_t)k && (uint32_t)k <= r.y) L[cur++] = off + j;
-      }
-    }
+    __syncthreads();  // the next window's counts take the places' room
   }
-  if (rank == 0 && tid == 0) {
-    J.band_off = s_bandbase;
-    set_status(J, A, job, kOk);
-  }
+  if (rank == 0 && tid == 0) set_status(J, A, job, status);
   sync();  // no CTA leaves while another may read its shared memory
 }
 

@@ -70,6 +70,58 @@ def test_segments_in_no_band(n, h, far):
             assert n > 2048 and "Path too complex" in str(e)
 
 
+def tall(n, w, h, seed, far=0):
+    """n short lines, quadratics and cubics wandering over a tall image, six edges
+    through all of it, and edges that end `far` beyond 32 bits."""
+    rs = np.random.RandomState(seed)
+    at = np.array([0.5 * w, 0.02 * h])
+    cmds = [1.0, *at]
+    for k in range(n):
+        kind = [0, 0, 1, 2, 0][k % 5]
+        pts = []
+        for _ in range(kind + 1):
+            at = np.clip(at + (rs.rand(2) - 0.5) * (w, 60.0) + (0, 0.9 * h / n / (kind + 1)), 0, (w, h - 0.25))
+            pts += [at[0], at[1]]
+        cmds += [[2.0, 7.0, 5.0][kind]] + pts
+    cmds += [0.0, 1.0, 0.1 * w, 0.0]
+    for k in range(6):
+        cmds += [2.0, (0.15 + 0.12 * k) * w, h if k % 2 == 0 else 0.0]
+    for k in range(far):
+        cmds += [0.0, 1.0, 0.2 * w, h * (0.3 + 0.1 * k), 2.0, 0.7 * w, 4294967296.0, 2.0, 0.8 * w, h * 0.9]
+    return np.asarray(cmds + [0.0], np.float32)
+
+
+# images around one, two and three windows of 1024 bands, with segments enough for a band every 4 rows
+@pytest.mark.parametrize("h", [4092, 4096, 4100, 8192, 8200, 12300])
+@pytest.mark.parametrize("n,far", [(700, 0), (2300, 0), (2300, 3)])
+def test_windows_of_bands(h, n, far):
+    check(tall(n, 11, h, h + n, far), 11, h)
+
+
+def test_windows_of_bands_in_batches():
+    """Masks and images of several heights in one launch, and strokes."""
+    hs = [37, 4100, 8300, 700, 9000]
+    cmds = [tall(1500, 11, h, h) for h in hs]
+    refs = []
+    for c, h in zip(cmds, hs):
+        refs.append(pxo.new_image(11, h))
+        pxo.fill_path(refs[-1], c, [1, 1, 1, 1], 1.0, 0, None, 0)
+    m = px.Masks()
+    m.add_paths([(c, 11, h, 0) for c, h in zip(cmds, hs)])
+    m.render()
+    imgs = [px.Image(11, h) for h in hs]
+    assert not px.fill_paths_batch(imgs, cmds, [(1, 1, 1, 1)] * len(hs)).any()
+    for k, ref in enumerate(refs):
+        assert np.array_equal(m.mask(k), ref[..., 3])
+        assert np.array_equal(imgs[k].to_numpy(), ref)
+    line = tall(150, 40, 8300, 5)
+    ref = pxo.new_image(40, 8300)
+    pxo.stroke_path(ref, line, [0.1, 0.7, 0.4, 0.8], 1.0, 0, None, 3.0, 1, 1)
+    img = px.Image(40, 8300)
+    img.stroke_path(line, px.Paint(color=(0.1, 0.7, 0.4, 0.8)), None, 3.0, 1, 1)
+    assert np.array_equal(img.to_numpy(), ref)
+
+
 def test_more_band_entries_than_32_bits():
     """262,200 edges through all 8191 bands of a 32,767-row image are 2^31 + 196,552
     entries: the call fails, leaves the image alone, and the next calls are whole."""
