@@ -955,7 +955,7 @@ __global__ void __launch_bounds__(kRowsLineThreads) k_rows_lines(PathJob* jobs, 
   pdl_trigger();
   pdl_wait();
   if (warp > 0) {
-    line_warps(S, warp, lane);
+    line_warps<true>(S, warp, lane);
     return;
   }
   init_fast_row(S.row, lane);
@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(kRowsLineThreads) k_rows_huge(PathJob* jobs, A
   pdl_trigger();
   pdl_wait();
   if (warp > 0) {
-    line_warps(S, warp, lane);
+    line_warps<true>(S, warp, lane);
     return;
   }
   init_fast_row(S.row, lane);
@@ -1178,7 +1178,7 @@ __global__ void __launch_bounds__(kLineWarps * 32) k_scene_huge(PathJob* jobs, A
   pdl_trigger();
   pdl_wait();
   if (warp > 0) {
-    line_warps(S, warp, lane);
+    line_warps<false>(S, warp, lane);
     return;
   }
   init_fast_row(S.row, lane);

@@ -248,9 +248,12 @@ __device__ __forceinline__ void cov_range(uint32_t* diff, const CovTile& T, int 
 }
 // One sample span (prevAt, at) of computeCoverage (paths.nim:1398-1431) in
 // 24.8 fixed point: coverage 51 per sample (255 / 5) with anti-aliasing, else
-// the pixels [prevAt / 256, at / 256) of a fillHits span at 255.
+// the pixels [prevAt / 256, at / 256) of a fillHits span at 255.  SKIP: spans
+// outside the tile, whose differences cancel at its edge, are left out.
+template <bool SKIP>
 __device__ __forceinline__ void cov_span(uint32_t* diff, CovTile& T, int prevAt, int at, bool aa) {
   const int pi = prevAt >> 8, ai = at >> 8;
+  if (SKIP && (ai < T.t0 || pi >= T.t1)) return;
   // differences at pi, pi + 1, ai, ai + 1; one pixel's span lies within it
   int d0, d1, d2 = 0, d3 = 0;
   if (!aa) {
@@ -358,10 +361,16 @@ __device__ __forceinline__ uint32_t crossing_key(FastRow<NB, XT>& S, int j, int 
 // With more, the entries are ordered once by where they cross the middle of the
 // row (or end nearest to it); a line's crossings, gathered in that order, are
 // then nearly sorted.  Only the exact sort of a line's own keys decides.
+// held: the row's spans left by the call for its first tile, which those for the
+// others take as they are; -1 before that, and where they were too many (a
+// stroke of 300 points on 16384 x 512, 16 tiles a row, takes 1080 us with its
+// lines sorted for each, 338 so).
 constexpr int kGroupN = 16;
+template <int XT>
+constexpr bool kHoldTiles = XT > 256;  // (the instance for glyphs, seldom wider than its tile, does without)
 template <bool GROUPED, int NB, int XT>
 __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, float Wf, int winding, bool aa,
-                                            CovTile& T, int lane) {
+                                            CovTile& T, int lane, int& held) {
   constexpr int TAG = tag_bits(NB);
   const unsigned lt = (1u << lane) - 1;
   uint32_t* keys = reinterpret_cast<uint32_t*>(S.key);
@@ -377,12 +386,29 @@ __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, fl
   const unsigned group = grouped ? ((1u << n) - 1) << kb : 0xffffffffu;
   const int cap = NB <= 64 || n <= 64 ? 64 : NB <= 512 ? NB : 0;
   int ns = 0, done = grouped ? 0 : -1;  // lines done (-1: the ordering is to come)
+  constexpr bool HOLD = GROUPED && kHoldTiles<XT>;
+  bool all = true;                            // every span so far is still there
+  if (HOLD && held >= 0) {
+    ns = held;
+    done = lines;
+  }
+  const auto draw = [&]() {
+#pragma unroll 1
+    for (int k = lane; k < ns; k += 32) cov_span<HOLD>(S.diff, T, sp[k].x, sp[k].y, opaque(aa) != 0);
+    __syncwarp();
+  };
   if (grouped) {                        // the first step's lines are s ahead
 #pragma unroll 1
     for (int k = 0; k < min(s, lines); k++) yLine += offset;
   }
 #pragma unroll 1
-  while (done < lines) {
+  while (HOLD || done < lines) {
+    if (HOLD && (ns > NB - max(n / 2, 16) || done >= lines)) {  // a step has at most n / 2 spans (16 by groups)
+      draw();
+      if (done >= lines) break;
+      ns = 0;
+      all = false;
+    }
     const bool ordering = !grouped && opaque(done) < 0;
     int nh = 0;  // the crossings of the lane's line
     if (!ordering) yLine += offset;
@@ -431,13 +457,12 @@ __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, fl
     }
     __syncwarp();
     done += sets;
-    if (ns > NB / 2 || done >= lines) {  // a line has at most NB / 2 spans, and there is room for NB
-#pragma unroll 1
-      for (int k = lane; k < ns; k += 32) cov_span(S.diff, T, sp[k].x, sp[k].y, opaque(aa) != 0);
+    if (!HOLD && (ns > NB / 2 || done >= lines)) {  // a line has at most NB / 2 spans, and there is room for NB
+      draw();
       ns = 0;
-      __syncwarp();
     }
   }
+  if (HOLD) held = all ? ns : -1;
 }
 
 // Rows whose time on one warp is what a launch waits for: a warp per sample
@@ -449,9 +474,10 @@ template <int NB>
 struct __align__(16) LineScratch {
   uint32_t keys[NB];
   int2 spans[NB / 2 + 32];
+  int ns;  // spans of the row's last tile: the same for its others
 };
 struct LineWork {  // what warp 0 publishes (n < 0: no more rows), and the warps' touched pixels
-  int n, y, winding, lines, x0, t0, t1;
+  int n, y, winding, lines, x0, t0, t1, held;
   float Wf;
   int lo[kLineWarps], hi[kLineWarps];
 };
@@ -479,14 +505,14 @@ static __device__ __noinline__ void sort_line(uint32_t* keys, int n, bool fresh,
   __syncwarp();
 }
 
-template <int NB, int XT>
+template <bool SKIP, int NB, int XT>
 __device__ __forceinline__ void one_line(FastRow<NB, XT>& S, LineWork& L, LineScratch<NB>& K, int q, int lane) {
   constexpr int TAG = tag_bits(NB);
   const unsigned lt = (1u << lane) - 1;
   CovTile T{L.x0, L.t0, L.t1, INT_MAX, INT_MIN};
   const int n = L.n;
   const bool aa = L.lines == 5;
-  if (q < L.lines) {
+  if (q < L.lines && !L.held) {
     const float offset = aa ? 1.0f / 5.0f : 1.0f;
     const float initialOffset = offset / 2 + kEps;
     float yLine = (float)L.y + initialOffset - offset;
@@ -507,9 +533,12 @@ __device__ __forceinline__ void one_line(FastRow<NB, XT>& S, LineWork& L, LineSc
 #pragma unroll 1
     for (int c0 = 0; c0 < nh; c0 += 32)
       walk_step<TAG>(K.keys, c0 + lane, nh, 0xffffffffu, false, count, prevAt, L.winding, K.spans, ns, lane);
+    if (lane == 0) K.ns = ns;
     __syncwarp();
+  }
+  if (q < L.lines) {
 #pragma unroll 1
-    for (int k = lane; k < ns; k += 32) cov_span(S.diff, T, K.spans[k].x, K.spans[k].y, opaque(aa) != 0);
+    for (int k = lane; k < K.ns; k += 32) cov_span<SKIP>(S.diff, T, K.spans[k].x, K.spans[k].y, opaque(aa) != 0);
   }
   const int lo = __reduce_min_sync(0xffffffffu, T.lo), hi = __reduce_max_sync(0xffffffffu, T.hi);
   if (lane == 0) {
@@ -517,21 +546,24 @@ __device__ __forceinline__ void one_line(FastRow<NB, XT>& S, LineWork& L, LineSc
     L.hi[q] = hi;
   }
 }
-// cov_samples by kLineWarps warps (called by warp 0).
-template <int NB, int XT>
+// cov_samples by kLineWarps warps (called by warp 0; a line's spans always fit).
+template <bool SKIP, int NB, int XT>
 __device__ __forceinline__ void cov_lines(FastRow<NB, XT>& S, LineWork& L, LineScratch<NB>& K, int n, int y, float Wf,
-                                          int winding, bool aa, CovTile& T, int lane) {
+                                          int winding, bool aa, CovTile& T, int lane, int& held) {
   constexpr int TAG = tag_bits(NB);
+  if (held < 0) {
 #pragma unroll 1
-  for (int i = lane; i < n; i += 32) {
-    const int j = S.idx[i];
-    K.keys[i] = crossing_key<TAG>(S, j, i, fminf(fmaxf((float)y + 0.5f, S.ay(j)), S.by(j)), Wf);
+    for (int i = lane; i < n; i += 32) {
+      const int j = S.idx[i];
+      K.keys[i] = crossing_key<TAG>(S, j, i, fminf(fmaxf((float)y + 0.5f, S.ay(j)), S.by(j)), Wf);
+    }
+    __syncwarp();
+    sort_line<NB>(K.keys, n, true, lane);
+#pragma unroll 1
+    for (int i = lane; i < n; i += 32) S.perm[i] = (uint16_t)((K.keys[i] >> 1) & ((1u << (TAG - 1)) - 1));
   }
-  __syncwarp();
-  sort_line<NB>(K.keys, n, true, lane);
-#pragma unroll 1
-  for (int i = lane; i < n; i += 32) S.perm[i] = (uint16_t)((K.keys[i] >> 1) & ((1u << (TAG - 1)) - 1));
   if (lane == 0) {
+    L.held = held >= 0;
     L.n = n;
     L.y = y;
     L.winding = winding;
@@ -541,8 +573,9 @@ __device__ __forceinline__ void cov_lines(FastRow<NB, XT>& S, LineWork& L, LineS
     L.t1 = T.t1;
     L.Wf = Wf;
   }
+  held = 0;
   line_barrier();
-  one_line(S, L, K, 0, lane);
+  one_line<SKIP>(S, L, K, 0, lane);
   line_barrier();
 #pragma unroll 1
   for (int q = 0; q < kLineWarps; q++) {
@@ -684,11 +717,13 @@ __device__ __forceinline__ float entry_x(float m, float b, float y) {  // solveX
 
 // The trapezoid test of a row whose n entries all span it (:1695-1750): their
 // crossings with its top and bottom in S.t0/t1, their order by midpoint in
-// S.perm; whether they form simple pairs.
-template <int NB, int XT>
-__device__ __forceinline__ bool trap_row(FastRow<NB, XT>& S, int n, float yTop, float yBottom, int winding, int lane) {
+// S.perm; whether they form simple pairs.  ordered: every position is exact as
+// an integer's floor and ceiling, so simple pairs lie one behind the other.
+template <bool ORDERED, int NB, int XT>
+__device__ __forceinline__ bool trap_row(FastRow<NB, XT>& S, int n, float yTop, float yBottom, int winding, int lane,
+                                         bool& ordered) {
   const unsigned le = 0xffffffffu >> (31 - lane);
-  bool nan = false;
+  bool nan = false, far = false;
 #pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     const int j = S.idx[i];
@@ -698,7 +733,9 @@ __device__ __forceinline__ bool trap_row(FastRow<NB, XT>& S, int n, float yTop, 
     S.t1[i] = t1;
     S.key[i] = key;
     nan |= isnan(key);
+    if (ORDERED) far |= !(fabsf(t0) < 1e18f && fabsf(t1) < 1e18f);
   }
+  if (ORDERED) ordered = !__any_sync(0xffffffffu, far);
   nan = __any_sync(0xffffffffu, nan);
   __syncwarp();
   if (!nan) {
@@ -743,16 +780,23 @@ __device__ __forceinline__ bool trap_row(FastRow<NB, XT>& S, int n, float yTop, 
 // 256 + the multiplier (0..255) its area rounds to, so that pixels blended
 // with nothing stay distinct from untouched ones (listed in S.zero when ZERO,
 // where only the multiplier is kept).  Returns true where a multiplier is
-// above 255 or the list is full: the general code's.
-template <bool ZERO, int NB, int XT>
-__device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const CovTile& T, int lane) {
+// above 255 or the list is full: the general code's.  dry: no more than that.
+// from: the first entry that reaches the tile or those to its right (advanced
+// where the entries are ordered: of 200 a row's 16 tiles have a dozen each).
+template <bool ZERO, bool ORDERED, int NB, int XT>
+__device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const CovTile& T, int lane, bool dry,
+                                         bool ordered, int& from) {
   constexpr int kBase = ZERO ? 0 : 256;
   bool odd = false;
 #pragma unroll 1
-  for (int s = 0; s < n; s++) {
+  for (int s = ORDERED ? from : 0; s < n; s++) {
     const int i = S.perm[s], j = S.idx[i];
     const float m = S.m(j), b = S.b(j), t0 = S.t0[i], t1 = S.t1[i];
     const float lo = nmin(t0, t1), end = ceilf(nmax(t0, t1));
+    if (ORDERED && ordered && !dry) {
+      if (!(s & 1) && lo >= (float)T.t1) break;
+      if ((s & 1) && end <= (float)T.t1) from = s + 1;
+    }
     const long long xs = nim_int(lo);
     const int x1 = nim_clamp(end, T.t0, T.t1);
 #pragma unroll 1
@@ -760,6 +804,7 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
       const float area = (s & 1) ? trap_right_area(m, b, t0, t1, x, xs, y) : trap_left_area(m, b, t0, t1, x, xs, y);
       const uint32_t v = area == 0.0f ? 0u : nim_u32(roundf(area * 255.0f));
       if (v > 255) odd = true;
+      else if (!ZERO && dry) continue;
       else if (!ZERO || v) cov_range(S.diff, T, x, x + 1, kBase + (int)v);
       else {
         const int z = atomicAdd(&S.nzero, 1);
@@ -767,7 +812,7 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
         else odd = true;
       }
     }
-    if (!(s & 1) && lane == 0) {  // the fully covered middle up to the next edge
+    if (!(s & 1) && lane == 0 && !(!ZERO && dry)) {  // the fully covered middle up to the next edge
       const int r = S.perm[s + 1];
       const int fe = nim_clamp(nmin(S.t0[r], S.t1[r]), T.t0, T.t1);
       if (fe > x1) cov_range(S.diff, T, x1, fe, kBase + 255);
@@ -783,7 +828,7 @@ template <int OUT, int NB, int XT, int LIST = 0, bool LINES = false>
 __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, const uint8_t* tbl, int job, int yA,
                                           int yB, FastRow<NB, XT>& S, int lane, LineWork* L = nullptr,
                                           LineScratch<NB>* K = nullptr) {
-  constexpr bool REC = OUT == kOutRec;
+  constexpr bool REC = OUT == kOutRec, ORDERED = !REC && kHoldTiles<XT>;
   const unsigned lt = (1u << lane) - 1;
   const int W = (int)J.W, startY = (int)J.startY, pathHeight = (int)J.pathHeight, ph = (int)J.ph;
   const int winding = J.winding, nb = J.nb;
@@ -813,6 +858,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
     const float yTop = (float)y, yBottom = (float)(y + 1);
     int n = 0;
     int kind = 0;             // 0: sample lines, 1: trapezoids, 2: a filled span
+    bool ordered = false;     // the trapezoids, one behind the other
     int dl = 0, dh = W;       // the pixels the row may touch
     if (two && !aa) {
       // (i) non-AA band with two spanning vertical edges (:1644-1668)
@@ -843,7 +889,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       // (ii) trapezoid fast path (:1695-1872), else (iii) computeCoverage
       // (:1350-1431) + fillCoverage / fillHits
       if (allSpan && (n & 1) == 0) {
-        if (trap_row(S, n, yTop, yBottom, winding, lane)) {
+        if (trap_row<ORDERED>(S, n, yTop, yBottom, winding, lane, ordered)) {
           kind = 1;
           // the pixels the pairs touch (the path's bounds do not limit them)
           int lo = W, hi = 0;
@@ -887,36 +933,41 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
     int covX = dl - off, covHi = dh;
     bool failed = false;
     // a row in several tiles whose trapezoids might be the general code's is
-    // gone through once before any of it is drawn
+    // gone through once, whole, before any of it is drawn
     bool dry = !REC && tiled && kind == 1;
+    int held = -1, from = 0;  // what the tiles before found: the row's spans, its first trapezoid to come
     if (REC && lane == 0) S.nzero = 0;
     __syncwarp();
 #pragma unroll 1
     for (int xt = dl - off; !failed; xt += XT) {
-      if (xt >= dh) {
-        if (!dry) break;
-        dry = false;
-        xt = dl - off;
-      }
-      CovTile T{xt, max(dl, xt), min(dh, xt + XT), INT_MAX, INT_MIN};
+      if (xt >= dh) break;
+      CovTile T{xt, max(dl, xt), dry ? dh : min(dh, xt + XT), INT_MAX, INT_MIN};
       if (kind == 0) {
         if (LINES && (REC || NB > 512 || n > kGroupN)) {
-          if constexpr (LINES) cov_lines(S, *L, *K, n, y, (float)W, winding, aa, T, lane);
+          if constexpr (LINES) cov_lines<!REC>(S, *L, *K, n, y, (float)W, winding, aa, T, lane, held);
         } else {
-          cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane);
+          cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane, held);
         }
       } else {
-        if (kind == 1) failed = trap_cov<REC>(S, n, y, T, lane);
+        if (kind == 1) failed = trap_cov<REC, ORDERED>(S, n, y, T, lane, dry, ordered, from);
         else if (lane == 0) cov_range(S.diff, T, dl, dh, 255);
         T.lo = T.t0;
         T.hi = T.t1;
+        if (!REC && dry) {
+          dry = false;
+          xt -= XT;
+          continue;
+        }
       }
       __syncwarp();
       const int lo = max(__reduce_min_sync(0xffffffffu, T.lo), T.t0);
       const int hi = min(__reduce_max_sync(0xffffffffu, T.hi), T.t1);
       int i0 = 0, iEnd = T.t1 - xt;
-      if (!tiled) {
-        if (hi <= lo) break;  // every difference cancelled or was dropped
+      if (!tiled || ORDERED) {
+        if (hi <= lo) {  // every difference cancelled or was dropped
+          if (ORDERED && tiled) continue;
+          break;
+        }
         i0 = (lo - xt) & ~15;
         iEnd = hi - xt;
       }
@@ -941,7 +992,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
           // pixel once: the blended alpha is the multiplier
           const uint32_t a = pack4(f[0], f[1]), b = pack4(f[2], f[3]);
           const int x = xt + i;
-          if (failed || dry || (a | b) == 0) return;
+          if (failed || (a | b) == 0) return;
           if (x >= 0 && x + 8 <= W) {
             *reinterpret_cast<uint2*>(dst + x) = make_uint2(a, b);
           } else {
@@ -953,7 +1004,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
           }
         } else {
           const uint32_t c[4] = {f[0] & 0xffffu, f[0] >> 16, f[1] & 0xffffu, f[1] >> 16};
-          if (failed || dry || (f[0] | f[1]) == 0) return;
+          if (failed || (f[0] | f[1]) == 0) return;
           const int x = xt + i;
           uint32_t* p = reinterpret_cast<uint32_t*>(base) + x;
           const bool vec = x >= 0 && x + 4 <= W;
@@ -1008,13 +1059,13 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
 
 // The warps of a CTA that take a row's other sample lines, until warp 0 has no
 // more rows; what warp 0 calls then.
-template <int NB, int XT>
+template <bool SKIP, int NB, int XT>
 __device__ __forceinline__ void line_warps(LineRow<NB, XT>& S, int warp, int lane) {
 #pragma unroll 1
   while (true) {
     line_barrier();
     if (S.work.n < 0) break;
-    one_line(S.row, S.work, S.line[warp], warp, lane);
+    one_line<SKIP>(S.row, S.work, S.line[warp], warp, lane);
     line_barrier();
   }
 }
