@@ -125,6 +125,7 @@ void launch_rows_lines(unsigned blocks, cudaStream_t st, PathJob* jobs, const lo
                        const Arena& A, const uint8_t* tbl, long long items);
 const void* rows_huge_kernel();
 size_t rows_huge_smem();
+bool rows_huge_fits(long long W);
 void launch_rows_huge(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, const uint8_t* tbl);
 __global__ void k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl, int list);
 __global__ void k_xclears(PathJob* jobs, Arena A);
@@ -761,6 +762,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
   for (int attempt = 0; attempt < 12 && !todo.empty(); attempt++) {
     const int nr = (int)todo.size();
     long long rows = 0, maxH = 1, maxWork = 0, items = 0;
+    bool huge = false;  // some image is one for k_rows_huge
     std::vector<long long> offs((size_t)nr);  // the jobs' first work items
     for (int r = 0; r < nr; r++) {
       const PathJob& j = jobs[(size_t)todo[(size_t)r]];
@@ -768,6 +770,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
       items += (j.H + cfg.rpi - 1) / cfg.rpi;
       rows += j.H;
       maxH = std::max<long long>(maxH, j.H);
+      huge |= cfg.variant == 0 && rows_huge_fits(j.W);
     }
     const int maxBands = setup_max_bands(maxH);
     ensure_arena(seg_need, list_need, (long long)nr * maxBands, nprims, rows);
@@ -799,10 +802,11 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
     // crossings 65 and 54.  Beyond two rows per resident CTA the warps' number
     // counts.  Rows of more than 256 crossings need some thousand lines in the
     // path: their kernel is launched along then (3 us for nothing), else only
-    // when the call has come back with such rows.
+    // when the call has come back with such rows.  Images too wide for it go to the
+    // general kernel at once.
     const bool byLines = v == 0 && cfg.rpi == 1 && opts.cfg.rpi == 0 && maxWork >= 512 &&
                          items <= 2LL * g.nsm * g.lines_ctas_per_sm;
-    const bool hugeAlong = v == 0 && maxWork >= 2048;
+    const bool hugeAlong = huge && maxWork >= 2048;
     long long blocks = (items + rows_warps(v) - 1) / rows_warps(v);
     blocks = std::min<long long>(blocks, (long long)g.nsm * g.rows_ctas_per_sm[v]);
     blocks = std::max<long long>(blocks, 1);
@@ -875,10 +879,10 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
       if ((long long)ctr[kCtrXClears] > A.xclear_cap) throw ApiError{"Out of workspace memory (cross-row clears)"};
       if (more > 0) {
         long long b = std::min<long long>((long long)more, (long long)g.nsm * 4);
-        if (v == 0 && !hugeAlong) {
+        if (huge && !hugeAlong) {
           launch_rows_huge((unsigned)std::min<long long>(b, g.nsm), g.stream, dj, A, g.tbl); note_launch();
         }
-        k_rows_wide<<<(unsigned)b, 32, rows_smem_wide(), g.stream>>>(dj, A, g.tbl, v == 0); note_launch();
+        k_rows_wide<<<(unsigned)b, 32, rows_smem_wide(), g.stream>>>(dj, A, g.tbl, huge); note_launch();
         CU(cudaGetLastError());
       }
       if (ctr[kCtrXClears] > 0) {

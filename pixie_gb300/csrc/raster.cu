@@ -984,6 +984,7 @@ __global__ void __launch_bounds__(kRowsLineThreads) k_rows_lines(PathJob* jobs, 
   line_warps_end(S.work, lane);
 }
 
+__host__ __device__ bool rows_huge_fits(long long W) { return W < fast_max_w(kWideMaxH); }
 // Rows of RGBX launches with more than kRowsNB crossings (list 0), up to
 // kWideMaxH of them; the rest to list 1.  They are few and each takes long: a
 // stroke of 300 points with round joins has five, 160 us by the general code
@@ -1007,7 +1008,7 @@ __global__ void __launch_bounds__(kRowsLineThreads) k_rows_huge(PathJob* jobs, A
     const PathJob& J = jobs[job];
     const int k = min((y - (int)J.startY) / (int)J.ph, J.nb - 1);
     // a band of more than kWideMaxH entries is an error, which the general kernel reports
-    if (J.W >= fast_max_w(kWideMaxH) || A.bands[J.band_off + k].count > kWideMaxH) push_row(A, job, y, lane, 1);
+    if (!rows_huge_fits(J.W) || A.bands[J.band_off + k].count > kWideMaxH) push_row(A, job, y, lane, 1);
     else fast_rows<kOutRgbx, kWideMaxH, kWideXT, 1, true>(J, A, tbl, job, y, y + 1, S.row, lane, &S.work, S.line);
   }
   line_warps_end(S.work, lane);
@@ -1062,14 +1063,20 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows(PathJob* jobs, const long l
 }
 
 // Rows the kernels before handed on (list 0 or 1), by the general row code: one
-// warp per CTA with room for kWideMaxH crossings.
+// warp per CTA with room for kWideMaxH crossings.  They come in the order in
+// which they were handed on and differ in length, so the CTAs take them from a
+// queue.
 __global__ void __launch_bounds__(32) k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl, int list) {
   extern __shared__ __align__(16) unsigned char rsm[];
   using Scratch = RowScratch<kWideMaxH, kWideXT>;
   Scratch& S = *reinterpret_cast<Scratch*>(rsm);
   const int lane = threadIdx.x & 31;
-  long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[list ? kCtrOvfRows2 : kCtrOvfRows]);
-  for (long long i = blockIdx.x; i < n; i += gridDim.x) {
+  const long long n = (long long)min((unsigned long long)A.ovf_cap, A.counters[list ? kCtrOvfRows2 : kCtrOvfRows]);
+  while (true) {
+    unsigned long long q = 0;
+    if (lane == 0) q = atomicAdd(&A.counters[kCtrQueue2], 1ull);
+    const long long i = (long long)__shfl_sync(0xffffffffu, q, 0);
+    if (i >= n) break;
     long long v = A.ovf_rows[list * A.ovf_cap + i];
     int job = (int)(v >> 32);
     long long y = v & 0xffffffffLL;

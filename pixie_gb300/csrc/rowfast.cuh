@@ -596,14 +596,20 @@ __device__ __forceinline__ int warp_scan_incl(int v, int lane) {
 // leaving it at zero, 2 N pixels (N = 2 or 4 words) per lane: out(i, f) gets the
 // prefix sums of indices i .. i + 2 N - 1, two per word.  A word's two prefix
 // sums are w + (w << 16), the sum before it is added to both halves at once;
-// the sums themselves are not negative, so the halves come out exact.
-template <int N, class Out>
+// the sums themselves are not negative, so the halves come out exact.  SPARSE:
+// steps of pixels that nothing covers are passed over (a wide row of a stroke is
+// mostly those).
+template <int N, bool SPARSE, class Out>
 __device__ __forceinline__ void flush_diff(uint32_t* diff, int i0, int iEnd, int lane, Out&& out) {
   int carry = 0;
 #pragma unroll 1
   for (int i = i0; i <= iEnd; i += 64 * N) {
     const int ii = i + lane * 2 * N;
     uint32_t w[N];
+    if (SPARSE && N == 2 && carry == 0) {
+      const uint2 q = *reinterpret_cast<const uint2*>(diff + (ii >> 1));
+      if (!__any_sync(0xffffffffu, q.x != kDiffZero || q.y != kDiffZero)) continue;
+    }
     if (N == 4) {
       uint4* p = reinterpret_cast<uint4*>(diff + (ii >> 1));
       const uint4 q = *p;
@@ -675,6 +681,7 @@ __device__ __forceinline__ int load_chunk(const PathJob& J, const Arena& A, cons
       }
     }
     n += __popc(msk);
+    if (n > NB) break;
   }
   __syncwarp();
   two = false;
@@ -983,7 +990,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
         failed = (long long)(cb + covBytes) > A.cov8_cap;
       }
       uint8_t* dst = REC ? A.cov8 + cov : base;
-      flush_diff<OUT == kOutRgbx ? 2 : 4>(S.diff, i0, iEnd, lane, [&](int i, const uint32_t* f) {
+      flush_diff<OUT == kOutRgbx ? 2 : 4, ORDERED>(S.diff, i0, iEnd, lane, [&](int i, const uint32_t* f) {
         if (REC) {
           const int o = xt + i - covX;
           if (i < XT && o < (int)covBytes && !failed)

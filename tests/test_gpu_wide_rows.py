@@ -98,3 +98,21 @@ def test_wide_strokes():
     img = px.Image(w, h)
     img.stroke_path(cmds, px.Paint(color=COLOR), None, 3.0, 1, 1)
     assert np.array_equal(img.to_numpy(), ref)
+
+
+@pytest.mark.parametrize("curves", [0, 90])  # with 90 short curves above the image the paths count as heavy
+def test_many_crossings_at_mixed_widths(curves):
+    """Rows of more than 256 crossings of images that the kernel for them takes and
+    of wider ones, in one launch and alone."""
+    ws = [4200, 900, 5000, 4095, 4096]
+    above = [1.0, 5.0, -20.0] + [5.0, 6.0, -20.5, 7.0, -21.0, 5.0, -20.0 - 0.01] * curves + [0.0]
+    cmds = [np.concatenate([comb(n, w, n), np.asarray(above, np.float32)]) for n, w in zip((400, 500, 20, 300, 700), ws)]
+    refs = []
+    for c, w in zip(cmds, ws):
+        refs.append(pxo.new_image(w, H))
+        pxo.fill_path(refs[-1], c, COLOR, 1.0, 0, None, 0)
+    for pick in ([0, 1, 2, 3, 4], [0], [2], [0, 4], [1, 3]):
+        imgs = [px.Image(ws[k], H) for k in pick]
+        assert not px.fill_paths_batch(imgs, [cmds[k] for k in pick], [COLOR] * len(pick)).any()
+        for im, k in zip(imgs, pick):
+            assert np.array_equal(im.to_numpy(), refs[k])
