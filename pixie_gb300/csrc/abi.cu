@@ -118,15 +118,17 @@ int rows_warps(int v);
 bool rows_fast(int mode, long long W);
 void launch_rows(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
                  const Arena& A, const uint8_t* tbl, long long items, int rpi);
-const void* rows_lines_kernel();
+bool rows_narrow(long long W);
+const void* rows_lines_kernel(bool narrow);
 size_t rows_lines_smem();
 int rows_lines_threads();
-void launch_rows_lines(unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
+void launch_rows_lines(bool narrow, unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
                        const Arena& A, const uint8_t* tbl, long long items);
-const void* rows_huge_kernel();
+const void* rows_huge_kernel(bool narrow);
 size_t rows_huge_smem();
 bool rows_huge_fits(long long W);
-void launch_rows_huge(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, const uint8_t* tbl);
+void launch_rows_huge(bool narrow, unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A,
+                      const uint8_t* tbl);
 __global__ void k_rows_wide(PathJob* jobs, Arena A, const uint8_t* tbl, int list);
 __global__ void k_xclears(PathJob* jobs, Arena A);
 const void* scene_rec_kernel();
@@ -320,8 +322,8 @@ struct Ctx {
   size_t ringSmemMax = 0;
   float last_ms = 0;
   long long stats[6] = {0, 0, 0, 0, 0, 0};  // last fill launch: paths, prims, segments, entries, blends, wide rows
-  int rows_ctas_per_sm[4] = {1, 1, 1, 1};  // resident CTAs of each row-kernel variant
-  int lines_ctas_per_sm = 1;               // and of the row kernel with a CTA per row
+  int rows_ctas_per_sm[5] = {1, 1, 1, 1, 1};  // resident CTAs of each row-kernel variant
+  int lines_ctas_per_sm[2] = {1, 1};          // and of the row kernels with a CTA per row
   int scene_ctas_per_sm[5] = {1, 1, 1, 1, 1};  // resident CTAs of the scene recording, drawing, rest and big-row kernels
   int scene_slice = 0;                // pixels of a row one warp of the drawing pass owns (0: chosen per launch)
   bool stroke_gpu = true;             // outline strokes without dashes on the GPU (stroke.cu)
@@ -377,20 +379,22 @@ void init_locked(int device) {
   }
   CU(cudaMalloc(&g.tbl, kTblBytes));
   CU(cudaMemcpy(g.tbl, t.data(), kTblBytes, cudaMemcpyHostToDevice));
-  for (int v = 0; v < 4; v++) {
+  for (int v = 0; v < 5; v++) {
     CU(cudaFuncSetAttribute(rows_kernel(v), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(v)));
     int per = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rows_kernel(v), rows_warps(v) * 32, rows_smem(v)));
     g.rows_ctas_per_sm[v] = std::max(1, per);
   }
-  {
+  for (int narrow = 0; narrow < 2; narrow++) {
     int per = 0;
-    CU(cudaFuncSetAttribute(rows_lines_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_lines_smem()));
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rows_lines_kernel(), rows_lines_threads(),
-                                                     rows_lines_smem()));
-    g.lines_ctas_per_sm = std::max(1, per);
+    const void* k = rows_lines_kernel(narrow);
+    CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_lines_smem()));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, rows_lines_threads(), rows_lines_smem()));
+    g.lines_ctas_per_sm[narrow] = std::max(1, per);
   }
-  CU(cudaFuncSetAttribute(rows_huge_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_huge_smem()));
+  for (int narrow = 0; narrow < 2; narrow++)
+    CU(cudaFuncSetAttribute(rows_huge_kernel(narrow), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)rows_huge_smem()));
   CU(cudaFuncSetAttribute(k_rows_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem_wide()));
   {
     CU(cudaFuncSetAttribute(scene_rec_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scene_rec_smem()));
@@ -707,7 +711,7 @@ void grow_needs(const unsigned long long* ctr, long long& seg_need, long long& l
 // Row-kernel configuration of a fill launch: scratch variant and rows per
 // work item.
 struct RowsCfg {
-  int variant = 0;  // 0 (masks: 3), 1 (masks only)
+  int variant = 0;  // 0 (masks: 3; narrow images: 4), 1 (masks only)
   int rpi = 0;      // 0: chosen per launch
 };
 
@@ -742,13 +746,18 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
               const RunOpts& opts = RunOpts()) {
   RowsCfg cfg = opts.cfg;
   if (cfg.variant == 0 && !jobs.empty() && jobs[0].a8) cfg.variant = 3;
+  bool narrow = cfg.variant == 0;
+  for (const PathJob& j : jobs) narrow &= rows_narrow(j.W);
+  if (narrow) cfg.variant = 4;
   if (cfg.rpi == 0) {
     // a row per warp while the launch's rows are few (the chain of a chunk is
-    // as long as its rows); whole band chunks once every resident warp has some
+    // as long as its rows); whole band chunks once every resident warp has two (8192
+    // rows of 1000 edges: 606 us by pairs, which are one and a third per warp, 440
+    // by single rows)
     long long rows = 0;
     for (const PathJob& j : jobs) rows += j.H;
     const long long slots = (long long)g.nsm * g.rows_ctas_per_sm[cfg.variant] * rows_warps(cfg.variant);
-    cfg.rpi = rows >= 4 * slots ? 4 : rows >= 2 * slots ? 2 : 1;
+    cfg.rpi = rows >= 8 * slots ? 4 : rows >= 4 * slots ? 2 : 1;
   }
   for (const PathJob& j : jobs)
     if (!rows_fast(j.mode, j.W)) cfg = RowsCfg{2, 1};  // the general row kernel, row by row
@@ -770,7 +779,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
       items += (j.H + cfg.rpi - 1) / cfg.rpi;
       rows += j.H;
       maxH = std::max<long long>(maxH, j.H);
-      huge |= cfg.variant == 0 && rows_huge_fits(j.W);
+      huge |= (cfg.variant == 0 || cfg.variant == 4) && rows_huge_fits(j.W);
     }
     const int maxBands = setup_max_bands(maxH);
     ensure_arena(seg_need, list_need, (long long)nr * maxBands, nprims, rows);
@@ -804,8 +813,8 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
     // path: their kernel is launched along then (3 us for nothing), else only
     // when the call has come back with such rows.  Images too wide for it go to the
     // general kernel at once.
-    const bool byLines = v == 0 && cfg.rpi == 1 && opts.cfg.rpi == 0 && maxWork >= 512 &&
-                         items <= 2LL * g.nsm * g.lines_ctas_per_sm;
+    const bool byLines = (v == 0 || v == 4) && cfg.rpi == 1 && opts.cfg.rpi == 0 && maxWork >= 512 &&
+                         items <= 2LL * g.nsm * g.lines_ctas_per_sm[narrow];
     const bool hugeAlong = huge && maxWork >= 2048;
     long long blocks = (items + rows_warps(v) - 1) / rows_warps(v);
     blocks = std::min<long long>(blocks, (long long)g.nsm * g.rows_ctas_per_sm[v]);
@@ -818,11 +827,11 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
       if (count) note_launch();
       if (timeRows) CU(cudaEventRecord(g.evr0, g.stream));
       const long long* doffs = reinterpret_cast<const long long*>(S.extra);
-      if (byLines) launch_rows_lines((unsigned)items, g.stream, dj, doffs, nr, A, g.tbl, items);
+      if (byLines) launch_rows_lines(narrow, (unsigned)items, g.stream, dj, doffs, nr, A, g.tbl, items);
       else launch_rows(v, (unsigned)blocks, g.stream, dj, doffs, nr, A, g.tbl, items, cfg.rpi);
       if (count) note_launch();
       if (hugeAlong) {
-        launch_rows_huge((unsigned)g.nsm, g.stream, dj, A, g.tbl);
+        launch_rows_huge(narrow, (unsigned)g.nsm, g.stream, dj, A, g.tbl);
         if (count) note_launch();
       }
       CU(cudaGetLastError());
@@ -880,7 +889,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
       if (more > 0) {
         long long b = std::min<long long>((long long)more, (long long)g.nsm * 4);
         if (huge && !hugeAlong) {
-          launch_rows_huge((unsigned)std::min<long long>(b, g.nsm), g.stream, dj, A, g.tbl); note_launch();
+          launch_rows_huge(narrow, (unsigned)std::min<long long>(b, g.nsm), g.stream, dj, A, g.tbl); note_launch();
         }
         k_rows_wide<<<(unsigned)b, 32, rows_smem_wide(), g.stream>>>(dj, A, g.tbl, huge); note_launch();
         CU(cudaGetLastError());

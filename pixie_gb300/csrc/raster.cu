@@ -914,7 +914,7 @@ constexpr int kWideMaxH = 2048, kWideXT = 1024;
 // height share the GPU evenly.  Rows the engine hands on go to the wide
 // kernel.  NB = 64 with a 256-pixel tile is for small paths such as glyphs:
 // a quarter of the shared memory per warp.
-template <int OUT, int NB, int XT, int WARPS>
+template <int OUT, int NB, int XT, int WARPS, int TILES>
 __global__ void __launch_bounds__(WARPS * 32) k_rows_fast(PathJob* jobs, const long long* offs, int njobs, Arena A,
                                                           const uint8_t* tbl, long long totalItems, int rpi) {
   extern __shared__ __align__(16) unsigned char rsm[];
@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows_fast(PathJob* jobs, const l
       r = (int)((J.pathHeight - J.startY + chunks - 1) / chunks);
     }
     const long long yA = J.startY + (item - J.row_off) * r, yB = min(yA + r, J.pathHeight);
-    if (yA < yB) fast_rows<OUT, NB, XT>(J, A, tbl, lo, (int)yA, (int)yB, S, lane);
+    if (yA < yB) fast_rows<OUT, NB, XT, TILES>(J, A, tbl, lo, (int)yA, (int)yB, S, lane);
   }
 }
 constexpr int kRowsNB = 256, kRowsXT = 1024, kRowsWarps = 4;
@@ -955,6 +955,7 @@ constexpr int kRowsNB = 256, kRowsXT = 1024, kRowsWarps = 4;
 // launch lasts as long as the busiest row, and a warp per sample line shortens
 // it (64 cubics on 512 x 512: 29 -> 21 us).
 constexpr int kRowsLineThreads = kLineWarps * 32;
+template <int TILES>
 __global__ void __launch_bounds__(kRowsLineThreads) k_rows_lines(PathJob* jobs, const long long* offs, int njobs,
                                                                  Arena A, const uint8_t* tbl, long long totalItems) {
   extern __shared__ __align__(16) unsigned char rsm[];
@@ -979,7 +980,7 @@ __global__ void __launch_bounds__(kRowsLineThreads) k_rows_lines(PathJob* jobs, 
     const PathJob& J = jobs[lo];
     const int y = (int)(J.startY + (item - J.row_off));
     if (J.status != kOk || y >= (int)J.pathHeight) continue;
-    fast_rows<kOutRgbx, kRowsNB, kRowsXT, 0, true>(J, A, tbl, lo, y, y + 1, S.row, lane, &S.work, S.line);
+    fast_rows<kOutRgbx, kRowsNB, kRowsXT, TILES, 0, true>(J, A, tbl, lo, y, y + 1, S.row, lane, &S.work, S.line);
   }
   line_warps_end(S.work, lane);
 }
@@ -989,6 +990,7 @@ __host__ __device__ bool rows_huge_fits(long long W) { return W < fast_max_w(kWi
 // kWideMaxH of them; the rest to list 1.  They are few and each takes long: a
 // stroke of 300 points with round joins has five, 160 us by the general code
 // on a warp each after a wait for the host, 56 so.
+template <int TILES>
 __global__ void __launch_bounds__(kRowsLineThreads) k_rows_huge(PathJob* jobs, Arena A, const uint8_t* tbl) {
   extern __shared__ __align__(16) unsigned char rsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1009,7 +1011,7 @@ __global__ void __launch_bounds__(kRowsLineThreads) k_rows_huge(PathJob* jobs, A
     const int k = min((y - (int)J.startY) / (int)J.ph, J.nb - 1);
     // a band of more than kWideMaxH entries is an error, which the general kernel reports
     if (!rows_huge_fits(J.W) || A.bands[J.band_off + k].count > kWideMaxH) push_row(A, job, y, lane, 1);
-    else fast_rows<kOutRgbx, kWideMaxH, kWideXT, 1, true>(J, A, tbl, job, y, y + 1, S.row, lane, &S.work, S.line);
+    else fast_rows<kOutRgbx, kWideMaxH, kWideXT, TILES, 1, true>(J, A, tbl, job, y, y + 1, S.row, lane, &S.work, S.line);
   }
   line_warps_end(S.work, lane);
 }
@@ -1153,7 +1155,7 @@ __global__ void __launch_bounds__(kRecRowWarps * 32, 7) k_scene_rec(PathJob* job
       for (int y = yA; y < yB; y++) push_row(A, job, y, lane);
       continue;
     }
-    fast_rows<kOutRec, kRecNB, kRecRowXT>(J, A, nullptr, job, yA, yB, S, lane);
+    fast_rows<kOutRec, kRecNB, kRecRowXT, kAgain>(J, A, nullptr, job, yA, yB, S, lane);
   }
 }
 
@@ -1175,7 +1177,7 @@ __global__ void __launch_bounds__(kBigWarps * 32) k_scene_big(PathJob* jobs, Are
     const int job = (int)(v >> 32), y = (int)(v & 0xffffffffLL);
     const PathJob& J = jobs[job];
     if (J.W >= fast_max_w(kBigNB)) push_row(A, job, y, lane, 1);
-    else fast_rows<kOutRec, kBigNB, kBigXT, 1>(J, A, nullptr, job, y, y + 1, S, lane);
+    else fast_rows<kOutRec, kBigNB, kBigXT, kAgain, 1>(J, A, nullptr, job, y, y + 1, S, lane);
   }
 }
 
@@ -1204,7 +1206,7 @@ __global__ void __launch_bounds__(kLineWarps * 32) k_scene_huge(PathJob* jobs, A
     const int job = (int)(v >> 32), y = (int)(v & 0xffffffffLL);
     const PathJob& J = jobs[job];
     if (J.W >= fast_max_w(kHugeNB)) push_row(A, job, y, lane, 2);
-    else fast_rows<kOutRec, kHugeNB, kHugeXT, 2, true>(J, A, nullptr, job, y, y + 1, S.row, lane, &S.work, S.line);
+    else fast_rows<kOutRec, kHugeNB, kHugeXT, kAgain, 2, true>(J, A, nullptr, job, y, y + 1, S.row, lane, &S.work, S.line);
   }
   line_warps_end(S.work, lane);
 }
@@ -1556,30 +1558,42 @@ size_t scene_wide_bytes() { return sizeof(RowScratch<kWideMaxH, kWideXT>); }
 
 size_t rows_smem_wide() { return sizeof(RowScratch<kWideMaxH, kWideXT>); }
 
-const void* rows_lines_kernel() { return (const void*)k_rows_lines; }
+// Whether every row of a job fits one tile of the row engine (which begins up to
+// 3 pixels before the row's first: RGBX images).
+bool rows_narrow(long long W) { return W + 3 <= kRowsXT; }
+const void* rows_lines_kernel(bool narrow) {
+  return narrow ? (const void*)k_rows_lines<kNoTiles> : (const void*)k_rows_lines<kOnce>;
+}
 size_t rows_lines_smem() { return sizeof(LineRow<kRowsNB, kRowsXT>); }
 int rows_lines_threads() { return kRowsLineThreads; }
-void launch_rows_lines(unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
+void launch_rows_lines(bool narrow, unsigned blocks, cudaStream_t st, PathJob* jobs, const long long* offs, int njobs,
                        const Arena& A, const uint8_t* tbl, long long items) {
-  launch_pdl(k_rows_lines, dim3(blocks), dim3(kRowsLineThreads), rows_lines_smem(), st, jobs, offs, njobs, A, tbl,
+  launch_pdl(narrow ? k_rows_lines<kNoTiles> : k_rows_lines<kOnce>, dim3(blocks), dim3(kRowsLineThreads), rows_lines_smem(), st, jobs, offs, njobs, A, tbl,
              items);
 }
-const void* rows_huge_kernel() { return (const void*)k_rows_huge; }
+const void* rows_huge_kernel(bool narrow) {
+  return narrow ? (const void*)k_rows_huge<kNoTiles> : (const void*)k_rows_huge<kOnce>;
+}
 size_t rows_huge_smem() { return sizeof(LineRow<kWideMaxH, kWideXT>); }
-void launch_rows_huge(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, const uint8_t* tbl) {
-  launch_pdl(k_rows_huge, dim3(blocks), dim3(kRowsLineThreads), rows_huge_smem(), st, jobs, A, tbl);
+void launch_rows_huge(bool narrow, unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A,
+                      const uint8_t* tbl) {
+  launch_pdl(narrow ? k_rows_huge<kNoTiles> : k_rows_huge<kOnce>, dim3(blocks), dim3(kRowsLineThreads), rows_huge_smem(), st, jobs, A, tbl);
 }
 
 // Row kernel variants: 0 = RGBX images, 1 = masks of small paths such as
 // glyphs (64 crossings and 256-px tiles, a quarter of the shared memory per
-// warp), 2 = the general code, 3 = masks.
-constexpr auto kRowsRgbx = k_rows_fast<kOutRgbx, kRowsNB, kRowsXT, kRowsWarps>;
-constexpr auto kRowsGlyph = k_rows_fast<kOutA8, kGlyphNB, kGlyphXT, kGlyphWarps>;
-constexpr auto kRowsMask = k_rows_fast<kOutA8, kRowsNB, kRowsXT, kRowsWarps>;
+// warp), 2 = the general code, 3 = masks, 4 = RGBX images whose rows fit a tile.
+constexpr auto kRowsRgbx = k_rows_fast<kOutRgbx, kRowsNB, kRowsXT, kRowsWarps, kOnce>;
+constexpr auto kRowsNarrow = k_rows_fast<kOutRgbx, kRowsNB, kRowsXT, kRowsWarps, kNoTiles>;
+constexpr auto kRowsGlyph = k_rows_fast<kOutA8, kGlyphNB, kGlyphXT, kGlyphWarps, kAgain>;
+constexpr auto kRowsMask = k_rows_fast<kOutA8, kRowsNB, kRowsXT, kRowsWarps, kOnce>;
 constexpr auto kRowsGeneral = k_rows<kFastMaxH, kFastXT, kFastWarps>;
 const void* rows_kernel(int v) {
-  return v == 0 ? (const void*)kRowsRgbx
-                : v == 1 ? (const void*)kRowsGlyph : v == 2 ? (const void*)kRowsGeneral : (const void*)kRowsMask;
+  return v == 0   ? (const void*)kRowsRgbx
+         : v == 1 ? (const void*)kRowsGlyph
+         : v == 2 ? (const void*)kRowsGeneral
+         : v == 3 ? (const void*)kRowsMask
+                  : (const void*)kRowsNarrow;
 }
 size_t rows_smem(int v) {
   return v == 1   ? sizeof(FastRow<kGlyphNB, kGlyphXT>) * kGlyphWarps
@@ -1596,7 +1610,8 @@ void launch_rows(int v, unsigned blocks, cudaStream_t st, PathJob* jobs, const l
   if (v == 0) launch_pdl(kRowsRgbx, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
   else if (v == 1) launch_pdl(kRowsGlyph, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
   else if (v == 2) launch_pdl(kRowsGeneral, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
-  else launch_pdl(kRowsMask, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
+  else if (v == 3) launch_pdl(kRowsMask, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
+  else launch_pdl(kRowsNarrow, b, t, sm, st, jobs, offs, njobs, A, tbl, items, rpi);
 }
 
 }  // namespace pxg

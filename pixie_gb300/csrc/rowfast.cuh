@@ -366,9 +366,12 @@ __device__ __forceinline__ uint32_t crossing_key(FastRow<NB, XT>& S, int j, int 
 // stroke of 300 points on 16384 x 512, 16 tiles a row, takes 1080 us with lines
 // and trapezoids gone through for each, 348 so.
 constexpr int kGroupN = 16;
-template <int XT>
-constexpr bool kHoldTiles = XT > 256;  // (the instance for glyphs, seldom wider than its tile, does without)
-template <bool GROUPED, int NB, int XT>
+// Rows in several tiles: none (the images are narrower than one), or gone through
+// again for each (recording, whose code is at the instruction cache's edge, and
+// glyphs, seldom so wide), or worked out once.  A call on 60000 rows of 16 pixels
+// takes 134 us with the code for none, 152 with that for the last.
+enum Tiles { kNoTiles = 0, kAgain = 1, kOnce = 2 };
+template <bool GROUPED, bool HOLD, int NB, int XT>
 __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, float Wf, int winding, bool aa,
                                             CovTile& T, int lane, int& held) {
   constexpr int TAG = tag_bits(NB);
@@ -386,7 +389,6 @@ __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, fl
   const unsigned group = grouped ? ((1u << n) - 1) << kb : 0xffffffffu;
   const int cap = NB <= 64 || n <= 64 ? 64 : NB <= 512 ? NB : 0;
   int ns = 0, done = grouped ? 0 : -1;  // lines done (-1: the ordering is to come)
-  constexpr bool HOLD = GROUPED && kHoldTiles<XT>;
   bool all = true;                            // every span so far is still there
   if (HOLD && held >= 0) {
     ns = held;
@@ -681,7 +683,6 @@ __device__ __forceinline__ int load_chunk(const PathJob& J, const Arena& A, cons
       }
     }
     n += __popc(msk);
-    if (n > NB) break;
   }
   __syncwarp();
   two = false;
@@ -831,11 +832,11 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
 // Rows [yA, yB) of job J (non-MaskBlend, narrower than fast_max_w(NB), within the
 // path's rows), drawn into an RGBX image or an 8-bit mask, or recorded; rows it
 // does not take are handed on to list LIST.
-template <int OUT, int NB, int XT, int LIST = 0, bool LINES = false>
+template <int OUT, int NB, int XT, int TILES, int LIST = 0, bool LINES = false>
 __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, const uint8_t* tbl, int job, int yA,
                                           int yB, FastRow<NB, XT>& S, int lane, LineWork* L = nullptr,
                                           LineScratch<NB>* K = nullptr) {
-  constexpr bool REC = OUT == kOutRec, ORDERED = !REC && kHoldTiles<XT>;
+  constexpr bool REC = OUT == kOutRec, ONCE = TILES == kOnce;
   const unsigned lt = (1u << lane) - 1;
   const int W = (int)J.W, startY = (int)J.startY, pathHeight = (int)J.pathHeight, ph = (int)J.ph;
   const int winding = J.winding, nb = J.nb;
@@ -897,7 +898,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       // (ii) trapezoid fast path (:1695-1872), else (iii) computeCoverage
       // (:1350-1431) + fillCoverage / fillHits
       if (allSpan && (n & 1) == 0) {
-        if (trap_row<ORDERED>(S, n, yTop, yBottom, winding, lane, ordered)) {
+        if (trap_row<ONCE>(S, n, yTop, yBottom, winding, lane, ordered)) {
           kind = 1;
           // the pixels the pairs touch (the path's bounds do not limit them)
           int lo = W, hi = 0;
@@ -935,7 +936,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
     const int off = REC ? dl & 15
                         : OUT == kOutA8 ? (int)((reinterpret_cast<uintptr_t>(base) + dl) & 7)
                                         : (int)(((reinterpret_cast<uintptr_t>(base) >> 2) + dl) & 3);
-    const bool tiled = dh - (dl - off) > XT;  // wider than the difference array
+    const bool tiled = TILES != kNoTiles && dh - (dl - off) > XT;  // wider than the difference array
     long long cov = -1;                       // REC: the row's bytes in cov8
     unsigned covBytes = 0;
     int covX = dl - off, covHi = dh;
@@ -954,10 +955,10 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
         if (LINES && (REC || NB > 512 || n > kGroupN)) {
           if constexpr (LINES) cov_lines<!REC>(S, *L, *K, n, y, (float)W, winding, aa, T, lane, held);
         } else {
-          cov_samples<!REC, NB, XT>(S, n, y, (float)W, winding, aa, T, lane, held);
+          cov_samples<!REC, ONCE, NB, XT>(S, n, y, (float)W, winding, aa, T, lane, held);
         }
       } else {
-        if (kind == 1) failed = trap_cov<REC, ORDERED>(S, n, y, T, lane, dry, ordered, from);
+        if (kind == 1) failed = trap_cov<REC, ONCE>(S, n, y, T, lane, dry, ordered, from);
         else if (lane == 0) cov_range(S.diff, T, dl, dh, 255);
         T.lo = T.t0;
         T.hi = T.t1;
@@ -971,9 +972,9 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       const int lo = max(__reduce_min_sync(0xffffffffu, T.lo), T.t0);
       const int hi = min(__reduce_max_sync(0xffffffffu, T.hi), T.t1);
       int i0 = 0, iEnd = T.t1 - xt;
-      if (!tiled || ORDERED) {
+      if (!tiled || ONCE) {
         if (hi <= lo) {  // every difference cancelled or was dropped
-          if (ORDERED && tiled) continue;
+          if (ONCE && tiled) continue;
           break;
         }
         i0 = (lo - xt) & ~15;
@@ -990,7 +991,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
         failed = (long long)(cb + covBytes) > A.cov8_cap;
       }
       uint8_t* dst = REC ? A.cov8 + cov : base;
-      flush_diff<OUT == kOutRgbx ? 2 : 4, ORDERED>(S.diff, i0, iEnd, lane, [&](int i, const uint32_t* f) {
+      flush_diff<OUT == kOutRgbx ? 2 : 4, ONCE>(S.diff, i0, iEnd, lane, [&](int i, const uint32_t* f) {
         if (REC) {
           const int o = xt + i - covX;
           if (i < XT && o < (int)covBytes && !failed)
