@@ -44,6 +44,7 @@ struct pxg_masks {
   std::vector<pxg::PathJob> jobs;
   std::vector<long long> offs;  // byte offset of each mask
   long long bytes = 0;
+  long long side = 1, work = 0;  // the longest side and the heaviest outline (setup_work)
   unsigned char* dev = nullptr;
   long long dev_cap = 0;
   bool rendered = false;
@@ -732,7 +733,7 @@ struct RunOpts {
   unsigned char* zero = nullptr;  // buffer cleared before the first launch (mask batches)
   long long zero_bytes = 0;
   GraphCache* graph = nullptr;    // capture / replay the first launch
-  float* rows_ms = nullptr;       // row-kernel time of the first launch (autotuning)
+  float* rows_ms = nullptr;       // the rows' time of the first launch (autotuning)
   const Prim* dprims = nullptr;   // primitives already on the device (else staged)
   long long ndprims = -1;         // how many, when `prims` does not hold them (a GPU outline)
   unsigned char* imgs = nullptr;  // the jobs' images: imgs + (*img_offs)[job] (mask batches), else job.img
@@ -747,7 +748,8 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
   RowsCfg cfg = opts.cfg;
   if (cfg.variant == 0 && !jobs.empty() && jobs[0].a8) cfg.variant = 3;
   bool narrow = cfg.variant == 0;
-  for (const PathJob& j : jobs) narrow &= rows_narrow(j.W);
+  if (narrow)
+    for (const PathJob& j : jobs) narrow &= rows_narrow(j.W);
   if (narrow) cfg.variant = 4;
   if (cfg.rpi == 0) {
     // a row per warp while the launch's rows are few (the chain of a chunk is
@@ -899,10 +901,12 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
         k_xclears<<<(unsigned)b, 256, 0, g.stream>>>(dj, A); note_launch();
         CU(cudaGetLastError());
       }
+      if (timeRows) CU(cudaEventRecord(g.evr1, g.stream));  // rows handed on are the configuration's too
       // (the wide kernel's failures are in the jobs alone)
       CU(cudaMemcpyAsync(g.h_up, g.d_up, S.jobsBytes, cudaMemcpyDeviceToHost, g.stream));
       Timed::mark();
       CU(cudaStreamSynchronize(g.stream));
+      if (timeRows) CU(cudaEventElapsedTime(opts.rows_ms, g.evr0, g.evr1));
       wide = reinterpret_cast<const PathJob*>(g.h_up);
     }
     std::vector<int> again;
@@ -1586,7 +1590,7 @@ void srv_step(pxg_server* sv) {
 // seen.  Every configuration computes the same bytes; only speed differs.
 // ---------------------------------------------------------------------------
 enum TuneOp { kTuneMaskRows = 0, kTuneMaskDraw = 1 };
-const RowsCfg kMaskRowsCands[] = {{0, 4}, {1, 1}, {1, 2}, {1, 4}};
+const RowsCfg kMaskRowsCands[] = {{0, 0}, {1, 1}, {1, 2}, {1, 4}};
 constexpr int kNumMaskRowsCands = 4;
 
 struct Tuner {
@@ -1610,10 +1614,16 @@ int count_bucket(long long n) {
   while (b < 20 && (1LL << b) < n) b++;
   return b;
 }
+// Heavy outlines are a class of their own: their rows cross more edges than the
+// instance for glyphs holds, which light ones of the same size run best on (64
+// cubics on 2000 x 1500: 312 us of kernels by that one, 167 by the other).
+constexpr long long kHeavyMasks = 1024;
+void note_mask(pxg_masks* m, const PathJob& j) {
+  m->side = std::max<long long>(m->side, std::max<long long>(j.W, j.H));
+  m->work = std::max(m->work, setup_work(j));
+}
 long long mask_class(const pxg_masks* m) {
-  long long side = 1;
-  for (const PathJob& j : m->jobs) side = std::max<long long>(side, std::max<long long>(j.W, j.H));
-  return size_bucket(side) * 32 + count_bucket((long long)m->jobs.size());
+  return size_bucket(m->side) * 32 + count_bucket((long long)m->jobs.size()) + (m->work >= 1024 ? kHeavyMasks : 0);
 }
 
 }  // namespace
@@ -2287,6 +2297,7 @@ int pxg_masks_add_path(pxg_masks* m, const float* cmds, int64_t n, int64_t width
     j.curves = count_curves(prims, 0, j.nprims);
     m->prims.insert(m->prims.end(), prims.begin(), prims.end());
     m->jobs.push_back(j);
+    note_mask(m, j);
     m->dirty = true;
     m->offs.push_back(m->bytes);
     m->bytes += (width * height + 15) / 16 * 16;
@@ -2368,6 +2379,7 @@ int pxg_masks_add_paths(pxg_masks* m, int64_t n, const float* cmds, const int64_
       r.job.curves = count_curves(r.prims, 0, r.job.nprims);
       m->prims.insert(m->prims.end(), r.prims.begin(), r.prims.end());
       m->jobs.push_back(r.job);
+      note_mask(m, r.job);
       m->offs.push_back(m->bytes);
       m->bytes += (r.job.W * r.job.H + 15) / 16 * 16;
     }
@@ -2620,8 +2632,9 @@ int64_t pxg_autotune_report(char* buf, int64_t cap) {
     const long long cls = kv.first.second;
     int c = kv.second;
     if (op == kTuneMaskRows)
-      snprintf(line, sizeof line, "mask_rows class(side<=%d,count<=%lld): variant=%d rows_per_item=%d",
-               32 << (int)(cls / 32), 1LL << (cls % 32), kMaskRowsCands[c].variant, kMaskRowsCands[c].rpi);
+      snprintf(line, sizeof line, "mask_rows class(side<=%d,count<=%lld%s): variant=%d rows_per_item=%d",
+               32 << (int)(cls / 32 % 32), 1LL << (cls % 32), cls >= kHeavyMasks ? ",heavy" : "",
+               kMaskRowsCands[c].variant, kMaskRowsCands[c].rpi);
     else
       snprintf(line, sizeof line, "mask_draw class(side<=%d,count<=%lld): tile=%s", 32 << (int)(cls / 32),
                1LL << (cls % 32), c == 0 ? "32x32" : (c == 1 ? "64x32" : "64x64"));
