@@ -12,6 +12,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <atomic>
 #include <vector>
@@ -2352,19 +2353,45 @@ int pxg_masks_add_paths(pxg_masks* m, int64_t n, const float* cmds, const int64_
         failed = 1;
       }
     };
-    int nt = threads > 0 ? threads : (int)std::thread::hardware_concurrency();
-    nt = std::max(1, std::min<int>(nt, (int)std::min<int64_t>(n / 16 + 1, 256)));
-    // an outline takes some 2 us and a thread 30 to 60 to start, one after the
-    // other: the shortest total is near the square root of their quotient (240
-    // outlines: 16 threads 1200 us, 8 716, 4 587, 2 622, 1 763)
-    if (threads <= 0) nt = std::max(1, std::min(nt, (int)std::sqrt((double)n / 16)));
     std::atomic<int64_t> next{0};
     auto worker = [&] {
       for (int64_t i = next.fetch_add(1); i < n; i = next.fetch_add(1)) build(i);
     };
     std::vector<std::thread> pool;
-    for (int t = 1; t < nt; t++) pool.emplace_back(worker);
-    worker();
+    auto grow = [&](int nt) {  // to nt threads with this one
+      try {
+        while ((int)pool.size() + 1 < nt) pool.emplace_back(worker);
+      } catch (const std::system_error&) {  // no more to be had: those there are do
+      }
+    };
+    if (threads > 0) {
+      grow(std::max(1, std::min<int>(threads, (int)std::min<int64_t>(n / 16 + 1, 256))));
+      worker();
+    } else {
+      // A thread takes 30 to 60 us to start, one after the other, and an outline
+      // from 2 us to some hundreds: with that pace, taken from the last outlines as
+      // the work goes on, the rest takes least time with about as many threads as
+      // the square root of what is left over what a thread costs.  240 outlines of 2
+      // us: 16 threads 1200 us, 4 587, 2 622, 1 763; 60 of 50 us: 1 thread 3220, 4
+      // 1270.
+      constexpr double kStart = 30e-6;
+      const int most = (int)std::min<int64_t>(std::max(1u, std::thread::hardware_concurrency()), std::max<int64_t>(n, 1));
+      double from = now_s(), look = 0;  // since when the pace is taken, when to look at it next
+      int64_t done = 0;
+      for (int64_t i = next.fetch_add(1); i < n; i = next.fetch_add(1)) {
+        build(i);
+        ++done;
+        if ((int)pool.size() + 1 >= most) continue;
+        const double t = now_s();
+        if (t < look || (done < 4 && t - from < 100e-6)) continue;
+        const double left = (double)std::max<int64_t>(n - next.load(), 0) * (t - from) / (double)done;
+        const int have = (int)pool.size() + 1, want = std::min(most, (int)std::sqrt(left / kStart));
+        if (left > 6 * kStart && 2 * want >= 3 * have) grow(want);  // (not for one more among several)
+        from = now_s();
+        look = from + 100e-6;
+        done = 0;
+      }
+    }
     for (auto& t : pool) t.join();
     if (failed)
       for (const Rec& r : rec)
