@@ -187,7 +187,11 @@ __device__ __forceinline__ float gradient_t(const GradientArgs& g, float fx, flo
 // STAGED: the stops are copied into shared memory once per CTA; otherwise
 // (more stops than 48 KB of shared memory holds) they are read from global
 // memory, through the read-only cache.
-template <int KIND, bool STAGED, int OUT>
+// PX: neighbours a thread takes: four, but one of the angular kind and of images
+// with no more than two pixels for every thread the chip holds, where four would
+// mostly follow one another (21 stops: 64 x 64 38.5 us a call with four, 34.3
+// with one; 8192 x 64 39.6 and 38.2; 1000 x 1000 44 with either).
+template <int KIND, bool STAGED, int OUT, int PX>
 __global__ void __launch_bounds__(256) k_gradient(uint32_t* __restrict__ img, long long W, long long n,
                                                   const __grid_constant__ GradientArgs g,
                                                   const float* __restrict__ gstops, const uint32_t* __restrict__ mask,
@@ -200,7 +204,6 @@ __global__ void __launch_bounds__(256) k_gradient(uint32_t* __restrict__ img, lo
     __syncthreads();
     stops = staged;
   }
-  constexpr int PX = KIND == 5 ? 1 : 4;
   const bool small = n < (1ll << 31);
   for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * PX; i < n;
        i += (long long)gridDim.x * blockDim.x * PX) {
@@ -369,11 +372,15 @@ struct CorrectTable<kNumBlends> {
 namespace {
 typedef void (*GradientKernel)(uint32_t*, long long, long long, GradientArgs, const float*, const uint32_t*, uint32_t,
                                int);
+template <int OUT, bool STAGED>
+GradientKernel gradient_kernel_of(int kind, int px) {
+  if (kind == 3) return px == 4 ? k_gradient<3, STAGED, OUT, 4> : k_gradient<3, STAGED, OUT, 1>;
+  if (kind == 4) return px == 4 ? k_gradient<4, STAGED, OUT, 4> : k_gradient<4, STAGED, OUT, 1>;
+  return k_gradient<5, STAGED, OUT, 1>;
+}
 template <int OUT>
-GradientKernel gradient_kernel(int kind, bool staged) {
-  if (kind == 3) return staged ? k_gradient<3, true, OUT> : k_gradient<3, false, OUT>;
-  if (kind == 4) return staged ? k_gradient<4, true, OUT> : k_gradient<4, false, OUT>;
-  return staged ? k_gradient<5, true, OUT> : k_gradient<5, false, OUT>;
+GradientKernel gradient_kernel(int kind, bool staged, int px) {
+  return staged ? gradient_kernel_of<OUT, true>(kind, px) : gradient_kernel_of<OUT, false>(kind, px);
 }
 }  // namespace
 
@@ -384,14 +391,15 @@ void launch_gradient(uint32_t* img, long long W, long long H, const GradientArgs
   const size_t need = sizeof(float) * 5 * (size_t)g.nstops;
   const bool staged = need <= 48 * 1024;
   const size_t smem = staged ? need : 0;
-  const long long per = g.kind == 5 ? 256 : 1024;
+  const int px = g.kind == 5 || n <= (long long)nsm * 4096 ? 1 : 4;
+  const long long per = 256 * px;
   long long blocks = (n + per - 1) / per;  // four waves of eight CTAs per SM at most
   if (blocks > (long long)nsm * 32) blocks = (long long)nsm * 32;
   const unsigned gb = (unsigned)(blocks < 1 ? 1 : blocks);
   const int vec = ((reinterpret_cast<uintptr_t>(img) | reinterpret_cast<uintptr_t>(mask)) & 15) == 0;
-  const GradientKernel k = out == kOutFill     ? gradient_kernel<kOutFill>(g.kind, staged)
-                           : out == kOutMasked ? gradient_kernel<kOutMasked>(g.kind, staged)
-                                               : gradient_kernel<kOutComposite>(g.kind, staged);
+  const GradientKernel k = out == kOutFill     ? gradient_kernel<kOutFill>(g.kind, staged, px)
+                           : out == kOutMasked ? gradient_kernel<kOutMasked>(g.kind, staged, px)
+                                               : gradient_kernel<kOutComposite>(g.kind, staged, px);
   k<<<gb, 256, smem, st>>>(img, W, n, g, stops, mask, o, vec);
   note_launch();
 }
