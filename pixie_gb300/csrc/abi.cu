@@ -1210,7 +1210,10 @@ void run_scene_chunk(std::vector<HostRun>& runs) {
 // rows took 82.  A path's coverage
 // is at most its canvas; from the second chunk on it is taken as what the chunk
 // before asked for, and half as much again.  At least 64 paths of a run go
-// together.
+// together.  A chunk is bounded by its paths' rows, too, whatever they cover:
+// each takes 40 bytes (its header, its places in the lists of rows handed on), so
+// a million small paths on 1000 rows would take 40 GB at once and take 1.3 so.
+constexpr long long kChunkPathRows = 32LL << 20;
 void run_scene_runs(std::vector<HostRun>& runs) {
   if (!g.cov8) {  // coverage-byte arena: up to 4 GB, at most an eighth of the free memory
     size_t fr = 0, tot = 0;
@@ -1226,22 +1229,25 @@ void run_scene_runs(std::vector<HostRun>& runs) {
   while (true) {
     std::vector<HostRun> part;
     std::vector<size_t> which;
-    double left = (double)g.cov8_cap, pixels = 0;
+    double left = (double)g.cov8_cap, pixels = 0, rows = (double)kChunkPathRows;
     for (size_t i = 0; i < runs.size(); i++) {
       const HostRun& r = runs[i];
       if (r.status != kOk || r.j0 >= r.j1) continue;
       const double canvas = (double)(r.canvas->width + 16) * (double)r.canvas->height;
-      const double fit = std::max(left, 0.0) / (canvas * density);
-      const size_t all = r.j1 - r.j0;
+      const double byRows = std::max(rows, 0.0) / (double)r.canvas->height;
+      const double fit = std::min(std::max(left, 0.0) / (canvas * density), byRows);
+      const size_t all = r.j1 - r.j0, least = std::min<size_t>(all, 64);
       size_t n = fit >= (double)all ? all : (size_t)fit;
-      if (n < all && n < 64) {
-        if (!part.empty()) continue;
-        n = std::min<size_t>(all, 64);
+      if (n < least) {
+        // left for a chunk of its own, unless that would not hold it either
+        if (!part.empty() && (byRows < (double)least || (double)least * canvas * density <= (double)g.cov8_cap)) continue;
+        n = least;
       }
       part.push_back(r);
       part.back().j1 = r.j0 + n;
       which.push_back(i);
       left -= (double)n * canvas * density;
+      rows -= (double)n * (double)r.canvas->height;
       pixels += (double)n * canvas;
     }
     if (part.empty()) break;
