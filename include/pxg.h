@@ -173,8 +173,9 @@ int64_t pxg_stroke_fixups(void);
 /* Blur kernels: 3 (default) runs radii 1..8 on register-blocked CUDA-core
  * passes and radii 9..128 on the tensor cores with input rings in tensor
  * memory, as it does radii 6..8 of images large enough to be faster there
- * (images with a side below 4 take mode 1's kernels); 1 runs radii 8..128 on the tensor cores with the warp-specialised
- * kernel that loads through registers; 2 uses the single-stage tensor-core
+ * (images with a side below 4 take mode 1's kernels); 1 runs radii 8..128 on
+ * the tensor cores with the warp-specialised kernel that loads through
+ * registers; 2 uses the single-stage tensor-core
  * kernel (radii 8..128); 0 the tiled CUDA-core kernels (which every mode uses
  * for the radii it does not take).  All write the same bytes.  No
  * counterpart in the reference. */
@@ -184,10 +185,17 @@ int pxg_blur_config(int use_tensor_cores);
  * mode 3 for radii 1..8, on images the library allocated whose device
  * address was never handed out: the result lands in the library's scratch
  * buffer and the two buffers change owners), 4 (the two small-radius passes
- * of mode 3, in place), 3 (the ring passes, sides multiples of 4), 1 (the ring
- * passes on other sizes, and mode 1's kernel), 2 or 0 as above (-1 before any
- * blur).  No counterpart in the reference. */
+ * of mode 3, in place), 3 (the ring passes, both sides multiples of 4), 1
+ * (mode 1's kernel, or the ring passes on an image with another side:
+ * pxg_last_blur_ring tells which), 2 or 0 as above (-1 before any blur).  No
+ * counterpart in the reference. */
 int pxg_last_blur_kernel(void);
+
+/* Whether the last blur ran on the ring passes: 1 if it did with the image
+ * read and written through tensor maps, 2 if by plain copies (its rows are
+ * not whole 16-byte units, or it does not begin at one), 0 if it did not.  No
+ * counterpart in the reference. */
+int pxg_last_blur_ring(void);
 
 /* Converter trace of the ring blur passes, a profiling aid: enable != 0
  * switches it on (and clears it) for the passes launched afterwards, 0 off.

@@ -620,8 +620,13 @@ def blur_config(mode):
 
 
 def last_blur_kernel() -> int:
-    """Kernel family the last blur ran on (3, 2, 1, 0; -1 before any)."""
+    """Kernel family the last blur ran on (5, 4, 3, 2, 1, 0; -1 before any)."""
     return int(lib().pxg_last_blur_kernel())
+
+
+def last_blur_ring() -> int:
+    """Whether the last blur ran on the ring passes: 1 through tensor maps, 2 by plain copies, 0 not."""
+    return int(lib().pxg_last_blur_ring())
 
 
 def ring_trace(enable: bool, fetch: bool = False):

@@ -198,7 +198,7 @@ bool ring_blur_init(size_t* maxSmem);
 bool weights_exact_f16(const uint16_t* hostKern, int r);
 long long blur_scratch_bytes(long long W, long long H);
 int ring_trace(int enable, long long* out, long long n);
-bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, int r, const uint16_t* kern,
+int launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, int r, const uint16_t* kern,
                       bool exactF16, uint32_t oob, int nsm, size_t maxSmem, int* err, cudaStream_t st);
 void launch_stroke_outline(const float2* pts, const StrokeShape* shapes, int nshapes, long long nthreads, Prim* out,
                            int2* amb, long long amb_cap, unsigned long long* amb_count, int nsm, cudaStream_t st);
@@ -321,6 +321,7 @@ struct Ctx {
   size_t tcSmemMax = 0;
   bool ring_ok = false;  // the ring kernels and the driver's tensor-map encoder are available
   int last_blur = -1;    // kernel family of the last blur (4: the small-radius passes)
+  int last_ring = 0;     // whether the last blur ran on the ring passes: 1, or 2 by plain copies (0: it did not)
   size_t ringSmemMax = 0;
   float last_ms = 0;
   long long stats[6] = {0, 0, 0, 0, 0, 0};  // last fill launch: paths, prims, segments, entries, blends, wide rows
@@ -486,14 +487,18 @@ bool ring_takes_small(const uint32_t* img, long long W, long long H, int64_t r) 
 // tmp holds tmp_bytes: W * H * 4 at least; the tensor-core passes need
 // blur_scratch_bytes(W, H) (a padded intermediate) and are skipped below that.
 // g.last_blur tells the ring passes' images by their sides: 3 if both are
-// multiples of 4, else 1.
+// multiples of 4, else 1; g.last_ring tells the passes.
 bool blur_dispatch(uint32_t* img, uint32_t* tmp, long long tmp_bytes, long long W, long long H, int64_t r,
                    uint32_t oob, bool swap_ok = false) {
   const uint16_t* kern = weights_for(r);
   const bool ring = g.blur_tensor == 3 && g.ring_ok && tmp_bytes >= blur_scratch_bytes(W, H);
-  if (ring && ring_takes_small(img, W, H, r) &&
-      launch_blur_ring(img, tmp, W, H, (int)r, kern, g.weights_f16[r], oob, g.nsm, g.ringSmemMax, g.dev_err,
-                       g.stream)) {
+  auto by_ring = [&] {
+    g.last_ring = launch_blur_ring(img, tmp, W, H, (int)r, kern, g.weights_f16[r], oob, g.nsm, g.ringSmemMax,
+                                   g.dev_err, g.stream);
+    return g.last_ring != 0;
+  };
+  g.last_ring = 0;
+  if (ring && ring_takes_small(img, W, H, r) && by_ring()) {
     g.last_blur = ((W | H) & 3) == 0 ? 3 : 1;
     return false;
   }
@@ -503,9 +508,7 @@ bool blur_dispatch(uint32_t* img, uint32_t* tmp, long long tmp_bytes, long long 
   }
   int used = -1;
   if (g.blur_tensor == 3 && launch_blur_small(img, tmp, W, H, (int)r, kern, oob, g.nsm, g.stream)) used = 4;
-  if (used < 0 && ring &&
-      launch_blur_ring(img, tmp, W, H, (int)r, kern, g.weights_f16[r], oob, g.nsm, g.ringSmemMax, g.dev_err,
-                       g.stream))
+  if (used < 0 && ring && by_ring())
     used = ((W | H) & 3) == 0 ? 3 : 1;
   if (used < 0 && g.blur_tensor == 2 &&
       launch_blur_tc(img, tmp, W, H, (int)r, kern, oob, g.nsm, g.tcSmemMax, g.dev_err, g.stream))
@@ -2641,6 +2644,11 @@ int pxg_blur_config(int use_tensor_cores) {
 int pxg_last_blur_kernel(void) {
   std::lock_guard<std::recursive_mutex> lk(g.mu);
   return g.last_blur;
+}
+
+int pxg_last_blur_ring(void) {
+  std::lock_guard<std::recursive_mutex> lk(g.mu);
+  return g.last_ring;
 }
 
 int pxg_ring_trace(int enable, int64_t* out, int64_t n) {

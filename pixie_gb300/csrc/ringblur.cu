@@ -712,8 +712,9 @@ long long ring_tmp_pitch(long long H) {
 // Bytes of the intermediate buffer a blur of W x H pixels needs.
 long long blur_scratch_bytes(long long W, long long H) { return W * ring_tmp_pitch(H) * 4; }
 
-// Both passes (img -> tmp transposed -> img) on the ring kernels.  Returns
-// false (and launches nothing) when the image or radius is not for this path:
+// Both passes (img -> tmp transposed -> img) on the ring kernels.  Returns 1, or 2
+// where the image went by plain copies; 0 (having launched nothing) when the
+// image or radius is not for this path:
 // r in 1..128, sides of 4 to 2^24, tmp 16-byte aligned.  An image whose rows
 // are not whole 16-byte units, or whose base is not at one, is read and
 // written by plain copies (kIoLoad4, kIoStore4); the intermediate always goes
@@ -721,10 +722,10 @@ long long blur_scratch_bytes(long long W, long long H) { return W * ring_tmp_pit
 // what pass 1 made of lines past the image, and pass 2 replaces them with the
 // outOfBounds colour as it does every position past the row.  tmp holds
 // blur_scratch_bytes(W, H) bytes (W rows of ring_tmp_pitch(H) pixels).
-bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, int r, const uint16_t* kern,
+int launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, int r, const uint16_t* kern,
                       bool exactF16, uint32_t oob, int nsm, size_t maxSmem, int* err, cudaStream_t st) {
-  if (!g_encode || r < 1 || r > 128 || W < 4 || H < 4 || W > (1 << 24) || H > (1 << 24)) return false;
-  if (reinterpret_cast<uintptr_t>(tmp) & 15) return false;
+  if (!g_encode || r < 1 || r > 128 || W < 4 || H < 4 || W > (1 << 24) || H > (1 << 24)) return 0;
+  if (reinterpret_cast<uintptr_t>(tmp) & 15) return 0;
   const bool mapped = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
   // plans and tensor maps of the last few (buffers, size, radius, colour)
   // keys, so a repeated blur costs its two launches on the host (callers
@@ -764,17 +765,17 @@ bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, in
     n.split = split;
     if (!plan_pass(n.a1, (int)W, (int)H, r, nsm, maxSmem, split, n.g1) ||
         !plan_pass(n.a2, (int)H, (int)W, r, nsm, maxSmem, split, n.g2))
-      return false;
+      return 0;
     n.a1.oob = n.a2.oob = oob;
     n.a1.opitch = (int)ring_tmp_pitch(H);  // pass 1 writes the intermediate
     if (!mapped) n.a1.delta = 0;
     const int Hp = (int)((H + 3) / 4 * 4);
     if (!encode_map(&n.m2, tmp, Hp, (int)W, ring_tmp_pitch(H), kRawW, kLines) ||
         !encode_map(&n.o1, tmp, Hp, (int)W, ring_tmp_pitch(H), kLines, kPos, true))
-      return false;
+      return 0;
     if (mapped && (!encode_map(&n.m1, img, (int)W, (int)H, W, kRawW, kLines) ||
                    !encode_map(&n.o2, img, (int)W, (int)H, W, kLines, kPos, true)))
-      return false;
+      return 0;
     cache[next] = n;
     pl = &cache[next];
     next = (next + 1) % 8;
@@ -787,7 +788,7 @@ bool launch_blur_ring(uint32_t* img, uint32_t* tmp, long long W, long long H, in
   const int late2 = dep_late(st, {im}, {tm});  // pass 2 (always waits: it reads pass 1's output)
   launch_ring_pass(pl->a2, split, mapped ? kIoTma : kIoStore4, pl->g2, pl->m2, pl->o2, kern, nullptr, img, err, late2,
                    st);
-  return true;
+  return mapped ? 1 : 2;
 }
 
 // The converter trace: enable != 0 switches it on for later passes (0 off);
