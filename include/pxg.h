@@ -322,12 +322,15 @@ int pxg_masks_add_paths(pxg_masks* masks, int64_t n, const float* cmds, const in
                         const int32_t* windings, int threads);
 int pxg_masks_render(pxg_masks* masks);
 /* Renders with a given row-kernel configuration instead of the tuned one
- * (variant 0: 256-crossing scratch, 1: 32-crossing scratch; rows per work
- * item 1..64); for tests and tuning. */
+ * (variant 0: rows of up to 256 crossings, 1: of up to 64, in a quarter of the
+ * memory; rows per work item 1..64); for tests and tuning. */
 int pxg_masks_render_config(pxg_masks* masks, int variant, int rows_per_item);
 int pxg_masks_download(const pxg_masks* masks, int64_t index, void* out, int64_t nbytes);
 const void* pxg_masks_device_ptr(const pxg_masks* masks, int64_t index);
 int pxg_image_draw_masks(pxg_image* page, const pxg_masks* masks, const int64_t* xy, int blend_mode);
+/* Draws with a given tile shape (0: 32 x 32, 1: 64 x 32, 2: 64 x 64) instead of
+ * the tuned one; for tests and tuning. */
+int pxg_image_draw_masks_config(pxg_image* page, const pxg_masks* masks, const int64_t* xy, int blend_mode, int tile);
 
 /* Serving: render jobs admitted against a device-memory budget and advanced
  * together by continuous batching.  A job paints a recorded scene onto a

@@ -139,6 +139,7 @@ def lib():
         L.pxg_masks_device_ptr.argtypes = [P, I64]
         L.pxg_masks_device_ptr.restype = P
         L.pxg_image_draw_masks.argtypes = [P, P, P, I]
+        L.pxg_image_draw_masks_config.argtypes = [P, P, P, I, I]
         L.pxg_server_new.restype = P
         L.pxg_server_new.argtypes = [I64, I64, I64]
         L.pxg_server_free.argtypes = [P]
@@ -530,11 +531,15 @@ class Masks:
         return out
 
 
-def draw_masks(page: "Image", masks: Masks, positions, blend_mode=BlendMode.NormalBlend):
-    """draw(page, mask_i, translate(x_i, y_i), blend_mode) for every mask in order."""
+def draw_masks(page: "Image", masks: Masks, positions, blend_mode=BlendMode.NormalBlend, tile=None):
+    """draw(page, mask_i, translate(x_i, y_i), blend_mode) for every mask in order;
+    tile: 0 (32x32), 1 (64x32) or 2 (64x64) instead of the tuned tile shape."""
     xy = np.ascontiguousarray(positions, np.int64).reshape(-1, 2)
     if len(xy) != len(masks):
         raise PixieError("one position per mask is required")
+    if tile is not None:
+        _check(lib().pxg_image_draw_masks_config(page._h, masks._h, _ptr(xy), int(blend_mode), int(tile)))
+        return
     _check(lib().pxg_image_draw_masks(page._h, masks._h, _ptr(xy), int(blend_mode)))
 
 

@@ -1716,7 +1716,8 @@ void render_masks(pxg_masks* m) {
   m->renders++;
 }
 
-void draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blend) {
+// forced: a tile shape, or -1 for the one that did best
+void draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blend, int forced = -1) {
   const int n = (int)m->jobs.size();
   if (n == 0) return;
   // one buffer: the rectangles, then the items (16 bytes each)
@@ -1750,7 +1751,9 @@ void draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blen
                                                         count_bucket(n)};
   auto it = g_tune.best.find(key);
   int tile = 1;  // 64x32: the fastest of most classes
-  if (g_tune.on && it == g_tune.best.end()) {
+  if (forced >= 0) {
+    tile = forced;
+  } else if (g_tune.on && it == g_tune.best.end()) {
     // time every tile shape on a copy of the page, then draw with the fastest
     unsigned char* tmp = (unsigned char*)scratch(pxBytes);
     std::vector<float> t((size_t)draw_masks_tiles(), 0.0f);
@@ -2476,7 +2479,7 @@ const void* pxg_masks_device_ptr(const pxg_masks* m, int64_t i) {
   return m->dev + m->offs[(size_t)i];
 }
 
-int pxg_image_draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blend) {
+static int draw_masks_call(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blend, int tile) {
   return guarded([&] {
     check_image(page);
     if (!m) throw ApiError{"Invalid mask batch handle"};
@@ -2485,9 +2488,17 @@ int pxg_image_draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy,
     if (!m->rendered && !m->jobs.empty()) throw ApiError{"Masks not rendered"};
     if (!xy && !m->jobs.empty()) throw ApiError{"Invalid positions"};
     Timed t;
-    draw_masks(page, m, xy, blend);
+    draw_masks(page, m, xy, blend, tile);
     t.done();
   });
+}
+int pxg_image_draw_masks(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blend) {
+  return draw_masks_call(page, m, xy, blend, -1);
+}
+int pxg_image_draw_masks_config(pxg_image* page, const pxg_masks* m, const int64_t* xy, int blend, int tile) {
+  return guarded_host([&] {
+    if (tile < 0 || tile >= draw_masks_tiles()) throw ApiError{"Invalid configuration"};
+  }) || draw_masks_call(page, m, xy, blend, tile);
 }
 
 pxg_server* pxg_server_new(int64_t budget_bytes, int64_t paths_per_job, int64_t paths_per_step) {
