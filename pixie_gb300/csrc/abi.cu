@@ -112,7 +112,7 @@ struct pxg_server {
 
 namespace pxg {
 __global__ void k_setup(PathJob* jobs, Arena A, int maxBands, int C);
-int setup_cluster(long long njobs, long long maxWork);
+int setup_cluster(long long njobs, long long maxWork, int nsm);
 cudaError_t launch_setup(int njobs, int C, int maxBands, cudaStream_t st, PathJob* jobs, const Arena& A);
 const void* rows_kernel(int v);
 size_t rows_smem(int v);
@@ -150,8 +150,8 @@ void launch_scene_rec(unsigned blocks, cudaStream_t st, PathJob* jobs, const Rec
                       long long items, int rpi, const Arena& A);
 void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Arena& A, unsigned char* wide,
                        long long slots);
-void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
-                  long long items, const Arena& A, const uint8_t* tbl, int sliceW);
+void launch_scene(int ppl, unsigned blocks, cudaStream_t st, const SceneRun* runs, int nruns, long long items,
+                  const Arena& A, const uint8_t* tbl, int sliceW);
 size_t scene_wide_bytes();
 int draw_masks_tiles();
 void launch_draw_masks(int tile, uint32_t* page, long long W, long long H, const int4* rects, const MaskDraw* items,
@@ -805,7 +805,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
                          maxWork = std::max(maxWork, setup_work(j));
                        }
                      });
-    const int setupC = setup_cluster(nr, maxWork);
+    const int setupC = setup_cluster(nr, maxWork, g.nsm);
     Arena& A = S.A;
     A.ovf_cap = g.ovf_cap / 2;
     PathJob* dj = S.dj;
@@ -1152,7 +1152,7 @@ void run_scene_chunk(std::vector<HostRun>& runs) {
       }
     });
     S.A.ovf_cap = g.ovf_cap / 3;  // three lists
-    CU(launch_setup(nj, setup_cluster(nj, maxWork), maxBands, g.stream, S.dj, S.A));
+    CU(launch_setup(nj, setup_cluster(nj, maxWork, g.nsm), maxBands, g.stream, S.dj, S.A));
     note_launch();
     CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
     launch_scene_rec((unsigned)recBlocks, g.stream, S.dj, reinterpret_cast<const RecOrder*>(S.extra + orderAt), nj,
@@ -1169,8 +1169,8 @@ void run_scene_chunk(std::vector<HostRun>& runs) {
     launch_scene_rest((unsigned)restBlocks, g.stream, S.dj, S.A, g.wide, g.wide_slots);
     note_launch();
     CU(cudaGetLastError());
-    launch_scene(ppl, (unsigned)blocks, g.stream, S.dj, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(), items,
-                 S.A, g.tbl, slice);
+    launch_scene(ppl, (unsigned)blocks, g.stream, reinterpret_cast<const SceneRun*>(S.extra), (int)sr.size(), items, S.A,
+                 g.tbl, slice);
     note_launch();
     CU(cudaGetLastError());
     S.read_back();

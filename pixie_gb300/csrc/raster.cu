@@ -1285,9 +1285,8 @@ static __device__ __noinline__ unsigned draw_program(RowPx<false> row, int mode,
 // PPL = 1 for launches with too few rows to fill the GPU, where a path's time
 // on its warp matters and not the instructions per pixel.
 template <int PPL, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 4) k_scene(PathJob* jobs, const SceneRun* runs, int nruns,
-                                                         long long totalItems, Arena A, const uint8_t* tbl,
-                                                         int sliceW) {
+__global__ void __launch_bounds__(WARPS * 32, 4) k_scene(const SceneRun* runs, int nruns, long long totalItems,
+                                                         Arena A, const uint8_t* tbl, int sliceW) {
   constexpr int SW = 32 * PPL;          // pixels of a step
   __shared__ int accs[WARPS][SW + 1];   // recorded programs: a coverage tile and the step's pixels
   __shared__ uint32_t pix[WARPS][SW];
@@ -1507,10 +1506,10 @@ void launch_scene_rest(unsigned blocks, cudaStream_t st, PathJob* jobs, const Ar
   launch_pdl(k_scene_rest<kRecMaxH, kRecWarps>, dim3(blocks), dim3(kRecWarps * 32), scene_rest_smem(), st, jobs, A,
              wide, slots);
 }
-void launch_scene(int ppl, unsigned blocks, cudaStream_t st, PathJob* jobs, const SceneRun* runs, int nruns,
-                  long long items, const Arena& A, const uint8_t* tbl, int sliceW) {
+void launch_scene(int ppl, unsigned blocks, cudaStream_t st, const SceneRun* runs, int nruns, long long items,
+                  const Arena& A, const uint8_t* tbl, int sliceW) {
   launch_pdl(ppl == 1 ? k_scene<1, kSceneWarps> : k_scene<4, kSceneWarps>, dim3(blocks), dim3(kSceneWarps * 32), 0, st,
-             jobs, runs, nruns, items, A, tbl, sliceW);
+             runs, nruns, items, A, tbl, sliceW);
 }
 
 // Dynamic shared memory of k_setup for a launch whose images have at most
@@ -1522,16 +1521,17 @@ size_t setup_smem(int maxBands) {
 }
 // CTAs per job: the longest job's time shrinks with them, while each CTA of a
 // launch beyond the first four per SM costs a wave's fixed part.  In
-// microseconds, as measured: 0.014 per unit of work, 15 per wave (0.025 per CTA
-// on 152 SMs), 4 for the cluster's barriers.  One heart: 10 us with 1 CTA, 15
+// microseconds, as measured: 0.014 per unit of work, 15.2 per wave, 4 for the
+// cluster's barriers.  One heart: 10 us with 1 CTA, 15
 // with 8; 64 cubics: 90 and 38; a 14,540-primitive stroke: 600 and 83; 4096
 // glyphs: 100 with 1, 243 with 2; 240 local paths: 970 and 175; 2000 paths over
 // 1024 x 1024: 6400 and 2250.
-int setup_cluster(long long njobs, long long maxWork) {
+int setup_cluster(long long njobs, long long maxWork, int nsm) {
+  const double cta = 15.2 / (4.0 * nsm);
   int best = 1;
   double cost = 0;
   for (int c = 1; c <= 8; c *= 2) {
-    const double t = 0.014 * (double)maxWork / c + 0.025 * (double)njobs * c + (c > 1 ? 4.0 : 0.0);
+    const double t = 0.014 * (double)maxWork / c + cta * (double)njobs * c + (c > 1 ? 4.0 : 0.0);
     if (c == 1 || t < cost) {
       best = c;
       cost = t;

@@ -387,7 +387,8 @@ __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, fl
   // the lane's place: line s of a step, entry i of its group, keys from kb on
   const int s = grouped ? lane / n : 0, kb = s * n, i = lane - kb;
   const unsigned group = grouped ? ((1u << n) - 1) << kb : 0xffffffffu;
-  const int cap = NB <= 64 || n <= 64 ? 64 : NB <= 512 ? NB : 0;
+  static_assert(NB <= 512, "a line's keys are sorted in registers");
+  const int cap = NB <= 64 || n <= 64 ? 64 : NB;
   int ns = 0, done = grouped ? 0 : -1;  // lines done (-1: the ordering is to come)
   bool all = true;                            // every span so far is still there
   if (HOLD && held >= 0) {
@@ -444,8 +445,7 @@ __device__ __forceinline__ void cov_samples(FastRow<NB, XT>& S, int n, int y, fl
       for (int k = nh + lane; k < cap; k += 32) keys[k] = kNoKey;
       __syncwarp();
       if (cap == 64) sort_keys<2>(keys, nh, ordering, lane);
-      else if (NB <= 512) sort_keys<NB <= 512 ? NB / 32 : 2>(keys, nh, ordering, lane);
-      else sort_keys_shared(keys, nh, ordering, lane);
+      else sort_keys<NB / 32>(keys, nh, ordering, lane);
     }
     __syncwarp();
     if (ordering) {
@@ -952,10 +952,15 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
       if (xt >= dh) break;
       CovTile T{xt, max(dl, xt), dry ? dh : min(dh, xt + XT), INT_MAX, INT_MIN};
       if (kind == 0) {
-        if (LINES && (REC || NB > 512 || n > kGroupN)) {
-          if constexpr (LINES) cov_lines<!REC>(S, *L, *K, n, y, (float)W, winding, aa, T, lane, held);
+        if constexpr (LINES && (REC || NB > 512)) {
+          cov_lines<!REC>(S, *L, *K, n, y, (float)W, winding, aa, T, lane, held);
         } else {
-          cov_samples<!REC, ONCE, NB, XT>(S, n, y, (float)W, winding, aa, T, lane, held);
+          bool byLines = false;
+          if constexpr (LINES) {
+            byLines = n > kGroupN;
+            if (byLines) cov_lines<!REC>(S, *L, *K, n, y, (float)W, winding, aa, T, lane, held);
+          }
+          if (!byLines) cov_samples<!REC, ONCE, NB, XT>(S, n, y, (float)W, winding, aa, T, lane, held);
         }
       } else {
         if (kind == 1) failed = trap_cov<REC, ONCE>(S, n, y, T, lane, dry, ordered, from);
