@@ -2197,6 +2197,9 @@ int pxg_scene_record_batch(pxg_scene* sc, int64_t n, const int32_t* kinds, const
         r.err = e.what();
       }
     };
+    // A thread for every four paths (a batch of masks goes by its outlines' pace): a
+    // scene's path, arcs and stroke outlines among them, takes 150 us and a thread 30
+    // to 60 to start (2000 paths 303 ms call by call, 26.5 on 16 cores).
     int nt = threads > 0 ? threads : (int)std::thread::hardware_concurrency();
     nt = std::max(1, std::min<int>(nt, (int)std::min<int64_t>(n / 4 + 1, 256)));
     std::atomic<int64_t> next{0};

@@ -2,16 +2,23 @@
 // shapesToSegments, computeBounds/snapToPixels, partitionSegments and the
 // fillShapes row loop (src/pixie/paths.nim:654-1912), restated for sm_103a.
 //
-// k_setup   one CTA per fill job: flatten primitives, emit pixie's segments
-//           (quantised, oriented, horizontals dropped) in the reference's
-//           order, reduce the bounds, derive the partition geometry, each
-//           segment's band range and each band's count and AA flag.
-// k_rows    one warp per image row: a ballot scan over the segments collects
-//           the row's band entries in segment order (clipped to the band as
-//           partitionSegments does), then the reference's per-row decision
-//           (the non-AA two-edge fill, the trapezoid fast path, or 5-sample
-//           coverage with the nonzero/even-odd walk) and the fused
-//           coverage -> paint -> blend write of the row.
+// k_setup       a cluster of 1 to 8 CTAs per fill job (setup.cuh): flatten the
+//               primitives, emit pixie's segments (quantised, oriented,
+//               horizontals dropped) in the reference's order, reduce the bounds,
+//               derive the partition geometry, each band's count, flag and list of
+//               segments.
+// k_rows_fast   the row engine (rowfast.cuh): a warp takes chunks of rows from a
+//               queue; a row's band entries are clipped as partitionSegments does,
+//               then the reference's per-row decision (the non-AA two-edge fill, the
+//               trapezoid fast path, or 5-sample coverage with the nonzero/even-odd
+//               walk) and the fused coverage -> paint -> blend write.
+// k_rows_lines  the same with a CTA per row and a warp per sample line, for few
+//               rows of many crossings; k_rows_huge for rows of more than 256.
+// k_rows        the general row code (process_row), one row a warp: MaskBlend and
+//               images too wide for the row engine's keys; k_rows_wide takes the
+//               rows that the other kernels hand on.
+// k_scene_rec, k_scene_big, k_scene_huge, k_scene_rest, k_scene  many paths on one
+//               canvas: rows recorded by the same code, then drawn in path order.
 // Float math is compiled with -fmad=false: every expression keeps the
 // reference's float32 operation order.
 #include <algorithm>

@@ -52,8 +52,12 @@ struct __align__(16) FastRow {
   __device__ __forceinline__ float& m(int j) { return ent[2][j]; }
   __device__ __forceinline__ float& b(int j) { return ent[3][j]; }
 };
-// Two signed 16-bit sums per word: the lower one is kept above zero, so adding
-// a negative difference to it never borrows from the upper one.
+// Two signed 16-bit sums per word.  Words add modulo 2^32 in any order, so only a
+// pixel's final difference has to fit: a sample line's spans are disjoint and their
+// bytes rounded down, a trapezoid row's pixels lie in one edge or span each, so a
+// pixel's sum is within 0..511 (256 + 255) and a difference within +-511; one at a
+// tile's edge, which takes what lies beyond, is a pixel's sum itself.  The lower
+// half begins at 0x4000, so its final value is positive and borrows nothing.
 constexpr uint32_t kDiffZero = 0x4000u;
 
 // A loop-invariant value the compiler is not to specialise loops for: a copy
