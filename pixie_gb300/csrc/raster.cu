@@ -497,8 +497,9 @@ __device__ void apply_hits(RowPx<A8> row, int mode, const uint8_t* tbl, uint32_t
 //   kRecCov8  coverage bytes of pixels [lo, hi) -- lo a multiple of 16 -- from
 //             unit `place` (16 bytes) of Arena::cov8 (the accumulation done
 //             once, at record time); zero: the pixel is left alone
-//   kRecCov8Z a list at unit `place` of Arena::prog: {cov8 unit, n} and n
-//             pixels that are blended with an empty source besides
+//   kRecCov8Z a list at unit `place` of Arena::prog: {cov8 unit, n, first, last}
+//             and n pixels besides (at most kZeroCap, between first and last), each
+//             {x, area}: blended with an empty source or a multiplier above 255
 //   kRecProg  a program at unit `place` of Arena::prog
 enum RecKind { kRecFill = 1, kRecCov = 2, kRecHits = 3, kRecTrap = 4, kRecCov8 = 5, kRecCov8Z = 6, kRecProg = 7 };
 
@@ -1366,12 +1367,16 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(const SceneRun* runs, i
         const int mode0 = (int)(in.y & 255u);
         const bool plain0 = mode0 < kMask && premultiplied(in.x);
         const unsigned masks = __ballot_sync(0xffffffffu, draws && mode0 >= kMask);
+        int unit0 = h.y, kind0 = h.x;
+        if (draws && kind0 == kRecCov8Z) {
+          const int4 g = A.prog[(unsigned)h.y];
+          unit0 = g.x;
+          if (g.z >= xb || g.w < xa) kind0 = kRecCov8;  // its listed pixels are in other steps
+        }
         const uint32_t pack0 = (uint32_t)max(h.z - xa, 0) | ((uint32_t)min(h.w - xa, xb - xa) << 8) |
-                               ((uint32_t)h.x << 16) | ((uint32_t)mode0 << 20) | (plain0 ? 1u << 30 : 0u) |
+                               ((uint32_t)kind0 << 16) | ((uint32_t)mode0 << 20) | (plain0 ? 1u << 30 : 0u) |
                                (plain0 && solid && (masks & ((1u << lane) - 1)) == 0 ? 1u << 31 : 0u);
         solid &= masks == 0;
-        int unit0 = h.y;
-        if (draws && h.x == kRecCov8Z) unit0 = A.prog[(unsigned)h.y].x;
         unit0 += ((xa & ~15) - h.z) >> 4;
         int next = -1;      // the path after the current one, and its coverage
         uint32_t nextCov = 0, nextPack = 0;
@@ -1453,14 +1458,13 @@ __global__ void __launch_bounds__(WARPS * 32, 4) k_scene(const SceneRun* runs, i
         const int4 ph = hdr[path];
         const uint2 pi = info[path];
         const int pmode = (int)(pi.y & 255u);
-        if (ph.x == kRecCov8Z) {  // the listed pixels with an empty source
-          const int nz = A.prog[ph.y].y;
-#pragma unroll 1
-          for (int z = 0; z < nz && lane == 0; z++) {
-            const int x = reinterpret_cast<const int*>(A.prog + ph.y + 1)[z];
-            if (x < xa || x >= xb) continue;
-            ++painted;
-            pix[warp][x - xa] = blend_any(pmode, tbl, pix[warp][x - xa], 0u);
+        if (ph.x == kRecCov8Z) {  // the listed pixels (no two the same)
+          if (lane < A.prog[ph.y].y) {
+            const int2 e = reinterpret_cast<const int2*>(A.prog + ph.y + 1)[lane];
+            if (e.x >= xa && e.x < xb) {
+              ++painted;
+              pix[warp][e.x - xa] = blend_any(pmode, tbl, pix[warp][e.x - xa], mul_f(pi.x, __int_as_float(e.y)));
+            }
           }
         } else {
           const RowPx<false> row{reinterpret_cast<unsigned char*>(pix[warp]), xa};

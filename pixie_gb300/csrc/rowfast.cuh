@@ -34,7 +34,7 @@ constexpr int tag_bits(int nb) { return nb <= 64 ? 7 : nb <= 128 ? 8 : nb <= 256
 constexpr int fast_max_w(int nb) { return 1 << (24 - tag_bits(nb)); }
 static_assert(tag_bits(2048) == 12 && fast_max_w(256) == 32768, "a key holds NB crossings");
 constexpr uint32_t kNoKey = 0xffffffffu;
-constexpr int kZeroCap = 32;  // blended pixels of coverage 0 a trapezoid row may record
+constexpr int kZeroCap = 32;  // pixels of a trapezoid row listed apart: what a byte of coverage cannot say
 enum RowOut { kOutRgbx = 0, kOutA8 = 1, kOutRec = 2 };
 
 template <int NB, int XT>
@@ -790,9 +790,10 @@ __device__ __forceinline__ bool trap_row(FastRow<NB, XT>& S, int n, float yTop, 
 
 // The pixels of a simple trapezoid row (:1752-1835) over tile T into S.diff:
 // 256 + the multiplier (0..255) its area rounds to, so that pixels blended
-// with nothing stay distinct from untouched ones (listed in S.zero when ZERO,
-// where only the multiplier is kept).  Returns true where a multiplier is
-// above 255 or the list is full: the general code's.  dry: no more than that.
+// with nothing stay distinct from untouched ones (listed in S.zero, their area in
+// S.key, free by now, when ZERO, where only the multiplier is kept).  Returns
+// true where a multiplier is above 255, which list_odd lists, or the list is
+// full: the general code's.  dry: no more than that.
 // from: the first entry that reaches the tile or those to its right (advanced
 // where the entries are ordered: of 200 a row's 16 tiles have a dozen each).
 template <bool ZERO, bool ORDERED, int NB, int XT>
@@ -820,8 +821,12 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
       else if (!ZERO || v) cov_range(S.diff, T, x, x + 1, kBase + (int)v);
       else {
         const int z = atomicAdd(&S.nzero, 1);
-        if (z < kZeroCap) S.zero[z] = x;
-        else odd = true;
+        if (z < kZeroCap) {
+          S.zero[z] = x;
+          S.key[z] = 0.0f;
+        } else {
+          odd = true;
+        }
       }
     }
     if (!(s & 1) && lane == 0 && !(!ZERO && dry)) {  // the fully covered middle up to the next edge
@@ -831,6 +836,53 @@ __device__ __forceinline__ bool trap_cov(FastRow<NB, XT>& S, int n, int y, const
     }
   }
   return __any_sync(0xffffffffu, odd) != 0;
+}
+
+// Lists the pixels of [dl, dh) whose multipliers are above 255, with their areas,
+// in S.zero and S.key; true if there is no room for them.  Where an edge crosses
+// the image's left side between pixels -1 and 0, pixel 0 has an area above 1, so
+// a shape that leaves the image there has such a pixel in many of its rows; as
+// rows handed on they cost a wait for the host or three kernels: 1000 edges on
+// 1500 x 1000 222 us, 120 so, 200 of them in a scene 10.99 ms and 1.48.  Out of
+// line, and a walk of its own: a list made in trap_cov took a fifth of the time of
+// rows that have none (50 lines on 2000 x 1500 96 us, 123).
+template <int NB, int XT>
+static __device__ __noinline__ bool list_odd(FastRow<NB, XT>* S, int n, int y, int dl, int dh, bool fresh, int lane) {
+  __syncwarp();
+  if (fresh && lane == 0) S->nzero = 0;
+  __syncwarp();
+#pragma unroll 1
+  for (int s = 0; s < n; s++) {
+    const int i = S->perm[s], j = S->idx[i];
+    const float m = S->m(j), b = S->b(j), t0 = S->t0[i], t1 = S->t1[i], lo = nmin(t0, t1);
+    const long long xs = nim_int(lo);
+    const int x1 = nim_clamp(ceilf(nmax(t0, t1)), dl, dh);
+#pragma unroll 1
+    for (int x = nim_clamp(lo, dl, dh) + lane; x < x1; x += 32) {
+      const float area = (s & 1) ? trap_right_area(m, b, t0, t1, x, xs, y) : trap_left_area(m, b, t0, t1, x, xs, y);
+      if (area == 0.0f || nim_u32(roundf(area * 255.0f)) <= 255) continue;
+      const int z = atomicAdd(&S->nzero, 1);
+      if (z < kZeroCap) {
+        S->zero[z] = x;
+        S->key[z] = area;
+      }
+    }
+  }
+  __syncwarp();
+  return S->nzero > kZeroCap;
+}
+// The listed pixels, drawn as the general code draws them.
+template <int OUT, int NB, int XT>
+static __device__ __noinline__ void draw_odd(FastRow<NB, XT>* S, uint8_t* base, int mode, const uint8_t* tbl,
+                                             uint32_t rgbx, int lane) {
+  if (lane < S->nzero) {
+    const int x = S->zero[lane];
+    const uint32_t c = mul_f(rgbx, S->key[lane]);
+    uint32_t* p = reinterpret_cast<uint32_t*>(base) + x;
+    if (OUT == kOutA8) base[x] = (uint8_t)(c >> 24);
+    else *p = blend_any(mode, tbl, *p, c);
+  }
+  __syncwarp();
 }
 
 // Rows [yA, yB) of job J (non-MaskBlend, narrower than fast_max_w(NB), within the
@@ -949,6 +1001,7 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
     // gone through once, whole, before any of it is drawn
     bool dry = !REC && tiled && kind == 1;
     int held = -1, from = 0;  // what the tiles before found: the row's spans, its first trapezoid to come
+    bool listed = false;      // the row's odd multipliers are in S.zero
     if (REC && lane == 0) S.nzero = 0;
     __syncwarp();
 #pragma unroll 1
@@ -967,8 +1020,12 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
           if (!byLines) cov_samples<!REC, ONCE, NB, XT>(S, n, y, (float)W, winding, aa, T, lane, held);
         }
       } else {
-        if (kind == 1) failed = trap_cov<REC, ONCE>(S, n, y, T, lane, dry, ordered, from);
-        else if (lane == 0) cov_range(S.diff, T, dl, dh, 255);
+        if (kind == 1) {
+          if (trap_cov<REC, ONCE>(S, n, y, T, lane, dry, ordered, from) && !listed) {
+            listed = true;
+            failed = list_odd(&S, n, y, dl, dh, !REC, lane);
+          }
+        } else if (lane == 0) cov_range(S.diff, T, dl, dh, 255);
         T.lo = T.t0;
         T.hi = T.t1;
         if (!REC && dry) {
@@ -1066,15 +1123,21 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
     }
     if (failed) {
       push_row(A, job, y, lane, LIST);
-    } else if (REC && cov >= 0) {
+    } else if (!REC) {
+      if (listed) draw_odd<OUT>(&S, base, J.mode, tbl, J.rgbx, lane);
+    } else if (cov >= 0) {
       const int nz = S.nzero;
-      if (nz == 0) {
+      if (nz > kZeroCap) {
+        push_row(A, job, y, lane, LIST);
+      } else if (nz == 0) {
         if (lane == 0) *hdr = make_int4(kRecCov8, (int)(cov >> 4), covX, covHi);
       } else {
-        const long long at = rec_alloc(J, A, y, kRecCov8Z, 1 + (nz + 3) / 4, covX, covHi, lane);
+        const long long at = rec_alloc(J, A, y, kRecCov8Z, 1 + (nz + 1) / 2, covX, covHi, lane);
+        const int x = S.zero[min(lane, nz - 1)];
+        const int lo = __reduce_min_sync(0xffffffffu, x), hi = __reduce_max_sync(0xffffffffu, x);
         if (at >= 0) {
-          if (lane == 0) A.prog[at] = make_int4((int)(cov >> 4), nz, 0, 0);
-          if (lane < nz) reinterpret_cast<int*>(A.prog + at + 1)[lane] = S.zero[lane];
+          if (lane == 0) A.prog[at] = make_int4((int)(cov >> 4), nz, lo, hi);
+          if (lane < nz) reinterpret_cast<int2*>(A.prog + at + 1)[lane] = make_int2(x, __float_as_int(S.key[lane]));
         }
       }
     }
