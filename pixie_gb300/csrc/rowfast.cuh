@@ -1079,13 +1079,26 @@ __device__ __forceinline__ void fast_rows(const PathJob& J, const Arena& A, cons
           }
         } else {
           const uint32_t c[4] = {f[0] & 0xffffu, f[0] >> 16, f[1] & 0xffffu, f[1] >> 16};
-          if (failed || (f[0] | f[1]) == 0) return;
           const int x = xt + i;
           uint32_t* p = reinterpret_cast<uint32_t*>(base) + x;
-          const bool vec = x >= 0 && x + 4 <= W;
+          const bool vec = x >= 0 && x + 4 <= W, some = !failed && (f[0] | f[1]) != 0;
+          const bool whole = vec && (f[0] & f[1] & 0x00ff00ffu) == 0x00ff00ffu;
+          // a step within a span, where it is Normal: no blend for parts of it (a
+          // translucent heart on 3000 x 3000 120 -> 108 us)
+          if (!LINES && J.mode == kNormal && !flat && !__any_sync(0xffffffffu, some && !whole)) {
+            if (!some) return;
+            uint4 v = *reinterpret_cast<const uint4*>(p);
+            v.x = blendNormal(v.x, J.rgbx);
+            v.y = blendNormal(v.y, J.rgbx);
+            v.z = blendNormal(v.z, J.rgbx);
+            v.w = blendNormal(v.w, J.rgbx);
+            *reinterpret_cast<uint4*>(p) = v;
+            return;
+          }
+          if (!some) return;
           // what a full coverage replaces is not read (a heart that overwrites 8192 x
           // 8192: 368 us reading, 183 not)
-          if (vec && (f[0] & f[1] & 0x00ff00ffu) == 0x00ff00ffu && flat) {
+          if (whole && flat) {
             *reinterpret_cast<uint4*>(p) = make_uint4(J.rgbx, J.rgbx, J.rgbx, J.rgbx);
             return;
           }
