@@ -200,10 +200,11 @@ __global__ void __launch_bounds__(256) k_blur_sy(const uint32_t* __restrict__ in
 // by vertical neighbours come from L2).  The arithmetic per output is the
 // two-pass kernels': the same sums, the same floor(S / 65280) between passes.
 constexpr int kFTW = 128;  // columns of a tile
-template <int R>
+template <int R, int TH>
 __global__ void __launch_bounds__(256) k_blur_fused(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                     int W, int H, const uint16_t* __restrict__ kern, uint32_t oob,
-                                                    int th, int vec, int late) {
+                                                    int thArg, int vec, int late) {
+  const int th = TH > 0 ? TH : thArg;  // rows of a tile
   constexpr int NI = kOut + 2 * R;
   constexpr int D = (4 - (R & 3)) & 3;
   constexpr int NC = (D + NI + 3) / 4;
@@ -307,28 +308,36 @@ __global__ void __launch_bounds__(256) k_blur_fused(const uint32_t* __restrict__
 // so: 97 x 97 at radius 8 12.0 / 5.3 us, 641 x 641 14.4 / 9.3, 1237 x 1001 at
 // radius 3 10.6 / 8.6 (24 rows) and at 8 19.3 / 16.4 (72), 4096 x 4096 at 5
 // 75.6 / 72.7 (72).
-int fused_rows(long long W, long long H, int r, int nsm) {
+// Tiles of 64 rows have an instance of their own, 3 % faster than one that is told
+// (4096 x 4096 at 3 63.3 and 60.1 us, 3733 x 1285 at 3 24.5 and 23.2), and other
+// numbers have to promise more than that: where rows are not whole 16-byte units,
+// and a staged row costs more, a sixth (3733 x 1285 with 56 rows, a tenth less by
+// this count: 3 26.2, 6 37.0 us; with 64 23.2 and 34.1).
+constexpr int kFusedRows = 64;
+int fused_rows(long long W, long long H, int r, int vec, int nsm) {
   const long long cols = (W + kFTW - 1) / kFTW;
-  long long best = 0;
-  int th = 64;
+  long long best = 0, usual = 0;
+  int th = kFusedRows;
   for (int t = 80; t >= 8; t -= 8) {
     const long long down = (H + t - 1) / t, rounds = (cols * down + nsm - 1) / nsm, cost = (2 * rounds + 1) * (t + 2 * r);
     if (down <= 65535 && (best == 0 || cost < best)) {
       best = cost;
       th = t;
     }
+    if (t == kFusedRows) usual = cost;
   }
-  return th;
+  return best * 100 <= usual * (vec ? 97 : 84) ? th : kFusedRows;
 }
 template <int R>
 void launch_fused(const uint32_t* in, uint32_t* out, int W, int H, const uint16_t* kern, uint32_t oob,
                   int nsm, cudaStream_t st) {
   const int vec = (W % 4 == 0) && ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
-  const int th = fused_rows(W, H, R, nsm);
+  const int th = fused_rows(W, H, R, vec, nsm);
   const dim3 grid((unsigned)((W + kFTW - 1) / kFTW), (unsigned)((H + th - 1) / th));
   const size_t bytes = (size_t)W * (size_t)H * 4;
   const int late = dep_late(st, {Span{out, bytes}}, {Span{in, bytes}});
-  launch_pdl(k_blur_fused<R>, grid, dim3(256), (size_t)(th + 2 * R) * kFTW * 4, st, in, out, W, H, kern, oob, th, vec,
+  const auto kernel = th == kFusedRows ? k_blur_fused<R, kFusedRows> : k_blur_fused<R, 0>;
+  launch_pdl(kernel, grid, dim3(256), (size_t)(th + 2 * R) * kFTW * 4, st, in, out, W, H, kern, oob, th, vec,
              late);
   note_launch();
 }
