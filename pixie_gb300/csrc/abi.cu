@@ -588,16 +588,36 @@ int64_t nim_round_int(float v) {
   return (int64_t)r;
 }
 
+// The steps of a curve's flattening, about: its deviation from a chord falls with
+// the square of their number.
+int curve_steps(const Prim& p, float ems) {
+  auto bend = [&](int i) { return hypotf(p.x[i] - 2 * p.x[i + 1] + p.x[i + 2], p.y[i] - 2 * p.y[i + 1] + p.y[i + 2]); };
+  const float d = p.kind == kPrimCubic ? 3 * std::max(bend(0), bend(1)) : bend(0), n = sqrtf(d / (4 * sqrtf(ems)));
+  return n < 1000 ? (int)n + 1 : 1000;  // (also for what is no number)
+}
 // Quadratics and cubics among a job's primitives (the setup kernel shares its
-// threads out over them).
-int count_curves(const std::vector<Prim>& prims, long long off, int n) {
-  int curves = 0;
-  for (int i = 0; i < n; i++) curves += prims[(size_t)(off + i)].kind != kPrimLine;
-  return curves;
+// threads out over them), and the steps of the longest of up to eight of them.
+void count_curves(PathJob& j, const std::vector<Prim>& prims, long long off) {
+  const Prim* P = prims.data() + off;
+  j.curves = j.curve_steps = 0;
+  for (int i = 0; i < j.nprims; i++) j.curves += P[i].kind != kPrimLine;
+  for (int s = 0, i = 0; s < 8 && j.curves > 0; s++) {
+    i = std::max(i, (int)((long long)j.nprims * s / 8));
+    while (i < j.nprims && P[i].kind == kPrimLine) i++;
+    if (i == j.nprims) break;
+    j.curve_steps = std::max(j.curve_steps, curve_steps(P[i++], j.ems));
+  }
 }
 // What the setup kernel spends on a job, in lines: a curve's search takes some
 // tens of them.
 long long setup_work(const PathJob& j) { return j.nprims + 24LL * j.curves; }
+// The same for the choice of its CTAs, where a glyph's curves of up to 8 steps count
+// less: 115 glyphs of 25 pixels take 58 us a rendering with a CTA each, 70 with the
+// four that 24 a curve would give them; 250 of 10 pixels 60 and 72.
+long long setup_cost(const PathJob& j) {
+  const bool few = j.curve_steps > 0 && j.curve_steps <= 8;
+  return j.nprims + (few ? j.curve_steps / 2 + 2LL : 24LL) * j.curves;
+}
 
 // Workspace of the fill kernels, grown on demand (never shrunk).
 void ensure_arena(long long seg_need, long long list_need, long long nbands, long long nprims, long long rows) {
@@ -776,7 +796,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
   long long list_need = seg_need * 4;
   for (int attempt = 0; attempt < 12 && !todo.empty(); attempt++) {
     const int nr = (int)todo.size();
-    long long rows = 0, maxH = 1, maxWork = 0, items = 0;
+    long long rows = 0, maxH = 1, maxWork = 0, maxCost = 0, items = 0;
     bool huge = false;  // some image is one for k_rows_huge
     std::vector<long long> offs((size_t)nr);  // the jobs' first work items
     for (int r = 0; r < nr; r++) {
@@ -797,15 +817,16 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
                          PathJob& j = dst[r];
                          j = jobs[i];
                          if (opts.imgs) j.img = opts.imgs + (*opts.img_offs)[i];
-                         if (j.curves < 0) j.curves = count_curves(prims, j.prim_off, j.nprims);
+                         if (j.curves < 0) count_curves(j, prims, j.prim_off);
                          j.pc_off = j.prim_off;
                          j.prims = opts.dprims;  // null: the staged copy
                          j.row_off = offs[(size_t)r];
                          j.status = kOk;
                          maxWork = std::max(maxWork, setup_work(j));
+                         maxCost = std::max(maxCost, setup_cost(j));
                        }
                      });
-    const int setupC = setup_cluster(nr, maxWork, g.nsm);
+    const int setupC = setup_cluster(nr, maxCost, g.nsm);
     Arena& A = S.A;
     A.ovf_cap = g.ovf_cap / 2;
     PathJob* dj = S.dj;
@@ -1053,7 +1074,7 @@ void run_scene_chunk(std::vector<HostRun>& runs) {
     int nj = 0;
     std::vector<SceneRun> sr;
     std::vector<size_t> which;  // launch run -> runs index
-    long long items = 0, riTotal = 0, maxH = 1, maxWork = 0;
+    long long items = 0, riTotal = 0, maxH = 1, maxCost = 0;
     int ppl = 4;
     const int slice = scene_slice_for(runs, ppl);
     long long pathRows = 0;
@@ -1136,7 +1157,7 @@ void run_scene_chunk(std::vector<HostRun>& runs) {
         for (size_t j = r.j0; j < r.j1; j++) {
           PathJob& pj = *dst++;
           pj = (*r.jobs)[j];
-          if (pj.curves < 0) pj.curves = count_curves(*r.prims, pj.prim_off, pj.nprims);
+          if (pj.curves < 0) count_curves(pj, *r.prims, pj.prim_off);
           pj.prims = pj.stroke_gpu ? r.dstroke : r.dprims;
           pj.pc_off = at;
           at += pj.nprims;
@@ -1147,12 +1168,12 @@ void run_scene_chunk(std::vector<HostRun>& runs) {
           pj.ri_off = s.ri_base + (long long)(j - r.j0);
           pj.ri_stride = s.j1 - s.j0;
           pj.status = kOk;
-          maxWork = std::max(maxWork, setup_work(pj));
+          maxCost = std::max(maxCost, setup_cost(pj));
         }
       }
     });
     S.A.ovf_cap = g.ovf_cap / 3;  // three lists
-    CU(launch_setup(nj, setup_cluster(nj, maxWork, g.nsm), maxBands, g.stream, S.dj, S.A));
+    CU(launch_setup(nj, setup_cluster(nj, maxCost, g.nsm), maxBands, g.stream, S.dj, S.A));
     note_launch();
     CU(cudaMemsetAsync(g.rowhdr, 0, sizeof(int4) * (size_t)std::max<long long>(riTotal, 1), g.stream));
     launch_scene_rec((unsigned)recBlocks, g.stream, S.dj, reinterpret_cast<const RecOrder*>(S.extra + orderAt), nj,
@@ -2086,7 +2107,7 @@ int pxg_scene_fill_path(pxg_scene* sc, const float* cmds, int64_t n, const float
     PathJob j = make_job(nullptr, rgbx, blend, mat, ps, winding);
     j.prim_off = (long long)sc->prims.size();
     j.nprims = (int)prims.size();
-    j.curves = count_curves(prims, 0, j.nprims);
+    count_curves(j, prims, 0);
     sc->prims.insert(sc->prims.end(), prims.begin(), prims.end());
     sc->jobs.push_back(j);
     sc->dirty = true;
@@ -2123,7 +2144,7 @@ int pxg_scene_stroke_path(pxg_scene* sc, const float* cmds, int64_t n, const flo
     build_stroke_prims(cmds, n, ps, width, cap, join, miterLimit, dashes, nd, prims);
     j.prim_off = (long long)sc->prims.size();
     j.nprims = (int)prims.size();
-    j.curves = count_curves(prims, 0, j.nprims);
+    count_curves(j, prims, 0);
     sc->prims.insert(sc->prims.end(), prims.begin(), prims.end());
     sc->jobs.push_back(j);
     sc->dirty = true;
@@ -2227,7 +2248,7 @@ int pxg_scene_record_batch(pxg_scene* sc, int64_t n, const int32_t* kinds, const
       } else {
         r.job.prim_off = (long long)sc->prims.size();
         r.job.nprims = (int)r.prims.size();
-        r.job.curves = count_curves(r.prims, 0, r.job.nprims);
+        count_curves(r.job, r.prims, 0);
         sc->prims.insert(sc->prims.end(), r.prims.begin(), r.prims.end());
       }
       sc->jobs.push_back(r.job);
@@ -2310,7 +2331,7 @@ int pxg_masks_add_path(pxg_masks* m, const float* cmds, int64_t n, int64_t width
     j.H = height;
     j.prim_off = (long long)m->prims.size();
     j.nprims = (int)prims.size();
-    j.curves = count_curves(prims, 0, j.nprims);
+    count_curves(j, prims, 0);
     m->prims.insert(m->prims.end(), prims.begin(), prims.end());
     m->jobs.push_back(j);
     note_mask(m, j);
@@ -2418,7 +2439,7 @@ int pxg_masks_add_paths(pxg_masks* m, int64_t n, const float* cmds, const int64_
       Rec& r = rec[(size_t)i];
       r.job.prim_off = (long long)m->prims.size();
       r.job.nprims = (int)r.prims.size();
-      r.job.curves = count_curves(r.prims, 0, r.job.nprims);
+      count_curves(r.job, r.prims, 0);
       m->prims.insert(m->prims.end(), r.prims.begin(), r.prims.end());
       m->jobs.push_back(r.job);
       note_mask(m, r.job);

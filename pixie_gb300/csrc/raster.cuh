@@ -64,7 +64,7 @@ struct PathJob {
   long long ri_off;     // scenes: row y of the job is Arena::rowhdr[ri_off + y * ri_stride]
   long long ri_stride;
   int stroke_gpu;       // host: the primitives are a GPU-outlined stroke (scene: in its stroke region)
-  int pad_;
+  int curve_steps;      // host: steps of the longest of some curves, 0 if unknown
   // outputs (setup kernel)
   int status, nseg, nb;
   uint32_t ph;
