@@ -796,7 +796,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
   long long list_need = seg_need * 4;
   for (int attempt = 0; attempt < 12 && !todo.empty(); attempt++) {
     const int nr = (int)todo.size();
-    long long rows = 0, maxH = 1, maxWork = 0, maxCost = 0, items = 0;
+    long long rows = 0, maxH = 1, maxWork = 0, maxCost = 0, maxPrims = 0, items = 0;
     bool huge = false;  // some image is one for k_rows_huge
     std::vector<long long> offs((size_t)nr);  // the jobs' first work items
     for (int r = 0; r < nr; r++) {
@@ -824,6 +824,7 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
                          j.status = kOk;
                          maxWork = std::max(maxWork, setup_work(j));
                          maxCost = std::max(maxCost, setup_cost(j));
+                         maxPrims = std::max<long long>(maxPrims, j.nprims);
                        }
                      });
     const int setupC = setup_cluster(nr, maxCost, g.nsm);
@@ -832,15 +833,16 @@ void run_jobs(const std::vector<PathJob>& jobs, const std::vector<Prim>& prims, 
     PathJob* dj = S.dj;
     const int v = cfg.variant;
     // A launch of few rows lasts as long as its busiest one, and a warp per
-    // sample line shortens rows of more than 16 crossings, as paths of some
-    // hundred lines (a curve counts 24) have them: one path of 64 cubics on 512 x
-    // 512 29 us by a warp per row, 21 by a CTA; a stroke's 767 rows of up to 256
-    // crossings 65 and 54.  Beyond two rows per resident CTA the warps' number
-    // counts.  Rows of more than 256 crossings need some thousand lines in the
+    // sample line shortens rows of more than 16 crossings, as paths of some tens of
+    // lines have them (a curve counts 24, for twenty or more): one path of 64 cubics
+    // on 512 x 512 29 us by a warp per row, 21 by a CTA; a stroke's 767 rows of up to
+    // 256 crossings 65 and 54; calls of 89 lines over 34 x 5 67 and 54, over 1000 x 700
+    // 91 and 79, of 50 lines 56 and 54, 80 and 78.  Beyond two rows per resident CTA
+    // the warps' number counts.  Rows of more than 256 crossings need some thousand lines in the
     // path: their kernel is launched along then (3 us for nothing), else only
     // when the call has come back with such rows.  Images too wide for it go to the
     // general kernel at once.
-    const bool byLines = (v == 0 || v == 4) && cfg.rpi == 1 && opts.cfg.rpi == 0 && maxWork >= 512 &&
+    const bool byLines = (v == 0 || v == 4) && cfg.rpi == 1 && opts.cfg.rpi == 0 && (maxWork >= 512 || maxPrims >= 64) &&
                          items <= 2LL * g.nsm * g.lines_ctas_per_sm[narrow];
     const bool hugeAlong = huge && maxWork >= 2048;
     long long blocks = (items + rows_warps(v) - 1) / rows_warps(v);
