@@ -20,7 +20,7 @@
 // 128 crossings; the rows of 4096 glyphs 1.23 -> 0.38 ms; of one 512 x 512
 // path of 64 cubics 46 -> 30 us.  The recording kernel's hot code is at the
 // instruction cache's edge: 49 KB of it run at 6.6 ms, 54 KB (with the groups
-// of cov_samples) at 8.6 ms, a miss rate of 8 against 18 per cent.
+// of cov_samples) at 8.6 ms.
 //
 // Included by raster.cu after the shared row helpers (make_entry, blends, the
 // trapezoid areas).
